@@ -1,0 +1,811 @@
+"""The work that is measured: batches of requests through ``Engine.step``.
+
+A pass takes a batch from its first prompt token to its last new one: requests are opened, their prompts go through
+the engine in portions under the token budget of a step, beside the single tokens of the requests that are already
+decoding, and they are closed again.  Every new token's logits are kept, as a scoring or replay program keeps them, and
+its draw is read one step late, as the scheduler reads it.  The tokens that are fed are given beforehand and not fed back, so
+that a rounding of the logits cannot send the rest of a pass another way.
+
+Models are the repository's own benchmark configurations with random weights.  An engine is kept for each model, as a
+serving program keeps it; a state is what new requests bring: their tokens, and room for their logits.
+"""
+
+import json
+import math
+import os
+import re
+import tempfile
+import zlib
+
+import numpy as np
+import torch
+
+from mini_llm_b200.config import config_from_dict
+from mini_llm_b200.config.registry import describe_model
+from mini_llm_b200.engine import Engine, SamplingParams, StepEntry
+from mini_llm_b200.sampling import request_seed
+from mini_llm_b200.weights import collect_specs, write_safetensors
+from mini_llm_b200.weights.random_init import model_parts
+
+VOCAB = 50257
+STEP_TOKENS = 2048      # the engine's default token budget of a step
+
+
+# ---- the models ----------------------------------------------------------------------------------
+
+def _gpt2(layers, width, heads):
+    return {"architectures": ["GPT2LMHeadModel"], "model_type": "gpt2", "n_layer": layers, "n_embd": width, "n_head": heads,
+            "n_inner": 4 * width, "vocab_size": VOCAB, "n_positions": 1024, "activation_function": "gelu_new",
+            "layer_norm_epsilon": 1e-5, "tie_word_embeddings": True}
+
+
+_ROT = {"base": 10000.0, "dims": 64}
+_YARN = {"factor": 8.0, "original": 1024, "fast": 32.0, "slow": 1.0}
+_HEADS = {"heads": 12, "kv_heads": 4, "dim": 64, "vdim": 64, "scale": 0.125}
+_LATENT = {"heads": 12, "dim": 64, "rot_dim": 32, "vdim": 64, "kv_rank": 256, "scale": 96 ** -0.5, "rot": {"base": 10000.0, "dims": 32}}
+_MOE = {"kind": "moe", "router": {"experts": 8, "top": 2}, "expert": {"ff": 768}, "shared": {"ff": 1536}}
+
+
+def _fuvolix():
+    dense = {"kind": "dense", "ff": 3072}
+    three = [{"type": "latent_attention", "mlp": dense, "mixer": _LATENT},
+             {"type": "mlstm", "mlp": None, "mixer": {"heads": 4, "dim": 96, "vdim": 192, "gate_cap": 15.0}},
+             {"type": "lightning", "mlp": dense,
+              "mixer": {"heads": 12, "dim": 64, "vdim": 64, "decay": [1.0 - 2.0 ** -(2 + 6 * h / 11) for h in range(12)]}}]
+    return {"architecture": "Fuvolix", "vocab": VOCAB, "width": 768, "norm": {"eps": 1e-5, "groups": 4}, "canon": {"taps": 4},
+            "layers": three * 4}
+
+
+def _sumozen():
+    parallel = {"type": "parallel", "mlp": _MOE, "mixer": {
+        "left": dict(_HEADS, conv=4, softcap=50.0, rot=dict(_ROT, scaling=_YARN)),
+        "right": {"heads": 6, "kv_heads": 3, "dim": 128, "vdim": 128, "conv": 4}, "left_scale": 1.0, "right_scale": 1.0}}
+    mamba = {"type": "mamba2", "mlp": _MOE, "mixer": {"heads": 24, "vdim": 64, "state": 128, "groups": 1, "norm_groups": 1, "conv": 4}}
+    return {"architecture": "Sumozen", "vocab": VOCAB, "width": 768, "norm": {"eps": 1e-5}, "layers": [parallel, parallel, mamba] * 4}
+
+
+def _lipulorn():
+    mlp = {"kind": "dense", "ff": 2048}
+    attention = {"type": "attention", "mlp": mlp, "mixer": dict(_HEADS, mask={"size": 512})}
+    memory = {"type": "channel_delta", "mlp": mlp,
+              "mixer": {"heads": 6, "kv_heads": 3, "dim": 128, "vdim": 128, "a_rank": 64, "g_rank": 64, "conv": 4}}
+    layers = []
+    for index in range(12):
+        mixer = dict(_LATENT, q_rank=384, mask={"size": 512})
+        if index % 6 == 3:
+            mixer["kv_from"] = index - 3
+        latent = {"type": "latent_attention", "mixer": mixer, "mlp": mlp}
+        layers.append([latent, attention, memory][index % 3])
+    return {"architecture": "Lipulorn", "vocab": VOCAB, "width": 768, "streams": 4, "norm": {"eps": 1e-5}, "layers": layers}
+
+
+def _deluvik():
+    banded = dict(_ROT, scaling={"factor": 8.0, "low": 1.0, "high": 4.0, "original": 1024})
+    layers = []
+    for first in (0, 4, 8):
+        layers += [{"type": "attention_2", "mixer": dict(_HEADS, conv=4, rot=_ROT), "mlp": {"kind": "dense", "ff": 3072}},
+                   {"type": "attention", "mixer": dict(_HEADS, kv_heads=1, rot=banded, softcap=50.0), "mlp": _MOE},
+                   {"type": "parallel", "mlp": _MOE, "mixer": {
+                       "left": dict(_HEADS, kv_heads=1, rot=dict(_ROT, dims=32), mask={"size": 512}),
+                       "right": {"width": 768, "blocks": 12, "conv": 4}, "left_scale": 1.0, "right_scale": 1.0}},
+                   {"type": "attention_2", "mixer": dict(_HEADS, conv=4, rot=_ROT, kv_from=first), "mlp": _MOE}]
+    return {"architecture": "Deluvik", "vocab": VOCAB, "width": 768, "norm": {"eps": 1e-5}, "logit_softcap": 30.0, "layers": layers}
+
+
+def _nufavik():
+    layer = {"type": "attention", "mixer": dict(_HEADS, conv=4, rot=_ROT, mask={"size": 512, "keep_first": 64}),
+             "mlp": {"kind": "moe", "router": {"experts": 8, "identity": 2, "top": 2, "scale": 1.5}, "expert": {"ff": 768}}}
+    return {"architecture": "Nufavik", "vocab": VOCAB, "width": 768, "norm": {"eps": 1e-5}, "embedding": {"scale": 1.0},
+            "layers": [layer] * 12}
+
+
+def _kerepel():
+    dense = {"kind": "dense", "ff": 3072}
+    routed = {"kind": "moe", "router": {"experts": 16, "top": 2, "groups": {"count": 4, "keep": 2}},
+              "expert": {"ff": 512, "limit": 7.0}, "shared": {"ff": 512, "limit": 7.0}}
+    latent = dict(_LATENT, rot=dict(_LATENT["rot"], scaling=_YARN))
+    windowed = dict(_HEADS, conv=4, softcap=50.0, mask={"size": 512})
+    layers = []
+    while len(layers) < 12:
+        layers += [{"type": "latent_attention", "mixer": latent, "mlp": dense}, {"type": "attention", "mixer": windowed, "mlp": routed},
+                   {"type": "attention", "mixer": dict(windowed, kv_from=len(layers) + 1), "mlp": dense}]
+    return {"architecture": "Kerepel", "vocab": VOCAB, "width": 768, "norm": {"eps": 1e-5}, "logit_scale": 0.5,
+            "embedding": {"bigram": {"buckets": 32749, "mul_prev": 10007, "mul_cur": 31}}, "token_side": {"dim": 64}, "layers": layers}
+
+
+MODELS = {"gpt2-small": lambda: _gpt2(12, 768, 12), "gpt2-medium": lambda: _gpt2(24, 1024, 16), "gpt2-xl": lambda: _gpt2(48, 1600, 25),
+          "fuvolix": _fuvolix, "sumozen": _sumozen, "lipulorn": _lipulorn, "deluvik": _deluvik, "nufavik": _nufavik, "kerepel": _kerepel}
+
+
+# ---- the cases -----------------------------------------------------------------------------------
+
+def _case(model, requests, prompt, spread, new, portion=STEP_TOKENS, temperature=0.0, top_p=1.0, dtype="bfloat16"):
+    """``requests`` prompts of up to ``prompt`` tokens (shorter by up to ``spread``), ``new`` tokens fed after each, in
+    portions of at most ``portion`` tokens."""
+    return {"model": model, "dtype": dtype, "requests": requests, "prompt": prompt, "spread": spread, "new": new,
+            "portion": portion, "temperature": temperature, "top_p": top_p}
+
+
+def listed():
+    named = {
+        # one user's short question: the latency of single steps, where launches and waits are what counts
+        "small, one request": _case("gpt2-small", 1, 9, 0, 24),
+        # a handful of requests decoding greedily behind half a context
+        "small, 8 requests": _case("gpt2-small", 8, 512, 31, 32),
+        # a full batch of short chats, drawn at a temperature
+        "small, 64 requests": _case("gpt2-small", 64, 128, 59, 24, temperature=0.8),
+        # scoring two documents of the whole context: prompts only
+        "small, 2 whole contexts": _case("gpt2-small", 2, 1024, 0, 0),
+        # a server under load: prompts of all lengths in portions beside decoding requests, nucleus sampling
+        "medium, portions beside decoding": _case("gpt2-medium", 24, 768, 700, 24, portion=512, temperature=1.0, top_p=0.95),
+        # the largest model with its batch full
+        "xl, 64 requests": _case("gpt2-xl", 64, 256, 0, 16, temperature=1.0),
+        # the 32-bit path, which checks and comparisons run on
+        "small in 32 bits, 4 requests": _case("gpt2-small", 4, 61, 17, 6, dtype="float32"),
+        # the other architectures, each from prompts to decoded tokens at another mix of the two
+        "fuvolix, 8 requests": _case("fuvolix", 8, 250, 87, 16),
+        "sumozen, 2 long prompts": _case("sumozen", 2, 1000, 13, 8),
+        "lipulorn, one request": _case("lipulorn", 1, 700, 0, 24),
+        "deluvik, 16 requests": _case("deluvik", 16, 120, 50, 12, temperature=0.8),
+        "kerepel, 3 long prompts": _case("kerepel", 3, 900, 211, 12, temperature=0.7, top_p=0.9),
+    }
+    return [dict(case, name=name) for name, case in named.items()]
+
+
+def draw(rng):
+    model = rng.choice(["gpt2-small", "gpt2-small", "gpt2-small", "gpt2-medium", "gpt2-xl", "fuvolix", "sumozen", "lipulorn", "deluvik",
+                        "nufavik", "kerepel"])
+    dtype = "float32" if model == "gpt2-small" and rng.random() < 0.2 else "bfloat16"
+
+    def spread_over(low, high):
+        return int(round(math.exp(rng.uniform(math.log(low), math.log(high)))))
+    if dtype == "float32":
+        most, prompt, new = 256, spread_over(5, 128), spread_over(1, 8)
+    else:
+        most = 8192 if model.startswith("gpt2") else 3072        # prompt tokens of the batch
+        prompt, new = spread_over(5, 960), rng.choice([0, spread_over(1, 32), spread_over(1, 32), spread_over(1, 32)])
+    requests = min(spread_over(1, 64), max(1, most // prompt))
+    return _case(model, requests, prompt, rng.randrange(prompt // 2 + 1), new, portion=rng.choice([STEP_TOKENS, STEP_TOKENS, 512, 300]),
+                 temperature=rng.choice([0.0, 0.8, 1.0]), top_p=rng.choice([1.0, 1.0, 0.95]), dtype=dtype)
+
+
+def _lengths(case):
+    return [case["prompt"] - (i * 37) % (case["spread"] + 1) for i in range(case["requests"])]
+
+
+def _plan(case):
+    """The steps of a pass, each a list of (request, first token, tokens, whether its last token's logits are wanted):
+    one token of every decoding request, then portions of prompts in the order of the requests."""
+    lengths, steps = _lengths(case), []
+    done = [0] * len(lengths)
+    while any(d < n + case["new"] for d, n in zip(done, lengths)):
+        entries = [(r, done[r], 1, True) for r, n in enumerate(lengths) if n <= done[r] < n + case["new"]]
+        budget = STEP_TOKENS - len(entries)
+        for r, n in enumerate(lengths):
+            count = min(n - done[r], case["portion"], budget)
+            if count > 0:
+                entries.append((r, done[r], count, done[r] + count == n))
+                budget -= count
+        for r, _, count, _ in entries:
+            done[r] += count
+        steps.append(entries)
+    return steps
+
+
+def _tokens(case, seed):
+    rng = np.random.default_rng([seed & 0xFFFFFFFF, 17])
+    return [rng.integers(0, VOCAB, size=n + case["new"]).tolist() for n in _lengths(case)]
+
+
+# ---- weights and engines -------------------------------------------------------------------------
+
+def _is_taps(spec):
+    return len(spec.shape) == 2 and spec.shape[1] <= 8 and spec.init == "matrix" and spec.role == "vector"
+
+
+def _weights(model, dtype):
+    """``{name: (values on the GPU in 32 bits, stored type)}``: what initialisation gives such models, with gains, shifts and
+    biases that are not all alike and with recurrences that remember tens to thousands of tokens."""
+    config = MODELS[model]()
+    spec = describe_model(config_from_dict(config))
+    layers = len(spec.layers)
+    tensors = {}
+    for name, w in collect_specs(model_parts(spec)).items():
+        if w.optional and w.fallback is not None:
+            continue
+        g = torch.Generator(device="cuda").manual_seed(zlib.crc32(name.encode()))
+        values = torch.randn(tuple(w.shape), generator=g, device="cuda")
+        uniform = torch.rand(tuple(w.shape), generator=g, device="cuda")
+        if name.endswith("A_log"):
+            values = torch.log(1.0 + 15.0 * uniform)
+        elif name.endswith("dt_bias"):
+            step = torch.exp(math.log(1e-3) + uniform * math.log(100.0))
+            values = step + torch.log(-torch.expm1(-step))          # softplus of it is the step
+        elif name.endswith(".lam"):
+            values = -8.0 + 4.0 * uniform
+        elif name.endswith(".dwa"):
+            # what a layer hands on: mostly its own result, a little of every earlier one
+            values = 0.05 * values
+            values[-1] += 1.0
+        elif _is_taps(w):
+            values = uniform - 0.5
+        elif w.init == "identity":
+            values = torch.eye(*w.shape, device="cuda") + 0.05 * values
+        elif w.init == "gain":
+            values = 1.0 + 0.1 * values
+        elif w.init == "shift":
+            values *= 0.1
+        elif re.search(r"\.e\d+\.", name):
+            # experts that began as copies of one feed-forward: which of two equally good ones a token takes hardly matters
+            common = torch.Generator(device="cuda").manual_seed(zlib.crc32(re.sub(r"\.e\d+\.", ".e.", name).encode()))
+            values = math.sqrt(0.97) * torch.randn(tuple(w.shape), generator=common, device="cuda") + math.sqrt(0.03) * values
+            values *= 0.02 / (math.sqrt(2.0 * layers) if w.init == "residual_matrix" else 1.0)
+        elif w.init == "residual_matrix":
+            values *= 0.02 / math.sqrt(2.0 * layers)
+        else:
+            values *= 0.02
+        stored = "BF16" if dtype == "bfloat16" and w.role != "vector" else "F32"
+        tensors[name] = (values.bfloat16().float() if stored == "BF16" else values, stored)
+    return config, tensors
+
+
+_engines = {}
+
+
+def _engine(model, dtype):
+    if (model, dtype) not in _engines:
+        config, tensors = _weights(model, dtype)
+        with tempfile.TemporaryDirectory() as folder:
+            with open(os.path.join(folder, "config.json"), "w", encoding="utf-8") as handle:
+                json.dump(config_from_dict(config).to_dict(), handle)
+            write_safetensors(os.path.join(folder, "model.safetensors"), {n: v.cpu().numpy() for n, (v, _) in tensors.items()},
+                              {n: stored for n, (_, stored) in tensors.items()})
+            del tensors
+            _engines[model, dtype] = Engine(folder, dtype=dtype, max_requests=64, cache_tokens=64 * 1024)
+    return _engines[model, dtype]
+
+
+# ---- a pass --------------------------------------------------------------------------------------
+
+def prepare(case, seed):
+    plan = _plan(case)
+    rows = sum(want for entries in plan for _, _, _, want in entries)
+    return {"engine": _engine(case["model"], case["dtype"]), "case": case, "plan": plan, "tokens": _tokens(case, seed),
+            "seeds": [request_seed(seed, r) for r in range(case["requests"])],
+            "logits": torch.empty(rows, VOCAB, dtype=torch.float32, device="cuda")}
+
+
+def run(state):
+    engine, case, tokens, logits = state["engine"], state["case"], state["tokens"], state["logits"]
+    slots = [engine.open_request() for _ in range(case["requests"])]
+    drawn, row, counts = [], 0, [0] * case["requests"]
+    for index, planned in enumerate(state["plan"]):
+        entries, sampling = [], []
+        for request, first, count, want in planned:
+            entries.append(StepEntry(slots[request], tokens[request][first:first + count], [count - 1] if want else []))
+            if want:
+                sampling.append(SamplingParams(case["temperature"], case["top_p"], state["seeds"][request], counts[request]))
+                counts[request] += 1
+        got = engine.step(entries, sampling)
+        if got is not None:
+            logits[row:row + got.shape[0]].copy_(got)
+            row += got.shape[0]
+        if index:
+            drawn.extend(engine.sampled_tokens(1))
+    drawn.extend(engine.sampled_tokens(0))
+    for slot in slots:
+        engine.close_request(slot)
+    if case["dtype"] == "float32":
+        return {"logits": logits, "tokens": np.array(drawn, dtype=np.int64)}
+    # A draw turns on the last bits of two logits that lie side by side: with 16-bit activations a few in a hundred
+    # of another correct implementation's draws differ, so what is compared there is the logits they are drawn from.
+    return {"logits": logits}
+
+
+def tolerance(case):
+    if case["dtype"] == "float32":
+        return {"rel": 1e-5, "differ": 0.01}
+    # Measured against the plain kernels, which sum in another order: rel 0.004 for GPT-2 at every size, 0.005 to 0.018 for the
+    # others, where a router's near tie may go the other way.
+    return {"rel": 0.016, "max": 0.1} if case["model"].startswith("gpt2") else {"rel": 0.03, "max": 0.7}
+
+
+# ---- what a pass cannot do without ---------------------------------------------------------------
+
+def _layers(model, config):
+    """Of every layer: (heads, entries of a query and of a value, keys a query sees at most, cached values a token, values of
+    state a request, operations a token on that state)."""
+    if model.startswith("gpt2"):
+        heads = config["n_head"]
+        return [(heads, 64, 64, None, 2 * config["n_embd"], 0, 0)] * config["n_layer"]
+    out = []
+
+    def attend(m, own):
+        mask = m.get("mask") or {}
+        seen = mask["size"] + mask.get("keep_first", 0) if mask else None
+        out.append((m["heads"], m["dim"], m["vdim"], seen, m["kv_heads"] * (m["dim"] + m["vdim"]) if own else 0, 0, 0))
+
+    def state(heads, values, times):
+        out.append((heads, 0, 0, 0, 0, heads * values, times * heads * values))
+    for layer in config["layers"]:
+        m, kind = layer["mixer"], layer["type"]
+        if kind == "latent_attention":
+            out.append((m["heads"], m["dim"] + m["rot_dim"], m["vdim"], (m.get("mask") or {}).get("size"),
+                        m["kv_rank"] + m["rot_dim"] if "kv_from" not in m else 0, 0, 0))
+        elif kind == "parallel":
+            attend(m["left"], True)
+            right = m["right"]
+            if "blocks" in right:
+                state(1, right["width"], 4)
+            else:
+                state(right["heads"], right["dim"] * right["vdim"], 6)
+        elif kind in ("attention", "attention_2"):
+            attend(m, "kv_from" not in m)
+        elif kind == "mamba2":
+            state(m["heads"], m["state"] * m["vdim"], 4)
+        else:
+            state(m["heads"], m["dim"] * m["vdim"], 6 if kind == "channel_delta" else 4)
+    return out
+
+
+def work(case):
+    """Per step: every weight that its tokens need once, the cached rows they see and the states they move, the logits that
+    come out; products of every token with those weights, scores and weighted sums of what it sees."""
+    config = MODELS[case["model"]]()
+    spec = describe_model(config_from_dict(config))
+    size = 4 if case["dtype"] == "float32" else 2
+    routers = [layer["mlp"]["router"] for layer in config.get("layers", ()) if layer.get("mlp") and layer["mlp"]["kind"] == "moe"]
+    share = routers[0]["top"] / (routers[0]["experts"] + routers[0].get("identity", 0)) if routers else 0.0
+    dense = routed = head = 0
+    for name, w in collect_specs(model_parts(spec)).items():
+        count = math.prod(w.shape)
+        if re.search(r"\.e\d+\.", name):
+            routed += count
+        elif name in ("head", "wte.weight") or (name == "embed" and "architecture" in config and config["architecture"] in
+                                                ("Fuvolix", "Nufavik", "Kerepel")):
+            head = count
+        elif w.role == "matrix":
+            dense += count
+    layers = _layers(case["model"], config)
+    total_bytes = flops = 0.0
+    for entries in _plan(case):
+        tokens = sum(count for _, _, count, _ in entries)
+        rows = sum(want for _, _, _, want in entries)
+        touched = min(1.0, tokens * share)              # of the experts, by the tokens that choose them
+        total_bytes += size * (dense + touched * routed + (head if rows else 0)) + rows * VOCAB * 4.0
+        flops += 2.0 * tokens * (dense + share * routed) + 2.0 * rows * head
+        for _, first, count, _ in entries:
+            for heads, dim, vdim, seen, cached, held, moved in layers:
+                if seen == 0:
+                    total_bytes += 8.0 * held
+                    flops += count * moved
+                    continue
+                last = first + count
+                pairs = sum(min(p + 1, seen or last) for p in range(first, last)) if seen else (first + 1 + last) * count / 2.0
+                total_bytes += size * cached * (count + min(first, seen or first))
+                flops += 2.0 * pairs * heads * (dim + vdim)
+    return {"bytes": total_bytes, "flops": flops}
+
+
+# ---- the same in 64 bits -------------------------------------------------------------------------
+# Whole sequences at once, padded at their end to one length; nothing here is shared with the package but the weights' values.
+
+def _rms(x, eps, gain=None):
+    y = x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps)
+    return y if gain is None else y * gain
+
+
+def _conv(u, w, bias=None):
+    n, taps = u.shape[1], w.shape[1]
+    padded = torch.nn.functional.pad(u, (0, 0, taps - 1, 0))
+    y = sum(padded[:, j:j + n] * w[:, j] for j in range(taps))
+    return y if bias is None else y + bias
+
+
+def _frequencies(rot):
+    dims, scaling = rot["dims"], rot.get("scaling")
+    f = [rot["base"] ** (-2.0 * i / dims) for i in range(dims // 2)]
+    if not scaling:
+        return f, 1.0
+    if "low" in scaling:                     # by bands of the wavelength
+        out = []
+        for one in f:
+            turns = scaling["original"] * one / (2.0 * math.pi)
+            s = min(max((turns - scaling["low"]) / (scaling["high"] - scaling["low"]), 0.0), 1.0)
+            out.append((1.0 - s) * one / scaling["factor"] + s * one)
+        return out, 1.0
+
+    def place(turns):
+        return dims * math.log(scaling["original"] / (2.0 * math.pi * turns)) / (2.0 * math.log(rot["base"]))
+    lo, hi = max(math.floor(place(scaling["fast"])), 0), min(math.ceil(place(scaling["slow"])), dims - 1)
+    ramp = [min(max((i - lo) / max(hi - lo, 0.001), 0.0), 1.0) for i in range(len(f))]
+    return [one / scaling["factor"] * r + one * (1.0 - r) for one, r in zip(f, ramp)], 0.1 * math.log(scaling["factor"]) + 1.0
+
+
+def _rotate(x, rot, half_apart):
+    """x [B, T, heads, size]: pairs among the first ``dims`` entries turn by position * frequency."""
+    f, amplitude = _frequencies(rot)
+    dims = rot["dims"]
+    angle = torch.arange(x.shape[1], device=x.device, dtype=x.dtype)[:, None] * torch.tensor(f, device=x.device, dtype=x.dtype)
+    c, s = torch.cos(angle)[:, None] * amplitude, torch.sin(angle)[:, None] * amplitude
+    first = slice(0, dims // 2) if half_apart else slice(0, dims, 2)
+    second = slice(dims // 2, dims) if half_apart else slice(1, dims, 2)
+    out = x.clone()
+    out[..., first] = x[..., first] * c - x[..., second] * s
+    out[..., second] = x[..., second] * c + x[..., first] * s
+    return out
+
+
+def _visible(n, device, window=None, keep=0, block=None):
+    i, j = torch.arange(n, device=device)[:, None], torch.arange(n, device=device)[None]
+    see = j <= i
+    if window is not None:
+        see = see & ((i - j < window) | (j < keep))
+    return see & (i // block == j // block) if block is not None else see
+
+
+def _attend(q, k, v, scale, visible, cap=None, sink=None, slopes=None):
+    """q [B, T, H, d], k [B, T, G, d], v [B, T, G, e] -> [B, T, H, e]."""
+    group = q.shape[2] // k.shape[2]
+    q, k, v = q.transpose(1, 2), k.repeat_interleave(group, 2).transpose(1, 2), v.repeat_interleave(group, 2).transpose(1, 2)
+    s = q @ k.transpose(-1, -2) * scale
+    if cap:
+        s = cap * torch.tanh(s / cap)
+    if slopes is not None:
+        at = torch.arange(s.shape[-1], device=s.device, dtype=s.dtype)
+        s = s - slopes[:, None, None] * (at[:, None] - at[None])
+    s = s.masked_fill(~visible, -math.inf)
+    if sink is not None:
+        s = torch.cat([s, sink[:, None, None].expand(s.shape[0], -1, s.shape[2], 1)], -1)
+    p = torch.softmax(s, -1)
+    return (p[..., :k.shape[2]] @ v).transpose(1, 2)
+
+
+def _gated(x, w, p, act):
+    return (act(x @ w(p + ".gate").T) * (x @ w(p + ".up").T)) @ w(p + ".down").T
+
+
+_silu = torch.nn.functional.silu
+_softplus = torch.nn.functional.softplus
+
+
+def _gelu(x):
+    return torch.nn.functional.gelu(x, approximate="tanh")
+
+
+def _routed(h, chosen, weight, count, expert):
+    """Sum over every token's chosen experts e < count of expert(e, the token's row, its weight)."""
+    x, out = h.reshape(-1, h.shape[-1]), torch.zeros_like(h).reshape(-1, h.shape[-1])
+    chosen, weight = chosen.reshape(x.shape[0], -1), weight.reshape(x.shape[0], -1)
+    for e in range(count):
+        at, place = torch.nonzero(chosen == e, as_tuple=True)
+        if at.numel():
+            out[at] += expert(e, x[at], weight[at, place][:, None])
+    return out.reshape(h.shape)
+
+
+def _latent(h, m, w, p, eps, q, half_apart, visible, kv=None):
+    b, n = h.shape[:2]
+    rank, dim = m["kv_rank"], m["dim"]
+    if kv is None:
+        down = h @ w(p + ".dkv").T
+        kv = _rms(down[..., :rank], eps, w(p + ".dkv.norm")), _rotate(down[..., None, rank:], m["rot"], half_apart)
+    c, shared = kv
+    q = q.reshape(b, n, m["heads"], -1)
+    q = torch.cat([q[..., :dim], _rotate(q[..., dim:], m["rot"], half_apart)], -1)
+    k = torch.cat([(c @ w(p + ".uk").T).reshape(b, n, m["heads"], dim), shared.expand(-1, -1, m["heads"], -1)], -1)
+    v = (c @ w(p + ".uv").T).reshape(b, n, m["heads"], m["vdim"])
+    return _attend(q, k, v, m["scale"], visible), kv
+
+
+def _delta(h, m, w, p, eps, decay, gate):
+    """S <- decay S; u = beta (v - S^T k); S <- S + k u^T; o = S^T q.  decay [B, T, heads, dim or 1]."""
+    b, n, heads, dim = h.shape[0], h.shape[1], m["heads"], m["dim"]
+
+    def stream(name, size):
+        return _silu(_conv(h @ w(f"{p}.{name}").T, w(f"{p}.{name}.conv"))).reshape(b, n, -1, size)
+    q, k, v = stream("q", dim), stream("k", dim), stream("v", m["vdim"])
+    group = heads // m["kv_heads"]
+    q = (q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * dim ** -0.5).repeat_interleave(group, 2)
+    k = (k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)).repeat_interleave(group, 2)
+    beta = torch.sigmoid(h @ w(p + ".b").T)[..., None]
+    state = h.new_zeros(b, heads, dim, m["vdim"])
+    out = torch.empty_like(v)
+    for t in range(n):
+        state = state * decay[:, t, :, :, None]
+        u = beta[:, t] * (v[:, t] - torch.einsum("bhde,bhd->bhe", state, k[:, t]))
+        state = state + k[:, t, :, :, None] * u[:, :, None]
+        out[:, t] = torch.einsum("bhde,bhd->bhe", state, q[:, t])
+    return (_rms(out, eps, w(p + ".norm")) * gate).reshape(b, n, -1) @ w(p + ".o").T
+
+
+def _gpt2_rows(config, w, ids):
+    eps, heads = config["layer_norm_epsilon"], config["n_head"]
+    b, n = ids.shape
+
+    def norm(x, p):
+        return torch.nn.functional.layer_norm(x, x.shape[-1:], w(p + ".weight"), w(p + ".bias"), eps)
+    x = w("wte.weight")[ids] + w("wpe.weight")[:n]
+    see = _visible(n, ids.device)
+    for i in range(config["n_layer"]):
+        p = f"h.{i}."
+        qkv = norm(x, p + "ln_1") @ w(p + "attn.c_attn.weight") + w(p + "attn.c_attn.bias")
+        q, k, v = (t.reshape(b, n, heads, -1) for t in qkv.chunk(3, -1))
+        x = x + _attend(q, k, v, 0.125, see).reshape(b, n, -1) @ w(p + "attn.c_proj.weight") + w(p + "attn.c_proj.bias")
+        up = _gelu(norm(x, p + "ln_2") @ w(p + "mlp.c_fc.weight") + w(p + "mlp.c_fc.bias"))
+        x = x + up @ w(p + "mlp.c_proj.weight") + w(p + "mlp.c_proj.bias")
+    return norm(x, "ln_f"), w("wte.weight"), lambda z: z
+
+
+def _fuvolix_rows(config, w, ids):
+    eps, groups = config["norm"]["eps"], config["norm"]["groups"]
+    b, n = ids.shape
+
+    def norm(x, name):
+        return _rms(x.reshape(b, n, groups, -1), eps).reshape(b, n, -1) * w(name)
+    x = norm(w("embed")[ids], "embed.norm")
+    results, see = [x], _visible(n, ids.device)
+    for i, layer in enumerate(config["layers"]):
+        p, m = f"l{i}.", layer["mixer"]
+        h = norm(x, p + "norm1")
+        h = h + _conv(h, w(p + "canon1"))
+        if layer["type"] == "latent_attention":
+            y, _ = _latent(h, m, w, p + "mix", eps, h @ w(p + "mix.q").T, False, see)
+            y = y.reshape(b, n, -1)
+        else:
+            gated = layer["type"] == "mlstm"
+            q, k, v = (h @ w(f"{p}mix.{name}").T for name in "qkv")
+            if not gated:
+                q, k, v = _silu(q), _silu(k), _silu(v)
+            q, k, v = (t.reshape(b, n, m["heads"], -1) for t in (q, k, v))
+            state, norm_state, top = h.new_zeros(b, m["heads"], m["dim"], m["vdim"]), h.new_zeros(b, m["heads"], m["dim"]), h.new_zeros(b, m["heads"])
+            y = torch.empty_like(v)
+            if gated:
+                q, cap = q * m["dim"] ** -0.5, m["gate_cap"]
+                log_in = cap * torch.tanh((h @ w(p + "mix.i").T + w(p + "mix.i.b")) / cap)
+                log_keep = -_softplus(-cap * torch.tanh((h @ w(p + "mix.f").T + w(p + "mix.f.b")) / cap))
+            else:
+                decay = torch.tensor(m["decay"], device=h.device, dtype=h.dtype)[:, None, None]
+            for t in range(n):
+                outer = k[:, t, :, :, None] * v[:, t, :, None]
+                if gated:
+                    new = torch.maximum(log_keep[:, t] + top, log_in[:, t])
+                    keep, take = torch.exp(log_keep[:, t] + top - new), torch.exp(log_in[:, t] - new)
+                    state = keep[..., None, None] * state + take[..., None, None] * outer
+                    norm_state, top = keep[..., None] * norm_state + take[..., None] * k[:, t], new
+                    below = torch.maximum((norm_state * q[:, t]).sum(-1).abs(), torch.exp(-top)) + 1e-6
+                    y[:, t] = torch.einsum("bhde,bhd->bhe", state, q[:, t]) / below[..., None]
+                else:
+                    state = decay * state + outer
+                    y[:, t] = torch.einsum("bhde,bhd->bhe", state, q[:, t])
+            y = _rms(y, eps).reshape(b, n, -1) if gated else _rms(y.reshape(b, n, -1), eps)
+            y = y * w(p + "mix.norm") * torch.sigmoid(h @ w(p + "mix.g").T)
+        x = x + norm(y @ w(p + "mix.o").T, p + "norm1b")
+        if layer["mlp"] is not None:
+            up = torch.relu(norm(x, p + "norm2") @ w(p + "mlp.up").T)
+            x = x + norm((up * up) @ w(p + "mlp.down").T, p + "norm2b")
+        results.append(x)
+        x = sum(a * r for a, r in zip(w(p + "dwa"), results))
+    return norm(x, "final.norm"), w("embed"), lambda z: z
+
+
+def _sumozen_rows(config, w, ids):
+    eps = config["norm"]["eps"]
+    b, n = ids.shape
+    x, see = w("embed")[ids], _visible(n, ids.device)
+    for i, layer in enumerate(config["layers"]):
+        p, m, mlp = f"l{i}.mix", layer["mixer"], layer["mlp"]
+        h = _rms(x, eps) * (1.0 + w(f"l{i}.norm1"))
+        if layer["type"] == "parallel":
+            a = m["left"]
+            q, k, v = (_conv(h @ w(f"{p}.left.{c}").T + w(f"{p}.left.{c}.b"), w(f"{p}.left.{c}.conv")).reshape(b, n, -1, a["dim"]) for c in "qkv")
+            left = _attend(_rotate(q, a["rot"], False), _rotate(k, a["rot"], False), v, a["scale"], see, a["softcap"]).reshape(b, n, -1)
+            left = left @ w(p + ".left.o").T + w(p + ".left.o.b")
+            r = p + ".right"
+            decay = torch.exp(-torch.exp(w(r + ".A_log")) * _softplus(h @ w(r + ".a").T + w(r + ".dt_bias")))
+            gate = _silu(h @ w(r + ".g").T).reshape(b, n, m["right"]["heads"], -1)
+            x = x + m["left_scale"] * left + m["right_scale"] * _delta(h, m["right"], w, r, eps, decay[..., None], gate)
+        else:
+            heads, inner, size = m["heads"], m["heads"] * m["vdim"], m["groups"] * m["state"]
+            z, xbc, dt = (h @ w(p + ".in").T).split([inner, inner + 2 * size, heads], -1)
+            u, k, q = _silu(_conv(xbc, w(p + ".conv"), w(p + ".conv.b"))).split([inner, size, size], -1)
+            u = u.reshape(b, n, heads, -1)
+            k, q = (t.reshape(b, n, m["groups"], -1).repeat_interleave(heads // m["groups"], 2) for t in (k, q))
+            dt = _softplus(dt + w(p + ".dt_bias"))
+            decay = torch.exp(-torch.exp(w(p + ".A_log")) * dt)
+            state, y = h.new_zeros(b, heads, m["state"], m["vdim"]), torch.empty_like(u)
+            for t in range(n):
+                state = decay[:, t, :, None, None] * state + dt[:, t, :, None, None] * k[:, t, :, :, None] * u[:, t, :, None]
+                y[:, t] = torch.einsum("bhde,bhd->bhe", state, q[:, t]) + w(p + ".D")[:, None] * u[:, t]
+            y = _rms((y.reshape(b, n, inner) * _silu(z)).reshape(b, n, m["norm_groups"], -1), eps).reshape(b, n, inner) * w(p + ".norm")
+            x = x + y @ w(p + ".o").T
+        p = f"l{i}.mlp"
+        h = _rms(x, eps) * (1.0 + w(f"l{i}.norm2"))
+        score, chosen = torch.sigmoid(h @ w(p + ".router").T).topk(mlp["router"]["top"])
+        x = x + _routed(h, chosen, score, mlp["router"]["experts"], lambda e, u, g: _gated(u * g, w, f"{p}.e{e}", _silu))
+        x = x + _gated(h, w, p + ".shared", _silu) * torch.sigmoid(h @ w(p + ".shared.sg").T)
+    return _rms(x, eps) * (1.0 + w("final.norm")), w("head"), lambda z: z
+
+
+def _lipulorn_rows(config, w, ids):
+    eps = config["norm"]["eps"]
+    b, n = ids.shape
+    streams, kept = w("embed")[ids].expand(config["streams"], -1, -1, -1), {}
+
+    def read(p, gain):
+        return _rms(torch.einsum("s,sbtc->btc", w(p + ".in"), streams), eps, w(gain))
+
+    def write(p, y):
+        return torch.einsum("st,sbnc->tbnc", w(p + ".mix"), streams) + w(p + ".out")[:, None, None, None] * y
+    for i, layer in enumerate(config["layers"]):
+        p, m = f"l{i}.mix", layer["mixer"]
+        h = read(f"l{i}.hc1", f"l{i}.norm1")
+        if layer["type"] == "latent_attention":
+            source = m.get("kv_from")
+            q = _rms(h @ w(p + ".dq").T, eps, w(p + ".dq.norm")) @ w(p + ".uq").T
+            y, kept[i] = _latent(h, m, w, p, eps, q, True, _visible(n, ids.device, m["mask"]["size"]), kept.get(source))
+            y = y.reshape(b, n, -1) @ w(p + ".o").T
+        elif layer["type"] == "attention":
+            q, k, v = ((h @ w(f"{p}.{c}").T + w(f"{p}.{c}.b")).reshape(b, n, -1, m["dim"]) for c in "qkv")
+            y = _attend(_rms(q, eps), _rms(k, eps), v, m["scale"], _visible(n, ids.device, block=m["mask"]["size"]))
+            y = (y * torch.sigmoid(h @ w(p + ".g").T)[..., None]).reshape(b, n, -1) @ w(p + ".o").T
+        else:
+            step = _softplus(h @ w(p + ".a1").T @ w(p + ".a2").T + w(p + ".dt_bias")).reshape(b, n, m["heads"], -1)
+            gate = torch.sigmoid(h @ w(p + ".g1").T @ w(p + ".g2").T).reshape(b, n, m["heads"], -1)
+            y = _delta(h, m, w, p, eps, torch.exp(-torch.exp(w(p + ".A_log"))[:, None] * step), gate)
+        streams = write(f"l{i}.hc1", y)
+        h, p = read(f"l{i}.hc2", f"l{i}.norm2"), f"l{i}.mlp"
+        y = _silu(h @ w(p + ".gate").T + w(p + ".gate.b")) * (h @ w(p + ".up").T + w(p + ".up.b"))
+        streams = write(f"l{i}.hc2", y @ w(p + ".down").T + w(p + ".down.b"))
+    return _rms(streams.sum(0), eps, w("final.norm")), w("head"), lambda z: z
+
+
+def _deluvik_rows(config, w, ids):
+    eps = config["norm"]["eps"]
+    b, n = ids.shape
+    x, see, rows = w("embed")[ids], _visible(n, ids.device), {}
+    for i, layer in enumerate(config["layers"]):
+        p, m, mlp = f"l{i}.mix", layer["mixer"], layer["mlp"]
+        if layer["type"] == "parallel":
+            a, u = m["left"], m["right"]
+            q, k, v = ((x @ w(f"{p}.left.{c}").T).reshape(b, n, -1, a["dim"]) for c in "qkv")
+            q, k = (_rotate(_rms(t, eps, w(f"{p}.left.{c}.norm")), a["rot"], False) for t, c in ((q, "q"), (k, "k")))
+            y = _attend(q, k, v, a["scale"], _visible(n, ids.device, a["mask"]["size"])).reshape(b, n, -1) @ w(p + ".left.o").T
+            r = p + ".right"
+            opened = _gelu(x @ w(r + ".y").T + w(r + ".y.b"))
+            c = _conv(x @ w(r + ".x").T + w(r + ".x.b"), w(r + ".conv"), w(r + ".conv.b"))
+            parts = c.reshape(b, n, u["blocks"], -1)
+            gates = [torch.sigmoid(torch.einsum("btki,koi->btko", parts, w(f"{r}.{g}")) + w(f"{r}.{g}.b")).reshape(b, n, -1) for g in ("ra", "ri")]
+            decay = torch.exp(-8.0 * gates[0] * _softplus(w(r + ".lam")))
+            add = torch.sqrt(1.0 - decay * decay) * gates[1] * c
+            state, out = torch.zeros_like(c[:, 0]), torch.empty_like(c)
+            for t in range(n):
+                state = decay[:, t] * state + add[:, t]
+                out[:, t] = state
+            y = m["left_scale"] * y + m["right_scale"] * ((out * opened) @ w(r + ".o").T)
+        else:
+            taps = layer["type"] == "attention_2"
+
+            def stream(name):
+                t = x @ w(f"{p}.{name}").T
+                return _conv(t, w(f"{p}.{name}.conv")) if taps else t
+            q = _rotate(_rms(stream("q"), eps, w(p + ".q.norm")).reshape(b, n, -1, m["dim"]), m["rot"], True)
+            if "kv_from" in m:
+                rows[i] = rows[m["kv_from"]]
+            else:
+                k = stream("k")
+                v = (stream("v") if taps else k).reshape(b, n, m["kv_heads"], -1)
+                rows[i] = _rotate(_rms(k, eps, w(p + ".k.norm")).reshape(b, n, -1, m["dim"]), m["rot"], True), v
+            y = _attend(q, *rows[i], m["scale"], see, m.get("softcap"), w(p + ".sink")).reshape(b, n, -1) @ w(p + ".o").T
+        x = x + _rms(y, eps, w(f"l{i}.norm1"))
+        p = f"l{i}.mlp"
+        if mlp["kind"] == "dense":
+            y = _gated(x, w, p, _gelu)
+        else:
+            value, chosen = (x @ w(p + ".router").T + w(p + ".router.b")).topk(mlp["router"]["top"])
+            y = _routed(x, chosen, torch.softmax(value, -1), mlp["router"]["experts"], lambda e, u, g: g * _gated(u, w, f"{p}.e{e}", _silu))
+            y = y + _gated(x, w, p + ".shared", _silu)
+        x = x + _rms(y, eps, w(f"l{i}.norm2"))
+    cap = config["logit_softcap"]
+    return _rms(x, eps, w("final.norm")), w("head"), lambda z: cap * torch.tanh(z / cap)
+
+
+def _nufavik_rows(config, w, ids):
+    eps = config["norm"]["eps"]
+    b, n = ids.shape
+    x = w("embed")[ids] * config["embedding"]["scale"]
+    for i, layer in enumerate(config["layers"]):
+        p, m, router = f"l{i}.mix", layer["mixer"], layer["mlp"]["router"]
+        h = _rms(x, eps, w(f"l{i}.norm1"))
+        q, k, v = (_conv(h @ w(f"{p}.{c}").T + w(f"{p}.{c}.b"), w(f"{p}.{c}.conv")).reshape(b, n, -1, m["dim"]) for c in "qkv")
+        see = _visible(n, ids.device, m["mask"]["size"], m["mask"]["keep_first"])
+        y = _attend(_rotate(q, m["rot"], True), _rotate(k, m["rot"], True), v, m["scale"], see, sink=x.new_zeros(m["heads"]))
+        x = x + y.reshape(b, n, -1) @ w(p + ".o").T
+        p = f"l{i}.mlp"
+        score = torch.softmax(h @ w(p + ".router").T, -1)
+        chosen = (score + w(p + ".correction")).topk(router["top"])[1]
+        weight = score.gather(-1, chosen)
+        weight = weight / (weight.sum(-1, keepdim=True) + 1e-20) * router["scale"]
+        x = x + _routed(h, chosen, weight, router["experts"] + router["identity"],
+                        lambda e, u, g: g * (torch.relu(u @ w(f"{p}.e{e}.up").T) ** 2 @ w(f"{p}.e{e}.down").T if e < router["experts"] else u))
+    return _rms(x, eps, w("final.norm")), w("embed"), lambda z: z
+
+
+def _kerepel_rows(config, w, ids):
+    eps, pair, side = config["norm"]["eps"], config["embedding"]["bigram"], config["token_side"]["dim"]
+    b, n = ids.shape
+    before = torch.cat([torch.full_like(ids[:, :1], -1), ids[:, :-1]], 1)
+    row = torch.where(before < 0, pair["buckets"], (before * pair["mul_prev"] + ids * pair["mul_cur"]) % pair["buckets"])
+    x, rows = w("embed")[ids] + w("bigram")[row], {}
+
+    def expert(u, p, limit):
+        g, up = (u @ w(p + ".gate").T).clamp(max=limit), (u @ w(p + ".up").T).clamp(-limit, limit)
+        return (g * torch.sigmoid(1.702 * g) * (up + 1.0)) @ w(p + ".down").T
+    for i, layer in enumerate(config["layers"]):
+        p, m, mlp = f"l{i}.mix", layer["mixer"], layer["mlp"]
+        h = _rms(x, eps, w(f"l{i}.norm1"))
+        if layer["type"] == "latent_attention":
+            y, _ = _latent(h, m, w, p, eps, h @ w(p + ".q").T, False, _visible(n, ids.device))
+            y = (y * torch.sigmoid(h @ w(p + ".g").T)[..., None]).reshape(b, n, -1)
+        else:
+            def stream(name):
+                return _conv(h @ w(f"{p}.{name}").T, w(f"{p}.{name}.conv")).reshape(b, n, -1, m["dim"])
+            q = _rms(stream("q"), eps, w(p + ".q.norm"))
+            rows[i] = rows[m["kv_from"]] if "kv_from" in m else (_rms(stream("k"), eps, w(p + ".k.norm")), stream("v"))
+            slopes = torch.tensor([2.0 ** (-8.0 * (a + 1) / m["heads"]) for a in range(m["heads"])], device=x.device, dtype=x.dtype)
+            y = _attend(q, *rows[i], m["scale"], _visible(n, ids.device, m["mask"]["size"]), m["softcap"], slopes=slopes)
+            y = y.reshape(b, n, -1) * torch.sigmoid(h @ w(p + ".g").T)
+        x = x + y @ w(p + ".o").T
+        h, p = _rms(x, eps, w(f"l{i}.norm2")), f"l{i}.mlp"
+        if mlp["kind"] == "dense":
+            x = x + torch.nn.functional.gelu(h @ w(p + ".up").T) @ w(p + ".down").T
+        else:
+            router, limit = mlp["router"], mlp["expert"]["limit"]
+            score = torch.sigmoid(h @ w(p + ".router").T)
+            ranked = (score + w(p + ".correction")).reshape(b, n, router["groups"]["count"], -1)
+            kept = ranked.topk(2)[0].sum(-1).topk(router["groups"]["keep"])[1]
+            open_ = torch.zeros(ranked.shape[:3], dtype=torch.bool, device=x.device).scatter_(2, kept, True)
+            chosen = ranked.masked_fill(~open_[..., None], -math.inf).reshape(b, n, -1).topk(router["top"])[1]
+            x = x + _routed(h, chosen, score.gather(-1, chosen), router["experts"], lambda e, u, g: g * expert(u, f"{p}.e{e}", limit))
+            x = x + expert(h, p + ".shared", mlp["shared"]["limit"]) * torch.sigmoid(h @ w(p + ".shared.sg").T)
+        own = w("side.embed")[ids][..., i * side:(i + 1) * side]
+        x = x + _rms((_gelu(x @ w(f"l{i}.side.gate").T) * own) @ w(f"l{i}.side.proj").T, eps, w(f"l{i}.side.norm"))
+    return _rms(x, eps, w("final.norm")), w("embed"), lambda z: z * config["logit_scale"]
+
+
+ROWS = {"gpt2-small": _gpt2_rows, "gpt2-medium": _gpt2_rows, "gpt2-xl": _gpt2_rows, "fuvolix": _fuvolix_rows, "sumozen": _sumozen_rows,
+        "lipulorn": _lipulorn_rows, "deluvik": _deluvik_rows, "nufavik": _nufavik_rows, "kerepel": _kerepel_rows}
+
+
+@torch.no_grad()
+def exact(case, seed):
+    config, tensors = _weights(case["model"], case["dtype"])
+    tokens, lengths = _tokens(case, seed), _lengths(case)
+    most = max(len(t) for t in tokens)
+    ids = torch.tensor([t + [0] * (most - len(t)) for t in tokens], device="cuda")
+    held = {}
+
+    def w(name):
+        # small tensors stay widened; the largest are widened when they are used
+        if name in held:
+            return held[name]
+        wide = tensors[name][0].double()
+        if wide.numel() < 1 << 24:
+            held[name] = wide
+        return wide
+    places = {}                  # (request, position) -> row of the output
+    for entries in _plan(case):
+        for request, first, count, want in entries:
+            if want:
+                places[request, first + count - 1] = len(places)
+    logits = torch.empty(len(places), VOCAB, dtype=torch.float64, device="cuda")
+    together = max(1, 4096 // most)
+    for start in range(0, len(lengths), together):
+        rows, head, last = ROWS[case["model"]](config, w, ids[start:start + together])
+        mine = [(r, t, row) for (r, t), row in places.items() if start <= r < start + together]
+        at = torch.tensor(mine, device="cuda")
+        logits[at[:, 2]] = last(rows[at[:, 0] - start, at[:, 1]] @ head.T)
+    out = {"logits": logits}
+    if case["dtype"] == "float32":
+        out["tokens"] = None
+    return out
