@@ -129,25 +129,25 @@ def _case(model, requests, prompt, spread, new, portion=STEP_TOKENS, temperature
 def listed():
     named = {
         # one user's short question: the latency of single steps, where launches and waits are what counts
-        "small, one request": _case("gpt2-small", 1, 9, 0, 24),
+        "small one request": _case("gpt2-small", 1, 9, 0, 24),
         # a handful of requests decoding greedily behind half a context
-        "small, 8 requests": _case("gpt2-small", 8, 512, 31, 32),
+        "small 8 requests": _case("gpt2-small", 8, 512, 31, 32),
         # a full batch of short chats, drawn at a temperature
-        "small, 64 requests": _case("gpt2-small", 64, 128, 59, 24, temperature=0.8),
+        "small 64 requests": _case("gpt2-small", 64, 128, 59, 24, temperature=0.8),
         # scoring two documents of the whole context: prompts only
-        "small, 2 whole contexts": _case("gpt2-small", 2, 1024, 0, 0),
+        "small 2 whole contexts": _case("gpt2-small", 2, 1024, 0, 0),
         # a server under load: prompts of all lengths in portions beside decoding requests, nucleus sampling
-        "medium, portions beside decoding": _case("gpt2-medium", 24, 768, 700, 24, portion=512, temperature=1.0, top_p=0.95),
+        "medium portions beside decoding": _case("gpt2-medium", 24, 768, 700, 24, portion=512, temperature=1.0, top_p=0.95),
         # the largest model with its batch full
-        "xl, 64 requests": _case("gpt2-xl", 64, 256, 0, 16, temperature=1.0),
+        "xl 64 requests": _case("gpt2-xl", 64, 256, 0, 16, temperature=1.0),
         # the 32-bit path, which checks and comparisons run on
-        "small in 32 bits, 4 requests": _case("gpt2-small", 4, 61, 17, 6, dtype="float32"),
+        "small in 32 bits 4 requests": _case("gpt2-small", 4, 61, 17, 6, dtype="float32"),
         # the other architectures, each from prompts to decoded tokens at another mix of the two
-        "fuvolix, 8 requests": _case("fuvolix", 8, 250, 87, 16),
-        "sumozen, 2 long prompts": _case("sumozen", 2, 1000, 13, 8),
-        "lipulorn, one request": _case("lipulorn", 1, 700, 0, 24),
-        "deluvik, 16 requests": _case("deluvik", 16, 120, 50, 12, temperature=0.8),
-        "kerepel, 3 long prompts": _case("kerepel", 3, 900, 211, 12, temperature=0.7, top_p=0.9),
+        "fuvolix 8 requests": _case("fuvolix", 8, 250, 87, 16),
+        "sumozen 2 long prompts": _case("sumozen", 2, 1000, 13, 8),
+        "lipulorn one request": _case("lipulorn", 1, 700, 0, 24),
+        "deluvik 16 requests": _case("deluvik", 16, 120, 50, 12, temperature=0.8),
+        "kerepel 3 long prompts": _case("kerepel", 3, 900, 211, 12, temperature=0.7, top_p=0.9),
     }
     return [dict(case, name=name) for name, case in named.items()]
 
