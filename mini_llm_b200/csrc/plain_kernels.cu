@@ -12,6 +12,8 @@
 //   attention   engine/src/attention.c:24-49 with the causal softmax of
 //               engine/src/softmax.c:29-55, in the online form of
 //               engine/src/attention.cu:98-123
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 MLLM_DEFINE_ERROR_API(mllm_plain)
@@ -107,12 +109,58 @@ __global__ void layernorm_kernel(O* __restrict__ out, const float* __restrict__ 
     }
 }
 
+// 32-bit rows whose width is a multiple of 4 (up to 4,096): the row is read once, 16 bytes a lane, and stays in registers
+// through both sums.  A few rows are bound by the latency of their dependent passes (loads, two sums over the block,
+// store), not by bytes: three passes over memory cost 5.7 us at 4 x 768, one costs 3.
+__global__ void __launch_bounds__(256)
+layernorm_float_kernel(float* __restrict__ out, const float* __restrict__ x, const float* __restrict__ gamma,
+                       const float* __restrict__ beta, const int* __restrict__ rows, int width, float eps) {
+    __shared__ float scratch[33];
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int r = blockIdx.x, quads = width / 4;
+    const float4* row = reinterpret_cast<const float4*>(x + (long)(rows ? rows[r] : r) * width);
+    float4 v[4];
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int c = threadIdx.x + i * 256;
+        v[i] = c < quads ? row[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        sum += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+    }
+    const float mean = block_sum(sum, scratch) / (float)width;
+    float sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (threadIdx.x + i * 256 < quads) {
+            v[i].x -= mean; v[i].y -= mean; v[i].z -= mean; v[i].w -= mean;
+            sq += (v[i].x * v[i].x + v[i].y * v[i].y) + (v[i].z * v[i].z + v[i].w * v[i].w);
+        }
+    }
+    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int c = threadIdx.x + i * 256;
+        if (c < quads) {
+            const float4 g = reinterpret_cast<const float4*>(gamma)[c], b = reinterpret_cast<const float4*>(beta)[c];
+            reinterpret_cast<float4*>(out + (long)r * width)[c] =
+                make_float4(v[i].x * inv * g.x + b.x, v[i].y * inv * g.y + b.y, v[i].z * inv * g.z + b.z, v[i].w * inv * g.w + b.w);
+        }
+    }
+}
+
+static bool on_16_bytes(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 extern "C" int mllm_plain_layernorm(void* out, const float* x, const float* gamma, const float* beta,
                                     const int* rows, int n_rows, int width, float eps, int out_dtype,
                                     void* stream) {
     if (n_rows <= 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     int threads = width >= 1024 ? 256 : (width >= 256 ? 128 : 64);
+    if (out_dtype == DT_F32 && width % 4 == 0 && width <= 4096 && on_16_bytes(out) && on_16_bytes(x) && on_16_bytes(gamma) &&
+        on_16_bytes(beta))
+        return launched(launch_kernel(g_dependent_launch != 0, layernorm_float_kernel, dim3(n_rows), dim3(256), 0, s, (float*)out,
+                                      x, gamma, beta, rows, width, eps), "layernorm_float_kernel");
     if (out_dtype == DT_F32)
         layernorm_kernel<float><<<n_rows, threads, 0, s>>>((float*)out, x, gamma, beta, rows, width, eps);
     else if (out_dtype == DT_BF16)
@@ -182,6 +230,247 @@ linear_plain_kernel(OT* __restrict__ out, const AT* __restrict__ a, const WT* __
     }
 }
 
+__device__ __forceinline__ float activate(int epilogue, float v) {
+    switch (epilogue) {
+    case EPI_GELU_TANH: return gelu_tanh_f(v);
+    case EPI_GELU_ERF: return gelu_erf_f(v);
+    case EPI_RELU_SQ: return apply_activation<EPI_RELU_SQ>(v);
+    case EPI_SILU: return apply_activation<EPI_SILU>(v);
+    default: return v;
+    }
+}
+
+// 32-bit operands, up to 8 rows: the product is a stream of the weights, bound by HBM and by the latency of one pass.
+// The rows of `a` lie in shared memory; `split` warps share the inner size of F output features between them (their sums meet
+// in shared memory in warp order), so that a product of 768 features still brings 3,072 warps.  The first four
+// 16-byte pieces of each feature are asked for before the kernels ahead have ended: no kernel writes weights.
+// 4 x 768 x 3072: 300 us with the 64-wide tiles below (12 blocks, 94 % of the rows padding), under 10 us so.
+template <int MT, int F>
+__global__ void __launch_bounds__(256)
+linear_float_rows_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ w,
+                         const float* __restrict__ bias, int M, int N, int K, long lda, long ldo, int epilogue, int split) {
+    extern __shared__ __align__(16) float rows_shared[];                  // [MT][K]
+    __shared__ float partial[8][F][MT];
+    constexpr int AHEAD = F == 1 ? 4 : 2;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quads = K / 4, part = warp % split;
+    const int per_part = ((quads + split - 1) / split + 31) / 32 * 32;
+    const int begin = part * per_part, end = min(quads, begin + per_part);
+    const int n0 = (blockIdx.x * (8 / split) + warp / split) * F;
+    const float4* wrow[F];
+#pragma unroll
+    for (int f = 0; f < F; f++) wrow[f] = reinterpret_cast<const float4*>(w + (long)min(n0 + f, N - 1) * K);
+    float4 ahead[F][AHEAD];
+    dependents_may_start();
+#pragma unroll
+    for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+        for (int f = 0; f < F; f++) {
+            const int c = begin + lane + 32 * i;
+            ahead[f][i] = c < end ? __ldg(wrow[f] + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+    wait_for_earlier_kernels();
+    for (int m = 0; m < MT; m++)
+        for (int c = threadIdx.x; c < quads; c += 256)
+            reinterpret_cast<float4*>(rows_shared + (long)m * K)[c] =
+                m < M ? reinterpret_cast<const float4*>(a + (long)m * lda)[c] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    __syncthreads();
+    float acc[F][MT];
+#pragma unroll
+    for (int f = 0; f < F; f++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) acc[f][m] = 0.0f;
+    for (int first = begin + lane; first < end; first += 32 * AHEAD) {
+        float4 now[F][AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+            for (int f = 0; f < F; f++) {
+                now[f][i] = ahead[f][i];
+                const int c = first + 32 * (AHEAD + i);
+                ahead[f][i] = c < end ? __ldg(wrow[f] + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) {
+            const int c = first + 32 * i;
+            if (c >= end) break;
+#pragma unroll
+            for (int m = 0; m < MT; m++) {
+                const float4 x = reinterpret_cast<const float4*>(rows_shared + (long)m * K)[c];
+#pragma unroll
+                for (int f = 0; f < F; f++) {
+                    acc[f][m] = fmaf(now[f][i].x, x.x, acc[f][m]);
+                    acc[f][m] = fmaf(now[f][i].y, x.y, acc[f][m]);
+                    acc[f][m] = fmaf(now[f][i].z, x.z, acc[f][m]);
+                    acc[f][m] = fmaf(now[f][i].w, x.w, acc[f][m]);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int f = 0; f < F; f++)
+#pragma unroll
+        for (int m = 0; m < MT; m++) {
+            const float total = warp_sum(acc[f][m]);
+            if (lane == 0) partial[warp][f][m] = total;
+        }
+    __syncthreads();
+    // one thread per (feature of the block, row)
+    for (int i = threadIdx.x; i < (8 / split) * F * MT; i += 256) {
+        const int m = i % MT, f = (i / MT) % F, group = i / (MT * F);
+        const int n = (blockIdx.x * (8 / split) + group) * F + f;
+        if (m >= M || n >= N) continue;
+        float v = 0.0f;
+        for (int s = 0; s < split; s++) v += partial[group * split + s][f][m];
+        v += bias ? bias[n] : 0.0f;
+        float* o = out + (long)m * ldo + n;
+        *o = epilogue == EPI_ADD ? *o + v : activate(epilogue, v);
+    }
+}
+
+// 32-bit operands, more rows: tiles of 64 x 64 by 256 threads, 4 x 4 sums a thread out of two 16-byte reads of shared
+// memory per step of K, the next 32 entries of K in registers while these are multiplied.  Where the tiles are fewer than
+// the SMs a cluster of 2, 4 or 8 blocks shares a tile's K: every block leaves its sums in its shared memory, and block r
+// finishes rows r * 64 / blocks and up, adding the parts in block order (the order is the tile's, never timing).
+// 240 x 768 x 768: 278 us with the kernel above on 48 blocks; scalar FMA either way.
+constexpr int FLOAT_TILE = 64, FLOAT_K = 32, FLOAT_LD = FLOAT_TILE + 4;
+__global__ void __launch_bounds__(256)
+linear_float_tile_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ w,
+                         const float* __restrict__ bias, int M, int N, int K, long lda, long ldo, int epilogue, int per_block) {
+    __shared__ __align__(16) float staged[2][2][FLOAT_K][FLOAT_LD];       // [buffer][a, w][k][row]
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int m0 = blockIdx.y * FLOAT_TILE, n0 = blockIdx.x * FLOAT_TILE;
+    const int blocks = gridDim.z, rank = blockIdx.z;
+    const int k_begin = rank * per_block, k_end = min(K, k_begin + per_block);
+    const int row = threadIdx.x >> 2, quad = threadIdx.x & 3;             // what this thread copies: 4 + 4 entries of one row each
+    const bool a_there = m0 + row < M, w_there = n0 + row < N;
+    const float* a_row = a + (long)(a_there ? m0 + row : 0) * lda;
+    const float* w_row = w + (long)(w_there ? n0 + row : 0) * K;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 ra[2], rw[2];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int k = k0 + (quad + 4 * i) * 4;
+            ra[i] = a_there && k < k_end ? *reinterpret_cast<const float4*>(a_row + k) : none;
+            rw[i] = w_there && k < k_end ? __ldg(reinterpret_cast<const float4*>(w_row + k)) : none;
+        }
+    };
+    auto stage = [&](int buffer) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+            const int k = (quad + 4 * i) * 4;
+            staged[buffer][0][k][row] = ra[i].x; staged[buffer][0][k + 1][row] = ra[i].y;
+            staged[buffer][0][k + 2][row] = ra[i].z; staged[buffer][0][k + 3][row] = ra[i].w;
+            staged[buffer][1][k][row] = rw[i].x; staged[buffer][1][k + 1][row] = rw[i].y;
+            staged[buffer][1][k + 2][row] = rw[i].z; staged[buffer][1][k + 3][row] = rw[i].w;
+        }
+    };
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+    if (k_begin < k_end) {
+        fetch(k_begin);
+        stage(0);
+    }
+    __syncthreads();
+    int buffer = 0;
+    for (int k0 = k_begin; k0 < k_end; k0 += FLOAT_K) {
+        const bool more = k0 + FLOAT_K < k_end;
+        if (more) fetch(k0 + FLOAT_K);
+#pragma unroll 8
+        for (int kk = 0; kk < FLOAT_K; kk++) {
+            const float4 x = *reinterpret_cast<const float4*>(&staged[buffer][0][kk][ty * 4]);
+            const float4 y = *reinterpret_cast<const float4*>(&staged[buffer][1][kk][tx * 4]);
+            const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+        }
+        if (more) stage(buffer ^ 1);           // the other buffer: every thread left it before the barrier below, a trip ago
+        __syncthreads();
+        buffer ^= 1;
+    }
+    auto finish = [&](int m, int n, float v) {
+        if (m >= M || n >= N) return;
+        v += bias ? bias[n] : 0.0f;
+        float* o = out + (long)m * ldo + n;
+        *o = epilogue == EPI_ADD ? *o + v : activate(epilogue, v);
+    };
+    if (blocks == 1) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) finish(m0 + ty * 4 + i, n0 + tx * 4 + j, acc[i][j]);
+        return;
+    }
+    float* sums = &staged[0][0][0][0];                                    // [64][68]: 17 KB of the 34
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        *reinterpret_cast<float4*>(sums + (ty * 4 + i) * FLOAT_LD + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    cluster.sync();
+    const int mine = FLOAT_TILE / blocks;
+    for (int i = threadIdx.x; i < mine * FLOAT_TILE; i += 256) {
+        const int r = rank * mine + i / FLOAT_TILE, c = i % FLOAT_TILE;
+        float v = 0.0f;
+        for (int b = 0; b < blocks; b++) v += cluster.map_shared_rank(sums, b)[r * FLOAT_LD + c];
+        finish(m0 + r, n0 + c, v);
+    }
+    cluster.sync();                                                       // no block leaves while another reads its sums
+}
+
+template <int MT, int F>
+static int launch_float_rows(float* out, const float* a, const float* w, const float* bias, int M, int N, int K, long lda, long ldo,
+                             int epilogue, int split, cudaStream_t s) {
+    const size_t shared = (size_t)MT * K * sizeof(float);
+    if (shared > 40 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(linear_float_rows_kernel<MT, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+        if (e != cudaSuccess) return fail("linear: cannot raise the shared memory limit");
+    }
+    const int per_block = 8 / split * F;
+    return launched(launch_kernel(g_dependent_launch != 0, linear_float_rows_kernel<MT, F>, dim3((N + per_block - 1) / per_block),
+                                  dim3(256), shared, s, out, a, w, bias, M, N, K, lda, ldo, epilogue, split),
+                    "linear_float_rows_kernel");
+}
+
+// Whether the two kernels above take the operands: rows on 16-byte boundaries (K and the stride of `a` multiples of 4).
+static bool linear_float_takes(const void* a, const void* w, int K, long lda) {
+    return K % 4 == 0 && lda % 4 == 0 && on_16_bytes(a) && on_16_bytes(w);
+}
+
+static int launch_linear_float(float* out, const float* a, const float* w, const float* bias, int M, int N, int K, long lda, long ldo,
+                               int epilogue, cudaStream_t s) {
+    // up to 8 rows that fit 128 KB of shared memory stream the weights; more rows reuse them in tiles
+    if (M <= 8 && (size_t)(M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : 8) * K * sizeof(float) <= 128 * 1024) {
+        // wide products (a vocabulary) take four features a warp, so that a row read from shared memory serves four; narrow
+        // ones share a feature's K among up to four warps, while each still has 128 pieces of 16 bytes
+        const bool wide = N >= 16384;
+        int split = 1;
+        while (!wide && split < 4 && N * split < 3072 && K / 4 >= split * 2 * 64) split *= 2;
+#define FLOAT_ROWS(MT) (wide ? launch_float_rows<MT, 4>(out, a, w, bias, M, N, K, lda, ldo, epilogue, 1, s) \
+                             : launch_float_rows<MT, 1>(out, a, w, bias, M, N, K, lda, ldo, epilogue, split, s))
+        if (M <= 1) return FLOAT_ROWS(1);
+        if (M <= 2) return FLOAT_ROWS(2);
+        if (M <= 4) return FLOAT_ROWS(4);
+        return FLOAT_ROWS(8);
+#undef FLOAT_ROWS
+    }
+    const dim3 tiles((N + FLOAT_TILE - 1) / FLOAT_TILE, (M + FLOAT_TILE - 1) / FLOAT_TILE);
+    // blocks that share a tile's K: while they stay within two to an SM and each has two steps of K or more
+    int blocks = 1;
+    while (blocks < 8 && (long)tiles.x * tiles.y * blocks * 2 <= 296 && K >= blocks * 2 * 2 * FLOAT_K) blocks *= 2;
+    const int per_block = ((K + blocks - 1) / blocks + FLOAT_K - 1) / FLOAT_K * FLOAT_K;
+    return launched(launch_kernel_in_clusters(g_dependent_launch != 0, blocks > 1 ? dim3(1, 1, blocks) : dim3(0, 1, 1),
+                                              linear_float_tile_kernel, dim3(tiles.x, tiles.y, blocks), dim3(256), 0, s, out, a, w, bias, M,
+                                              N, K, lda, ldo, epilogue, per_block), "linear_float_tile_kernel");
+}
+
 template <typename AT, typename WT, typename OT>
 static int launch_linear_plain(void* out, const void* a, const void* w, const float* bias, int M, int N, int K,
                                long lda, long ldo, int epilogue, cudaStream_t s) {
@@ -211,6 +500,8 @@ extern "C" int mllm_plain_linear(void* out, const void* a, const void* w, const 
     if ((M + 63) / 64 > 65535) return fail("linear: too many rows for one launch");
     if (epilogue == EPI_ADD && out_dtype != DT_F32) return fail("linear: the residual sum is kept in 32-bit");
     cudaStream_t s = (cudaStream_t)stream;
+    if (in_dtype == DT_F32 && out_dtype == DT_F32 && linear_float_takes(a, w, K, lda))
+        return launch_linear_float((float*)out, (const float*)a, (const float*)w, bias, M, N, K, lda, ldo, epilogue, s);
     if (in_dtype == DT_F32 && out_dtype == DT_F32)
         return launch_linear_plain<float, float, float>(out, a, w, bias, M, N, K, lda, ldo, epilogue, s);
     if (in_dtype == DT_BF16 && out_dtype == DT_BF16)
@@ -343,6 +634,86 @@ attention_plain_kernel(T* __restrict__ out, long ld_out, const T* __restrict__ q
     }
 }
 
+// 32-bit queries, keys and values whose head size is a multiple of 4 up to 128: a lane owns four of the head's entries, LPK
+// lanes own a key, and a warp has four keys a lane group in flight before it uses the first (one key at a time, each with its own
+// block-table look-up and a reduction over 32 lanes, waited 1.4 us a key: 21 us for 60 keys of 4 tokens).  Eight warps a
+// block; their states are merged in warp and group order.
+template <int LPK>
+__global__ void __launch_bounds__(256)
+attention_float_kernel(float* __restrict__ out, long ld_out, const float* __restrict__ q, long ld_q, const float* __restrict__ k_pages,
+                       const float* __restrict__ v_pages, const int* __restrict__ block_table, int max_blocks,
+                       const int* __restrict__ positions, const int* __restrict__ token_item, int n_heads, int n_kv_heads,
+                       int head_size, int page_size, float scale, int window) {
+    constexpr int KPW = 32 / LPK, STATES = 8 * KPW, DEEP = 4;
+    __shared__ float state_m[STATES], state_l[STATES];
+    __shared__ __align__(16) float state_acc[STATES][LPK * 4];
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int t = blockIdx.x, h = blockIdx.y;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane % LPK, group = lane / LPK;
+    const int p = positions[t];
+    const int* bt = block_table + (long)token_item[t] * max_blocks;
+    const long width = (long)n_kv_heads * head_size, column = (long)(h / (n_heads / n_kv_heads)) * head_size + sub * 4;
+    const bool there = sub * 4 < head_size;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const float4 mine = there ? *reinterpret_cast<const float4*>(q + (long)t * ld_q + (long)h * head_size + sub * 4) : none;
+    float4 acc = none;
+    float m = -INFINITY, l = 0.0f;
+    const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
+    // every lane of a warp runs the same trips (the shuffles need all of them)
+    for (int base = lo + warp * KPW * DEEP; base <= p; base += STATES * DEEP) {
+        float4 k[DEEP], v[DEEP];
+        float s[DEEP];
+#pragma unroll
+        for (int i = 0; i < DEEP; i++) {
+            const int j = base + i * KPW + group;
+            k[i] = v[i] = none;
+            if (j <= p && there) {
+                const long at = ((long)bt[j / page_size] * page_size + j % page_size) * width + column;
+                k[i] = *reinterpret_cast<const float4*>(k_pages + at);
+                v[i] = *reinterpret_cast<const float4*>(v_pages + at);
+            }
+        }
+        float top = m;
+#pragma unroll
+        for (int i = 0; i < DEEP; i++) {
+            float dot = fmaf(mine.x, k[i].x, fmaf(mine.y, k[i].y, fmaf(mine.z, k[i].z, mine.w * k[i].w)));
+#pragma unroll
+            for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+            s[i] = base + i * KPW + group <= p ? dot * scale : -INFINITY;
+            top = fmaxf(top, s[i]);
+        }
+        if (top != -INFINITY) {
+            const float keep = expf(m - top);
+            l *= keep;
+            acc.x *= keep; acc.y *= keep; acc.z *= keep; acc.w *= keep;
+#pragma unroll
+            for (int i = 0; i < DEEP; i++) {
+                const float e = expf(s[i] - top);
+                l += e;
+                acc.x = fmaf(e, v[i].x, acc.x); acc.y = fmaf(e, v[i].y, acc.y);
+                acc.z = fmaf(e, v[i].z, acc.z); acc.w = fmaf(e, v[i].w, acc.w);
+            }
+            m = top;
+        }
+    }
+    const int cell = warp * KPW + group;
+    if (sub == 0) {
+        state_m[cell] = m;
+        state_l[cell] = l;
+    }
+    *reinterpret_cast<float4*>(&state_acc[cell][sub * 4]) = acc;
+    __syncthreads();
+    float big = -INFINITY, total = 0.0f;
+    for (int c = 0; c < STATES; c++) big = fmaxf(big, state_m[c]);
+    for (int c = 0; c < STATES; c++) total += state_m[c] == -INFINITY ? 0.0f : state_l[c] * expf(state_m[c] - big);
+    for (int d = threadIdx.x; d < head_size; d += 256) {
+        float o = 0.0f;
+        for (int c = 0; c < STATES; c++) o += state_m[c] == -INFINITY ? 0.0f : state_acc[c][d] * expf(state_m[c] - big);
+        out[(long)t * ld_out + (long)h * head_size + d] = o / total;
+    }
+}
+
 extern "C" int mllm_plain_attention(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,
                                     const void* v_pages, const int* block_table, int max_blocks,
                                     const int* positions, const int* token_item, int n_tokens, int n_heads,
@@ -355,6 +726,19 @@ extern "C" int mllm_plain_attention(void* out, long ld_out, const void* q, long 
     if (n_heads > 65535) return fail("attention: too many heads for one launch");
     cudaStream_t s = (cudaStream_t)stream;
     dim3 grid(n_tokens, n_heads);
+    if (dtype == DT_F32 && head_size % 4 == 0 && head_size <= 128 && ld_q % 4 == 0 && on_16_bytes(q) && on_16_bytes(k_pages) &&
+        on_16_bytes(v_pages)) {
+#define FLOAT_ATTENTION(LPK)                                                                                                     \
+    return launched(launch_kernel(g_dependent_launch != 0, attention_float_kernel<LPK>, grid, dim3(256), 0, s, (float*)out, ld_out, \
+                                  (const float*)q, ld_q, (const float*)k_pages, (const float*)v_pages, block_table, max_blocks,  \
+                                  positions, token_item, n_heads, n_kv_heads, head_size, page_size, scale, window),              \
+                    "attention_float_kernel")
+        if (head_size <= 16) FLOAT_ATTENTION(4);
+        if (head_size <= 32) FLOAT_ATTENTION(8);
+        if (head_size <= 64) FLOAT_ATTENTION(16);
+        FLOAT_ATTENTION(32);
+#undef FLOAT_ATTENTION
+    }
     if (dtype == DT_F32)
         attention_plain_kernel<float><<<grid, 128, 0, s>>>((float*)out, ld_out, (const float*)q, ld_q,
                                                            (const float*)k_pages, (const float*)v_pages, block_table,

@@ -1,0 +1,72 @@
+"""Products, norms and attention of few rows at the sizes where their tiles, shares of K and chunks end, against 64-bit sums."""
+
+import math
+
+import numpy as np
+import pytest
+import torch
+
+import plain_gpt2 as plain
+from test_kernels_gpu import attention_expected, dev, f64, paged_case, tol
+
+pytestmark = pytest.mark.gpu
+
+
+# rows: the few-row kernel's 1 to 8, then tiles of 64; features: a warp's, a block's and a tile's edges, four features a warp
+# from 16,384 on; K: one 16-byte piece, less than a warp's share, shares that are no multiple of a load, K shared by 2, 4 and 8
+@pytest.mark.parametrize("m", [1, 2, 3, 8, 9, 64, 65])
+@pytest.mark.parametrize("n, k", [(1, 4), (63, 100), (65, 768), (768, 3076), (130, 516), (16385, 132)])
+@pytest.mark.parametrize("epilogue", ["store", "add", "gelu_erf"])
+def test_linear_in_32_bits(m, n, k, epilogue):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(m * 31 + n + k)
+    a = dev(rng.normal(size=(m, k + 4)), torch.float32)[:, 4:]
+    w, bias = dev(rng.normal(size=(n, k)) / math.sqrt(k), torch.float32), dev(rng.normal(size=n), torch.float32)
+    out = dev(rng.normal(size=(m, n + 3)), torch.float32)
+    before = f64(out)
+    acc = f64(a) @ f64(w).T + f64(bias)
+    expected = {"store": acc, "add": before[:, :n] + acc, "gelu_erf": plain.gelu_erf(acc)}[epilogue]
+    ops.linear_plain(out[:, :n], a, w, bias, epilogue)
+    # every product and every sum rounds by at most 2^-24 of values below 2^3; their roots-of-K walk stays under 2e-5
+    np.testing.assert_allclose(f64(out)[:, :n], expected, rtol=0, atol=2e-5)
+    np.testing.assert_array_equal(f64(out)[:, n:], before[:, n:])
+
+
+def test_linear_in_32_bits_off_16_byte_boundaries_and_with_infinities():
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(8)
+    base, w = dev(rng.normal(size=(5, 131)), torch.float32), dev(rng.normal(size=(70, 128)) / 11, torch.float32)
+    out = torch.empty(5, 70, device="cuda")
+    for a in (base[:, 1:129], base[:, 3:131]):            # rows that start on 4-byte boundaries only
+        ops.linear_plain(out, a, w, None, "store")
+        np.testing.assert_allclose(f64(out), f64(a) @ f64(w).T, rtol=0, atol=2e-5)
+    a = dev(rng.normal(size=(3, 128)), torch.float32)
+    a[1, 127] = math.inf                                  # stays in its row, and in no other share of K
+    ops.linear_plain(out[:3], a, w, None, "store")
+    np.testing.assert_array_equal(f64(out)[1], np.sign(f64(w)[:, 127]) * math.inf)
+    assert np.isfinite(f64(out)[[0, 2]]).all()
+
+
+@pytest.mark.parametrize("width", [4, 1020, 1024, 4096, 4100, 771])
+def test_layernorm_in_32_bits(width):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(width)
+    x = dev(rng.normal(3.0, 5.0, size=(5, width)), torch.float32)
+    gain, shift = dev(rng.uniform(0.5, 1.5, width), torch.float32), dev(rng.normal(0, 0.1, width), torch.float32)
+    out = torch.empty(3, width, device="cuda")
+    ops.layernorm(out, x, gain, shift, 1e-5, dev([4, 0, 4], torch.int32))
+    np.testing.assert_allclose(f64(out), plain.layer_norm(f64(x), f64(gain), f64(shift), 1e-5)[[4, 0, 4]], rtol=0, atol=tol(torch.float32, 4))
+
+
+# every number of lanes a key, head sizes that leave lanes idle, one that no lane layout takes; 1 key up to several rounds
+@pytest.mark.parametrize("head", [4, 12, 20, 32, 48, 64, 100, 128, 144, 10])
+@pytest.mark.parametrize("window", [0, 33])
+def test_attention_in_32_bits(head, window):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(head)
+    k_pages, v_pages, table, positions, items, dense = paged_case(rng, [1, 37, 300, 64], [1, 5, 2, 1], 4, 2, head, 8, torch.float32)
+    q = dev(rng.normal(size=(len(f64(positions)), 4 * head)), torch.float32)
+    out = torch.full_like(q, float("nan"))
+    expected = attention_expected(f64(q), dense, f64(positions).astype(int), f64(items).astype(int), 4, 2, head, head ** -0.5, window)
+    ops.attention_plain(out, q, k_pages, v_pages, table, positions, items, 4, 2, head, 8, head ** -0.5, window)
+    np.testing.assert_allclose(f64(out), expected, rtol=0, atol=tol(torch.float32))
