@@ -250,6 +250,8 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     if (block > 0) lo = max(lo, p - p % block);
     const int n_kept = min(keep, lo), gap = lo - n_kept;        // key number i is position i (i < n_kept) or i + gap
     const int n_seen = n_kept + p - lo + 1;
+    // the chunk that is asked for, or what makes the launch's chunks cover this token's keys (a multiple of 64 then)
+    if ((long)chunk * max_chunks < n_seen) chunk = ((n_seen + max_chunks - 1) / max_chunks + 63) / 64 * 64;
     const int c_last = (n_seen - 1) / chunk;
     if (c > c_last) return;
     const int begin = c * chunk, end = min(n_seen, begin + chunk) - 1;             // key numbers, inclusive
@@ -434,6 +436,13 @@ extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const vo
     const int size = most <= 16 ? 16 : (most <= 32 ? 32 : (most <= 64 ? 64 : (most <= 128 ? 128 : 256)));
     const bool full = dim == size && vdim == size;
     cudaStream_t s = (cudaStream_t)stream;
+    // Chunks a (token, head) pair is launched with.  max_chunks follows the block table's reach, which without a limit on
+    // positions is the whole cache: 65,536 keys are 256 to 1,024 chunks a pair, nearly all of which have no keys and only come
+    // and go (16 tokens x 12 heads at 120 keys: 51 us for 49,152 blocks, 7.6 us for 1,536).  A wave of 1,184 blocks (8 an SM) is shared among
+    // the pairs, at least 4 each; a token that sees more keys than so many chunks hold takes longer chunks (in the kernel).
+    const long pairs = (long)n_tokens * n_heads;
+    const long share = (1184 + pairs - 1) / pairs;
+    if (max_chunks > share && max_chunks > 4) max_chunks = (int)(share > 4 ? share : 4);
     dim3 grid(n_tokens, n_heads, max_chunks);
 #define LAUNCH_SPLIT(D, FULL)                                                                                        \
     launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL>, grid, dim3(128), 0, s, (bf16*)out, ld_out, \

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import plain_gpt2 as plain
-from test_kernels_gpu import attention_expected, dev, f64, paged_case, tol
+from test_kernels_gpu import attention_expected, dev, f64, paged_case, split_scratch, tol
 
 pytestmark = pytest.mark.gpu
 
@@ -70,3 +70,25 @@ def test_attention_in_32_bits(head, window):
     expected = attention_expected(f64(q), dense, f64(positions).astype(int), f64(items).astype(int), 4, 2, head, head ** -0.5, window)
     ops.attention_plain(out, q, k_pages, v_pages, table, positions, items, 4, 2, head, 8, head ** -0.5, window)
     np.testing.assert_allclose(f64(out), expected, rtol=0, atol=tol(torch.float32))
+
+
+@pytest.mark.parametrize("lengths, heads", [([9000, 3, 2200], 12), ([700] * 33, 16)])
+def test_split_attention_with_more_keys_than_the_launch_has_chunks(lengths, heads):
+    """A block table that reaches over a whole cache: a launch has far fewer chunks than the reach would take, and tokens that
+    see more keys than those chunks hold at the asked length take longer ones."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(len(lengths))
+    head, page, chunk = 64, 64, 64
+    k_pages, v_pages, table, positions, items, dense = paged_case(rng, lengths, [1] * len(lengths), heads, heads, head, page, torch.bfloat16)
+    dense = [(f64(dev(k, torch.bfloat16)), f64(dev(v, torch.bfloat16))) for k, v in dense]
+    n, max_chunks = len(lengths), 1024
+    table = torch.cat([table, torch.full((n, max_chunks - table.shape[1]), -1, dtype=torch.int32, device="cuda")], 1).contiguous()
+    q = dev(rng.normal(size=(n, heads * head)), torch.bfloat16)
+    out = torch.full_like(q, float("nan"))
+    scratch = split_scratch(n, heads, max_chunks, head)
+    expected = attention_expected(f64(q), dense, f64(positions).astype(int), f64(items).astype(int), heads, heads, head, head ** -0.5, 0)
+    for _ in range(2):
+        ops.split_attention(out, q, k_pages, v_pages, table, positions, items, heads, heads, head, page, head ** -0.5, 0, chunk,
+                            max_chunks, *scratch)
+        np.testing.assert_allclose(f64(out), expected, rtol=0, atol=tol(torch.bfloat16, 2))
+        assert int(scratch[2].abs().sum()) == 0
