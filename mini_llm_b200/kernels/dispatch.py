@@ -297,6 +297,10 @@ class Kernels:
     def _memory_scratch(self, device, floats):
         held = getattr(self, "_memory_passes", None)
         if held is None or any(t.numel() < n for t, n in zip(held, floats)):
+            # each buffer as large as any layer has asked for: memories of two shapes that take turns in a model would else
+            # move the scratch at every layer, and every move drops the captured graphs
+            if held is not None:
+                floats = [max(t.numel(), n) for t, n in zip(held, floats)]
             self._memory_passes = held = tuple(torch.empty(max(n, 1), dtype=torch.float32, device=device) for n in floats)
             self.scratch_generation += 1
         return held

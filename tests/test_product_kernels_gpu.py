@@ -92,3 +92,15 @@ def test_split_attention_with_more_keys_than_the_launch_has_chunks(lengths, head
                             max_chunks, *scratch)
         np.testing.assert_allclose(f64(out), expected, rtol=0, atol=tol(torch.bfloat16, 2))
         assert int(scratch[2].abs().sum()) == 0
+
+
+def test_two_memory_shapes_share_scratch_without_moving_it():
+    from mini_llm_b200.kernels.dispatch import Kernels
+    kernels = Kernels(torch.bfloat16)
+    first = kernels._memory_scratch("cuda", (100, 20, 30))
+    second = kernels._memory_scratch("cuda", (50, 40, 10))
+    moved = kernels.scratch_generation
+    assert [t.numel() for t in second] == [100, 40, 30] and [t.numel() for t in first] == [100, 20, 30]
+    for floats in ((100, 20, 30), (50, 40, 10)):
+        assert kernels._memory_scratch("cuda", floats) is second
+    assert kernels.scratch_generation == moved
