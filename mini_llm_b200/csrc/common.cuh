@@ -97,6 +97,27 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return scratch[32];
 }
 
+// The same with one barrier, for a kernel's first use of `slots` (one float a warp): every thread adds the warps' sums itself,
+// in warp order.
+__device__ __forceinline__ float block_sum_once(float v, float* slots) {
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) slots[threadIdx.x >> 5] = v;
+    __syncthreads();
+    const int n_warps = (blockDim.x + 31) >> 5;
+    float total = 0.0f;
+    for (int w = 0; w < n_warps; w++) total += slots[w];
+    return total;
+}
+
+// c[16 x 8] += a[16 x 16] b[16 x 8] over the lanes of a warp, bfloat16 operands, 32-bit sums.
+__device__ __forceinline__ void mma_bf16_16816(float& c0, float& c1, float& c2, float& c3, uint32_t a0, uint32_t a1,
+                                               uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+                 "{%0, %1, %2, %3};"
+                 : "+f"(c0), "+f"(c1), "+f"(c2), "+f"(c3)
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
 #define MLLM_ERROR_BUFFER 512
 
 // ---- programmatic dependent launch ---------------------------------------------------------
@@ -112,6 +133,15 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // dependency as an edge of the graph.
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_earlier_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A kernel that reads weights before that wait takes what other kernels of the step wrote through a pointer that has passed
+// here behind it: loads through a `const ... __restrict__` parameter count as loads of memory that nobody writes, and the
+// compiler may move them ahead of the wait (a filter kernel read rows that the product before it had not yet written, once
+// in a few replayed steps).
+template <typename T> __device__ __forceinline__ T* behind_the_wait(T* p) {
+    asm volatile("" : "+l"(p) : : "memory");
+    return p;
+}
 
 // (cluster: the CTAs of a thread block cluster, or x = 0 for a launch without clusters)
 template <typename... Params, typename... Args>

@@ -118,6 +118,8 @@ layernorm_float_kernel(float* __restrict__ out, const float* __restrict__ x, con
     __shared__ float scratch[33];
     dependents_may_start();
     wait_for_earlier_kernels();
+    x = behind_the_wait(x);
+    rows = behind_the_wait(rows);
     const int r = blockIdx.x, quads = width / 4;
     const float4* row = reinterpret_cast<const float4*>(x + (long)(rows ? rows[r] : r) * width);
     float4 v[4];
@@ -270,6 +272,7 @@ linear_float_rows_kernel(float* __restrict__ out, const float* __restrict__ a, c
             ahead[f][i] = c < end ? __ldg(wrow[f] + c) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     wait_for_earlier_kernels();
+    a = behind_the_wait(a);
     for (int m = 0; m < MT; m++)
         for (int c = threadIdx.x; c < quads; c += 256)
             reinterpret_cast<float4*>(rows_shared + (long)m * K)[c] =
@@ -340,6 +343,7 @@ linear_float_tile_kernel(float* __restrict__ out, const float* __restrict__ a, c
     __shared__ __align__(16) float staged[2][2][FLOAT_K][FLOAT_LD];       // [buffer][a, w][k][row]
     dependents_may_start();
     wait_for_earlier_kernels();
+    a = behind_the_wait(a);
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     const int m0 = blockIdx.y * FLOAT_TILE, n0 = blockIdx.x * FLOAT_TILE;
     const int blocks = gridDim.z, rank = blockIdx.z;
@@ -649,6 +653,9 @@ attention_float_kernel(float* __restrict__ out, long ld_out, const float* __rest
     __shared__ __align__(16) float state_acc[STATES][LPK * 4];
     dependents_may_start();
     wait_for_earlier_kernels();
+    q = behind_the_wait(q);
+    k_pages = behind_the_wait(k_pages);
+    v_pages = behind_the_wait(v_pages);
     const int t = blockIdx.x, h = blockIdx.y;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane % LPK, group = lane / LPK;
     const int p = positions[t];
