@@ -234,13 +234,22 @@ gemm_swapped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
-    wait_for_earlier_kernels();          // nothing above reads or writes the step's memory
 
     if (warp == 8) {
         // ---- producer ----
         if (lane == 0) {
-            int issued = 0;
-            for (int kb = 0; kb < num_k; kb++) {
+            // No kernel of a step writes weights: as many blocks of them as there are stages are asked for before the kernels
+            // ahead have ended, x behind that wait.
+            const int ahead = min(num_k, STAGES);
+            for (int kb = 0; kb < ahead; kb++) {
+                mbar_expect_tx(&full[kb], A_BYTES + B_BYTES);
+                tma_load_2d(stage_a + kb * A_BYTES, &map_a, &full[kb], (kb_first + kb) * BK, tile_a * BM);
+            }
+            wait_for_earlier_kernels();
+            for (int kb = 0; kb < ahead; kb++)
+                tma_load_2d(stage_b + kb * B_BYTES, &map_b, &full[kb], (kb_first + kb) * BK, tile_b * BN);
+            int issued = ahead;
+            for (int kb = ahead; kb < num_k; kb++) {
                 const int s = kb % STAGES;
                 if (!mbar_wait(&empty[s], ((kb / STAGES) & 1) ^ 1) || *failed) {
                     if (!*failed) {
@@ -264,6 +273,7 @@ gemm_swapped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     } else if (warp == 9) {
         // ---- MMA issue ----
         if (lane == 0) {
+            wait_for_earlier_kernels();          // (the bounded waits below count from here)
             const uint32_t idesc = make_instr_desc(BM, BN);
             for (int kb = 0; kb < num_k; kb++) {
                 const int s = kb % STAGES;
@@ -288,6 +298,7 @@ gemm_swapped_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
         }
     } else {
         // ---- epilogue: warps w and w + 4 own TMEM lanes 32w .. 32w+31 and split the columns ----
+        wait_for_earlier_kernels();
         const int quarter = warp & 3, col_half = warp >> 2;
         if (p.k_pages != nullptr) {
             const int t = tile_b * BN + threadIdx.x;
@@ -669,7 +680,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         __syncthreads();
     }
 
-    wait_for_earlier_kernels();          // nothing above reads or writes the step's memory (the stamps are the caller's own)
+    // (nothing above reads or writes the step's memory; the stamps are the caller's own)
     if (stamps && threadIdx.x == 0) p.timeline[1] = now_ns();
     // Each issuing thread has a ring of stages of its own (the first RING0 stages, the rest),
     // filled by the producer in the order in which that thread takes its blocks.  A stage that
@@ -684,9 +695,32 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             uint32_t phase[2] = {0u, 0u};            // the parity of the round that stage is in
             int issued[2] = {0, 0};
             bool ok = true;
+            auto took = [&](int ring) {
+                issued[ring]++;
+                if (++pos[ring] == (ring == 0 ? RING0 : RING1)) {
+                    pos[ring] = 0;
+                    phase[ring] ^= 1u;
+                }
+            };
+            // No kernel of a step writes weights: the first tile's first blocks of them are asked for before the kernels ahead
+            // have ended, the tokens' rows behind that wait.
+            constexpr int AHEAD = ISSUERS == 2 ? 2 * RING1 : STAGES;
+            const int ahead = PAIR || walker >= n_tiles ? 0 : min(num_k, AHEAD);
+            auto stage_of = [&](int kb) { return ISSUERS == 2 ? (kb & 1 ? RING0 : 0) + kb / 2 : kb; };
+            for (int kb = 0; kb < ahead; kb++) {
+                const int s = stage_of(kb);
+                mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
+                tma_load_2d(stage_b + s * B_BYTES, &map_b, &full[s], kb * BK, walker / tiles_m * BN);
+            }
+            wait_for_earlier_kernels();
+            for (int kb = 0; kb < ahead; kb++) {
+                const int s = stage_of(kb);
+                tma_load_2d(stage_a + s * A_BYTES, &map_a, &full[s], kb * BK, walker % tiles_m * TILE_ROWS);
+                took(ISSUERS == 2 ? (kb & 1) : 0);
+            }
             for (int tile = walker; tile < n_tiles && ok && !*failed; tile += walkers) {
                 const int tile_m = tile % tiles_m, tile_n = tile / tiles_m;
-                for (int kb = 0; kb < num_k; kb++) {
+                for (int kb = tile == walker ? ahead : 0; kb < num_k; kb++) {
                     const int ring = ISSUERS == 2 ? (kb & 1) : 0;
                     const int s = ring == 0 ? pos[0] : RING0 + pos[1];
                     if (!mbar_wait(&empty[s], phase[ring] ^ 1u) || *failed) {
@@ -705,11 +739,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         tma_load_2d(stage_a + s * A_BYTES, &map_a, &full[s], kb * BK, tile_m * BM);
                         tma_load_2d(stage_b + s * B_BYTES, &map_b, &full[s], kb * BK, tile_n * BN);
                     }
-                    issued[ring]++;
-                    if (++pos[ring] == (ring == 0 ? RING0 : RING1)) {
-                        pos[ring] = 0;
-                        phase[ring] ^= 1u;
-                    }
+                    took(ring);
                 }
             }
             if (*failed && leader) {
@@ -728,6 +758,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         // by a wait running out.
         const int issuer = warp - 9;
         if (lane == 0 && leader) {
+            wait_for_earlier_kernels();          // (the bounded waits below count from here)
             // This thread's instructions between two blocks are what bounds the loop, so it keeps
             // the ring's position and the descriptors as running values.
             const uint32_t idesc = make_instr_desc(TILE_ROWS, BN);
@@ -794,6 +825,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else {
         // ---- epilogue: warps w and w + 4 own TMEM lanes 32 (w % 4) .. +31 and take the tile's
         // blocks of 32 columns in turn ----
+        wait_for_earlier_kernels();
         const int quarter = warp & 3, col_half = warp >> 2;
         BlockOut out_ctx{&map_out, turn_all + warp * (WARP_BLOCKS_BYTES / 4), nullptr, nullptr, quarter, lane, 0};
         const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
@@ -975,13 +1007,20 @@ gemm_rows_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             atomicExch(p.status, code);
         }
     };
-    wait_for_earlier_kernels();
     if (stamps && threadIdx.x == 0) p.timeline[1] = now_ns();
     const uint32_t exchange = smem_u32(smem);        // [block of this CTA][other CTA][8 pieces of 4 columns][BM rows][4 floats]: a warp's rows lie side by side
     if (warp == 8) {
         if (lane == 0) {
-            int issued = 0;
-            for (int kb = kb_lo; kb < kb_hi; kb++) {
+            // (weights ahead of the wait, as in the other kernels)
+            const int ahead = min(kb_hi - kb_lo, STAGES);
+            for (int i = 0; i < ahead; i++) {
+                mbar_expect_tx(&full[i], A_BYTES + B_BYTES);
+                tma_load_2d(stage_b + i * B_BYTES, &map_b, &full[i], (kb_lo + i) * BK, tile_n * BN);
+            }
+            wait_for_earlier_kernels();
+            for (int i = 0; i < ahead; i++) tma_load_2d(stage_a + i * A_BYTES, &map_a, &full[i], (kb_lo + i) * BK, tile_m * BM);
+            int issued = ahead;
+            for (int kb = kb_lo + ahead; kb < kb_hi; kb++) {
                 const int i = kb - kb_lo, s = i % STAGES;
                 if (!mbar_wait(&empty[s], (((uint32_t)(i / STAGES)) & 1u) ^ 1u) || *failed) {
                     give_up(STATUS_TIMEOUT_SPLIT_PRODUCER);
@@ -997,6 +1036,7 @@ gemm_rows_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp == 9) {
         if (lane == 0) {
+            wait_for_earlier_kernels();          // (the bounded waits below count from here)
             const uint32_t idesc = make_instr_desc(BM, BN);
             const uint64_t desc_a0 = make_smem_desc(smem_u32(stage_a)), desc_b0 = make_smem_desc(smem_u32(stage_b));
             for (int kb = kb_lo; kb < kb_hi; kb++) {
@@ -1020,6 +1060,7 @@ gemm_rows_split_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
         }
     } else {
+        wait_for_earlier_kernels();
         if (threadIdx.x < BN) {
             const int n = tile_n * BN + threadIdx.x;
             bias_s[threadIdx.x] = (p.bias != nullptr && n < p.N) ? p.bias[n] : 0.0f;
@@ -1468,13 +1509,13 @@ static int gemm_bf16(void* out, const void* x, const void* w, const float* bias,
                 break;
             }
     }
-    // (many tiles, as for a vocabulary: fewer stages, so that two or three CTAs share an SM and
-    // one's start and end fall under another's main loop)
-    const bool many_tiles = (long)grid.x * grid.y > 2L * sms && p.splits <= 1;
-    if (bn == 16) return many_tiles ? launch_swapped<16, 4>(map_w, map_x, p, grid, s) : launch_swapped<16, 8>(map_w, map_x, p, grid, s);
-    if (bn == 32) return many_tiles ? launch_swapped<32, 4>(map_w, map_x, p, grid, s) : launch_swapped<32, 8>(map_w, map_x, p, grid, s);
-    if (bn == 64 && many_tiles) return launch_swapped<64, 4>(map_w, map_x, p, grid, s);
-    if (bn == 64) return launch_swapped<64, 8>(map_w, map_x, p, grid, s);
+    // Fewer stages where a CTA walks few blocks of K (a split product at a width of 768: three) or where many tiles share the
+    // SMs (a vocabulary): two CTAs then fit an SM, so that one's start falls under another's end, of this launch or of the next.
+    const int walked = (blocks_of_k + p.splits - 1) / p.splits;
+    const bool few_stages = walked <= 4 || ((long)grid.x * grid.y > 2L * sms && p.splits <= 1);
+    if (bn == 16) return few_stages ? launch_swapped<16, 4>(map_w, map_x, p, grid, s) : launch_swapped<16, 8>(map_w, map_x, p, grid, s);
+    if (bn == 32) return few_stages ? launch_swapped<32, 4>(map_w, map_x, p, grid, s) : launch_swapped<32, 8>(map_w, map_x, p, grid, s);
+    if (bn == 64) return few_stages ? launch_swapped<64, 4>(map_w, map_x, p, grid, s) : launch_swapped<64, 8>(map_w, map_x, p, grid, s);
     if (bn == 128) return launch_swapped<128, 6>(map_w, map_x, p, grid, s);
     return launch_swapped<256, 4>(map_w, map_x, p, grid, s);
 }
