@@ -16,8 +16,9 @@ import torch
 
 from . import ops
 
-SKINNY_MAX_ROWS = 8           # up to here a product streams the weights once through the SIMT kernel (measured:
-                              # from 9 rows on the tensor-core kernel with swapped operands is faster)
+SKINNY_MAX_ROWS = 16          # up to here a product streams the weights once through small tiles (measured at 12 rows, against
+                              # the tensor-core kernel with swapped operands: 2.6 against 4.2 us at 768 x 768, 4.5 against
+                              # 6.1 at 1024 x 4096, and 12.1 against 8.8 at 1600 x 6400: a K this long only up to 8 rows)
 SPLIT_ATTENTION_MAX_ROWS = 64 # up to here attention runs one CTA per (token, head, chunk of keys)
 
 
@@ -241,6 +242,9 @@ class Kernels:
                 ops.gemm_bf16(out[:, h * o_head:h * o_head + n], a[:, h * a_head:h * a_head + k], w[h], None, "store", status)
             return out
         self.launches += 1
+        if not self.plain_only and ops.skinny_heads_takes(a, w, a_head):
+            self.chose("head_linear", "skinny_heads", m, n, k, heads)
+            return ops.skinny_heads(out, a, w, heads, a_head, o_head)
         self.chose("head_linear", "head_linear_plain", m, n, k, heads)
         return ops.head_linear(out, a, w, heads, a_head, o_head)
 
@@ -381,7 +385,7 @@ class Kernels:
     def _skinny(self, m, k, n=0) -> bool:
         # a product as wide as a vocabulary streams faster through the tensor-core kernel from
         # three rows on (measured at 50,257 x 768: 23 against 51 us at eight rows)
-        rows = 2 if n >= 8192 and k % 8 == 0 else SKINNY_MAX_ROWS
+        rows = 2 if n >= 8192 and k % 8 == 0 else (SKINNY_MAX_ROWS if k <= 4096 else 8)
         return not self.plain_only and m <= rows and ops.skinny_linear_takes(m, k)
 
     def linear(self, ctx, out, a, w, bias=None, epilogue="store"):

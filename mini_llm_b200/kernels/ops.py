@@ -224,7 +224,8 @@ class _SkinnyParams(ctypes.Structure):
     _fields_ = [("out", P), ("x", P), ("w", P), ("bias", P), ("gamma", P), ("beta", P), ("rows", P),
                 ("eps", F), ("M", I), ("N", I), ("K", I), ("ldx", L), ("ldo", L), ("epilogue", I), ("out_f32", I),
                 ("k_pages", P), ("v_pages", P), ("positions", P), ("token_item", P), ("block_table", P),
-                ("max_blocks", I), ("page_size", I), ("q_width", I), ("kv_width", I)]
+                ("max_blocks", I), ("page_size", I), ("q_width", I), ("kv_width", I),
+                ("batch", I), ("x_step", L), ("w_step", L), ("out_step", L)]
 
 
 _skinny = Function("decode", "mllm_decode_skinny_linear", [ctypes.POINTER(_SkinnyParams), P])
@@ -291,7 +292,7 @@ def skinny_linear(out, x, w, bias=None, epilogue="store", norm=None, scatter=Non
         if bias.shape[0] != n:
             raise KernelError("skinny_linear: bias has another length")
     params.out, params.x, params.w, params.bias = out.data_ptr(), x.data_ptr(), w.data_ptr(), _ptr(bias)
-    params.M, params.N, params.K = m, n, k
+    params.M, params.N, params.K, params.batch = m, n, k, 1
     params.ldx, params.ldo = x.stride(0), out.stride(0)
     params.epilogue = EPILOGUES[epilogue]
     params.out_f32 = int(out.dtype == torch.float32 and epilogue != "add")
@@ -306,6 +307,34 @@ def skinny_linear(out, x, w, bias=None, epilogue="store", norm=None, scatter=Non
         params.positions, params.token_item = positions.data_ptr(), token_item.data_ptr()
         params.block_table, params.max_blocks = block_table.data_ptr(), block_table.shape[1]
         params.page_size, params.q_width, params.kv_width = page_size, q_width, kv_width
+    _skinny(ctypes.byref(params), _stream())
+    return out
+
+
+def skinny_heads_takes(a, w, a_head) -> bool:
+    """Whether ``skinny_heads`` takes a product per head: bfloat16, rows, heads and strides on 16-byte boundaries."""
+    return (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and a.stride(1) == 1 and a.stride(0) % 8 == 0 and a_head % 8 == 0
+            and w.shape[2] % 8 == 0 and a.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0)
+
+
+def skinny_heads(out, a, w, heads, a_head, o_head):
+    """``head_linear`` for few rows on the tiles of ``skinny_linear``: out[:, h * o_head + n] = sum_k a[:, h * a_head + k] * w[h, n, k]
+    for every head in one launch; a and w [heads, N, K] bf16, out bf16 or fp32."""
+    _check(a, "skinny_heads.a", torch.bfloat16, 2)
+    _check(w, "skinny_heads.w", torch.bfloat16, 3)
+    _check(out, "skinny_heads.out", None, 2)
+    n, k = w.shape[1], w.shape[2]
+    if out.dtype not in (torch.float32, torch.bfloat16):
+        raise KernelError("skinny_heads: out must be bfloat16 or float32")
+    if (w.shape[0] != heads or not w.is_contiguous() or out.shape[0] != a.shape[0] or out.shape[1] < (heads - 1) * o_head + n
+            or a.shape[1] < (heads - 1) * a_head + k or not skinny_heads_takes(a, w, a_head)):
+        raise KernelError("skinny_heads: sizes do not agree, or rows are off 16-byte boundaries")
+    params = _SkinnyParams()
+    params.out, params.x, params.w = out.data_ptr(), a.data_ptr(), w.data_ptr()
+    params.M, params.N, params.K, params.batch = a.shape[0], n, k, heads
+    params.ldx, params.ldo = a.stride(0), out.stride(0)
+    params.x_step, params.w_step, params.out_step = a_head, n * k, o_head
+    params.epilogue, params.out_f32 = EPILOGUES["store"], int(out.dtype == torch.float32)
     _skinny(ctypes.byref(params), _stream())
     return out
 
