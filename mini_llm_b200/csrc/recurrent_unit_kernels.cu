@@ -458,17 +458,23 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(256)
 add_normed_cast_kernel(float* __restrict__ hidden, const float* __restrict__ y, const float* __restrict__ gain, float eps,
                        T* __restrict__ act, int width) {
-    dependents_may_start();
-    wait_for_earlier_kernels();
     __shared__ float scratch[33];
     const long row = blockIdx.x;
     float* h = hidden + row * width;
     const float* v = y != nullptr ? y + row * width : nullptr;
     T* a = act != nullptr ? act + row * width : nullptr;
+    dependents_may_start();
     if (VEC) {
-        // 16-byte vectors; a thread's first vector of y stays in registers between the two passes
+        // 16-byte vectors; a thread's first vectors of y and of the stream stay in registers between the two passes, and its
+        // first of the gain is there before the kernels ahead have ended (no kernel of a step writes it)
         const int n = width / 4;
-        float4 kept = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float4 kept = make_float4(0.0f, 0.0f, 0.0f, 0.0f), gain_ahead = kept, old = kept;
+        const bool there = (int)threadIdx.x < n;
+        if (there && v != nullptr) gain_ahead = __ldg(reinterpret_cast<const float4*>(gain) + threadIdx.x);
+        wait_for_earlier_kernels();
+        h = behind_the_wait(h);
+        v = behind_the_wait(v);
+        if (there) old = reinterpret_cast<const float4*>(h)[threadIdx.x];
         float inv = 0.0f;
         if (v != nullptr) {
             float sq = 0.0f;
@@ -477,13 +483,14 @@ add_normed_cast_kernel(float* __restrict__ hidden, const float* __restrict__ y, 
                 if (i == (int)threadIdx.x) kept = x;
                 sq = fmaf(x.x, x.x, fmaf(x.y, x.y, fmaf(x.z, x.z, fmaf(x.w, x.w, sq))));
             }
-            inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+            inv = 1.0f / sqrtf(block_sum_once(sq, scratch) / (float)width + eps);
         }
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            float4 sum = reinterpret_cast<const float4*>(h)[i];
+            const bool first = i == (int)threadIdx.x;
+            float4 sum = first ? old : reinterpret_cast<const float4*>(h)[i];
             if (v != nullptr) {
-                const float4 x = i == (int)threadIdx.x ? kept : reinterpret_cast<const float4*>(v)[i];
-                const float4 g = reinterpret_cast<const float4*>(gain)[i];
+                const float4 x = first ? kept : reinterpret_cast<const float4*>(v)[i];
+                const float4 g = first ? gain_ahead : reinterpret_cast<const float4*>(gain)[i];
                 sum.x = fmaf(x.x * inv, g.x, sum.x), sum.y = fmaf(x.y * inv, g.y, sum.y);
                 sum.z = fmaf(x.z * inv, g.z, sum.z), sum.w = fmaf(x.w * inv, g.w, sum.w);
                 reinterpret_cast<float4*>(h)[i] = sum;
@@ -495,6 +502,7 @@ add_normed_cast_kernel(float* __restrict__ hidden, const float* __restrict__ y, 
         }
         return;
     }
+    wait_for_earlier_kernels();
     float inv = 0.0f;
     if (v != nullptr) {
         float sq = 0.0f;
@@ -518,7 +526,7 @@ extern "C" int mllm_unit_add_normed_cast(float* hidden, const float* y, const fl
     if (y != nullptr && gain == nullptr) return fail("add_normed_cast: a norm needs its gain");
     cudaStream_t s = (cudaStream_t)stream;
     const bool vec = width % 4 == 0 && (((unsigned long long)hidden | (unsigned long long)y | (unsigned long long)gain) & 15ull) == 0;
-    const int threads = width >= 1024 ? 256 : 128;
+    const int threads = width >= 513 ? 256 : 128;          // (a 16-byte vector a thread up to 1,024 wide)
 #define RUN(T, VEC)                                                                                                       \
     launch_kernel(g_dependent_launch != 0, add_normed_cast_kernel<T, VEC>, dim3(n_rows), dim3(threads), 0, s, hidden, y, gain, eps, \
                   (T*)act, width)

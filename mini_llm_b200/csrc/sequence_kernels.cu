@@ -63,19 +63,80 @@ __global__ void grouped_rms_norm_kernel(O* __restrict__ out, long ld_out, const 
     }
 }
 
+// The same where a piece is a multiple of 4 up to 4,096 entries and every row starts on a boundary of four: four entries a
+// thread, everything that is read (the piece, gate, gain, old sum) asked for in one pass, the gain before the kernels ahead have
+// ended; one barrier.  Against a pass for the sum and a second one for the result: 8 rows of 768 3.2 -> 1.4 us, 2,048 rows 4.8 -> 3.1.
+template <typename T> struct alignas(4 * sizeof(T)) Four { T e[4]; };
+
+template <typename O, typename G, bool ADD, int GATE>
+__global__ void __launch_bounds__(1024)
+grouped_rms_norm_quads_kernel(O* __restrict__ out, long ld_out, const float* x, long ld_x, const float* __restrict__ gain,
+                              const int* __restrict__ rows, const G* __restrict__ gate, long ld_gate, int size, float eps) {
+    __shared__ float slots[32];
+    const int r = blockIdx.x, g = blockIdx.y, d = threadIdx.x * 4, c = g * size + d;
+    const bool there = d < size;
+    dependents_may_start();
+    float4 gains = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (there) gains = __ldg(reinterpret_cast<const float4*>(gain + c));
+    wait_for_earlier_kernels();
+    x = behind_the_wait(x);
+    gate = behind_the_wait(gate);
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, opened[4];
+    Four<O> old;
+    if (there) {
+        const float4 mine = *reinterpret_cast<const float4*>(x + (long)(rows ? rows[r] : r) * ld_x + c);
+        v[0] = mine.x, v[1] = mine.y, v[2] = mine.z, v[3] = mine.w;
+        if (GATE != 0) {
+            const Four<G> raw = *reinterpret_cast<const Four<G>*>(gate + (long)r * ld_gate + c);
+#pragma unroll
+            for (int i = 0; i < 4; i++) opened[i] = GATE == 1 ? sigmoid_f(to_f32(raw.e[i])) : silu_f(to_f32(raw.e[i]));
+        }
+        if (ADD) old = *reinterpret_cast<const Four<O>*>(out + (long)r * ld_out + c);
+    }
+    float sq = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        if (GATE == 3 && there) v[i] *= opened[i];
+        sq = fmaf(v[i], v[i], sq);
+    }
+    const float inv = 1.0f / sqrtf(block_sum_once(sq, slots) / (float)size + eps);
+    if (!there) return;
+    const float w[4] = {gains.x, gains.y, gains.z, gains.w};
+    Four<O> result;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        float y = v[i] * inv * w[i];
+        if (GATE == 1 || GATE == 2) y *= opened[i];
+        if (ADD) y += to_f32(old.e[i]);
+        result.e[i] = from_f32<O>(y);
+    }
+    *reinterpret_cast<Four<O>*>(out + (long)r * ld_out + c) = result;
+}
+
 template <typename O, typename G>
 static void launch_grouped_rms_norm(void* out, long ld_out, const float* x, long ld_x, const float* gain, const int* rows,
                                     const void* gate, long ld_gate, int n_rows, int size, int groups, float eps, int add,
                                     int gate_mode, cudaStream_t s) {
-    const int threads = size >= 1024 ? 256 : (size >= 256 ? 128 : (size >= 64 ? 64 : 32));
-    dim3 grid(n_rows, groups);
+    const dim3 grid(n_rows, groups);
     O* o = (O*)out;
     const G* g = (const G*)gate;
-    if (add) launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, true, 0>, dim3(grid), dim3(threads), 0, s, o, ld_out, x, ld_x, gain, rows, g, ld_gate, size, eps);
-    else if (gate != nullptr && gate_mode == 3) launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, false, 3>, dim3(grid), dim3(threads), 0, s, o, ld_out, x, ld_x, gain, rows, g, ld_gate, size, eps);
-    else if (gate != nullptr && gate_mode == 2) launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, false, 2>, dim3(grid), dim3(threads), 0, s, o, ld_out, x, ld_x, gain, rows, g, ld_gate, size, eps);
-    else if (gate != nullptr) launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, false, 1>, dim3(grid), dim3(threads), 0, s, o, ld_out, x, ld_x, gain, rows, g, ld_gate, size, eps);
-    else launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, false, 0>, dim3(grid), dim3(threads), 0, s, o, ld_out, x, ld_x, gain, rows, g, ld_gate, size, eps);
+    auto on = [](const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+    const bool quads = size % 4 == 0 && size <= 4096 && ld_x % 4 == 0 && ld_out % 4 == 0 && on(x, 16) && on(gain, 16) &&
+                       on(out, 4 * sizeof(O)) && (gate == nullptr || (ld_gate % 4 == 0 && on(gate, 4 * sizeof(G))));
+    const int threads = quads ? (size / 4 + 31) / 32 * 32 : (size >= 1024 ? 256 : (size >= 256 ? 128 : (size >= 64 ? 64 : 32)));
+#define GROUPED(ADD, GATE)                                                                                                     \
+    do {                                                                                                                       \
+        if (quads) launch_kernel(g_dependent_launch != 0, grouped_rms_norm_quads_kernel<O, G, ADD, GATE>, grid, dim3(threads), 0, s, o, ld_out, \
+                                 x, ld_x, gain, rows, g, ld_gate, size, eps);                                                  \
+        else launch_kernel(g_dependent_launch != 0, grouped_rms_norm_kernel<O, G, ADD, GATE>, grid, dim3(threads), 0, s, o, ld_out, x, ld_x,    \
+                           gain, rows, g, ld_gate, size, eps);                                                                 \
+    } while (0)
+    if (add) GROUPED(true, 0);
+    else if (gate != nullptr && gate_mode == 3) GROUPED(false, 3);
+    else if (gate != nullptr && gate_mode == 2) GROUPED(false, 2);
+    else if (gate != nullptr) GROUPED(false, 1);
+    else GROUPED(false, 0);
+#undef GROUPED
 }
 
 // out_dtype / gate_dtype: element types of out and gate.  add != 0: out is fp32 and is added to.
@@ -127,7 +188,7 @@ __global__ void causal_taps_kernel(T* __restrict__ out, long ld_out, const T* __
     const int item = token_item[t];
     const int local = positions[t] - item_start[item];          // tokens of this request before t in this step
     float* held = state + (long)item_slot[item] * state_stride;
-    for (int c = threadIdx.x; c < width; c += blockDim.x) {
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
         const float mine = to_f32(h[(long)t * ld_h + c]);
         float acc = identity ? mine : 0.0f;
         if (bias != nullptr) acc += bias[c];
@@ -145,6 +206,96 @@ __global__ void causal_taps_kernel(T* __restrict__ out, long ld_out, const T* __
             for (int s = 0; s + 1 < taps - 1; s++) held[(long)s * width + c] = held[(long)(s + 1) * width + c];
             if (taps > 1) held[(long)(taps - 2) * width + c] = mine;
         }
+    }
+}
+
+// Four taps, a step of single tokens (every earlier input lies in the state, which moves here): a thread a channel, its
+// taps in registers before the kernels ahead have ended.  One block a token walked 1,536 channels in six dependent trips:
+// two tokens 12.5 us against 2.1.
+template <typename T>
+__global__ void __launch_bounds__(128)
+causal_taps_single_kernel(T* __restrict__ out, long ld_out, const T* __restrict__ h, long ld_h, const float* __restrict__ w,
+                          const float* __restrict__ bias, float* state, long state_stride, const int* __restrict__ token_item,
+                          const int* __restrict__ item_slot, int width, int identity, int silu) {
+    const int t = blockIdx.x, c = blockIdx.y * 128 + threadIdx.x;
+    dependents_may_start();
+    if (c >= width) return;
+    const float4 taps = __ldg(reinterpret_cast<const float4*>(w) + c);
+    const float b = bias != nullptr ? __ldg(bias + c) : 0.0f;
+    wait_for_earlier_kernels();
+    h = behind_the_wait(h);
+    const float mine = to_f32(h[(long)t * ld_h + c]);
+    float* held = behind_the_wait(state) + (long)item_slot[token_item[t]] * state_stride + c;
+    const float first = held[0], second = held[width], third = held[2L * width];
+    float acc = (identity ? mine : 0.0f) + b;
+    acc = fmaf(taps.x, first, acc);
+    acc = fmaf(taps.y, second, acc);
+    acc = fmaf(taps.z, third, acc);
+    acc = fmaf(taps.w, mine, acc);
+    if (silu) acc = silu_f(acc);
+    out[(long)t * ld_out + c] = from_f32<T>(acc);
+    held[0] = second;
+    held[width] = third;
+    held[2L * width] = mine;
+}
+
+// Four taps, bfloat16 rows on 16-byte boundaries, prompt portions: a thread takes eight channels of four tokens one behind
+// the other, so that a row is read seven times for four results (four times for one) and 16 bytes at a time.  Two
+// bytes a load, four rows a result: 2,048 tokens of 1,280 to 1,536 channels 25 us against 15.
+constexpr int TAPS_RUN = 4;
+__global__ void __launch_bounds__(128)
+causal_taps_rows_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restrict__ h, long ld_h, const float* __restrict__ w,
+                        const float* __restrict__ bias, const float* __restrict__ state, long state_stride,
+                        const int* __restrict__ positions, const int* __restrict__ token_item, const int* __restrict__ item_slot,
+                        const int* __restrict__ item_start, int n_tokens, int width, int identity, int silu) {
+    const int groups = width / 8;
+    const long index = (long)blockIdx.x * 128 + threadIdx.x;
+    const int c = (int)(index % groups) * 8, t0 = (int)(index / groups) * TAPS_RUN;
+    dependents_may_start();
+    if (t0 >= n_tokens) return;
+    float4 taps[8];
+    float b[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        taps[i] = __ldg(reinterpret_cast<const float4*>(w) + c + i);
+        b[i] = bias != nullptr ? __ldg(bias + c + i) : 0.0f;
+    }
+    wait_for_earlier_kernels();
+    h = behind_the_wait(h);
+    state = behind_the_wait(state);
+    uint4 rows[TAPS_RUN + 3];
+#pragma unroll
+    for (int j = 0; j < TAPS_RUN + 3; j++) {
+        const int t = t0 - 3 + j;
+        rows[j] = t >= 0 && t < n_tokens ? *reinterpret_cast<const uint4*>(h + (long)t * ld_h + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    auto entry = [](const uint4& v, int i) {
+        const uint32_t word = i < 2 ? v.x : i < 4 ? v.y : i < 6 ? v.z : v.w;
+        return __uint_as_float((i & 1) ? word & 0xffff0000u : word << 16);
+    };
+#pragma unroll
+    for (int k = 0; k < TAPS_RUN; k++) {
+        const int t = t0 + k;
+        if (t >= n_tokens) break;
+        const int item = token_item[t], local = positions[t] - item_start[item];      // tokens of this request before t in this step
+        const float* held = state + (long)item_slot[item] * state_stride + c;
+        alignas(16) bf16 result[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float mine = entry(rows[k + 3], i);
+            float v[3];
+#pragma unroll
+            for (int back = 3; back >= 1; back--)
+                v[3 - back] = local >= back ? entry(rows[k + 3 - back], i) : held[(long)(3 + local - back) * width + i];
+            float acc = (identity ? mine : 0.0f) + b[i];
+            acc = fmaf(taps[i].x, v[0], acc);
+            acc = fmaf(taps[i].y, v[1], acc);
+            acc = fmaf(taps[i].z, v[2], acc);
+            acc = fmaf(taps[i].w, mine, acc);
+            if (silu) acc = silu_f(acc);
+            result[i] = __float2bfloat16_rn(acc);
+        }
+        *reinterpret_cast<uint4*>(out + (long)t * ld_out + c) = *reinterpret_cast<const uint4*>(result);
     }
 }
 
@@ -211,6 +362,63 @@ __global__ void norm_taps_step_kernel(T* __restrict__ out, const float* __restri
     }
 }
 
+// The same with four taps, four entries a thread: the row, the gain, the taps and the state each in one pass of 16-byte
+// loads, gain and taps before the kernels ahead have ended.  Two passes over the row and the state an entry at a time:
+// 8 tokens of 768 7.6 us against 2.8.
+template <typename T>
+__global__ void __launch_bounds__(1024)
+norm_taps_quads_kernel(T* __restrict__ out, const float* __restrict__ x, const float* __restrict__ gain, const float* __restrict__ w,
+                       float* __restrict__ state, long state_stride, const int* __restrict__ token_item, const int* __restrict__ item_slot,
+                       int width, int groups, float eps, int writes) {
+    extern __shared__ float norm_taps_shared[];                  // [quads of the row], then [groups]
+    const int t = blockIdx.x, quads = width / 4, q = threadIdx.x, c = 4 * q, warp = q >> 5, lane = q & 31;
+    float* squares = norm_taps_shared;
+    float* scales = norm_taps_shared + quads;
+    const bool there = q < quads;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 g = none, taps[4] = {none, none, none, none}, v = none, held[3] = {none, none, none};
+    dependents_may_start();
+    if (there) {
+        g = __ldg(reinterpret_cast<const float4*>(gain + c));
+#pragma unroll
+        for (int i = 0; i < 4; i++) taps[i] = __ldg(reinterpret_cast<const float4*>(w) + c + i);
+    }
+    wait_for_earlier_kernels();
+    x = behind_the_wait(x);
+    float* mine = behind_the_wait(state) + (long)item_slot[token_item[t]] * state_stride + c;
+    if (there) {
+        v = *reinterpret_cast<const float4*>(x + (long)t * width + c);
+#pragma unroll
+        for (int s = 0; s < 3; s++) held[s] = *reinterpret_cast<const float4*>(mine + (long)s * width);
+        squares[q] = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w)));
+    }
+    __syncthreads();
+    const int size = quads / groups;                             // quads of a group
+    for (int i = warp; i < groups; i += blockDim.x >> 5) {
+        float sum = 0.0f;
+        for (int j = lane; j < size; j += 32) sum += squares[i * size + j];
+        sum = warp_sum(sum);
+        if (lane == 0) scales[i] = 1.0f / sqrtf(sum / (float)(4 * size) + eps);
+    }
+    __syncthreads();
+    if (!there) return;
+    const float scale = scales[q / size];
+    const float normed[4] = {to_f32(from_f32<T>(v.x * scale * g.x)), to_f32(from_f32<T>(v.y * scale * g.y)),
+                             to_f32(from_f32<T>(v.z * scale * g.z)), to_f32(from_f32<T>(v.w * scale * g.w))};
+    const float a[4] = {held[0].x, held[0].y, held[0].z, held[0].w}, b[4] = {held[1].x, held[1].y, held[1].z, held[1].w};
+    const float d[4] = {held[2].x, held[2].y, held[2].z, held[2].w};
+    Four<T> result;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        result.e[i] = from_f32<T>(fmaf(taps[i].w, normed[i], fmaf(taps[i].z, d[i], fmaf(taps[i].y, b[i], fmaf(taps[i].x, a[i], normed[i])))));
+    *reinterpret_cast<Four<T>*>(out + (long)t * width + c) = result;
+    if (writes) {
+        *reinterpret_cast<float4*>(mine) = held[1];
+        *reinterpret_cast<float4*>(mine + width) = held[2];
+        *reinterpret_cast<float4*>(mine + 2L * width) = make_float4(normed[0], normed[1], normed[2], normed[3]);
+    }
+}
+
 extern "C" int mllm_sequence_norm_taps_step(void* out, const float* x, const float* gain, const float* w, float* state,
                                             long state_stride, const int* token_item, const int* item_slot, int n_tokens,
                                             int width, int groups, float eps, int taps, int writes, int dtype, void* stream) {
@@ -220,6 +428,19 @@ extern "C" int mllm_sequence_norm_taps_step(void* out, const float* x, const flo
     const int threads = width >= 256 ? 256 : 64;
     const size_t shared = (size_t)groups * sizeof(float);
     if (shared > 48 * 1024) return fail("norm_taps_step: too many groups");
+    auto on = [](const void* p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+    if (taps == 4 && width <= 4096 && (width / groups) % 4 == 0 && state_stride % 4 == 0 && on(x, 16) && on(gain, 16) && on(w, 16) &&
+        on(state, 16) && on(out, dtype == DT_F32 ? 16 : 8) && (dtype == DT_F32 || dtype == DT_BF16)) {
+        const int quads = width / 4, block = (quads + 31) / 32 * 32;
+        const size_t bytes = (size_t)(quads + groups) * sizeof(float);
+        if (dtype == DT_F32)
+            launch_kernel(g_dependent_launch != 0, norm_taps_quads_kernel<float>, dim3(n_tokens), dim3(block), bytes, s, (float*)out, x, gain,
+                          w, state, state_stride, token_item, item_slot, width, groups, eps, writes);
+        else
+            launch_kernel(g_dependent_launch != 0, norm_taps_quads_kernel<bf16>, dim3(n_tokens), dim3(block), bytes, s, (bf16*)out, x, gain, w,
+                          state, state_stride, token_item, item_slot, width, groups, eps, writes);
+        return check_launch("norm_taps_quads_kernel");
+    }
     if (dtype == DT_F32)
         launch_kernel(g_dependent_launch != 0, norm_taps_step_kernel<float>, dim3(n_tokens), dim3(threads), shared, s, (float*)out, x,
                       gain, w, state, state_stride, token_item, item_slot, width, groups, eps, taps, writes);
@@ -252,15 +473,39 @@ extern "C" int mllm_sequence_causal_taps(void* out, long ld_out, const void* h, 
     if (out == h && taps > 1) return fail("causal_taps: the filter does not run in place");
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = width >= 256 ? 256 : 64;
+    auto on_16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+    if (writes == 2 && taps == 4 && on_16(w)) {
+        const dim3 blocks(n_tokens, (width + 127) / 128);
+        if (dtype == DT_F32)
+            launch_kernel(g_dependent_launch != 0, causal_taps_single_kernel<float>, blocks, dim3(128), 0, s, (float*)out, ld_out,
+                          (const float*)h, ld_h, w, bias, state, state_stride, token_item, item_slot, width, identity, silu);
+        else if (dtype == DT_BF16)
+            launch_kernel(g_dependent_launch != 0, causal_taps_single_kernel<bf16>, blocks, dim3(128), 0, s, (bf16*)out, ld_out,
+                          (const bf16*)h, ld_h, w, bias, state, state_stride, token_item, item_slot, width, identity, silu);
+        else return fail("causal_taps: unknown dtype");
+        return check_launch("causal_taps_single_kernel");
+    }
+    if (writes != 2 && taps == 4 && dtype == DT_BF16 && width % 8 == 0 && ld_h % 8 == 0 && ld_out % 8 == 0 && on_16(w) && on_16(h) &&
+        on_16(out)) {
+        const long threads_needed = (long)((n_tokens + TAPS_RUN - 1) / TAPS_RUN) * (width / 8);
+        launch_kernel(g_dependent_launch != 0, causal_taps_rows_kernel, dim3((unsigned)((threads_needed + 127) / 128)), dim3(128), 0, s,
+                      (bf16*)out, ld_out, (const bf16*)h, ld_h, w, bias, (const float*)state, state_stride, positions, token_item,
+                      item_slot, item_start, n_tokens, width, identity, silu);
+        if (writes == 1)
+            launch_kernel(g_dependent_launch != 0, causal_taps_state_kernel<bf16>, taps_state_grid(n_items, width), dim3(threads), 0, s, state,
+                          state_stride, (const bf16*)h, ld_h, item_slot, item_offset, item_count, width, taps);
+        return check_launch("causal_taps_rows_kernel");
+    }
+    const dim3 token_blocks(n_tokens, n_tokens <= 64 ? (width + threads - 1) / threads : 1);
     if (dtype == DT_F32) {
-        launch_kernel(g_dependent_launch != 0, causal_taps_kernel<float>, dim3(n_tokens), dim3(threads), 0, s, (float*)out, ld_out,
+        launch_kernel(g_dependent_launch != 0, causal_taps_kernel<float>, token_blocks, dim3(threads), 0, s, (float*)out, ld_out,
                       (const float*)h, ld_h, w, bias, state, state_stride, positions, token_item, item_slot, item_start, width,
                       taps, identity, silu, (int)(writes == 2));
         if (writes == 1 && taps > 1)
             launch_kernel(g_dependent_launch != 0, causal_taps_state_kernel<float>, taps_state_grid(n_items, width), dim3(threads), 0, s, state,
                           state_stride, (const float*)h, ld_h, item_slot, item_offset, item_count, width, taps);
     } else if (dtype == DT_BF16) {
-        launch_kernel(g_dependent_launch != 0, causal_taps_kernel<bf16>, dim3(n_tokens), dim3(threads), 0, s, (bf16*)out, ld_out,
+        launch_kernel(g_dependent_launch != 0, causal_taps_kernel<bf16>, token_blocks, dim3(threads), 0, s, (bf16*)out, ld_out,
                       (const bf16*)h, ld_h, w, bias, state, state_stride, positions, token_item, item_slot, item_start, width,
                       taps, identity, silu, (int)(writes == 2));
         if (writes == 1 && taps > 1)

@@ -48,17 +48,23 @@ streams_step_kernel(float* __restrict__ streams, const float* __restrict__ y, lo
     constexpr int BOUND = NS > 0 ? NS : (NS == 0 ? 8 : MAX_STREAMS);
     if (NS > 0) n_streams = NS;
     dependents_may_start();
-    wait_for_earlier_kernels();
     extern __shared__ float u_row[];                 // [width]: the read-out, until it is normed
-    __shared__ float scratch[33];
+    __shared__ float slots[32];
     __shared__ float m[MAX_STREAMS * MAX_STREAMS], o[MAX_STREAMS], in[MAX_STREAMS];
     const int t = blockIdx.x;
+    // (weights: no kernel of a step writes them, so they are read before the kernels ahead have ended)
     if (threadIdx.x < n_streams * n_streams && y != nullptr) m[threadIdx.x] = mix[threadIdx.x];
     if (threadIdx.x < n_streams) {
         if (y != nullptr) o[threadIdx.x] = w_out[threadIdx.x];
         in[threadIdx.x] = w_in != nullptr ? w_in[threadIdx.x] : 1.0f;
     }
+    alignas(16) float gain_ahead[VEC];               // of this thread's first columns
+#pragma unroll
+    for (int e = 0; e < VEC; e++) gain_ahead[e] = normed != nullptr && threadIdx.x * VEC + e < width ? gain[threadIdx.x * VEC + e] : 0.0f;
     __syncthreads();
+    wait_for_earlier_kernels();
+    streams = behind_the_wait(streams);
+    y = behind_the_wait(y);
     float* mine = streams + (long)t * n_streams * width;
     float sq = 0.0f;
     for (int c = threadIdx.x * VEC; c < width; c += blockDim.x * VEC) {
@@ -123,10 +129,10 @@ streams_step_kernel(float* __restrict__ streams, const float* __restrict__ y, lo
     }
     if (!read || normed == nullptr) return;
     // (every thread reads back the columns it wrote itself: no barrier is needed before the sum's own)
-    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+    const float inv = 1.0f / sqrtf(block_sum_once(sq, slots) / (float)width + eps);
     for (int c = threadIdx.x * VEC; c < width; c += blockDim.x * VEC) {
 #pragma unroll
-        for (int e = 0; e < VEC; e++) normed[(long)t * ld_normed + c + e] = from_f32<T>(u_row[c + e] * inv * gain[c + e]);
+        for (int e = 0; e < VEC; e++) normed[(long)t * ld_normed + c + e] = from_f32<T>(u_row[c + e] * inv * (c == (int)threadIdx.x * VEC ? gain_ahead[e] : gain[c + e]));
     }
 }
 

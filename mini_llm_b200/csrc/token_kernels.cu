@@ -204,12 +204,24 @@ template <typename T, bool VEC>
 __global__ void __launch_bounds__(512)
 add_normed_norm_kernel(float* __restrict__ hidden, const float* __restrict__ y, const float* __restrict__ gain, float eps,
                        T* __restrict__ normed, const float* __restrict__ next_gain, float next_eps, int width) {
-    dependents_may_start();
-    wait_for_earlier_kernels();
-    __shared__ float scratch[33];
+    __shared__ float scratch[33], next_scratch[33];
     extern __shared__ __align__(16) float row[];             // [width]
     const long at = (long)blockIdx.x * width;
     float sq = 0.0f;
+    dependents_may_start();
+    // a thread's first entries of the gains are there before the kernels ahead have ended (no kernel of a step writes
+    // them), those of the stream are asked for beside the result's
+    const int mine = threadIdx.x * 4;
+    const bool there = VEC && mine < width;
+    float4 gain_ahead = make_float4(0.0f, 0.0f, 0.0f, 0.0f), next_ahead = gain_ahead, old = gain_ahead;
+    if (there) {
+        gain_ahead = four(gain + mine);
+        if (normed != nullptr) next_ahead = four(next_gain + mine);
+    }
+    wait_for_earlier_kernels();
+    hidden = behind_the_wait(hidden);
+    y = behind_the_wait(y);
+    if (there) old = four(hidden + at + mine);
     if (VEC) {
         for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
             const float4 v = four(y + at + c);
@@ -223,12 +235,12 @@ add_normed_norm_kernel(float* __restrict__ hidden, const float* __restrict__ y, 
             sq = fmaf(v, v, sq);
         }
     }
-    const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)width + eps);
+    const float inv = 1.0f / sqrtf(block_sum_once(sq, scratch) / (float)width + eps);
     float next = 0.0f;
     if (VEC) {
         for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {      // (a thread's own entries of the row)
-            const float4 v = four(row + c), g = four(gain + c);
-            float4 h = four(hidden + at + c);
+            const float4 v = four(row + c), g = c == mine ? gain_ahead : four(gain + c);
+            float4 h = c == mine ? old : four(hidden + at + c);
             h.x = fmaf(v.x * inv, g.x, h.x), h.y = fmaf(v.y * inv, g.y, h.y), h.z = fmaf(v.z * inv, g.z, h.z), h.w = fmaf(v.w * inv, g.w, h.w);
             put_four(hidden + at + c, h);
             put_four(row + c, h);
@@ -243,10 +255,10 @@ add_normed_norm_kernel(float* __restrict__ hidden, const float* __restrict__ y, 
         }
     }
     if (normed == nullptr) return;
-    const float next_inv = 1.0f / sqrtf(block_sum(next, scratch) / (float)width + next_eps);
+    const float next_inv = 1.0f / sqrtf(block_sum_once(next, next_scratch) / (float)width + next_eps);
     if (VEC) {
         for (int c = threadIdx.x * 4; c < width; c += blockDim.x * 4) {
-            const float4 h = four(row + c), g = four(next_gain + c);
+            const float4 h = four(row + c), g = c == mine ? next_ahead : four(next_gain + c);
             put_four(normed + at + c, make_float4(h.x * next_inv * g.x, h.y * next_inv * g.y, h.z * next_inv * g.z, h.w * next_inv * g.w));
         }
     } else {
