@@ -774,7 +774,7 @@ static int launch_capped_block(void* out, long ld_out, const void* q, long ld_q,
     if (e != cudaSuccess) return fail("capped_attention: the register tiles' shared memory was refused");
     cudaFuncSetAttribute(capped_attention_block_kernel<T, VG>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     dim3 grid((n_tokens + tokens_per_block - 1) / tokens_per_block, n_kv_heads * chunks);
-    launch_kernel(g_dependent_launch != 0, capped_attention_block_kernel<T, VG>, grid, dim3(BLOCK_THREADS), shared, s, (T*)out, ld_out, (const T*)q,
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, capped_attention_block_kernel<T, VG>, grid, dim3(BLOCK_THREADS), shared, s, (T*)out, ld_out, (const T*)q,
                   ld_q, (const T*)k_pages, (const T*)v_pages, block_table, max_blocks, positions, token_item, n_tokens, n_heads,
                   n_kv_heads, dim, vdim, page_size, scale, cap, window, keep, gate, ld_gate, gate_wide, sink, slopes,
                   tokens_per_block, heads_per_block);
@@ -809,7 +809,7 @@ static int launch_capped_tiles(void* out, long ld_out, const void* q, long ld_q,
     // several blocks an SM: as much of the SM's memory as shared memory as they need
     cudaFuncSetAttribute(capped_attention_tiled_kernel<T, R, SIZE>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     dim3 grid((n_tokens + tokens_per_block - 1) / tokens_per_block, n_kv_heads * chunks);
-    launch_kernel(g_dependent_launch != 0, capped_attention_tiled_kernel<T, R, SIZE>, grid, dim3(TILE_WARPS * 32), shared, s, (T*)out,
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, capped_attention_tiled_kernel<T, R, SIZE>, grid, dim3(TILE_WARPS * 32), shared, s, (T*)out,
                   ld_out, (const T*)q, ld_q, (const T*)k_pages, (const T*)v_pages, block_table, max_blocks, positions, token_item,
                   n_tokens, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, chunk, keep, gate, ld_gate, gate_wide, sink,
                   slopes, tokens_per_block, heads_per_block);
@@ -1156,7 +1156,7 @@ static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStr
     if (shared > 48 * 1024 &&
         cudaFuncSetAttribute(linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess)
         return fail("linear_recurrence: the staged rows' shared memory was refused");
-    launch_kernel(g_dependent_launch != 0, linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, grid, dim3(128), shared, s, pp);
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, grid, dim3(128), shared, s, pp);
     return check_launch("linear_recurrence_kernel");
 }
 

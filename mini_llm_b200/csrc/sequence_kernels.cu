@@ -488,7 +488,7 @@ extern "C" int mllm_sequence_causal_taps(void* out, long ld_out, const void* h, 
     if (writes != 2 && taps == 4 && dtype == DT_BF16 && width % 8 == 0 && ld_h % 8 == 0 && ld_out % 8 == 0 && on_16(w) && on_16(h) &&
         on_16(out)) {
         const long threads_needed = (long)((n_tokens + TAPS_RUN - 1) / TAPS_RUN) * (width / 8);
-        launch_kernel(g_dependent_launch != 0, causal_taps_rows_kernel, dim3((unsigned)((threads_needed + 127) / 128)), dim3(128), 0, s,
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, causal_taps_rows_kernel, dim3((unsigned)((threads_needed + 127) / 128)), dim3(128), 0, s,
                       (bf16*)out, ld_out, (const bf16*)h, ld_h, w, bias, (const float*)state, state_stride, positions, token_item,
                       item_slot, item_start, n_tokens, width, identity, silu);
         if (writes == 1)
@@ -1193,7 +1193,7 @@ template <typename T, int R, int RPT, int CT, int BK = 32>
 static int launch_latent_tiled(const LatentTiledParams& p, dim3 grid, size_t shared, cudaStream_t s) {
     if (shared > 48 * 1024)
         cudaFuncSetAttribute(latent_attention_tiled_kernel<T, R, RPT, CT, BK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-    launch_kernel(g_dependent_launch != 0, latent_attention_tiled_kernel<T, R, RPT, CT, BK>, dim3(grid), dim3(256), shared, s, p);
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, latent_attention_tiled_kernel<T, R, RPT, CT, BK>, dim3(grid), dim3(256), shared, s, p);
     return check_launch("latent_attention_tiled_kernel");
 }
 
@@ -1382,10 +1382,10 @@ extern "C" int mllm_sequence_memory_scan(const MemoryScanParams* params, int n_i
     dim3 grid(n_items, p.heads, (p.vdim + VS - 1) / VS);
     if (dtype == DT_F32) {
         if (shared > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<float, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-        launch_kernel(g_dependent_launch != 0, memory_scan_kernel<float, VS>, dim3(grid), dim3(VS), shared, s, p);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_scan_kernel<float, VS>, dim3(grid), dim3(VS), shared, s, p);
     } else if (dtype == DT_BF16) {
         if (shared > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<bf16, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-        launch_kernel(g_dependent_launch != 0, memory_scan_kernel<bf16, VS>, dim3(grid), dim3(VS), shared, s, p);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_scan_kernel<bf16, VS>, dim3(grid), dim3(VS), shared, s, p);
     } else {
         return fail("memory_scan: unknown dtype");
     }
@@ -1702,10 +1702,10 @@ extern "C" int mllm_sequence_memory_chunk(const MemoryScanParams* params, int n_
     dim3 grid(n_items, p.heads, (p.vdim + 31) / 32);
     if (dtype == DT_F32) {
         if (shared > 48 * 1024) cudaFuncSetAttribute(memory_chunk_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-        launch_kernel(g_dependent_launch != 0, memory_chunk_kernel<float>, dim3(grid), dim3(256), shared, s, p);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_chunk_kernel<float>, dim3(grid), dim3(256), shared, s, p);
     } else if (dtype == DT_BF16) {
         if (shared > 48 * 1024) cudaFuncSetAttribute(memory_chunk_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
-        launch_kernel(g_dependent_launch != 0, memory_chunk_kernel<bf16>, dim3(grid), dim3(256), shared, s, p);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_chunk_kernel<bf16>, dim3(grid), dim3(256), shared, s, p);
     } else {
         return fail("memory_chunk: unknown dtype");
     }
@@ -2120,17 +2120,17 @@ extern "C" int mllm_sequence_memory_passes(const MemoryPassParams* params, int d
             cudaFuncSetAttribute(memory_sums_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
             cudaFuncSetAttribute(memory_read_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         }
-        launch_kernel(g_dependent_launch != 0, memory_sums_kernel<float>, dim3(over_chunks), dim3(256), shared, s, pp);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_sums_kernel<float>, dim3(over_chunks), dim3(256), shared, s, pp);
         launch_kernel(g_dependent_launch != 0, memory_carry_kernel, dim3(over_items), dim3(256), 0, s, pp);
-        launch_kernel(g_dependent_launch != 0, memory_read_kernel<float>, dim3(over_chunks), dim3(256), shared, s, pp);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_read_kernel<float>, dim3(over_chunks), dim3(256), shared, s, pp);
     } else if (dtype == DT_BF16) {
         if (shared > 48 * 1024) {
             cudaFuncSetAttribute(memory_sums_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
             cudaFuncSetAttribute(memory_read_kernel<bf16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
         }
-        launch_kernel(g_dependent_launch != 0, memory_sums_kernel<bf16>, dim3(over_chunks), dim3(256), shared, s, pp);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_sums_kernel<bf16>, dim3(over_chunks), dim3(256), shared, s, pp);
         launch_kernel(g_dependent_launch != 0, memory_carry_kernel, dim3(over_items), dim3(256), 0, s, pp);
-        launch_kernel(g_dependent_launch != 0, memory_read_kernel<bf16>, dim3(over_chunks), dim3(256), shared, s, pp);
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_read_kernel<bf16>, dim3(over_chunks), dim3(256), shared, s, pp);
     } else {
         return fail("memory_passes: unknown dtype");
     }
