@@ -20,6 +20,7 @@
 // Every kernel is templated on the element type of the activations (float: the true 32-bit path;
 // bfloat16: the serving path) and is launched as a programmatic dependent of the kernel before it.
 #include "common.cuh"
+#include "mma_tiles.cuh"
 
 MLLM_DEFINE_ERROR_API(mllm_hybrid)
 
@@ -1724,7 +1725,7 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
                                    const long long* gate_of, const long long* up_of, const long long* down_of,
                                    const int* inner_of, long ld_down, int max_inner, int width, int pairs,
                                    const float* identity_weight, int form, float limit, float shared_limit, float alpha,
-                                   int n_experts, int n_tokens, int assign, int dtype, void* stream) {
+                                   int n_experts, int n_tokens, int assign, int n_tables, int dtype, void* stream) {
     if (n_tokens <= 0) return 0;
     if (form < EXPERT_GATED_SILU || form > EXPERT_CLAMPED_GLU || (form != EXPERT_RELU_SQUARED && gate_of == nullptr))
         return fail("experts: unknown form of an expert, or one without its gate matrices");
@@ -1775,3 +1776,278 @@ extern "C" int mllm_hybrid_scaled_add(float* x, const float* u, float a, const f
     launch_kernel(g_dependent_launch != 0, scaled_add_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, x, u, a, v, b, n, assign);
     return check_launch("scaled_add_kernel");
 }
+// ---- the pairs of few tokens, by expert ----------------------------------------------------------
+// Up to EXPERT_TILE_TOKENS tokens, bfloat16, inner sizes and the width multiples of 8: the pairs of one expert are the rows of
+// mma.sync tiles (m16n8k16, as the few-row products), so that an expert's weights cross the chip once however many tokens
+// chose it, and the sums are the tensor cores'.  A block a pair read them once a pair and spent its time unpacking: 16 tokens of 8 experts of
+// 768 and a shared one of 1,536 at a width of 768 took 23.4 + 14.7 us (floor 5.4 at measured copy bandwidth).
+// Now 11.9 + 13.4 us, and two tokens of eight choices 7.3 + 11.1 (in a step, one kernel after the other).
+constexpr int EXPERT_TILE_TOKENS = 31, EXPERT_TABLES = 64, EXPERT_UNITS = 64, EXPERT_UNIT_K = 256;
+
+// The pairs that chose expert e, in their order, by one warp; returns how many.
+__device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, int e, int* list, int* place) {
+    const int lane = threadIdx.x & 31;
+    int count = 0;
+    for (int first = 0; first < n_pairs; first += 32) {
+        const int pair = first + lane;
+        const bool mine = pair < n_pairs && choice[pair] == e;
+        const unsigned all = __ballot_sync(0xffffffffu, mine);
+        const int at = count + __popc(all & ((1u << lane) - 1u));
+        if (mine && at < 32) {
+            list[at] = pair;
+            if (place != nullptr) place[pair] = at;
+        }
+        count += __popc(all);
+    }
+    return min(count, 32);
+}
+
+// A block: 16 inner features of an expert, in two tiles of 8 whose K four warps share.
+template <int FORM>
+__global__ void __launch_bounds__(256)
+expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long ld_x, const int* choice, const float* in_weight,
+                       const long long* __restrict__ gate_of, const long long* __restrict__ up_of, const int* __restrict__ inner_of,
+                       int width, int pairs, int n_tokens, float limit, float shared_limit, float alpha, int n_experts) {
+    constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
+    constexpr int AHEAD = 4;
+    __shared__ int list[32], found;
+    __shared__ float sums[2][8][16][9];                      // [gate, up][warp][row][feature]
+    const int e = blockIdx.y, inner = __ldg(inner_of + e);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int f_block = blockIdx.x * 16, f0 = f_block + (warp >> 2) * 8;
+    dependents_may_start();
+    if (f_block >= inner) return;
+    const int pieces = width / 8, all = (width + 31) / 32, each = (all + 3) / 4;
+    const int begin = (warp & 3) * each, end = f0 < inner ? min(all, begin + each) : begin;
+    const long row = (long)min(f0 + g, inner - 1) * pieces;
+    const uint4* up = reinterpret_cast<const uint4*>(__ldg(up_of + e)) + row;
+    const uint4* gate = GATED ? reinterpret_cast<const uint4*>(__ldg(gate_of + e)) + row : up;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    uint4 wu[AHEAD], wg[AHEAD];
+    auto weights = [&](int i, int block) {
+        const int c = block * 4 + tq;
+        const bool there = block < end && c < pieces;
+        wu[i] = there ? __ldg(up + c) : none;
+        if (GATED) wg[i] = there ? __ldg(gate + c) : none;
+    };
+    // (ahead of the wait only where nearly every expert will have a token: a step of one reads four of eight)
+    const bool early = n_tokens * (pairs > 1 ? pairs - 1 : 1) >= n_experts;
+    if (early)
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) weights(i, begin + i);
+    wait_for_earlier_kernels();
+    choice = behind_the_wait(choice);
+    x = behind_the_wait(x);
+    in_weight = behind_the_wait(in_weight);
+    if (warp == 0) {
+        const int count = pairs_of_expert(choice, n_tokens * pairs, e, list, nullptr);
+        if (lane == 0) found = count;
+    }
+    __syncthreads();
+    const int count = found;
+    for (int m0 = 0; m0 < count; m0 += 16) {
+        if (m0 > 0 || !early)
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++) weights(i, begin + i);
+        // rows g and g + 8 of the tile: the tokens of two pairs and the weight their entries get
+        const uint4* xr[2];
+        float scale[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const bool there = m0 + r * 8 + g < count;
+            const int pair = there ? list[m0 + r * 8 + g] : 0;
+            xr[r] = there ? reinterpret_cast<const uint4*>(x + (long)(pair / pairs) * ld_x) : nullptr;
+            scale[r] = there ? in_weight[pair] : 1.0f;
+        }
+        float zg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, zu[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int first = begin; first < end; first += AHEAD) {
+            uint4 xv[AHEAD][2];
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const int c = (first + i) * 4 + tq;
+                    xv[i][r] = xr[r] != nullptr && first + i < end && c < pieces ? xr[r][c] : none;
+                }
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++) {
+                const uint4 u = wu[i], v = GATED ? wg[i] : none;
+                weights(i, first + AHEAD + i);
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+                    if (scale[r] != 1.0f) {                  // the input's weight, rounded as an activation
+                        float y[8];
+                        Vec16<bf16>::unpack(xv[i][r], y);
+                        __nv_bfloat162 two[4];
+#pragma unroll
+                        for (int k = 0; k < 4; k++) two[k] = __floats2bfloat162_rn(scale[r] * y[2 * k], scale[r] * y[2 * k + 1]);
+                        xv[i][r] = *reinterpret_cast<const uint4*>(two);
+                    }
+                mma_bf16_16816(zu[0], zu[1], zu[2], zu[3], xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y, u.x, u.y);
+                mma_bf16_16816(zu[0], zu[1], zu[2], zu[3], xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w, u.z, u.w);
+                if (GATED) {
+                    mma_bf16_16816(zg[0], zg[1], zg[2], zg[3], xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y, v.x, v.y);
+                    mma_bf16_16816(zg[0], zg[1], zg[2], zg[3], xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w, v.z, v.w);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            sums[1][warp][g + (i >> 1) * 8][2 * tq + (i & 1)] = zu[i];
+            if (GATED) sums[0][warp][g + (i >> 1) * 8][2 * tq + (i & 1)] = zg[i];
+        }
+        __syncthreads();
+        const int f = threadIdx.x & 15, r = threadIdx.x >> 4;
+        if (m0 + r < count && f_block + f < inner) {
+            float a = 0.0f, b = 0.0f;
+            for (int s = 0; s < 4; s++) {
+                if (GATED) a += sums[0][(f >> 3) * 4 + s][r][f & 7];
+                b += sums[1][(f >> 3) * 4 + s][r][f & 7];
+            }
+            act[(long)list[m0 + r] * ld_act + f_block + f] =
+                __float2bfloat16_rn(expert_form<FORM>(a, b, e == n_experts ? shared_limit : limit, alpha));
+        }
+        __syncthreads();
+    }
+}
+
+// A block: eight columns of the sum, all tokens.  A unit is an expert's pairs and EXPERT_UNIT_K of its inner size (all of it
+// where the chosen experts would bring more units than there is room for); sixteen warps take the units in turn, and a
+// token's column adds its pairs' units in their order.
+__global__ void __launch_bounds__(512)
+expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld_act, const int* choice, const float* out_weight,
+                         const long long* __restrict__ down_of, const int* __restrict__ inner_of, int n_tables, long ld_down,
+                         int width, int pairs, int n_tokens, int assign, const bf16* x, long ld_x, const float* identity_weight) {
+    constexpr int BLOCKS = EXPERT_UNIT_K / 32;
+    __shared__ int list[EXPERT_TABLES][32], count_of[EXPERT_TABLES], first_unit[EXPERT_TABLES + 1], unit_k;
+    extern __shared__ float down_shared[];                   // [units][32 rows][8 columns], then the pairs' places as ints
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int c0 = blockIdx.x * 8, n_pairs = n_tokens * pairs;
+    int* place = reinterpret_cast<int*>(down_shared + EXPERT_UNITS * 32 * 8);
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    choice = behind_the_wait(choice);
+    act = behind_the_wait(act);
+    out_weight = behind_the_wait(out_weight);
+    x = behind_the_wait(x);
+    for (int e = warp; e < n_tables; e += 16) {
+        const int count = pairs_of_expert(choice, n_pairs, e, list[e], place);
+        if (lane == 0) count_of[e] = count;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // how many units every expert has, and where they begin: two experts a lane
+        int size = EXPERT_UNIT_K, total = 0;
+        for (int attempt = 0; attempt < 2; attempt++) {
+            int mine[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = 2 * lane + h;
+                mine[h] = e < n_tables && count_of[e] > 0 ? (attempt == 0 ? (__ldg(inner_of + e) + EXPERT_UNIT_K - 1) / EXPERT_UNIT_K : 1) : 0;
+            }
+            int sum = mine[0] + mine[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int before = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += before;
+            }
+            total = __shfl_sync(0xffffffffu, sum, 31);
+            const int start = sum - mine[0] - mine[1];
+            if (2 * lane < n_tables) first_unit[2 * lane] = start;
+            if (2 * lane + 1 < n_tables) first_unit[2 * lane + 1] = start + mine[0];
+            size = attempt == 0 ? EXPERT_UNIT_K : 0;
+            if (total <= EXPERT_UNITS) break;
+        }
+        if (lane == 0) {
+            first_unit[n_tables] = total;
+            unit_k = size;
+        }
+    }
+    __syncthreads();
+    const int units = first_unit[n_tables];
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    for (int unit = warp; unit < units; unit += 16) {
+        int e = 0;                                           // the last expert that begins at or before this unit and has units
+        for (int first = 0; first < n_tables; first += 32) {
+            const int at = first + lane;
+            const unsigned here = __ballot_sync(0xffffffffu, at < n_tables && count_of[at] > 0 && first_unit[at] <= unit);
+            if (here != 0u) e = first + 31 - __clz(here);
+        }
+        const int inner = __ldg(inner_of + e), count = count_of[e];
+        const int k_first = unit_k > 0 ? (unit - first_unit[e]) * unit_k : 0, k_end = unit_k > 0 ? min(inner, k_first + unit_k) : inner;
+        const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(__ldg(down_of + e)) + (long)min(c0 + g, width - 1) * ld_down);
+        for (int m0 = 0; m0 < count; m0 += 16) {
+            const uint4* ar[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+                ar[r] = m0 + r * 8 + g < count ? reinterpret_cast<const uint4*>(act + (long)list[e][m0 + r * 8 + g] * ld_act) : nullptr;
+            float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int k0 = k_first; k0 < k_end; k0 += EXPERT_UNIT_K) {
+                uint4 wv[BLOCKS], av[BLOCKS][2];
+#pragma unroll
+                for (int i = 0; i < BLOCKS; i++) {
+                    const int c = k0 / 8 + i * 4 + tq;
+                    const bool there = c * 8 < k_end;
+                    wv[i] = there ? __ldg(w + c) : none;
+#pragma unroll
+                    for (int r = 0; r < 2; r++) av[i][r] = there && ar[r] != nullptr ? ar[r][c] : none;
+                }
+#pragma unroll
+                for (int i = 0; i < BLOCKS; i++) {
+                    mma_bf16_16816(z[0], z[1], z[2], z[3], av[i][0].x, av[i][1].x, av[i][0].y, av[i][1].y, wv[i].x, wv[i].y);
+                    mma_bf16_16816(z[0], z[1], z[2], z[3], av[i][0].z, av[i][1].z, av[i][0].w, av[i][1].w, wv[i].z, wv[i].w);
+                }
+            }
+            float* mine = down_shared + (unit * 32 + m0 + g) * 8 + 2 * tq;
+            mine[0] = z[0], mine[1] = z[1];
+            mine[64] = z[2], mine[65] = z[3];
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_tokens * 8; i += 512) {
+        const int t = i / 8, c = c0 + i % 8;
+        if (c >= width) continue;
+        float total = 0.0f;
+        for (int k = 0; k < pairs; k++) {
+            const int pair = t * pairs + k, e = choice[pair];
+            if (e < 0) continue;
+            const int last = unit_k > 0 ? first_unit[e] + (__ldg(inner_of + e) + EXPERT_UNIT_K - 1) / EXPERT_UNIT_K : first_unit[e] + 1;
+            float z = 0.0f;
+            for (int u = first_unit[e]; u < last; u++) z += down_shared[(u * 32 + place[pair]) * 8 + i % 8];
+            total = fmaf(out_weight[pair], z, total);
+        }
+        if (identity_weight != nullptr) total = fmaf(behind_the_wait(identity_weight)[t], to_f32(x[(long)t * ld_x + c]), total);
+        float* h = hidden + (long)t * ld_hidden + c;
+        *h = assign ? total : *h + total;
+    }
+}
+
+    if (n_tables > 0) {
+        // the caller's word that every inner size is a multiple of 8; what else the tiles need is looked at here
+        auto on_16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+        if (dtype != DT_BF16 || n_tokens > EXPERT_TILE_TOKENS || n_tables > EXPERT_TABLES || width % 8 != 0 || ld_x % 8 != 0 ||
+            ld_act % 8 != 0 || ld_down % 8 != 0 || !on_16(x) || !on_16(act))
+            return fail("experts: the tiles take up to 31 bfloat16 tokens, 64 experts, rows on 16-byte boundaries");
+        const dim3 tiles((max_inner + 15) / 16, n_tables);
+        const bf16* xb = (const bf16*)x;
+        bf16* ab = (bf16*)act;
+#define UP_TILES(FORM)                                                                                                           \
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_up_tiles_kernel<FORM>, tiles, dim3(256), 0, s, ab, ld_act, xb, ld_x, choice, in_weight, \
+                  gate_of, up_of, inner_of, width, pairs, n_tokens, limit, shared_limit, alpha, n_experts)
+        if (form == EXPERT_GATED_SILU) UP_TILES(EXPERT_GATED_SILU);
+        else if (form == EXPERT_RELU_SQUARED) UP_TILES(EXPERT_RELU_SQUARED);
+        else UP_TILES(EXPERT_CLAMPED_GLU);
+#undef UP_TILES
+        const size_t bytes = sizeof(float) * EXPERT_UNITS * 32 * 8 + sizeof(int) * (size_t)n_tokens * pairs;
+        static bool configured = false;
+        if (!configured) {
+            if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
+                return fail("experts: cannot raise the shared memory limit");
+            configured = true;
+        }
+        if (bytes > 128 * 1024) return fail("experts: too many pairs for the tiles");
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_down_tiles_kernel, dim3((width + 7) / 8), dim3(512), bytes, s, hidden, ld_hidden,
+                      (const bf16*)act, ld_act, choice, out_weight, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, assign, xb,
+                      ld_x, identity_weight);
+        return check_launch("expert tiles");
+    }

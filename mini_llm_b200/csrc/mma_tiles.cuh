@@ -1,0 +1,45 @@
+// Pieces of attention kernels on mma.sync m16n8k16 tiles: operands from shared memory, asynchronous copies into it, and a
+// 32-bit operand as three bfloat16 terms.
+#pragma once
+
+#include "common.cuh"
+
+// Four 8 x 8 blocks of 16-bit entries; lane l names row l % 8 of block l / 8.
+__device__ __forceinline__ void load_blocks(uint32_t (&r)[4], const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(row))
+                 : "memory");
+}
+__device__ __forceinline__ void load_blocks_turned(uint32_t (&r)[4], const void* row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(row))
+                 : "memory");
+}
+
+__device__ __forceinline__ void mma_tile(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    mma_bf16_16816(c[0], c[1], c[2], c[3], a[0], a[1], a[2], a[3], b0, b1);
+}
+
+// 16 bytes to shared memory, zeros where there is nothing to copy.
+__device__ __forceinline__ void copy_16(void* to, const void* from, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to)), "l"(from),
+                 "r"(there ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_end() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+
+// Two 32-bit numbers as three pairs of bfloat16 whose sums they are: 8 bits of the significand a term, all 24 in three.  A
+// product of such an operand with a bfloat16 one is three products with 32-bit sums, and rounds where those sums do.
+__device__ __forceinline__ void three_terms(float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
+    __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
+    first = *reinterpret_cast<uint32_t*>(&t);
+    x -= __low2float(t), y -= __high2float(t);
+    t = __floats2bfloat162_rn(x, y);
+    second = *reinterpret_cast<uint32_t*>(&t);
+    x -= __low2float(t), y -= __high2float(t);
+    t = __floats2bfloat162_rn(x, y);
+    third = *reinterpret_cast<uint32_t*>(&t);
+}

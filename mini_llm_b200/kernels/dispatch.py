@@ -169,10 +169,13 @@ class Kernels:
         return ops.route(x, router, shared_gate, top, choice, in_weight, out_weight, **how)
 
     def experts(self, hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
-                ld_down=None, assign=False, identity_weight=None, **form):
+                ld_down=None, assign=False, identity_weight=None, eights=False, **form):
+        """``eights``: every expert's inner size is a multiple of 8."""
         self.launches += 2
+        tiles = eights and not self.plain_only and ld_down is not None and ops.expert_tiles_take(x, act, inner_of.shape[0], ld_down)
+        self.chose("experts", "expert_tiles" if tiles else "expert_pairs", x.shape[0], max_inner, x.shape[1])
         return ops.experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
-                           ld_down, assign, identity_weight, **form)
+                           ld_down, assign, identity_weight, tiles=tiles, **form)
 
     EXPERTS_AT_ONCE_TOKENS = 32    # from here on a step's tokens go through all experts as two products
 

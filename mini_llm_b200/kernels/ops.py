@@ -1387,7 +1387,7 @@ def linear_recurrence(out, q, k, v, gate_a, gate_b, log_rate, step_bias, state, 
 
 
 _route = Function("hybrid", "mllm_hybrid_route", [P, L, P, P, P, P, I, I, F, I, I, I, I, I, I, P, P, P, P, I, I, P])
-_experts = Function("hybrid", "mllm_hybrid_experts", [P, L, P, L, P, L, P, P, P, P, P, P, P, L, I, I, I, P, I, F, F, F, I, I, I, I, P])
+_experts = Function("hybrid", "mllm_hybrid_experts", [P, L, P, L, P, L, P, P, P, P, P, P, P, L, I, I, I, P, I, F, F, F, I, I, I, I, I, P])
 _expert_combine = Function("hybrid", "mllm_hybrid_expert_combine",
                            [P, L, P, L, P, P, P, I, I, I, I, I, I, F, F, F, P, L, P, L, P, I, I, I, I, P])
 ROUTE_RULES = {"sigmoid_on_input": 0, "softmax_of_chosen": 1, "softmax_of_all": 2, "sigmoid": 3}
@@ -1448,7 +1448,7 @@ def _check_identity(identity_weight, x, n, who):
 
 
 def experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs, ld_down=None,
-            assign=False, identity_weight=None, form=None, limit=0.0, shared_limit=0.0, alpha=0.0, n_experts=-1):
+            assign=False, identity_weight=None, form=None, limit=0.0, shared_limit=0.0, alpha=0.0, n_experts=-1, tiles=False):
     """hidden[t] += sum over the token's ``pairs`` of out_weight * W_down[e] (silu(W_gate[e] x') * (W_up[e] x')),
     x' = in_weight * x[t] rounded to the activations' type; expert e's matrices are named by the
     int64 pointer tables ``gate_of``, ``up_of``, ``down_of`` and its inner size by ``inner_of`` (int32);
@@ -1457,7 +1457,8 @@ def experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_
     W_down[e] relu(W_up[e] x')^2.  ``form`` "clamped_glu": between the products g' sigmoid(alpha g') (u' + 1) with
     g' = min(g, limit) and u' = clamp(u, -limit, limit); expert ``n_experts`` (the shared one) has ``shared_limit``.  ``act`` [T * pairs, max_inner] is scratch.  A pair whose choice is negative has no
     expert; with ``identity_weight`` [T] identity_weight[t] * x[t] joins the sum.  ``assign``: ``hidden`` is set
-    to the sum instead of added to."""
+    to the sum instead of added to.  ``tiles``: the pairs go through the tensor cores expert by expert (``expert_tiles_take``;
+    the caller says with it that every inner size is a multiple of 8 and that no token chose an expert twice)."""
     _check(hidden, "experts.hidden", torch.float32, 2)
     _check(x, "experts.x", None, 2)
     _check(act, "experts.act", x.dtype, 2)
@@ -1474,8 +1475,17 @@ def experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_
              in_weight.data_ptr(), out_weight.data_ptr(), _ptr(gate_of), up_of.data_ptr(), down_of.data_ptr(),
              inner_of.data_ptr(), int(ld_down if ld_down is not None else max_inner), int(max_inner), width, int(pairs),
              _ptr(identity_weight), EXPERT_FORMS[form], float(limit), float(shared_limit), float(alpha), int(n_experts), n,
-             int(bool(assign)), dtype_code(x.dtype), _stream())
+             int(bool(assign)), inner_of.shape[0] if tiles else 0, dtype_code(x.dtype), _stream())
     return hidden
+
+
+EXPERT_TILE_TOKENS, EXPERT_TABLES = 31, 64
+
+
+def expert_tiles_take(x, act, n_tables, ld_down) -> bool:
+    """Whether ``experts(..., tiles=True)`` takes the step: few bfloat16 tokens, rows on 16-byte boundaries."""
+    return (x.dtype == torch.bfloat16 and x.shape[0] <= EXPERT_TILE_TOKENS and n_tables <= EXPERT_TABLES and x.shape[1] % 8 == 0
+            and x.stride(0) % 8 == 0 and act.stride(0) % 8 == 0 and ld_down % 8 == 0 and x.data_ptr() % 16 == 0 and act.data_ptr() % 16 == 0)
 
 
 def expert_combine(act, gu, choice, in_weight, out_weight, n_experts, inner, top, pairs, form="gated_silu", hidden=None, x=None,

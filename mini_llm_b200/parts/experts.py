@@ -139,6 +139,7 @@ class RoutedExperts(FeedForward):
         self.down_of = table(self.down_matrix.data_ptr(), starts)
         self.inner_of = torch.tensor([inner for _, inner in experts], dtype=torch.int32, device=device)
         self.max_inner = max(inner for _, inner in experts)
+        self.eights = all(inner % 8 == 0 for _, inner in experts)
         # the loaded matrices are held in the stacked ones now
         self.weights = {name: tensor for name, tensor in self.weights.items()
                         if name in [self.full_name(n[key]) for key in ("router", "shared_gate", "router_bias", "correction")]}
@@ -168,7 +169,7 @@ class RoutedExperts(FeedForward):
         act = ctx.buffer("expert_act", (n * self.pairs, self.max_inner), ctx.act_dtype)
         k.experts(hidden, act, x, choice, in_weight, out_weight, self.gate_of, self.up_of, self.down_of, self.inner_of,
                   self.max_inner, self.pairs, ld_down=self.total, assign=assign, identity_weight=identity,
-                  n_experts=self.n_experts, **self.form_constants)
+                  n_experts=self.n_experts, eights=self.eights, **self.form_constants)
 
     def compute(self, ctx, x):
         out = ctx.buffer("mlp_out", (x.shape[0], self.width), torch.float32)

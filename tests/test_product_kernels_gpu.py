@@ -104,3 +104,51 @@ def test_two_memory_shapes_share_scratch_without_moving_it():
     for floats in ((100, 20, 30), (50, 40, 10)):
         assert kernels._memory_scratch("cuda", floats) is second
     assert kernels.scratch_generation == moved
+
+
+# one expert and many, pairs that name none, inner sizes that end inside a tile of 16 features and a unit of 256, every form
+@pytest.mark.parametrize("tokens, experts, top, inners, width, form", [
+    (1, 8, 2, (24, 40), 64, "gated_silu"), (31, 3, 3, (264, 8), 768, "gated_silu"), (17, 40, 4, (512, 776), 72, "relu_squared"),
+    (8, 5, 1, (16, 96), 1160, "clamped_glu"), (9, 1, 1, (256, 256), 8, "clamped_glu")])
+def test_experts_in_tiles(tokens, experts, top, inners, width, form):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(tokens + experts)
+    sizes = [inners[e % 2] for e in range(experts)]
+    total, most = sum(sizes), max(sizes)
+    x = dev(rng.normal(size=(tokens, width)), torch.bfloat16)
+    gates, ups, downs = (dev(rng.normal(size=s) / math.sqrt(s[1]), torch.bfloat16) for s in ((total, width), (total, width), (width, total)))
+    starts = np.cumsum([0] + sizes[:-1])
+    chosen = np.stack([rng.permutation(experts)[:top] for _ in range(tokens)]).astype(np.int32)
+    chosen[rng.random(chosen.shape) < 0.1] = -1
+    in_weight, out_weight = rng.uniform(0.5, 1.0, (tokens, top)).astype(np.float32), rng.uniform(0.1, 1.0, (tokens, top)).astype(np.float32)
+    before = rng.normal(size=(tokens, width)).astype(np.float32)
+    constants = dict(limit=1.5, shared_limit=0.5, alpha=1.702, n_experts=experts - 1) if form == "clamped_glu" else {}
+    expected = before.astype(np.float64)
+    xs, gs, us, ds = f64(x), f64(gates), f64(ups), f64(downs)
+    for t in range(tokens):
+        for e, a, b in zip(chosen[t], in_weight[t], out_weight[t]):
+            if e < 0:
+                continue
+            part = slice(starts[e], starts[e] + sizes[e])
+            into = f64(dev(np.float32(a) * f64(x)[t].astype(np.float32), torch.bfloat16))
+            g, u = gs[part] @ into, us[part] @ into
+            if form == "gated_silu":
+                act = g / (1 + np.exp(-g)) * u
+            elif form == "relu_squared":
+                act = np.maximum(u, 0) ** 2
+            else:
+                limit = 0.5 if e == experts - 1 else 1.5
+                g = np.minimum(g, limit)
+                act = g / (1 + np.exp(-1.702 * g)) * (np.clip(u, -limit, limit) + 1)
+            expected[t] += b * (ds[:, part] @ act)
+    at = lambda matrix, step: torch.tensor([matrix.data_ptr() + 2 * step * int(s) for s in starts], dtype=torch.int64, device="cuda")
+    act = torch.full((tokens * top, most), float("nan"), dtype=torch.bfloat16, device="cuda")
+    assert ops.expert_tiles_take(x, act, experts, total)
+    for tiles in (True, False):
+        hidden = dev(before)
+        ops.experts(hidden, act, x, dev(chosen.reshape(-1)), dev(in_weight.reshape(-1)), dev(out_weight.reshape(-1)),
+                    at(gates, width) if form != "relu_squared" else None, at(ups, width), at(downs, 1), dev(np.array(sizes, np.int32)), most, top,
+                    ld_down=total, form=form, tiles=tiles, **constants)
+        # activations are rounded to 8 bits once: each of a sum's terms is off by 2^-9 of itself at most, and the largest sums here
+        # hold 3 experts x 264 terms of squares' size 1 / 264
+        np.testing.assert_allclose(f64(hidden), expected, rtol=0, atol=2e-2, err_msg=f"tiles={tiles}")
