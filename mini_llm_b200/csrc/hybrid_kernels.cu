@@ -750,6 +750,216 @@ capped_attention_block_kernel(T* __restrict__ out, long ld_out, const T* __restr
     }
 }
 
+// ---------------------------------------------------------------------------
+// The same attention on tensor-core tiles, bfloat16, keys and values of up to 128 entries (multiples of 8).  A block of four
+// warps takes 64 (token, head) rows of one key/value head, a warp 16 of them, and walks the keys 64 at a time, keys and
+// values copied a tile ahead.  Scores are products of bfloat16 operands with 32-bit sums; the weights stay 32-bit: each goes into the
+// second product as three bfloat16 terms, which hold all 24 bits of it, against the values as they are.  Maxima, sums,
+// weights and results are 32-bit in the rows' threads, four threads a row; cap, slopes, masks, sink and gate as above.
+// The products no longer bound it: a tile of 16 x 64 takes 128 of them (KEY 64, VALUE 64) against 32,768 FMAs of the
+// register tiles, and the exponentials and masks stand beside them.
+// Three prompts of 640 to 2,048 tokens (12 heads over 4, sizes 64): 169 us a launch on register tiles, 115 here.
+// ---------------------------------------------------------------------------
+template <int KEY, int VALUE>          // entries of a key and of a value: 64 or 128, zeros past dim and vdim
+__global__ void __launch_bounds__(128)
+capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, long ld_q, const bf16* k_pages, const bf16* v_pages,
+                            const int* block_table, int max_blocks, const int* positions, const int* token_item, int n_tokens,
+                            int n_heads, int n_kv_heads, int dim, int vdim, int page_size, float scale, float cap, int window, int chunk,
+                            int keep, const float* gate, long ld_gate, int gate_wide, const float* sink, const float* slopes,
+                            int tokens_per_block, int heads_per_block) {
+    constexpr int KEYS = 64, LDK = KEY + 8, LDV = VALUE + 8;           // rows an odd number of 16 bytes apart: no bank twice
+    extern __shared__ __align__(16) unsigned char mma_shared[];
+    bf16* q_rows = reinterpret_cast<bf16*>(mma_shared);               // [64][LDK]
+    bf16* keys = q_rows + 64 * LDK;                                    // [2][64][LDK]
+    bf16* values = keys + 2 * KEYS * LDK;                              // [2][64][LDV]
+    __shared__ int row_pos[64], row_item[64];
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int group = n_heads / n_kv_heads, chunks = (group + heads_per_block - 1) / heads_per_block;
+    const int hk = blockIdx.y / chunks, first_head = hk * group + (blockIdx.y % chunks) * heads_per_block;
+    const int n_heads_here = min(heads_per_block, hk * group + group - first_head);
+    // (the step's last tokens first, as above)
+    const int first_token = (gridDim.x - 1 - blockIdx.x) * tokens_per_block;
+    const int n_tok = min(tokens_per_block, n_tokens - first_token), n_rows = n_tok * n_heads_here;
+    const float inv_cap = cap > 0.0f ? 1.0f / cap : 0.0f;
+    if (tid < 64) {
+        const int token = tid < n_rows ? first_token + tid / n_heads_here : -1;
+        row_pos[tid] = token >= 0 ? positions[token] : -1;
+        row_item[tid] = token >= 0 ? token_item[token] : -1;
+    }
+    for (int u = tid; u < 64 * (KEY / 8); u += 128) {
+        const int r = u / (KEY / 8), d = (u % (KEY / 8)) * 8;
+        const bool there = r < n_rows && d < dim;
+        const bf16* from = there ? q + (long)(first_token + r / n_heads_here) * ld_q + (long)(first_head + r % n_heads_here) * dim + d : q;
+        copy_16(q_rows + r * LDK + d, from, there);
+    }
+    copies_end();
+    copies_landed<0>();
+    __syncthreads();
+    uint32_t qa[KEY / 16][4];
+#pragma unroll
+    for (int k = 0; k < KEY / 16; k++) load_blocks(qa[k], q_rows + (warp * 16 + (lane & 15)) * LDK + k * 16 + (lane >> 4) * 8);
+    int my_pos[2], my_item[2], my_first[2];
+    float my_slope[2], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, o[VALUE / 8][4];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int r = warp * 16 + h * 8 + g;
+        my_pos[h] = row_pos[r], my_item[h] = row_item[r], my_first[h] = first_visible(my_pos[h], window, chunk);
+        my_slope[h] = r < n_rows && slopes != nullptr ? slopes[first_head + r % n_heads_here] : 0.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < VALUE / 8; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+    const int page_shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;
+
+    int run_first = 0;
+    while (run_first < n_tok) {
+        const int item = token_item[first_token + run_first];
+        int run_last = run_first;
+        while (run_last + 1 < n_tok && token_item[first_token + run_last + 1] == item) run_last++;
+        const int p_first = positions[first_token + run_first], p_last = positions[first_token + run_last];
+        const int lo = first_visible(p_first, window, chunk);
+        const int* bt = block_table + (long)item * max_blocks;
+        const int first_base = (lo / KEYS) * KEYS;
+        auto ask = [&](int base, int buffer) {
+            bf16* into_k = keys + buffer * KEYS * LDK;
+            bf16* into_v = values + buffer * KEYS * LDV;
+            for (int u = tid; u < KEYS * (KEY / 8 + VALUE / 8); u += 128) {
+                const bool value = u >= KEYS * (KEY / 8);
+                const int v = value ? u - KEYS * (KEY / 8) : u, pieces = value ? VALUE / 8 : KEY / 8;
+                const int j = v / pieces, d = (v % pieces) * 8, kp = base + j, size = value ? vdim : dim;
+                // (pages before the first visible key may be gone)
+                const bool there = d < size && kp <= p_last && key_visible(kp, lo, keep);
+                const bf16* from = k_pages;
+                if (there) {
+                    const int block = page_shift >= 0 ? kp >> page_shift : kp / page_size;
+                    const long slot = (long)bt[block] * page_size + (kp - block * page_size);
+                    from = (value ? v_pages : k_pages) + (slot * n_kv_heads + hk) * size + d;
+                }
+                copy_16(value ? into_v + j * LDV + d : into_k + j * LDK + d, from, there);
+            }
+            copies_end();
+        };
+        int base = first_tile(first_base, keep), next = 0, buffer = 0;
+        ask(base, 0);
+        for (; base <= p_last; base = next, buffer ^= 1) {
+            next = next_tile(base, KEYS, first_base, keep);
+            // (the other buffer was left by every warp before the barrier that ended the last round)
+            if (next <= p_last) ask(next, buffer ^ 1);
+            else copies_end();
+            copies_landed<1>();
+            __syncthreads();
+            bool any = false;
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                any = any || (my_item[h] == item && base <= my_pos[h] && (base + KEYS > my_first[h] || base < keep));
+            if (__any_sync(0xffffffffu, any)) {
+                const bf16* kt = keys + buffer * KEYS * LDK;
+                const bf16* vt = values + buffer * KEYS * LDV;
+                float s[8][4];
+#pragma unroll
+                for (int j = 0; j < 8; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
+#pragma unroll
+                for (int k = 0; k < KEY / 16; k++)
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        uint32_t b[4];
+                        load_blocks(b, kt + (j * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * LDK + k * 16 + ((lane >> 3) & 1) * 8);
+                        mma_tile(s[j], qa[k], b[0], b[1]);
+                        mma_tile(s[j + 1], qa[k], b[2], b[3]);
+                    }
+                float corr[2];
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const bool row_here = my_item[h] == item;
+                    float top = -INFINITY;
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const int pos = base + j * 8 + 2 * tq + e;
+                            const bool seen = row_here && pos <= my_pos[h] && key_visible(pos, my_first[h], keep);
+                            float& x = s[j][2 * h + e];
+                            x = seen ? capped(x * scale, cap, inv_cap) - my_slope[h] * (float)(my_pos[h] - pos) : -INFINITY;
+                            top = fmaxf(top, x);
+                        }
+                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                    const float m_new = fmaxf(m[h], top), from = m_new == -INFINITY ? 0.0f : m_new;
+                    corr[h] = expf(m[h] - from);
+                    float sum = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 8; j++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            s[j][2 * h + e] = expf(s[j][2 * h + e] - from);
+                            sum += s[j][2 * h + e];
+                        }
+                    l[h] = l[h] * corr[h] + sum;             // this thread's share of the row
+                    m[h] = m_new;
+                }
+                if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
+#pragma unroll
+                    for (int j = 0; j < VALUE / 8; j++) o[j][0] *= corr[0], o[j][1] *= corr[0], o[j][2] *= corr[1], o[j][3] *= corr[1];
+                }
+#pragma unroll
+                for (int k = 0; k < KEYS / 16; k++) {
+                    uint32_t a[3][4];
+                    three_terms(s[2 * k][0], s[2 * k][1], a[0][0], a[1][0], a[2][0]);
+                    three_terms(s[2 * k][2], s[2 * k][3], a[0][1], a[1][1], a[2][1]);
+                    three_terms(s[2 * k + 1][0], s[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
+                    three_terms(s[2 * k + 1][2], s[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+                    for (int j = 0; j < VALUE / 8; j += 2) {
+                        uint32_t b[4];
+                        load_blocks_turned(b, vt + (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + j * 8 + ((lane >> 4) & 1) * 8);
+#pragma unroll
+                        for (int t = 0; t < 3; t++) {
+                            mma_tile(o[j], a[t], b[0], b[1]);
+                            mma_tile(o[j + 1], a[t], b[2], b[3]);
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        copies_landed<0>();
+        run_first = run_last + 1;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        float sum = l[h];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const int r = warp * 16 + h * 8 + g;
+        if (r >= n_rows) continue;
+        const int token = first_token + r / n_heads_here, head = first_head + r % n_heads_here;
+        float shrink = 1.0f;
+        if (sink != nullptr) {
+            const float top = fmaxf(m[h], sink[head]);
+            shrink = expf(m[h] - top);
+            sum = sum * shrink + expf(sink[head] - top);
+        }
+        const float inv = (gate != nullptr && !gate_wide ? sigmoid_f(gate[(long)token * ld_gate + head]) : 1.0f) * shrink / sum;
+        const float* open = gate != nullptr && gate_wide ? gate + (long)token * ld_gate + (long)head * vdim : nullptr;
+#pragma unroll
+        for (int j = 0; j < VALUE / 8; j++)
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const int d = j * 8 + 2 * tq + e;
+                if (d < vdim)
+                    out[(long)token * ld_out + (long)head * vdim + d] =
+                        __float2bfloat16_rn(o[j][2 * h + e] * inv * (open != nullptr ? sigmoid_f(open[d]) : 1.0f));
+            }
+    }
+}
+
+// (rows of queries, keys and values in whole 16-byte pieces)
+static bool capped_mma_takes(const void* q, long ld_q, const void* k_pages, const void* v_pages, int dim, int vdim) {
+    return dim % 8 == 0 && vdim % 8 == 0 && dim <= 128 && vdim <= 128 && ld_q % 8 == 0 &&
+           ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_pages) | reinterpret_cast<uintptr_t>(v_pages)) & 15) == 0;
+}
+
 static size_t capped_block_shared(int dim, int vdim) {
     return sizeof(float) * ((size_t)2 * BLOCK_ROWS * (dim + 4) + (size_t)BLOCK_KEYS * (vdim + 4) + (size_t)BLOCK_ROWS * (BLOCK_KEYS + 4)) +
            (2 * sizeof(int) + sizeof(float)) * BLOCK_ROWS;
@@ -830,8 +1040,35 @@ static int launch_capped_attention(bool tiled, void* out, long ld_out, const voi
                       sink, slopes);
         return check_launch("capped_attention_plain_kernel");
     }
-    // the common sizes go to the register tiles
-    if (chunk == 0 && n_tokens * (long)n_heads >= 2048 && capped_block_takes(dim, vdim, 16 / (int)sizeof(T)) &&
+    // bfloat16 of the common sizes goes to the tensor-core tiles
+    if constexpr (sizeof(T) == 2) {
+        if (capped_mma_takes(q, ld_q, k_pages, v_pages, dim, vdim)) {
+            const int group = n_heads / n_kv_heads, heads_per_block = group < 64 ? group : 64, tokens_per_block = 64 / heads_per_block;
+            const int key = dim <= 64 ? 64 : 128, value = vdim <= 64 ? 64 : 128;
+            const size_t shared = sizeof(bf16) * (size_t)(192 * (key + 8) + 128 * (value + 8));
+            const dim3 grid((n_tokens + tokens_per_block - 1) / tokens_per_block, n_kv_heads * ((group + heads_per_block - 1) / heads_per_block));
+#define CAPPED_MMA(KEY, VALUE)                                                                                                    \
+    do {                                                                                                                          \
+        if (cudaFuncSetAttribute(capped_attention_mma_kernel<KEY, VALUE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) !=  \
+            cudaSuccess)                                                                                                          \
+            return fail("capped_attention: the tiles' shared memory was refused");                                               \
+        cudaFuncSetAttribute(capped_attention_mma_kernel<KEY, VALUE>, cudaFuncAttributePreferredSharedMemoryCarveout,             \
+                             cudaSharedmemCarveoutMaxShared);                                                                     \
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, capped_attention_mma_kernel<KEY, VALUE>, grid, dim3(128), shared, s, (bf16*)out, ld_out,  \
+                      (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks, positions, token_item, \
+                      n_tokens, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, chunk, keep, gate, ld_gate, gate_wide, sink, \
+                      slopes, tokens_per_block, heads_per_block);                                                                 \
+        return check_launch("capped_attention_mma_kernel");                                                                       \
+    } while (0)
+            if (key == 64 && value == 64) CAPPED_MMA(64, 64);
+            if (key == 64) CAPPED_MMA(64, 128);
+            if (value == 64) CAPPED_MMA(128, 64);
+            CAPPED_MMA(128, 128);
+#undef CAPPED_MMA
+        }
+    }
+    // 32-bit rows of the common sizes go to the register tiles
+    if constexpr (sizeof(T) == 4) if (chunk == 0 && n_tokens * (long)n_heads >= 2048 && capped_block_takes(dim, vdim, 16 / (int)sizeof(T)) &&
         (ld_q * sizeof(T)) % 16 == 0) {
         if (vdim <= 64)
             return launch_capped_block<T, 1>(out, ld_out, q, ld_q, k_pages, v_pages, block_table, max_blocks, positions, token_item,

@@ -152,3 +152,36 @@ def test_experts_in_tiles(tokens, experts, top, inners, width, form):
         # activations are rounded to 8 bits once: each of a sum's terms is off by 2^-9 of itself at most, and the largest sums here
         # hold 3 experts x 264 terms of squares' size 1 / 264
         np.testing.assert_allclose(f64(hidden), expected, rtol=0, atol=2e-2, err_msg=f"tiles={tiles}")
+
+
+# what the launcher gives a whole tile row: groups of 1, 5, 64 and more heads; sizes that end inside a tile; each mask and option
+@pytest.mark.parametrize("heads, kv_heads, dim, vdim, window, chunk, keep, cap, options", [
+    (1, 1, 8, 8, 0, 0, 0, 0.0, ()), (5, 1, 64, 64, 0, 0, 0, 30.0, ("sink",)), (8, 4, 72, 56, 0, 32, 0, 0.0, ("gate",)),
+    (64, 1, 24, 128, 65, 0, 7, 0.0, ("slopes", "gate_wide")), (70, 1, 128, 128, 1, 0, 130, 0.0, ("sink", "slopes")), (6, 6, 128, 40, 200, 0, 0, 5.0, ("gate",))])
+def test_capped_attention_in_tensor_core_tiles(heads, kv_heads, dim, vdim, window, chunk, keep, cap, options):
+    """Three requests' portions whose borders fall inside a block's rows, against one block per (token, head)."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(heads + dim)
+    page, lengths, new = 16, [3, 210, 333], [3, 101, 64]
+    blocks = [-(-n // page) for n in lengths]
+    table = torch.zeros(3, max(blocks), dtype=torch.int32)
+    order = rng.permutation(sum(blocks))
+    for i, count in enumerate(blocks):
+        table[i, :count] = torch.tensor(order[sum(blocks[:i]):sum(blocks[:i]) + count])
+    k_pages, v_pages = (dev(rng.normal(size=(sum(blocks), page, kv_heads, d)), torch.bfloat16) for d in (dim, vdim))
+    positions = dev(np.concatenate([np.arange(l - m, l) for l, m in zip(lengths, new)]).astype(np.int32))
+    items = dev(np.repeat(np.arange(3), new).astype(np.int32))
+    n = sum(new)
+    q = dev(rng.normal(size=(n, heads * dim + 8)), torch.bfloat16)[:, 8:]
+    how = dict(window=window, chunk=chunk, keep=keep, cap=cap)
+    if "sink" in options:
+        how["sink"] = dev(rng.normal(size=heads), torch.float32)
+    if "slopes" in options:
+        how["slopes"] = dev(rng.uniform(0, 0.5, heads), torch.float32)
+    if "gate" in options or "gate_wide" in options:
+        how.update(gate=dev(rng.normal(size=(n, heads * (vdim if "gate_wide" in options else 1))), torch.float32), gate_wide="gate_wide" in options)
+    want, got = (torch.full((n, heads * vdim), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for out, tiled in ((want, False), (got, True)):
+        ops.capped_attention(out, q, k_pages, v_pages, table.cuda(), positions, items, heads, kv_heads, dim, vdim, page, dim ** -0.5, tiled=tiled, **how)
+    # both keep scores, weights and sums in 32 bits, so they may differ by the last rounding to 8 bits: 2^-8 of values below 4
+    np.testing.assert_allclose(f64(got), f64(want), rtol=2 ** -7, atol=2 ** -10)
