@@ -15,6 +15,7 @@
 // kernel before it on its stream: its blocks may be scheduled while that one still runs, and the
 // first thing each does is to wait for it, before any memory is touched.
 #include "common.cuh"
+#include "mma_tiles.cuh"
 
 MLLM_DEFINE_ERROR_API(mllm_sequence)
 
@@ -1155,6 +1156,218 @@ latent_attention_tiled_kernel(LatentTiledParams p) {
     }
 }
 
+// ---------------------------------------------------------------------------
+// Prompt portions over a latent of 128 or 256 entries, bfloat16 rows, on tensor-core tiles.  All heads read the same rows, so a
+// portion's (token, head) pairs in memory order are the rows of one matrix: a block takes 64 of them and walks the cached
+// rows 64 at a time (copied a tile ahead).  Warp w has rows 16 (w % 4) .. and keys 32 (w / 4) .. of every tile; the two warps of a row
+// group keep their own maximum, sum and weighted sum and are merged at the end.  Queries and weights stay 32-bit: each enters its
+// product as three bfloat16 terms that hold all its 24 bits, the cached rows are bfloat16 as they are, sums are 32-bit.
+// A tile of 64 x 64 pairs is 3,264 m16n8k16 products (latent 256, row 288); as 32-bit FMAs, 2.2 million of them, with a quarter of a load
+// from shared memory each, it was what the step waited for.
+// Three prompts of 640 to 2,048 tokens, 12 heads over a latent of 256: 550 us a launch then, 134 now.
+// ---------------------------------------------------------------------------
+constexpr int LATENT_MMA_ROWS = 64, LATENT_MMA_KEYS = 64;
+
+template <int RANK>
+__global__ void __launch_bounds__(256, 1)
+latent_attention_mma_kernel(LatentTiledParams p) {
+    extern __shared__ __align__(16) unsigned char latent_shared[];
+    const int row_width = p.rank + p.rot, ld = row_width + 8;                     // (an odd number of 16 bytes)
+    bf16* q_terms = reinterpret_cast<bf16*>(latent_shared);                       // [3][64][ld]
+    bf16* rows_of = q_terms + 3 * LATENT_MMA_ROWS * ld;                           // [2][64][ld]
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int per_record = 128 * p.heads / LATENT_MMA_ROWS;
+    const int* record = p.tiles + (long)(blockIdx.x / per_record) * 8;
+    // (a record's last rows, which see the most keys, first)
+    const int first = (per_record - 1 - (int)blockIdx.x % per_record) * LATENT_MMA_ROWS, n_rows = min(LATENT_MMA_ROWS, record[2] * p.heads - first);
+    if (record[4] != 0 || n_rows <= 0) return;
+    const int* bt = p.block_table + (long)record[0] * p.max_blocks;
+    const long row0 = (long)record[1] * p.heads + first;                          // of the step's (token, head) pairs
+    const int position0 = record[3];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int quarter = warp & 3, half = warp >> 2;
+    const int key_end = position0 + (first + n_rows - 1) / p.heads + 1;
+    const int key_begin = p.window > 0 ? max(0, position0 + first / p.heads - p.window + 1) : 0;
+    auto ask = [&](int k0, int buffer) {
+        bf16* into = rows_of + buffer * LATENT_MMA_KEYS * ld;
+        const int pieces = row_width / 8;
+        for (int u = tid; u < LATENT_MMA_KEYS * pieces; u += 256) {
+            const int j = u / pieces, d = (u % pieces) * 8, key = k0 + j;
+            const bool there = key < key_end;
+            const bf16* from = reinterpret_cast<const bf16*>(p.pages);
+            if (there) from += ((long)bt[key / p.page_size] * p.page_size + key % p.page_size) * row_width + d;
+            copy_16(into + j * ld + d, from, there);
+        }
+        copies_end();
+    };
+    ask(key_begin, 0);
+    for (int u = tid; u < LATENT_MMA_ROWS * (row_width / 4); u += 256) {
+        const int r = u / (row_width / 4), d = (u % (row_width / 4)) * 4;
+        float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (r < n_rows) x = *reinterpret_cast<const float4*>(p.q_eff + (row0 + r) * row_width + d);
+        uint2 t[3];
+        three_terms(x.x, x.y, t[0].x, t[1].x, t[2].x);
+        three_terms(x.z, x.w, t[0].y, t[1].y, t[2].y);
+#pragma unroll
+        for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(q_terms + (i * LATENT_MMA_ROWS + r) * ld + d) = t[i];
+    }
+    int my_pos[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) my_pos[h] = position0 + (first + min(quarter * 16 + h * 8 + g, n_rows - 1)) / p.heads;
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, o[RANK / 8][4];
+#pragma unroll
+    for (int j = 0; j < RANK / 8; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+    const float scale_log2 = p.scale * 1.4426950408889634f;                       // exp(x) = 2^(x log2 e)
+    int buffer = 0;
+    for (int k0 = key_begin; k0 < key_end; k0 += LATENT_MMA_KEYS, buffer ^= 1) {
+        // (the other buffer was left by every warp before the barrier that ended the last round)
+        if (k0 + LATENT_MMA_KEYS < key_end) ask(k0 + LATENT_MMA_KEYS, buffer ^ 1);
+        else copies_end();
+        copies_landed<1>();
+        __syncthreads();                                                          // (the queries' terms are written, too)
+        const bf16* kt = rows_of + (buffer * LATENT_MMA_KEYS + half * 32) * ld;
+        const int key0 = k0 + half * 32;
+        if (__any_sync(0xffffffffu, key0 <= max(my_pos[0], my_pos[1]))) {         // (else no row of the warp sees these keys yet)
+            float s[4][4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
+            const bf16* q_at = q_terms + (quarter * 16 + (lane & 15)) * ld + (lane >> 4) * 8;
+            const bf16* k_at = kt + ((lane & 7) + ((lane >> 4) & 1) * 8) * ld + ((lane >> 3) & 1) * 8;
+#pragma unroll 2
+            for (int k = 0; k < row_width; k += 16) {
+                uint32_t b0[4], b1[4];
+                load_blocks(b0, k_at + k);
+                load_blocks(b1, k_at + 16 * ld + k);
+#pragma unroll
+                for (int i = 2; i >= 0; i--) {                                    // the small terms first
+                    uint32_t a[4];
+                    load_blocks(a, q_at + i * LATENT_MMA_ROWS * ld + k);
+                    mma_tile(s[0], a, b0[0], b0[1]);
+                    mma_tile(s[1], a, b0[2], b0[3]);
+                    mma_tile(s[2], a, b1[0], b1[1]);
+                    mma_tile(s[3], a, b1[2], b1[3]);
+                }
+            }
+            float corr[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float top = -INFINITY;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        const int key = key0 + j * 8 + 2 * tq + e;
+                        const bool seen = key <= my_pos[h] && (p.window <= 0 || key > my_pos[h] - p.window);
+                        float& x = s[j][2 * h + e];
+                        x = seen ? x * scale_log2 : -INFINITY;
+                        top = fmaxf(top, x);
+                    }
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+                top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+                const float m_new = fmaxf(m[h], top), from = m_new == -INFINITY ? 0.0f : m_new;
+                corr[h] = exp2f(m[h] - from);
+                float sum = 0.0f;
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        s[j][2 * h + e] = exp2f(s[j][2 * h + e] - from);
+                        sum += s[j][2 * h + e];
+                    }
+                l[h] = l[h] * corr[h] + sum;                                      // this thread's share of the row
+                m[h] = m_new;
+            }
+            if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
+#pragma unroll
+                for (int j = 0; j < RANK / 8; j++) o[j][0] *= corr[0], o[j][1] *= corr[0], o[j][2] *= corr[1], o[j][3] *= corr[1];
+            }
+            const bf16* v_at = kt + ((lane & 7) + ((lane >> 3) & 1) * 8) * ld + ((lane >> 4) & 1) * 8;
+#pragma unroll
+            for (int k = 0; k < 2; k++) {
+                uint32_t a[3][4];
+                three_terms(s[2 * k][0], s[2 * k][1], a[0][0], a[1][0], a[2][0]);
+                three_terms(s[2 * k][2], s[2 * k][3], a[0][1], a[1][1], a[2][1]);
+                three_terms(s[2 * k + 1][0], s[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
+                three_terms(s[2 * k + 1][2], s[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+                for (int j = 0; j < RANK / 8; j += 2) {
+                    uint32_t b[4];
+                    load_blocks_turned(b, v_at + k * 16 * ld + j * 8);
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        mma_tile(o[j], a[i], b[0], b[1]);
+                        mma_tile(o[j + 1], a[i], b[2], b[3]);
+                    }
+                }
+            }
+        }
+        __syncthreads();
+    }
+    copies_landed<0>();
+    // the second half's states go through shared memory (the queries' terms are used up) to the first half's warps
+    float* other = reinterpret_cast<float*>(latent_shared) + (quarter * 32 + lane) * (RANK / 2 + 4 + 4);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    }
+    if (half == 1) {
+#pragma unroll
+        for (int j = 0; j < RANK / 8; j++) *reinterpret_cast<float4*>(other + 4 * j) = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+        *reinterpret_cast<float4*>(other + RANK / 2) = make_float4(m[0], m[1], l[0], l[1]);
+    }
+    __syncthreads();
+    if (half == 1) return;
+    const float4 state = *reinterpret_cast<const float4*>(other + RANK / 2);
+    const float m_other[2] = {state.x, state.y}, l_other[2] = {state.z, state.w};
+    float mine[2], theirs[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const float big = fmaxf(m[h], m_other[h]);
+        mine[h] = exp2f(m[h] - big), theirs[h] = exp2f(m_other[h] - big);
+        const int r = quarter * 16 + h * 8 + g;
+        const long pair = row0 + min(r, n_rows - 1);
+        const float open = p.gate != nullptr ? gate_open(p.gate[pair / p.heads * p.ld_gate + pair % p.heads]) : 1.0f;
+        const float inv = open / (l[h] * mine[h] + l_other[h] * theirs[h]);
+        mine[h] *= inv, theirs[h] *= inv;
+    }
+#pragma unroll
+    for (int j = 0; j < RANK / 8; j++) {
+        const float4 x = *reinterpret_cast<const float4*>(other + 4 * j);
+        const float y[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = quarter * 16 + h * 8 + g;
+            if (r >= n_rows) continue;
+            const float a = o[j][2 * h] * mine[h] + y[2 * h] * theirs[h], b = o[j][2 * h + 1] * mine[h] + y[2 * h + 1] * theirs[h];
+            const long at = (row0 + r) * RANK + j * 8 + 2 * tq;
+            if (p.out_bf16) *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<bf16*>(p.out) + at) = __floats2bfloat162_rn(a, b);
+            else *reinterpret_cast<float2*>(reinterpret_cast<float*>(p.out) + at) = make_float2(a, b);
+        }
+    }
+}
+
+static size_t latent_mma_shared(int row_width) { return sizeof(bf16) * (size_t)(3 * LATENT_MMA_ROWS + 2 * LATENT_MMA_KEYS) * (row_width + 8); }
+
+// Whole 16-byte pieces of a row and of a latent the accumulators are made for; the shared memory holds rows of up to 336 entries.
+static bool latent_mma_takes(const LatentTiledParams& p, int dtype) {
+    const int row_width = p.rank + p.rot;
+    return dtype == DT_BF16 && p.tiles != nullptr && (p.rank == 128 || p.rank == 256) && row_width % 16 == 0 &&
+           latent_mma_shared(row_width) <= 220 * 1024 && (reinterpret_cast<uintptr_t>(p.pages) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(p.q_eff) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+}
+
+template <int RANK>
+static int launch_latent_mma(const LatentTiledParams& p, int n_units, cudaStream_t s) {
+    const size_t shared = latent_mma_shared(p.rank + p.rot);
+    if (cudaFuncSetAttribute(latent_attention_mma_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess)
+        return fail("latent_attention: the tiles' shared memory was refused");
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, latent_attention_mma_kernel<RANK>, dim3(n_units * (128 * p.heads / LATENT_MMA_ROWS)), dim3(256),
+                  shared, s, p);
+    return check_launch("latent_attention_mma_kernel");
+}
+
 // The parts of a (token, head) into one result, in the order of the parts.
 __global__ void latent_merge_kernel(void* __restrict__ out, int out_bf16, const float* __restrict__ part_out,
                                     const float* __restrict__ part_ml, int parts, int rank, int heads,
@@ -1229,6 +1442,8 @@ extern "C" int mllm_sequence_latent_attention_tiled(const LatentTiledParams* par
     if (p.tiles == nullptr && p.TQ != 1) return fail("latent_attention_tiled: single tokens come one per block");
     if (p.parts < 1 || p.parts > 32 || (p.parts > 1 && (p.tiles != nullptr || p.part_out == nullptr || p.part_ml == nullptr)))
         return fail("latent_attention_tiled: parts are for single tokens and need scratch");
+    if (latent_mma_takes(p, dtype))
+        return p.rank == 128 ? launch_latent_mma<128>(p, n_units, (cudaStream_t)stream) : launch_latent_mma<256>(p, n_units, (cudaStream_t)stream);
     const int element_bytes = dtype == DT_F32 ? 4 : 2;
     // prompt portions take 64 keys a block where two such blocks, or one, fit beside the queries
     int keys = 32;

@@ -185,3 +185,30 @@ def test_capped_attention_in_tensor_core_tiles(heads, kv_heads, dim, vdim, windo
         ops.capped_attention(out, q, k_pages, v_pages, table.cuda(), positions, items, heads, kv_heads, dim, vdim, page, dim ** -0.5, tiled=tiled, **how)
     # both keep scores, weights and sums in 32 bits, so they may differ by the last rounding to 8 bits: 2^-8 of values below 4
     np.testing.assert_allclose(f64(got), f64(want), rtol=2 ** -7, atol=2 ** -10)
+
+
+@pytest.mark.parametrize("heads, rank, rot, window, gated", [(1, 128, 0, 0, False), (3, 128, 64, 50, True), (12, 256, 32, 0, False), (5, 256, 80, 1, True)])
+@pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
+def test_latent_attention_in_tensor_core_tiles(heads, rank, rot, window, gated, out_dtype):
+    """bfloat16 pages: portions that end inside a tile of 64 pairs and of 64 keys, against one block per (token, head)."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(heads + rank)
+    page, lengths, new, row = 8, [331, 9, 64], [260, 9, 1], rank + rot
+    blocks = [-(-n // page) for n in lengths]
+    table = torch.zeros(3, max(blocks), dtype=torch.int32)
+    order = rng.permutation(sum(blocks))
+    for i, count in enumerate(blocks):
+        table[i, :count] = torch.tensor(order[sum(blocks[:i]):sum(blocks[:i]) + count])
+    pages = dev(rng.normal(size=(sum(blocks), page, 1, row)), torch.bfloat16)
+    starts, offsets = [n - m for n, m in zip(lengths, new)], [0, 260, 269]
+    positions = dev(np.concatenate([np.arange(s, l) for s, l in zip(starts, lengths)]).astype(np.int32))
+    items, n = dev(np.repeat(np.arange(3), new).astype(np.int32)), sum(new)
+    q = dev(rng.normal(size=(n, heads * row)) * 0.7, torch.float32)
+    gate = dev(rng.normal(size=(n, heads)), torch.float32) if gated else None
+    want, got = torch.empty(n, heads * rank, device="cuda"), torch.full((n, heads * rank), float("nan"), dtype=out_dtype, device="cuda")
+    ops.latent_attention_plain(want, q, pages, table.cuda(), positions, items, heads, rank, rot, page, 0.1, window=window, gate=gate)
+    tiles, _, _ = ops.attention_tiles(offsets, new, starts)
+    ops.latent_attention_tiled(got, q, pages, table.cuda(), positions, items, heads, rank, rot, page, 0.1,
+                               tiles=dev(np.array(tiles, dtype=np.int32)), n_tiles=len(tiles), window=window, gate=gate)
+    # queries and weights keep all 24 bits and sums are 32-bit; a result of 16 bits is rounded once
+    np.testing.assert_allclose(f64(got), f64(want), rtol=2 ** -8 if out_dtype == torch.bfloat16 else 2e-5, atol=3e-5)
