@@ -331,52 +331,72 @@ linear_float_rows_kernel(float* __restrict__ out, const float* __restrict__ a, c
     }
 }
 
-// 32-bit operands, more rows: tiles of 64 x 64 by 256 threads, 4 x 4 sums a thread out of two 16-byte reads of shared
-// memory per step of K, the next 32 entries of K in registers while these are multiplied.  Where the tiles are fewer than
-// the SMs a cluster of 2, 4 or 8 blocks shares a tile's K: every block leaves its sums in its shared memory, and block r
-// finishes rows r * 64 / blocks and up, adding the parts in block order (the order is the tile's, never timing).
-// 240 x 768 x 768: 278 us with the kernel above on 48 blocks; scalar FMA either way.
-constexpr int FLOAT_TILE = 64, FLOAT_K = 32, FLOAT_LD = FLOAT_TILE + 4;
-__global__ void __launch_bounds__(256)
-linear_float_tile_kernel(float* __restrict__ out, const float* __restrict__ a, const float* __restrict__ w,
+// 32-bit operands, more rows: tiles of BM x 64 by 128 threads, BM / 16 x 8 sums a thread out of 16-byte reads of shared memory
+// (a step of K of 128 rows: 64 FMAs for 16 values read), the next step's values and the next 16 entries of K in registers while
+// these are multiplied.  Where the tiles are fewer than the SMs a cluster of 2, 4 or 8 blocks shares a tile's K: every
+// block leaves its sums in its shared memory, and block r finishes rows r * BM / blocks and up, adding the parts in block order
+// (the order is the tile's, never timing).  Scalar FMA.
+// 256 rows: 35 us at 768 x 768 (73 as tiles of 64 rows launched early, 41 launched late), 38 at 2,304 x 768.
+constexpr int FLOAT_BN = 64, FLOAT_K = 16;
+template <int BM>
+__global__ void __launch_bounds__(128)
+linear_float_tile_kernel(float* __restrict__ out, const float* a, const float* __restrict__ w,
                          const float* __restrict__ bias, int M, int N, int K, long lda, long ldo, int epilogue, int per_block) {
-    __shared__ __align__(16) float staged[2][2][FLOAT_K][FLOAT_LD];       // [buffer][a, w][k][row]
+    constexpr int TM = BM / 16, LDA = BM + 4, LDW = FLOAT_BN + 4, LDS = FLOAT_BN + 4;
+    constexpr int STAGED = 2 * FLOAT_K * (LDA + LDW), SUMS = BM * LDS;
+    __shared__ __align__(16) float staged[STAGED > SUMS ? STAGED : SUMS];     // [buffer][k][row] of a, then of w; the sums at the end
     dependents_may_start();
     wait_for_earlier_kernels();
-    a = behind_the_wait(a);
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * FLOAT_TILE, n0 = blockIdx.x * FLOAT_TILE;
+    const int tid = threadIdx.x, tx = tid & 7, ty = tid >> 3;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * FLOAT_BN;
     const int blocks = gridDim.z, rank = blockIdx.z;
     const int k_begin = rank * per_block, k_end = min(K, k_begin + per_block);
-    const int row = threadIdx.x >> 2, quad = threadIdx.x & 3;             // what this thread copies: 4 + 4 entries of one row each
-    const bool a_there = m0 + row < M, w_there = n0 + row < N;
-    const float* a_row = a + (long)(a_there ? m0 + row : 0) * lda;
-    const float* w_row = w + (long)(w_there ? n0 + row : 0) * K;
+    // what this thread copies of 16 entries of K: four of them (a quad) of rows row, row + 32, ...
+    const int row = tid >> 2, quad = (tid & 3) * 4;
+    constexpr int AR = BM / 32, WR = FLOAT_BN / 32;
     const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float4 ra[2], rw[2];
+    float4 ra[AR], rw[WR];
     auto fetch = [&](int k0) {
+        const int k = k0 + quad;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int k = k0 + (quad + 4 * i) * 4;
-            ra[i] = a_there && k < k_end ? *reinterpret_cast<const float4*>(a_row + k) : none;
-            rw[i] = w_there && k < k_end ? __ldg(reinterpret_cast<const float4*>(w_row + k)) : none;
+        for (int i = 0; i < AR; i++) {
+            const int r = m0 + row + 32 * i;
+            ra[i] = r < M && k < k_end ? *reinterpret_cast<const float4*>(a + (long)r * lda + k) : none;
+        }
+#pragma unroll
+        for (int i = 0; i < WR; i++) {
+            const int r = n0 + row + 32 * i;
+            rw[i] = r < N && k < k_end ? __ldg(reinterpret_cast<const float4*>(w + (long)r * K + k)) : none;
         }
     };
     auto stage = [&](int buffer) {
+        float* as = staged + buffer * FLOAT_K * LDA;
+        float* ws = staged + 2 * FLOAT_K * LDA + buffer * FLOAT_K * LDW;
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-            const int k = (quad + 4 * i) * 4;
-            staged[buffer][0][k][row] = ra[i].x; staged[buffer][0][k + 1][row] = ra[i].y;
-            staged[buffer][0][k + 2][row] = ra[i].z; staged[buffer][0][k + 3][row] = ra[i].w;
-            staged[buffer][1][k][row] = rw[i].x; staged[buffer][1][k + 1][row] = rw[i].y;
-            staged[buffer][1][k + 2][row] = rw[i].z; staged[buffer][1][k + 3][row] = rw[i].w;
+        for (int i = 0; i < AR; i++) {
+            float* to = as + quad * LDA + row + 32 * i;
+            to[0] = ra[i].x; to[LDA] = ra[i].y; to[2 * LDA] = ra[i].z; to[3 * LDA] = ra[i].w;
+        }
+#pragma unroll
+        for (int i = 0; i < WR; i++) {
+            float* to = ws + quad * LDW + row + 32 * i;
+            to[0] = rw[i].x; to[LDW] = rw[i].y; to[2 * LDW] = rw[i].z; to[3 * LDW] = rw[i].w;
         }
     };
-    float acc[4][4];
+    // a thread's rows: 4 ty .. and (of 128) 64 + 4 ty ..; its columns: 4 tx .. and 32 + 4 tx ..
+    float acc[TM][8];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < TM; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+        for (int j = 0; j < 8; j++) acc[i][j] = 0.0f;
+    auto load = [&](int buffer, int kk, float (&x)[TM], float (&y)[8]) {
+        const float* as = staged + (buffer * FLOAT_K + kk) * LDA;
+        const float* ws = staged + 2 * FLOAT_K * LDA + (buffer * FLOAT_K + kk) * LDW;
+#pragma unroll
+        for (int i = 0; i < TM / 4; i++) *reinterpret_cast<float4*>(x + 4 * i) = *reinterpret_cast<const float4*>(as + 64 * i + 4 * ty);
+#pragma unroll
+        for (int j = 0; j < 2; j++) *reinterpret_cast<float4*>(y + 4 * j) = *reinterpret_cast<const float4*>(ws + 32 * j + 4 * tx);
+    };
     if (k_begin < k_end) {
         fetch(k_begin);
         stage(0);
@@ -386,15 +406,15 @@ linear_float_tile_kernel(float* __restrict__ out, const float* __restrict__ a, c
     for (int k0 = k_begin; k0 < k_end; k0 += FLOAT_K) {
         const bool more = k0 + FLOAT_K < k_end;
         if (more) fetch(k0 + FLOAT_K);
-#pragma unroll 8
+        alignas(16) float x[2][TM], y[2][8];
+        load(buffer, 0, x[0], y[0]);
+#pragma unroll
         for (int kk = 0; kk < FLOAT_K; kk++) {
-            const float4 x = *reinterpret_cast<const float4*>(&staged[buffer][0][kk][ty * 4]);
-            const float4 y = *reinterpret_cast<const float4*>(&staged[buffer][1][kk][tx * 4]);
-            const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+            if (kk + 1 < FLOAT_K) load(buffer, kk + 1, x[(kk + 1) & 1], y[(kk + 1) & 1]);
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xs[i], ys[j], acc[i][j]);
+                for (int j = 0; j < 8; j++) acc[i][j] = fmaf(x[kk & 1][i], y[kk & 1][j], acc[i][j]);
         }
         if (more) stage(buffer ^ 1);           // the other buffer: every thread left it before the barrier below, a trip ago
         __syncthreads();
@@ -408,25 +428,40 @@ linear_float_tile_kernel(float* __restrict__ out, const float* __restrict__ a, c
     };
     if (blocks == 1) {
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < TM; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) finish(m0 + ty * 4 + i, n0 + tx * 4 + j, acc[i][j]);
+            for (int j = 0; j < 8; j++) finish(m0 + i / 4 * 64 + 4 * ty + i % 4, n0 + j / 4 * 32 + 4 * tx + j % 4, acc[i][j]);
         return;
     }
-    float* sums = &staged[0][0][0][0];                                    // [64][68]: 17 KB of the 34
 #pragma unroll
-    for (int i = 0; i < 4; i++)
-        *reinterpret_cast<float4*>(sums + (ty * 4 + i) * FLOAT_LD + tx * 4) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+    for (int i = 0; i < TM; i++)
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+            *reinterpret_cast<float4*>(staged + (i / 4 * 64 + 4 * ty + i % 4) * LDS + j / 4 * 32 + 4 * tx) =
+                make_float4(acc[i][j], acc[i][j + 1], acc[i][j + 2], acc[i][j + 3]);
     cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
     cluster.sync();
-    const int mine = FLOAT_TILE / blocks;
-    for (int i = threadIdx.x; i < mine * FLOAT_TILE; i += 256) {
-        const int r = rank * mine + i / FLOAT_TILE, c = i % FLOAT_TILE;
+    const int mine = BM / blocks;
+    for (int i = tid; i < mine * FLOAT_BN; i += 128) {
+        const int r = rank * mine + i / FLOAT_BN, c = i % FLOAT_BN;
         float v = 0.0f;
-        for (int b = 0; b < blocks; b++) v += cluster.map_shared_rank(sums, b)[r * FLOAT_LD + c];
+        for (int b = 0; b < blocks; b++) v += cluster.map_shared_rank(staged, b)[r * LDS + c];
         finish(m0 + r, n0 + c, v);
     }
     cluster.sync();                                                       // no block leaves while another reads its sums
+}
+
+template <int BM>
+static int launch_float_tiles(float* out, const float* a, const float* w, const float* bias, int M, int N, int K, long lda, long ldo,
+                              int epilogue, cudaStream_t s) {
+    const dim3 tiles((N + FLOAT_BN - 1) / FLOAT_BN, (M + BM - 1) / BM);
+    // blocks that share a tile's K: while they stay within three to an SM and each has 64 entries of K or more
+    int blocks = 1;
+    while (blocks < 8 && (long)tiles.x * tiles.y * blocks * 2 <= 444 && K >= blocks * 2 * 64) blocks *= 2;
+    const int per_block = ((K + blocks - 1) / blocks + FLOAT_K - 1) / FLOAT_K * FLOAT_K;
+    return launched(launch_kernel_in_clusters(AFTER_THE_KERNELS_AHEAD, blocks > 1 ? dim3(1, 1, blocks) : dim3(0, 1, 1),
+                                              linear_float_tile_kernel<BM>, dim3(tiles.x, tiles.y, blocks), dim3(128), 0, s, out, a, w, bias, M,
+                                              N, K, lda, ldo, epilogue, per_block), "linear_float_tile_kernel");
 }
 
 template <int MT, int F>
@@ -465,14 +500,8 @@ static int launch_linear_float(float* out, const float* a, const float* w, const
         return FLOAT_ROWS(8);
 #undef FLOAT_ROWS
     }
-    const dim3 tiles((N + FLOAT_TILE - 1) / FLOAT_TILE, (M + FLOAT_TILE - 1) / FLOAT_TILE);
-    // blocks that share a tile's K: while they stay within two to an SM and each has two steps of K or more
-    int blocks = 1;
-    while (blocks < 8 && (long)tiles.x * tiles.y * blocks * 2 <= 296 && K >= blocks * 2 * 2 * FLOAT_K) blocks *= 2;
-    const int per_block = ((K + blocks - 1) / blocks + FLOAT_K - 1) / FLOAT_K * FLOAT_K;
-    return launched(launch_kernel_in_clusters(g_dependent_launch != 0, blocks > 1 ? dim3(1, 1, blocks) : dim3(0, 1, 1),
-                                              linear_float_tile_kernel, dim3(tiles.x, tiles.y, blocks), dim3(256), 0, s, out, a, w, bias, M,
-                                              N, K, lda, ldo, epilogue, per_block), "linear_float_tile_kernel");
+    return M <= 64 ? launch_float_tiles<64>(out, a, w, bias, M, N, K, lda, ldo, epilogue, s)
+                   : launch_float_tiles<128>(out, a, w, bias, M, N, K, lda, ldo, epilogue, s);
 }
 
 template <typename AT, typename WT, typename OT>
