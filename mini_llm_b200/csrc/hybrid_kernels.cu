@@ -1814,205 +1814,6 @@ expert_down_kernel(float* __restrict__ hidden, long ld_hidden, const T* __restri
     }
 }
 
-// gu: [T, 2 * total] = [gates of all experts | ups of all experts]; act: [T, total].  Columns
-// [e * inner, (e + 1) * inner) belong to routed expert e, columns from n_experts * inner on to the
-// shared expert (pair index `top` of every token, if there is one).
-// (VEC: a thread takes the 16 bytes of columns that lie side by side, all of one expert: inner sizes that are
-// multiples of a vector's elements.  The token's weights per expert lie in shared memory, 0 for an expert it
-// did not choose, whose columns are written as zeros without reading the products.)
-// (EXPERT_RELU_SQUARED: experts without a gate matrix; gu holds the ups alone, [T, total], and act is the square of relu.
-// With `identity_weight` the block's share of the token's columns of `hidden` also gets identity_weight[t] * x[t]:
-// set to it with `assign`, else added.)
-template <typename T, bool VEC, int FORM>
-__global__ void __launch_bounds__(256)
-expert_combine_kernel(T* __restrict__ act, long ld_act, const T* __restrict__ gu, long ld_gu, const int* __restrict__ choice,
-                      const float* __restrict__ in_weight, const float* __restrict__ out_weight, int n_experts, int inner,
-                      int total, int top, int pairs, float* __restrict__ hidden, long ld_hidden, const T* __restrict__ x,
-                      long ld_x, const float* __restrict__ identity_weight, int width, int assign, float limit,
-                      float shared_limit, float alpha) {
-    constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
-    dependents_may_start();
-    wait_for_earlier_kernels();
-    extern __shared__ float weights[];             // [n_experts + 1][2]: input weight, output weight
-    const int t = blockIdx.x;
-    for (int e = threadIdx.x; e <= n_experts; e += blockDim.x) {
-        float s = 0.0f, o = 1.0f;
-        if (e == n_experts) {
-            if (pairs > top) s = in_weight[(long)t * pairs + top], o = out_weight[(long)t * pairs + top];
-        } else {
-            for (int k = 0; k < top; k++)
-                if (choice[(long)t * pairs + k] == e) s = in_weight[(long)t * pairs + k], o = out_weight[(long)t * pairs + k];
-        }
-        weights[2 * e] = s, weights[2 * e + 1] = o;
-    }
-    __syncthreads();
-    constexpr int N = VEC ? Vec16<T>::N : 1;
-    const T* row = gu + (long)t * ld_gu;
-    T* dst = act + (long)t * ld_act;
-    for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * N; c < total; c += gridDim.y * blockDim.x * N) {
-        const int e = c < n_experts * inner ? c / inner : n_experts;
-        const float s = weights[2 * e], o = weights[2 * e + 1];
-        const float most = e == n_experts ? shared_limit : limit;
-        if (VEC) {
-            uint4 packed = make_uint4(0u, 0u, 0u, 0u);
-            if (s != 0.0f) {
-                float g[N], u[N];
-                if (GATED) Vec16<T>::load(row + c, g);
-                Vec16<T>::load(row + (GATED ? total : 0) + c, u);
-                T* lanes = reinterpret_cast<T*>(&packed);
-#pragma unroll
-                for (int i = 0; i < N; i++)
-                    lanes[i] = from_f32<T>(expert_form<FORM>(GATED ? s * g[i] : 0.0f, s * u[i], most, alpha) * o);
-            }
-            *reinterpret_cast<uint4*>(dst + c) = packed;
-        } else {
-            float v = 0.0f;
-            if (s != 0.0f)
-                v = expert_form<FORM>(GATED ? s * to_f32(row[c]) : 0.0f, s * to_f32(row[(GATED ? total : 0) + c]), most, alpha) * o;
-            dst[c] = from_f32<T>(v);
-        }
-    }
-    if (identity_weight != nullptr) {
-        const float passed = identity_weight[t];
-        if (assign || passed != 0.0f)
-            for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
-                const float v = passed * to_f32(x[(long)t * ld_x + c]);
-                float* h = hidden + (long)t * ld_hidden + c;
-                *h = assign ? v : *h + v;
-            }
-    }
-}
-
-extern "C" int mllm_hybrid_expert_combine(void* act, long ld_act, const void* gu, long ld_gu, const int* choice,
-                                          const float* in_weight, const float* out_weight, int n_experts, int inner, int total,
-                                          int top, int pairs, int form, float limit, float shared_limit, float alpha, float* hidden, long ld_hidden, const void* x, long ld_x,
-                                          const float* identity_weight, int width, int assign, int n_tokens, int dtype,
-                                          void* stream) {
-    if (n_tokens <= 0) return 0;
-    if (dtype != DT_F32 && dtype != DT_BF16) return fail("expert_combine: unknown dtype");
-    cudaStream_t s = (cudaStream_t)stream;
-    const int n = dtype == DT_F32 ? 4 : 8;
-    const bool vec = inner % n == 0 && total % n == 0 && ld_act % n == 0 && ld_gu % n == 0 && aligned_host(act) && aligned_host(gu);
-    const int per_block = 256 * (vec ? n : 1);
-    int y = (total + per_block - 1) / per_block;
-    if (y > 64) y = 64;
-    dim3 grid(n_tokens, y);
-    const size_t shared = sizeof(float) * 2 * ((size_t)n_experts + 1);
-    if (shared > 48 * 1024) return fail("expert_combine: too many experts for the table of weights");
-    if (form < EXPERT_GATED_SILU || form > EXPERT_CLAMPED_GLU) return fail("expert_combine: unknown form of an expert");
-#define RUN(T, VEC, FORM)                                                                                                       \
-    launch_kernel(g_dependent_launch != 0, expert_combine_kernel<T, VEC, FORM>, grid, dim3(256), shared, s, (T*)act, ld_act,    \
-                  (const T*)gu, ld_gu, choice, in_weight, out_weight, n_experts, inner, total, top, pairs, hidden, ld_hidden,    \
-                  (const T*)x, ld_x, identity_weight, width, assign, limit, shared_limit, alpha)
-#define PICK(T, VEC)                                                                                                            \
-    do {                                                                                                                        \
-        if (form == EXPERT_GATED_SILU) RUN(T, VEC, EXPERT_GATED_SILU);                                                          \
-        else if (form == EXPERT_RELU_SQUARED) RUN(T, VEC, EXPERT_RELU_SQUARED);                                                 \
-        else RUN(T, VEC, EXPERT_CLAMPED_GLU);                                                                                   \
-    } while (0)
-#define RUN_AS(T)                                                                                                               \
-    do {                                                                                                                        \
-        if (vec) PICK(T, true);                                                                                                 \
-        else PICK(T, false);                                                                                                    \
-    } while (0)
-    if (dtype == DT_F32) RUN_AS(float);
-    else RUN_AS(bf16);
-#undef RUN_AS
-#undef PICK
-#undef RUN
-    return check_launch("expert_combine_kernel");
-}
-
-extern "C" int mllm_hybrid_route(const void* x, long ld_x, const void* router, const float* router_bias, const float* correction,
-                                 const void* shared_gate, int shared_plain, int rule, float scale, int width, int n_outputs,
-                                 int n_identity, int groups, int keep_groups, int top, int* choice, float* in_weight,
-                                 float* out_weight, float* identity_weight, int n_tokens, int dtype, void* stream) {
-    if (n_tokens <= 0) return 0;
-    if (top <= 0 || top > n_outputs) return fail("route: every token takes between one and all experts");
-    if (shared_plain && shared_gate != nullptr) return fail("route: the shared expert has a gate or none");
-    if (rule < ROUTE_SIGMOID_ON_INPUT || rule > ROUTE_SIGMOID) return fail("route: unknown rule");
-    if (groups < 0 || (groups > 0 && (n_outputs % groups != 0 || keep_groups < 1 || keep_groups > groups || keep_groups * (n_outputs / groups) < top)))
-        return fail("route: equal groups of experts, and enough of them kept to choose from");
-    if (n_identity < 0 || n_identity > n_outputs) return fail("route: more identity experts than experts");
-    if (n_identity > 0 && (identity_weight == nullptr || rule == ROUTE_SIGMOID_ON_INPUT))
-        return fail("route: identity experts need weights on the outputs and room for the token's sum of them");
-    cudaStream_t s = (cudaStream_t)stream;
-    const int pairs = top + (shared_gate != nullptr || shared_plain ? 1 : 0);
-    const size_t one = sizeof(float) * ((size_t)width + 2 * (size_t)n_outputs + 1 + (size_t)groups);
-    if (one > 48 * 1024) return fail("route: the token and the scores do not fit shared memory");
-    const bool four = n_tokens >= 512 && 4 * one <= 48 * 1024;
-    // a warp for every output in steps of few tokens, four to sixteen of them
-    const int warps = four ? 8 : (n_tokens >= 512 || n_outputs <= 4 ? 4 : (n_outputs < 16 ? n_outputs : 16));
-#define RUN(T, TOKENS)                                                                                                          \
-    launch_kernel(g_dependent_launch != 0, route_kernel<T, TOKENS>, dim3((n_tokens + TOKENS - 1) / TOKENS), dim3(32 * warps),   \
-                  TOKENS * one, s, (const T*)x, ld_x, (const T*)router, router_bias, correction, (const T*)shared_gate,         \
-                  shared_plain, rule, scale, width, n_outputs, n_identity, groups, keep_groups, top, pairs, n_tokens, choice,  \
-                  in_weight, out_weight, identity_weight)
-    if (dtype == DT_F32) { if (four) RUN(float, 4); else RUN(float, 1); }
-    else if (dtype == DT_BF16) { if (four) RUN(bf16, 4); else RUN(bf16, 1); }
-    else return fail("route: unknown dtype");
-#undef RUN
-    return check_launch("route_kernel");
-}
-
-// (form: an ExpertForm, with its constants; EXPERT_RELU_SQUARED has no gate matrices; expert `n_experts` is the shared one;
-// identity_weight: see expert_down)
-extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, long ld_act, const void* x, long ld_x,
-                                   const int* choice, const float* in_weight, const float* out_weight,
-                                   const long long* gate_of, const long long* up_of, const long long* down_of,
-                                   const int* inner_of, long ld_down, int max_inner, int width, int pairs,
-                                   const float* identity_weight, int form, float limit, float shared_limit, float alpha,
-                                   int n_experts, int n_tokens, int assign, int n_tables, int dtype, void* stream) {
-    if (n_tokens <= 0) return 0;
-    if (form < EXPERT_GATED_SILU || form > EXPERT_CLAMPED_GLU || (form != EXPERT_RELU_SQUARED && gate_of == nullptr))
-        return fail("experts: unknown form of an expert, or one without its gate matrices");
-    cudaStream_t s = (cudaStream_t)stream;
-    const size_t shared = sizeof(float) * (size_t)width;
-    if (shared > 48 * 1024) return fail("experts: the token does not fit shared memory");
-    constexpr int F = 4, C = 2;
-    dim3 up_grid(n_tokens * pairs, (max_inner + 8 * F - 1) / (8 * F)), down_grid(n_tokens, (width + 8 * C - 1) / (8 * C));
-    if (up_grid.y > 65535 || down_grid.y > 65535) return fail("experts: the sizes are too large for one launch");
-#define UP(T, FORM)                                                                                                             \
-    launch_kernel(g_dependent_launch != 0, expert_up_kernel<T, FORM, F>, up_grid, dim3(256), shared, s, (T*)act, ld_act,        \
-                  (const T*)x, ld_x, choice, in_weight, gate_of, up_of, inner_of, width, pairs, limit, shared_limit, alpha, n_experts)
-#define RUN(T)                                                                                                                  \
-    do {                                                                                                                        \
-        if (form == EXPERT_GATED_SILU) UP(T, EXPERT_GATED_SILU);                                                                \
-        else if (form == EXPERT_RELU_SQUARED) UP(T, EXPERT_RELU_SQUARED);                                                       \
-        else UP(T, EXPERT_CLAMPED_GLU);                                                                                         \
-        launch_kernel(g_dependent_launch != 0, expert_down_kernel<T, C>, down_grid, dim3(256), 0, s, hidden, ld_hidden,         \
-                      (const T*)act, ld_act, choice, out_weight, down_of, inner_of, ld_down, width, pairs, assign, (const T*)x, \
-                      ld_x, identity_weight);                                                                                   \
-    } while (0)
-    if (dtype == DT_F32) RUN(float);
-    else if (dtype == DT_BF16) RUN(bf16);
-    else return fail("experts: unknown dtype");
-#undef RUN
-#undef UP
-    return check_launch("expert kernels");
-}
-
-// ---------------------------------------------------------------------------
-// x[r, c] += a * u[r, c] + b * v[r, c]  (32-bit; v may be null; with `assign` x is set to the sum instead)
-// ---------------------------------------------------------------------------
-__global__ void scaled_add_kernel(float* __restrict__ x, const float* __restrict__ u, float a, const float* __restrict__ v,
-                                  float b, long n, int assign) {
-    dependents_may_start();
-    wait_for_earlier_kernels();
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        float sum = a * u[i];
-        if (v != nullptr) sum = fmaf(b, v[i], sum);
-        x[i] = assign ? sum : x[i] + sum;
-    }
-}
-
-extern "C" int mllm_hybrid_scaled_add(float* x, const float* u, float a, const float* v, float b, long n, int assign, void* stream) {
-    if (n <= 0) return 0;
-    long blocks = (n + 255) / 256;
-    if (blocks > 4096) blocks = 4096;
-    launch_kernel(g_dependent_launch != 0, scaled_add_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, x, u, a, v, b, n, assign);
-    return check_launch("scaled_add_kernel");
-}
 // ---- the pairs of few tokens, by expert ----------------------------------------------------------
 // Up to EXPERT_TILE_TOKENS tokens, bfloat16, inner sizes and the width multiples of 8: the pairs of one expert are the rows of
 // mma.sync tiles (m16n8k16, as the few-row products), so that an expert's weights cross the chip once however many tokens
@@ -2259,6 +2060,161 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
     }
 }
 
+// gu: [T, 2 * total] = [gates of all experts | ups of all experts]; act: [T, total].  Columns
+// [e * inner, (e + 1) * inner) belong to routed expert e, columns from n_experts * inner on to the
+// shared expert (pair index `top` of every token, if there is one).
+// (VEC: a thread takes the 16 bytes of columns that lie side by side, all of one expert: inner sizes that are
+// multiples of a vector's elements.  The token's weights per expert lie in shared memory, 0 for an expert it
+// did not choose, whose columns are written as zeros without reading the products.)
+// (EXPERT_RELU_SQUARED: experts without a gate matrix; gu holds the ups alone, [T, total], and act is the square of relu.
+// With `identity_weight` the block's share of the token's columns of `hidden` also gets identity_weight[t] * x[t]:
+// set to it with `assign`, else added.)
+template <typename T, bool VEC, int FORM>
+__global__ void __launch_bounds__(256)
+expert_combine_kernel(T* __restrict__ act, long ld_act, const T* __restrict__ gu, long ld_gu, const int* __restrict__ choice,
+                      const float* __restrict__ in_weight, const float* __restrict__ out_weight, int n_experts, int inner,
+                      int total, int top, int pairs, float* __restrict__ hidden, long ld_hidden, const T* __restrict__ x,
+                      long ld_x, const float* __restrict__ identity_weight, int width, int assign, float limit,
+                      float shared_limit, float alpha) {
+    constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    extern __shared__ float weights[];             // [n_experts + 1][2]: input weight, output weight
+    const int t = blockIdx.x;
+    for (int e = threadIdx.x; e <= n_experts; e += blockDim.x) {
+        float s = 0.0f, o = 1.0f;
+        if (e == n_experts) {
+            if (pairs > top) s = in_weight[(long)t * pairs + top], o = out_weight[(long)t * pairs + top];
+        } else {
+            for (int k = 0; k < top; k++)
+                if (choice[(long)t * pairs + k] == e) s = in_weight[(long)t * pairs + k], o = out_weight[(long)t * pairs + k];
+        }
+        weights[2 * e] = s, weights[2 * e + 1] = o;
+    }
+    __syncthreads();
+    constexpr int N = VEC ? Vec16<T>::N : 1;
+    const T* row = gu + (long)t * ld_gu;
+    T* dst = act + (long)t * ld_act;
+    for (int c = (blockIdx.y * blockDim.x + threadIdx.x) * N; c < total; c += gridDim.y * blockDim.x * N) {
+        const int e = c < n_experts * inner ? c / inner : n_experts;
+        const float s = weights[2 * e], o = weights[2 * e + 1];
+        const float most = e == n_experts ? shared_limit : limit;
+        if (VEC) {
+            uint4 packed = make_uint4(0u, 0u, 0u, 0u);
+            if (s != 0.0f) {
+                float g[N], u[N];
+                if (GATED) Vec16<T>::load(row + c, g);
+                Vec16<T>::load(row + (GATED ? total : 0) + c, u);
+                T* lanes = reinterpret_cast<T*>(&packed);
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    lanes[i] = from_f32<T>(expert_form<FORM>(GATED ? s * g[i] : 0.0f, s * u[i], most, alpha) * o);
+            }
+            *reinterpret_cast<uint4*>(dst + c) = packed;
+        } else {
+            float v = 0.0f;
+            if (s != 0.0f)
+                v = expert_form<FORM>(GATED ? s * to_f32(row[c]) : 0.0f, s * to_f32(row[(GATED ? total : 0) + c]), most, alpha) * o;
+            dst[c] = from_f32<T>(v);
+        }
+    }
+    if (identity_weight != nullptr) {
+        const float passed = identity_weight[t];
+        if (assign || passed != 0.0f)
+            for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < width; c += gridDim.y * blockDim.x) {
+                const float v = passed * to_f32(x[(long)t * ld_x + c]);
+                float* h = hidden + (long)t * ld_hidden + c;
+                *h = assign ? v : *h + v;
+            }
+    }
+}
+
+extern "C" int mllm_hybrid_expert_combine(void* act, long ld_act, const void* gu, long ld_gu, const int* choice,
+                                          const float* in_weight, const float* out_weight, int n_experts, int inner, int total,
+                                          int top, int pairs, int form, float limit, float shared_limit, float alpha, float* hidden, long ld_hidden, const void* x, long ld_x,
+                                          const float* identity_weight, int width, int assign, int n_tokens, int dtype,
+                                          void* stream) {
+    if (n_tokens <= 0) return 0;
+    if (dtype != DT_F32 && dtype != DT_BF16) return fail("expert_combine: unknown dtype");
+    cudaStream_t s = (cudaStream_t)stream;
+    const int n = dtype == DT_F32 ? 4 : 8;
+    const bool vec = inner % n == 0 && total % n == 0 && ld_act % n == 0 && ld_gu % n == 0 && aligned_host(act) && aligned_host(gu);
+    const int per_block = 256 * (vec ? n : 1);
+    int y = (total + per_block - 1) / per_block;
+    if (y > 64) y = 64;
+    dim3 grid(n_tokens, y);
+    const size_t shared = sizeof(float) * 2 * ((size_t)n_experts + 1);
+    if (shared > 48 * 1024) return fail("expert_combine: too many experts for the table of weights");
+    if (form < EXPERT_GATED_SILU || form > EXPERT_CLAMPED_GLU) return fail("expert_combine: unknown form of an expert");
+#define RUN(T, VEC, FORM)                                                                                                       \
+    launch_kernel(g_dependent_launch != 0, expert_combine_kernel<T, VEC, FORM>, grid, dim3(256), shared, s, (T*)act, ld_act,    \
+                  (const T*)gu, ld_gu, choice, in_weight, out_weight, n_experts, inner, total, top, pairs, hidden, ld_hidden,    \
+                  (const T*)x, ld_x, identity_weight, width, assign, limit, shared_limit, alpha)
+#define PICK(T, VEC)                                                                                                            \
+    do {                                                                                                                        \
+        if (form == EXPERT_GATED_SILU) RUN(T, VEC, EXPERT_GATED_SILU);                                                          \
+        else if (form == EXPERT_RELU_SQUARED) RUN(T, VEC, EXPERT_RELU_SQUARED);                                                 \
+        else RUN(T, VEC, EXPERT_CLAMPED_GLU);                                                                                   \
+    } while (0)
+#define RUN_AS(T)                                                                                                               \
+    do {                                                                                                                        \
+        if (vec) PICK(T, true);                                                                                                 \
+        else PICK(T, false);                                                                                                    \
+    } while (0)
+    if (dtype == DT_F32) RUN_AS(float);
+    else RUN_AS(bf16);
+#undef RUN_AS
+#undef PICK
+#undef RUN
+    return check_launch("expert_combine_kernel");
+}
+
+extern "C" int mllm_hybrid_route(const void* x, long ld_x, const void* router, const float* router_bias, const float* correction,
+                                 const void* shared_gate, int shared_plain, int rule, float scale, int width, int n_outputs,
+                                 int n_identity, int groups, int keep_groups, int top, int* choice, float* in_weight,
+                                 float* out_weight, float* identity_weight, int n_tokens, int dtype, void* stream) {
+    if (n_tokens <= 0) return 0;
+    if (top <= 0 || top > n_outputs) return fail("route: every token takes between one and all experts");
+    if (shared_plain && shared_gate != nullptr) return fail("route: the shared expert has a gate or none");
+    if (rule < ROUTE_SIGMOID_ON_INPUT || rule > ROUTE_SIGMOID) return fail("route: unknown rule");
+    if (groups < 0 || (groups > 0 && (n_outputs % groups != 0 || keep_groups < 1 || keep_groups > groups || keep_groups * (n_outputs / groups) < top)))
+        return fail("route: equal groups of experts, and enough of them kept to choose from");
+    if (n_identity < 0 || n_identity > n_outputs) return fail("route: more identity experts than experts");
+    if (n_identity > 0 && (identity_weight == nullptr || rule == ROUTE_SIGMOID_ON_INPUT))
+        return fail("route: identity experts need weights on the outputs and room for the token's sum of them");
+    cudaStream_t s = (cudaStream_t)stream;
+    const int pairs = top + (shared_gate != nullptr || shared_plain ? 1 : 0);
+    const size_t one = sizeof(float) * ((size_t)width + 2 * (size_t)n_outputs + 1 + (size_t)groups);
+    if (one > 48 * 1024) return fail("route: the token and the scores do not fit shared memory");
+    const bool four = n_tokens >= 512 && 4 * one <= 48 * 1024;
+    // a warp for every output in steps of few tokens, four to sixteen of them
+    const int warps = four ? 8 : (n_tokens >= 512 || n_outputs <= 4 ? 4 : (n_outputs < 16 ? n_outputs : 16));
+#define RUN(T, TOKENS)                                                                                                          \
+    launch_kernel(g_dependent_launch != 0, route_kernel<T, TOKENS>, dim3((n_tokens + TOKENS - 1) / TOKENS), dim3(32 * warps),   \
+                  TOKENS * one, s, (const T*)x, ld_x, (const T*)router, router_bias, correction, (const T*)shared_gate,         \
+                  shared_plain, rule, scale, width, n_outputs, n_identity, groups, keep_groups, top, pairs, n_tokens, choice,  \
+                  in_weight, out_weight, identity_weight)
+    if (dtype == DT_F32) { if (four) RUN(float, 4); else RUN(float, 1); }
+    else if (dtype == DT_BF16) { if (four) RUN(bf16, 4); else RUN(bf16, 1); }
+    else return fail("route: unknown dtype");
+#undef RUN
+    return check_launch("route_kernel");
+}
+
+// (form: an ExpertForm, with its constants; EXPERT_RELU_SQUARED has no gate matrices; expert `n_experts` is the shared one;
+// identity_weight: see expert_down)
+extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, long ld_act, const void* x, long ld_x,
+                                   const int* choice, const float* in_weight, const float* out_weight,
+                                   const long long* gate_of, const long long* up_of, const long long* down_of,
+                                   const int* inner_of, long ld_down, int max_inner, int width, int pairs,
+                                   const float* identity_weight, int form, float limit, float shared_limit, float alpha,
+                                   int n_experts, int n_tokens, int assign, int n_tables, int dtype, void* stream) {
+    if (n_tokens <= 0) return 0;
+    if (form < EXPERT_GATED_SILU || form > EXPERT_CLAMPED_GLU || (form != EXPERT_RELU_SQUARED && gate_of == nullptr))
+        return fail("experts: unknown form of an expert, or one without its gate matrices");
+    cudaStream_t s = (cudaStream_t)stream;
+    const size_t shared = sizeof(float) * (size_t)width;
+    if (shared > 48 * 1024) return fail("experts: the token does not fit shared memory");
     if (n_tables > 0) {
         // the caller's word that every inner size is a multiple of 8; what else the tiles need is looked at here
         auto on_16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
@@ -2288,3 +2244,47 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
                       ld_x, identity_weight);
         return check_launch("expert tiles");
     }
+    constexpr int F = 4, C = 2;
+    dim3 up_grid(n_tokens * pairs, (max_inner + 8 * F - 1) / (8 * F)), down_grid(n_tokens, (width + 8 * C - 1) / (8 * C));
+    if (up_grid.y > 65535 || down_grid.y > 65535) return fail("experts: the sizes are too large for one launch");
+#define UP(T, FORM)                                                                                                             \
+    launch_kernel(g_dependent_launch != 0, expert_up_kernel<T, FORM, F>, up_grid, dim3(256), shared, s, (T*)act, ld_act,        \
+                  (const T*)x, ld_x, choice, in_weight, gate_of, up_of, inner_of, width, pairs, limit, shared_limit, alpha, n_experts)
+#define RUN(T)                                                                                                                  \
+    do {                                                                                                                        \
+        if (form == EXPERT_GATED_SILU) UP(T, EXPERT_GATED_SILU);                                                                \
+        else if (form == EXPERT_RELU_SQUARED) UP(T, EXPERT_RELU_SQUARED);                                                       \
+        else UP(T, EXPERT_CLAMPED_GLU);                                                                                         \
+        launch_kernel(g_dependent_launch != 0, expert_down_kernel<T, C>, down_grid, dim3(256), 0, s, hidden, ld_hidden,         \
+                      (const T*)act, ld_act, choice, out_weight, down_of, inner_of, ld_down, width, pairs, assign, (const T*)x, \
+                      ld_x, identity_weight);                                                                                   \
+    } while (0)
+    if (dtype == DT_F32) RUN(float);
+    else if (dtype == DT_BF16) RUN(bf16);
+    else return fail("experts: unknown dtype");
+#undef RUN
+#undef UP
+    return check_launch("expert kernels");
+}
+
+// ---------------------------------------------------------------------------
+// x[r, c] += a * u[r, c] + b * v[r, c]  (32-bit; v may be null; with `assign` x is set to the sum instead)
+// ---------------------------------------------------------------------------
+__global__ void scaled_add_kernel(float* __restrict__ x, const float* __restrict__ u, float a, const float* __restrict__ v,
+                                  float b, long n, int assign) {
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+        float sum = a * u[i];
+        if (v != nullptr) sum = fmaf(b, v[i], sum);
+        x[i] = assign ? sum : x[i] + sum;
+    }
+}
+
+extern "C" int mllm_hybrid_scaled_add(float* x, const float* u, float a, const float* v, float b, long n, int assign, void* stream) {
+    if (n <= 0) return 0;
+    long blocks = (n + 255) / 256;
+    if (blocks > 4096) blocks = 4096;
+    launch_kernel(g_dependent_launch != 0, scaled_add_kernel, dim3((unsigned)blocks), dim3(256), 0, (cudaStream_t)stream, x, u, a, v, b, n, assign);
+    return check_launch("scaled_add_kernel");
+}
