@@ -751,17 +751,20 @@ capped_attention_block_kernel(T* __restrict__ out, long ld_out, const T* __restr
 }
 
 // ---------------------------------------------------------------------------
-// The same attention on tensor-core tiles, bfloat16, keys and values of up to 128 entries (multiples of 8).  A block of four
-// warps takes 64 (token, head) rows of one key/value head, a warp 16 of them, and walks the keys 64 at a time, keys and
-// values copied a tile ahead.  Scores are products of bfloat16 operands with 32-bit sums; the weights stay 32-bit: each goes into the
+// The same attention on tensor-core tiles, bfloat16, keys and values of up to 128 entries (multiples of 8).  A block of eight
+// warps takes 64 (token, head) rows of one key/value head and walks the keys 64 at a time, keys and values copied a tile ahead;
+// warp w has rows 16 (w % 4) .. and keys 32 (w / 4) .. of every tile, and the two warps of a row group are merged at the end (four warps
+// with all 64 keys left a scheduler one warp, whose products, exponentials and exchanges then stood one behind the other).  Scores are products of bfloat16 operands with 32-bit sums; the weights stay 32-bit: each goes into the
 // second product as three bfloat16 terms, which hold all 24 bits of it, against the values as they are.  Maxima, sums,
 // weights and results are 32-bit in the rows' threads, four threads a row; cap, slopes, masks, sink and gate as above.
 // The products no longer bound it: a tile of 16 x 64 takes 128 of them (KEY 64, VALUE 64) against 32,768 FMAs of the
 // register tiles, and the exponentials and masks stand beside them.
-// Three prompts of 640 to 2,048 tokens (12 heads over 4, sizes 64): 169 us a launch on register tiles, 115 here.
+// Three prompts of 640, 1,200 and 2,048 tokens (12 heads over 4, sizes 64, capped): 480 us a launch on register tiles, 175 here (four warps 210).
+// A tile's product is added with a rounded FMA: left in the tensor cores' accumulators, whose sums are cut off, the error against 64 bits
+// was twice the register tiles'; so it is two thirds of theirs.
 // ---------------------------------------------------------------------------
 template <int KEY, int VALUE>          // entries of a key and of a value: 64 or 128, zeros past dim and vdim
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256, KEY + VALUE == 128 ? 2 : 1)
 capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, long ld_q, const bf16* k_pages, const bf16* v_pages,
                             const int* block_table, int max_blocks, const int* positions, const int* token_item, int n_tokens,
                             int n_heads, int n_kv_heads, int dim, int vdim, int page_size, float scale, float cap, int window, int chunk,
@@ -776,6 +779,7 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
     dependents_may_start();
     wait_for_earlier_kernels();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int quarter = warp & 3, half = warp >> 2;
     const int group = n_heads / n_kv_heads, chunks = (group + heads_per_block - 1) / heads_per_block;
     const int hk = blockIdx.y / chunks, first_head = hk * group + (blockIdx.y % chunks) * heads_per_block;
     const int n_heads_here = min(heads_per_block, hk * group + group - first_head);
@@ -788,7 +792,7 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
         row_pos[tid] = token >= 0 ? positions[token] : -1;
         row_item[tid] = token >= 0 ? token_item[token] : -1;
     }
-    for (int u = tid; u < 64 * (KEY / 8); u += 128) {
+    for (int u = tid; u < 64 * (KEY / 8); u += 256) {
         const int r = u / (KEY / 8), d = (u % (KEY / 8)) * 8;
         const bool there = r < n_rows && d < dim;
         const bf16* from = there ? q + (long)(first_token + r / n_heads_here) * ld_q + (long)(first_head + r % n_heads_here) * dim + d : q;
@@ -799,12 +803,12 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
     __syncthreads();
     uint32_t qa[KEY / 16][4];
 #pragma unroll
-    for (int k = 0; k < KEY / 16; k++) load_blocks(qa[k], q_rows + (warp * 16 + (lane & 15)) * LDK + k * 16 + (lane >> 4) * 8);
+    for (int k = 0; k < KEY / 16; k++) load_blocks(qa[k], q_rows + (quarter * 16 + (lane & 15)) * LDK + k * 16 + (lane >> 4) * 8);
     int my_pos[2], my_item[2], my_first[2];
     float my_slope[2], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f}, o[VALUE / 8][4];
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-        const int r = warp * 16 + h * 8 + g;
+        const int r = quarter * 16 + h * 8 + g;
         my_pos[h] = row_pos[r], my_item[h] = row_item[r], my_first[h] = first_visible(my_pos[h], window, chunk);
         my_slope[h] = r < n_rows && slopes != nullptr ? slopes[first_head + r % n_heads_here] : 0.0f;
     }
@@ -824,7 +828,7 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
         auto ask = [&](int base, int buffer) {
             bf16* into_k = keys + buffer * KEYS * LDK;
             bf16* into_v = values + buffer * KEYS * LDV;
-            for (int u = tid; u < KEYS * (KEY / 8 + VALUE / 8); u += 128) {
+            for (int u = tid; u < KEYS * (KEY / 8 + VALUE / 8); u += 256) {
                 const bool value = u >= KEYS * (KEY / 8);
                 const int v = value ? u - KEYS * (KEY / 8) : u, pieces = value ? VALUE / 8 : KEY / 8;
                 const int j = v / pieces, d = (v % pieces) * 8, kp = base + j, size = value ? vdim : dim;
@@ -849,24 +853,25 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
             else copies_end();
             copies_landed<1>();
             __syncthreads();
+            const int key0 = base + half * 32;
             bool any = false;
 #pragma unroll
             for (int h = 0; h < 2; h++)
-                any = any || (my_item[h] == item && base <= my_pos[h] && (base + KEYS > my_first[h] || base < keep));
+                any = any || (my_item[h] == item && key0 <= my_pos[h] && (key0 + 32 > my_first[h] || key0 < keep));
             if (__any_sync(0xffffffffu, any)) {
-                const bf16* kt = keys + buffer * KEYS * LDK;
-                const bf16* vt = values + buffer * KEYS * LDV;
-                float s[8][4];
+                const bf16* kt = keys + (buffer * KEYS + half * 32) * LDK;
+                const bf16* vt = values + (buffer * KEYS + half * 32) * LDV;
+                float s[4][4];
 #pragma unroll
-                for (int j = 0; j < 8; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
+                for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
 #pragma unroll
                 for (int k = 0; k < KEY / 16; k++)
 #pragma unroll
-                    for (int j = 0; j < 8; j += 2) {
+                    for (int j = 0; j < 4; j += 2) {
                         uint32_t b[4];
                         load_blocks(b, kt + (j * 8 + (lane & 7) + ((lane >> 4) & 1) * 8) * LDK + k * 16 + ((lane >> 3) & 1) * 8);
-                        mma_tile(s[j], qa[k], b[0], b[1]);
-                        mma_tile(s[j + 1], qa[k], b[2], b[3]);
+                        mma_added(s[j], qa[k], b[0], b[1]);
+                        mma_added(s[j + 1], qa[k], b[2], b[3]);
                     }
                 float corr[2];
 #pragma unroll
@@ -874,10 +879,10 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
                     const bool row_here = my_item[h] == item;
                     float top = -INFINITY;
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
+                    for (int j = 0; j < 4; j++)
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
-                            const int pos = base + j * 8 + 2 * tq + e;
+                            const int pos = key0 + j * 8 + 2 * tq + e;
                             const bool seen = row_here && pos <= my_pos[h] && key_visible(pos, my_first[h], keep);
                             float& x = s[j][2 * h + e];
                             x = seen ? capped(x * scale, cap, inv_cap) - my_slope[h] * (float)(my_pos[h] - pos) : -INFINITY;
@@ -889,7 +894,7 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
                     corr[h] = expf(m[h] - from);
                     float sum = 0.0f;
 #pragma unroll
-                    for (int j = 0; j < 8; j++)
+                    for (int j = 0; j < 4; j++)
 #pragma unroll
                         for (int e = 0; e < 2; e++) {
                             s[j][2 * h + e] = expf(s[j][2 * h + e] - from);
@@ -898,26 +903,21 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
                     l[h] = l[h] * corr[h] + sum;             // this thread's share of the row
                     m[h] = m_new;
                 }
-                if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
+                uint32_t a[2][3][4];
 #pragma unroll
-                    for (int j = 0; j < VALUE / 8; j++) o[j][0] *= corr[0], o[j][1] *= corr[0], o[j][2] *= corr[1], o[j][3] *= corr[1];
-                }
+                for (int k = 0; k < 2; k++) terms_of(a[k], s[2 * k], s[2 * k + 1]);
 #pragma unroll
-                for (int k = 0; k < KEYS / 16; k++) {
-                    uint32_t a[3][4];
-                    three_terms(s[2 * k][0], s[2 * k][1], a[0][0], a[1][0], a[2][0]);
-                    three_terms(s[2 * k][2], s[2 * k][3], a[0][1], a[1][1], a[2][1]);
-                    three_terms(s[2 * k + 1][0], s[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
-                    three_terms(s[2 * k + 1][2], s[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+                for (int j = 0; j < VALUE / 8; j += 2) {
+                    uint32_t b[2][4];
+                    float x[2][4];
 #pragma unroll
-                    for (int j = 0; j < VALUE / 8; j += 2) {
-                        uint32_t b[4];
-                        load_blocks_turned(b, vt + (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + j * 8 + ((lane >> 4) & 1) * 8);
+                    for (int k = 0; k < 2; k++)
+                        load_blocks_turned(b[k], vt + (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + j * 8 + ((lane >> 4) & 1) * 8);
+                    weighted_rows(x, a, b);
 #pragma unroll
-                        for (int t = 0; t < 3; t++) {
-                            mma_tile(o[j], a[t], b[0], b[1]);
-                            mma_tile(o[j + 1], a[t], b[2], b[3]);
-                        }
+                    for (int e = 0; e < 4; e++) {
+                        o[j][e] = fmaf(o[j][e], corr[e >> 1], x[0][e]);
+                        o[j + 1][e] = fmaf(o[j + 1][e], corr[e >> 1], x[1][e]);
                     }
                 }
             }
@@ -926,12 +926,42 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
         copies_landed<0>();
         run_first = run_last + 1;
     }
+    // the second half's states go through shared memory (the tiles are used up) to the first half's warps
+    float* other = reinterpret_cast<float*>(mma_shared) + (quarter * 32 + lane) * (VALUE / 2 + 8);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+        l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    }
+    if (half == 1) {
+#pragma unroll
+        for (int j = 0; j < VALUE / 8; j++) *reinterpret_cast<float4*>(other + 4 * j) = make_float4(o[j][0], o[j][1], o[j][2], o[j][3]);
+        *reinterpret_cast<float4*>(other + VALUE / 2) = make_float4(m[0], m[1], l[0], l[1]);
+    }
+    __syncthreads();
+    if (half == 1) return;
+    {
+        const float4 state = *reinterpret_cast<const float4*>(other + VALUE / 2);
+        const float m_other[2] = {state.x, state.y}, l_other[2] = {state.z, state.w};
+        float mine[2], theirs[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const float big = fmaxf(m[h], m_other[h]), from = big == -INFINITY ? 0.0f : big;
+            mine[h] = expf(m[h] - from), theirs[h] = expf(m_other[h] - from);
+            l[h] = fmaf(l[h], mine[h], l_other[h] * theirs[h]);
+            m[h] = big;
+        }
+#pragma unroll
+        for (int j = 0; j < VALUE / 8; j++) {
+            const float4 x = *reinterpret_cast<const float4*>(other + 4 * j);
+            o[j][0] = fmaf(o[j][0], mine[0], x.x * theirs[0]), o[j][1] = fmaf(o[j][1], mine[0], x.y * theirs[0]);
+            o[j][2] = fmaf(o[j][2], mine[1], x.z * theirs[1]), o[j][3] = fmaf(o[j][3], mine[1], x.w * theirs[1]);
+        }
+    }
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         float sum = l[h];
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const int r = warp * 16 + h * 8 + g;
+        const int r = quarter * 16 + h * 8 + g;
         if (r >= n_rows) continue;
         const int token = first_token + r / n_heads_here, head = first_head + r % n_heads_here;
         float shrink = 1.0f;
@@ -1054,7 +1084,7 @@ static int launch_capped_attention(bool tiled, void* out, long ld_out, const voi
             return fail("capped_attention: the tiles' shared memory was refused");                                               \
         cudaFuncSetAttribute(capped_attention_mma_kernel<KEY, VALUE>, cudaFuncAttributePreferredSharedMemoryCarveout,             \
                              cudaSharedmemCarveoutMaxShared);                                                                     \
-        launch_kernel(AFTER_THE_KERNELS_AHEAD, capped_attention_mma_kernel<KEY, VALUE>, grid, dim3(128), shared, s, (bf16*)out, ld_out,  \
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, capped_attention_mma_kernel<KEY, VALUE>, grid, dim3(256), shared, s, (bf16*)out, ld_out,  \
                       (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks, positions, token_item, \
                       n_tokens, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, chunk, keep, gate, ld_gate, gate_wide, sink, \
                       slopes, tokens_per_block, heads_per_block);                                                                 \

@@ -43,3 +43,33 @@ __device__ __forceinline__ void three_terms(float x, float y, uint32_t& first, u
     t = __floats2bfloat162_rn(x, y);
     third = *reinterpret_cast<uint32_t*>(&t);
 }
+
+// The accumulators of two tiles, 16 rows by 16, as the first operand of the next product.
+__device__ __forceinline__ void terms_of(uint32_t (&a)[3][4], const float (&x)[4], const float (&y)[4]) {
+    three_terms(x[0], x[1], a[0][0], a[1][0], a[2][0]);
+    three_terms(x[2], x[3], a[0][1], a[1][1], a[2][1]);
+    three_terms(y[0], y[1], a[0][2], a[1][2], a[2][2]);
+    three_terms(y[2], y[3], a[0][3], a[1][3], a[2][3]);
+}
+
+// A tile's sum is cut off at 24 bits when it is added to what the accumulators held: over a long row of products that adds up.
+// The product by itself, added with a rounded addition, keeps a sum as near as a chain of FMAs does.
+__device__ __forceinline__ void mma_added(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    mma_tile(x, a, b0, b1);
+#pragma unroll
+    for (int e = 0; e < 4; e++) c[e] += x[e];
+}
+
+// x = the weights of 16 rows and 32 keys, as three terms, times two tiles of eight value columns: the small terms first.
+__device__ __forceinline__ void weighted_rows(float (&x)[2][4], const uint32_t (&a)[2][3][4], const uint32_t (&b)[2][4]) {
+#pragma unroll
+    for (int e = 0; e < 8; e++) x[e / 4][e % 4] = 0.0f;
+#pragma unroll
+    for (int term = 2; term >= 0; term--)
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            mma_tile(x[0], a[k][term], b[k][0], b[k][1]);
+            mma_tile(x[1], a[k][term], b[k][2], b[k][3]);
+        }
+}

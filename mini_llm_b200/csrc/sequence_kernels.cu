@@ -1164,7 +1164,9 @@ latent_attention_tiled_kernel(LatentTiledParams p) {
 // product as three bfloat16 terms that hold all its 24 bits, the cached rows are bfloat16 as they are, sums are 32-bit.
 // A tile of 64 x 64 pairs is 3,264 m16n8k16 products (latent 256, row 288); as 32-bit FMAs, 2.2 million of them, with a quarter of a load
 // from shared memory each, it was what the step waited for.
-// Three prompts of 640 to 2,048 tokens, 12 heads over a latent of 256: 550 us a launch then, 134 now.
+// Every 16 entries of a row and every tile's product are added with rounded additions: left in the tensor cores' accumulators, whose
+// sums are cut off, the error against 64 bits was 2.1e-6 (FMAs 7.0e-7); so it is 2.5e-7.  Three prompts of 640, 1,200 and 2,048 tokens, 12 heads
+// over a latent of 256: 2,330 us a launch then, 500 now; the products bound it (22 cycles each on a scheduler).
 // ---------------------------------------------------------------------------
 constexpr int LATENT_MMA_ROWS = 64, LATENT_MMA_KEYS = 64;
 
@@ -1234,20 +1236,23 @@ latent_attention_mma_kernel(LatentTiledParams p) {
             for (int j = 0; j < 4; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0f;
             const bf16* q_at = q_terms + (quarter * 16 + (lane & 15)) * ld + (lane >> 4) * 8;
             const bf16* k_at = kt + ((lane & 7) + ((lane >> 4) & 1) * 8) * ld + ((lane >> 3) & 1) * 8;
-#pragma unroll 2
+#pragma unroll 1
             for (int k = 0; k < row_width; k += 16) {
                 uint32_t b0[4], b1[4];
+                float x[4][4] = {};
                 load_blocks(b0, k_at + k);
                 load_blocks(b1, k_at + 16 * ld + k);
 #pragma unroll
                 for (int i = 2; i >= 0; i--) {                                    // the small terms first
                     uint32_t a[4];
                     load_blocks(a, q_at + i * LATENT_MMA_ROWS * ld + k);
-                    mma_tile(s[0], a, b0[0], b0[1]);
-                    mma_tile(s[1], a, b0[2], b0[3]);
-                    mma_tile(s[2], a, b1[0], b1[1]);
-                    mma_tile(s[3], a, b1[2], b1[3]);
+                    mma_tile(x[0], a, b0[0], b0[1]);
+                    mma_tile(x[1], a, b0[2], b0[3]);
+                    mma_tile(x[2], a, b1[0], b1[1]);
+                    mma_tile(x[3], a, b1[2], b1[3]);
                 }
+#pragma unroll
+                for (int e = 0; e < 16; e++) s[e / 4][e % 4] += x[e / 4][e % 4];  // (rounded, not cut off)
             }
             float corr[2];
 #pragma unroll
@@ -1278,27 +1283,21 @@ latent_attention_mma_kernel(LatentTiledParams p) {
                 l[h] = l[h] * corr[h] + sum;                                      // this thread's share of the row
                 m[h] = m_new;
             }
-            if (__any_sync(0xffffffffu, corr[0] != 1.0f || corr[1] != 1.0f)) {
-#pragma unroll
-                for (int j = 0; j < RANK / 8; j++) o[j][0] *= corr[0], o[j][1] *= corr[0], o[j][2] *= corr[1], o[j][3] *= corr[1];
-            }
             const bf16* v_at = kt + ((lane & 7) + ((lane >> 3) & 1) * 8) * ld + ((lane >> 4) & 1) * 8;
+            uint32_t a[2][3][4];
 #pragma unroll
-            for (int k = 0; k < 2; k++) {
-                uint32_t a[3][4];
-                three_terms(s[2 * k][0], s[2 * k][1], a[0][0], a[1][0], a[2][0]);
-                three_terms(s[2 * k][2], s[2 * k][3], a[0][1], a[1][1], a[2][1]);
-                three_terms(s[2 * k + 1][0], s[2 * k + 1][1], a[0][2], a[1][2], a[2][2]);
-                three_terms(s[2 * k + 1][2], s[2 * k + 1][3], a[0][3], a[1][3], a[2][3]);
+            for (int k = 0; k < 2; k++) terms_of(a[k], s[2 * k], s[2 * k + 1]);
 #pragma unroll
-                for (int j = 0; j < RANK / 8; j += 2) {
-                    uint32_t b[4];
-                    load_blocks_turned(b, v_at + k * 16 * ld + j * 8);
+            for (int j = 0; j < RANK / 8; j += 2) {
+                uint32_t b[2][4];
+                float x[2][4];
 #pragma unroll
-                    for (int i = 0; i < 3; i++) {
-                        mma_tile(o[j], a[i], b[0], b[1]);
-                        mma_tile(o[j + 1], a[i], b[2], b[3]);
-                    }
+                for (int k = 0; k < 2; k++) load_blocks_turned(b[k], v_at + k * 16 * ld + j * 8);
+                weighted_rows(x, a, b);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    o[j][e] = fmaf(o[j][e], corr[e >> 1], x[0][e]);
+                    o[j + 1][e] = fmaf(o[j + 1][e], corr[e >> 1], x[1][e]);
                 }
             }
         }
