@@ -1428,6 +1428,376 @@ static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStr
     return check_launch("linear_recurrence_kernel");
 }
 
+// ---- prompt portions, 16 tokens at a time --------------------------------------------------------
+// bfloat16 rows, one decay per head.  The walk above is a chain of one token after the other; over a chunk of 16 tokens the
+// same sums are products of small matrices.  With S the state before the chunk, G(t) the product of the decays up to token t, R(t, s) that of
+// the decays after s up to t, and k, q normed:
+//   delta rule:  M u = b (v - G S^T k),  M(t, s) = b_t R(t, s) (k_t . k_s) below a diagonal of ones  (else u = b v)
+//   out_t = G(t) S^T q_t + sum over s <= t of R(t, s) (q_t . k_s) u_s (+ skip v_t)
+//   S <- G(15) S + sum over s of R(15, s) k_s u_s^T
+// A block takes 16 columns of a head's state, transposed, in the accumulators of four warps, a quarter of the key entries each: as
+// the first operand of the next product the accumulators of m16n8k16 tiles need no exchange.  Those warps are the chain; what does not read the
+// state is prepared by six more while the chunk before is worked on: four bring the rows and take k . k and q . k, one solves
+// M T = 1 row by row, one makes the gates and the products of the decays (as products: no difference of logarithms).  Decays, S, u, T and
+// every sum are 32-bit: 32-bit operands enter a product as three bfloat16 terms that hold all their bits, the rows are bfloat16 as they
+// come and their norms are factors of the sums.  T is bounded: with |k| = 1 and b <= 1 every factor of the recurrence shrinks.
+// What bounds it: issue slots (4,900 warp instructions a chunk, a quarter of them splitting operands) and the chain from S to S.  Two portions of
+// 1,024 tokens, 6 heads of 128 x 128: 513 us a launch token by token, 114 here; 24 heads of 128 x 64 without the delta rule 662 and 94.
+// Errors against 64 bits (relative, 1,000 + 777 tokens): 2.83e-7 token by token, 2.43e-7 here; without the delta rule 1.0e-7 and 8.3e-8.
+constexpr int REC_TOKENS = 16, REC_ROW_SLOTS = 6, REC_SLOTS = 4, REC_LD = 24;     // (rows of 16 terms, 48 bytes apart: no bank twice)
+
+template <int DIM> struct RecurrenceRows {
+    bf16 k[REC_TOKENS * (DIM + 8)], q[REC_TOKENS * (DIM + 8)], v[REC_TOKENS * REC_LD];
+};
+struct RecurrenceChunk {
+    bf16 solve[3][REC_TOKENS * REC_LD], read[3][REC_TOKENS * REC_LD];             // T and R (q . k), [term][t][s]
+    float below[REC_TOKENS * 20];                                                 // M below the diagonal, [s][t]
+    float rest[REC_TOKENS * 17];                                                  // R(t, s), [t][s]
+    float until[REC_TOKENS];                                                      // G(t)
+    float strength[REC_TOKENS], old_k[REC_TOKENS], old_q[REC_TOKENS], write[REC_TOKENS];      // b, b G |k|, G |q|, R(15, s) |k|
+};
+template <int DIM> struct RecurrenceShared {
+    RecurrenceRows<DIM> rows[REC_ROW_SLOTS];
+    RecurrenceChunk chunk[REC_SLOTS];
+    float4 sums[4][4][32];                                                        // [quarter][k or q, 8 tokens][lane]
+    float unit[2][REC_TOKENS];                                                    // 1 / |k|, q_scale / |q|
+};
+
+__device__ __forceinline__ void barrier_of_128(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
+
+// c = a b, both 32-bit as three terms; the products whose terms are together below 2^-24 of the largest are left out.
+__device__ __forceinline__ void mma_terms(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int half) {
+    c[0] = c[1] = c[2] = c[3] = 0.0f;
+#pragma unroll
+    for (int order = 2; order >= 1; order--)
+#pragma unroll
+        for (int i = 0; i <= order; i++) mma_tile(c, a[i], half ? b[order - i][2] : b[order - i][0], half ? b[order - i][3] : b[order - i][1]);
+    mma_added(c, a[0], half ? b[0][2] : b[0][0], half ? b[0][3] : b[0][1]);
+}
+
+template <int DIM, bool DELTA>
+__global__ void __launch_bounds__(320, 1) recurrence_chunks_kernel(RecurrenceParams pp) {
+    extern __shared__ __align__(16) unsigned char recurrence_shared[];
+    RecurrenceShared<DIM>& sh = *reinterpret_cast<RecurrenceShared<DIM>*>(recurrence_shared);
+    constexpr int LD = DIM + 8, QUARTER = DIM / 4, TILES = QUARTER / 8;
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const int item = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * 16;
+    const int count = pp.item_count[item];
+    if (count <= 0) return;
+    const long first = pp.item_offset[item];
+    const int dim = pp.dim, vdim = pp.vdim, chunks = (count + REC_TOKENS - 1) / REC_TOKENS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const long qk_at = (long)(head / (pp.heads / pp.qk_heads)) * dim, v_at = (long)head * vdim + col0;
+    float* S = pp.state + (long)pp.item_slot[item] * pp.state_stride + (long)head * dim * vdim;
+
+    // the state's warps
+    float s[TILES][4];
+    if (warp < 4) {
+#pragma unroll
+        for (int j = 0; j < TILES; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int d = warp * QUARTER + j * 8 + 2 * tq + (e & 1), c = col0 + g + 8 * (e >> 1);
+                s[j][e] = d < dim && c < vdim ? S[(long)d * vdim + c] : 0.0f;
+            }
+    }
+    const float skip = pp.skip != nullptr ? pp.skip[head] : 0.0f;
+    auto walk = [&](int i) {
+        const RecurrenceRows<DIM>& rows = sh.rows[i % REC_ROW_SLOTS];
+        const RecurrenceChunk& ch = sh.chunk[i % REC_SLOTS];
+        float sums[4][4];                                                         // S^T k of 2 x 8 tokens, S^T q
+#pragma unroll
+        for (int j = 0; j < 4; j++) sums[j][0] = sums[j][1] = sums[j][2] = sums[j][3] = 0.0f;
+        const int at = ((lane & 7) + ((lane >> 4) & 1) * 8) * LD + warp * QUARTER + ((lane >> 3) & 1) * 8;
+#pragma unroll
+        for (int j = 0; j < TILES; j += 2) {
+            uint32_t a[3][4], bk[4], bq[4];
+            float x[4][4] = {};
+            terms_of(a, s[j], s[j + 1]);
+            if (DELTA) load_blocks(bk, rows.k + at + j * 8);
+            load_blocks(bq, rows.q + at + j * 8);
+#pragma unroll
+            for (int term = 2; term >= 0; term--) {
+                if (DELTA) mma_tile(x[0], a[term], bk[0], bk[1]), mma_tile(x[1], a[term], bk[2], bk[3]);
+                mma_tile(x[2], a[term], bq[0], bq[1]), mma_tile(x[3], a[term], bq[2], bq[3]);
+            }
+#pragma unroll
+            for (int e = 0; e < 16; e++) sums[e / 4][e % 4] += x[e / 4][e % 4];
+        }
+#pragma unroll
+        for (int j = DELTA ? 0 : 2; j < 4; j++) sh.sums[warp][j][lane] = make_float4(sums[j][0], sums[j][1], sums[j][2], sums[j][3]);
+        float v[2][4], u[2][4];
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) v[j][e] = to_f32(rows.v[(j * 8 + 2 * tq + (e & 1)) * REC_LD + g + 8 * (e >> 1)]);
+        barrier_of_128(1);
+        if (DELTA) {
+            float r[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const float4 x = sh.sums[0][j][lane], y = sh.sums[1][j][lane], z = sh.sums[2][j][lane], w = sh.sums[3][j][lane];
+                const float old[4] = {(x.x + y.x) + (z.x + w.x), (x.y + y.y) + (z.y + w.y), (x.z + y.z) + (z.z + w.z), (x.w + y.w) + (z.w + w.w)};
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const int t = j * 8 + 2 * tq + (e & 1);
+                    r[j][e] = ch.strength[t] * v[j][e] - ch.old_k[t] * old[e];
+                }
+            }
+            uint32_t a[3][4], b[3][4];
+            terms_of(a, r[0], r[1]);
+#pragma unroll
+            for (int term = 0; term < 3; term++) load_blocks(b[term], ch.solve[term] + ((lane & 7) + ((lane >> 4) & 1) * 8) * REC_LD + ((lane >> 3) & 1) * 8);
+            mma_terms(u[0], a, b, 0);
+            mma_terms(u[1], a, b, 1);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) u[j][e] = ch.strength[j * 8 + 2 * tq + (e & 1)] * v[j][e];
+        }
+        // the state moves on first: it is what the next chunk waits for
+        {
+            float w[2][4];
+            uint32_t a[3][4];
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int e = 0; e < 4; e++) w[j][e] = ch.write[j * 8 + 2 * tq + (e & 1)] * u[j][e];
+            terms_of(a, w[0], w[1]);
+            const float whole = ch.until[REC_TOKENS - 1];
+#pragma unroll
+            for (int j = 0; j < TILES; j += 2) {
+                uint32_t b[4];
+                load_blocks_turned(b, rows.k + ((lane & 7) + ((lane >> 3) & 1) * 8) * LD + warp * QUARTER + j * 8 + ((lane >> 4) & 1) * 8);
+                float x[2][4] = {};
+#pragma unroll
+                for (int term = 2; term >= 0; term--) mma_tile(x[0], a[term], b[0], b[1]), mma_tile(x[1], a[term], b[2], b[3]);
+#pragma unroll
+                for (int e = 0; e < 4; e++) s[j][e] = fmaf(s[j][e], whole, x[0][e]), s[j + 1][e] = fmaf(s[j + 1][e], whole, x[1][e]);
+            }
+        }
+        if (warp < 2) {                                                           // eight tokens' results a warp
+            uint32_t a[3][4], b[3][4];
+            terms_of(a, u[0], u[1]);
+#pragma unroll
+            for (int term = 0; term < 3; term++) load_blocks(b[term], ch.read[term] + ((lane & 7) + ((lane >> 4) & 1) * 8) * REC_LD + ((lane >> 3) & 1) * 8);
+            float o[4];
+            mma_terms(o, a, b, warp);
+            const float4 x = sh.sums[0][2 + warp][lane], y = sh.sums[1][2 + warp][lane], z = sh.sums[2][2 + warp][lane], w = sh.sums[3][2 + warp][lane];
+            const float old[4] = {(x.x + y.x) + (z.x + w.x), (x.y + y.y) + (z.y + w.y), (x.z + y.z) + (z.z + w.z), (x.w + y.w) + (z.w + w.w)};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int t = warp * 8 + 2 * tq + (e & 1), c = g + 8 * (e >> 1);
+                const float value = warp == 0 ? v[0][e] : v[1][e];
+                if (i * REC_TOKENS + t < count && col0 + c < vdim)
+                    pp.out[(first + i * REC_TOKENS + t) * pp.ld_out + v_at + c] = fmaf(ch.old_q[t], old[e], o[e]) + skip * value;
+            }
+        }
+    };
+
+    // the rows' warps
+    const int p = tid - 128, rows_warp = warp - 4;
+    // (a thread's pieces of a chunk lie where those of the chunk before lay, 16 rows on)
+    constexpr int PIECES = DIM / 8, STEP = 128 / PIECES;
+    const int piece_t = p / PIECES, piece_d = p % PIECES * 8, value_t = (p >> 1) & (REC_TOKENS - 1), value_c = (p & 1) * 8;
+    const bf16* k_from = (const bf16*)pp.k + (first + piece_t) * pp.ld_k + qk_at + piece_d;
+    const bf16* q_from = (const bf16*)pp.q + (first + piece_t) * pp.ld_q + qk_at + piece_d;
+    const bf16* v_from = (const bf16*)pp.v + (first + value_t) * pp.ld_v + v_at + value_c;
+    auto bring = [&](int i) {
+        if (i < chunks) {
+            RecurrenceRows<DIM>& rows = sh.rows[i % REC_ROW_SLOTS];
+            const int n = count - i * REC_TOKENS;
+#pragma unroll
+            for (int j = 0; j < REC_TOKENS / STEP; j++) {
+                const bool there = piece_t + j * STEP < n && piece_d < dim;
+                const int to = (piece_t + j * STEP) * LD + piece_d;
+                copy_16(rows.k + to, there ? k_from + j * STEP * pp.ld_k : (const bf16*)pp.k, there);
+                copy_16(rows.q + to, there ? q_from + j * STEP * pp.ld_q : (const bf16*)pp.q, there);
+            }
+            if (p < 2 * REC_TOKENS) {
+                const bool there = value_t < n && col0 + value_c < vdim;
+                copy_16(rows.v + value_t * REC_LD + value_c, there ? v_from : (const bf16*)pp.v, there);
+            }
+            k_from += REC_TOKENS * pp.ld_k, q_from += REC_TOKENS * pp.ld_q, v_from += REC_TOKENS * pp.ld_v;
+        }
+        copies_end();
+    };
+    auto pairs = [&](int i) {
+        bring(i + 3);
+        copies_landed<3>();
+        barrier_of_128(2);                                                        // the rows of chunk i are there
+        const RecurrenceRows<DIM>& rows = sh.rows[i % REC_ROW_SLOTS];
+        RecurrenceChunk& ch = sh.chunk[i % REC_SLOTS];
+        {
+            const int row = p >> 2, t = row & (REC_TOKENS - 1);
+            const bf16* x = (row < REC_TOKENS ? rows.k : rows.q) + t * LD + (p & 3) * QUARTER;
+            float sum = 0.0f;
+            if (pp.unit_norm) {
+#pragma unroll
+                for (int d = 0; d < QUARTER; d += 8) {
+                    const uint4 eight = *reinterpret_cast<const uint4*>(x + d);
+                    const uint32_t twos[4] = {eight.x, eight.y, eight.z, eight.w};
+#pragma unroll
+                    for (int r = 0; r < 4; r++) {
+                        const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&twos[r]));
+                        sum = fmaf(f.x, f.x, fmaf(f.y, f.y, sum));
+                    }
+                }
+                sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+                sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            }
+            const float scale = row < REC_TOKENS ? 1.0f : pp.q_scale;
+            if ((p & 3) == 0) sh.unit[row >> 4][t] = pp.unit_norm ? scale / sqrtf(sum + 1e-6f) : scale;
+        }
+        // warps 0 and 1: k . k with tokens s of 0..7, 8..15; warps 2 and 3: q . k
+        const bool is_q = rows_warp >= 2;
+        float even[4] = {0.0f, 0.0f, 0.0f, 0.0f}, odd[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (DELTA || is_q) {
+            const bf16* a_at = (is_q ? rows.q : rows.k) + (lane & 15) * LD + (lane >> 4) * 8;
+            const bf16* b_at = rows.k + ((rows_warp & 1) * 8 + (lane & 7)) * LD + (lane >> 3) * 8;
+#pragma unroll
+            for (int d = 0; d < DIM; d += 32) {
+                uint32_t a[4], b[4];
+                load_blocks(b, b_at + d);
+                load_blocks(a, a_at + d);
+                mma_added(even, a, b[0], b[1]);
+                load_blocks(a, a_at + d + 16);
+                mma_added(odd, a, b[2], b[3]);
+            }
+        }
+        barrier_of_128(2);                                                        // the norms are written
+        if (DELTA || is_q) {
+            const int s0 = (rows_warp & 1) * 8 + 2 * tq;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int t = g + 8 * h;
+                const float left = sh.unit[is_q][t];
+                float x[2];
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int s_ = s0 + e;
+                    x[e] = (is_q ? s_ <= t : s_ < t) ? (even[2 * h + e] + odd[2 * h + e]) * (left * sh.unit[0][s_]) * ch.rest[t * 17 + s_] : 0.0f;
+                    if (!is_q) ch.below[s_ * 20 + t] = ch.strength[t] * x[e];
+                }
+                if (is_q) {
+                    uint32_t terms[3];
+                    three_terms(x[0], x[1], terms[0], terms[1], terms[2]);
+#pragma unroll
+                    for (int term = 0; term < 3; term++) *reinterpret_cast<uint32_t*>(ch.read[term] + t * REC_LD + s0) = terms[term];
+                }
+            }
+        }
+        if (p < REC_TOKENS) {
+            const float unit_k = sh.unit[0][p], until = ch.until[p];
+            ch.old_k[p] = ch.strength[p] * until * unit_k;
+            ch.old_q[p] = until * sh.unit[1][p];
+            ch.write[p] = ch.rest[(REC_TOKENS - 1) * 17 + p] * unit_k;
+        }
+    };
+    // T: lane l has column l mod 16
+    auto solve = [&](int i) {
+        RecurrenceChunk& ch = sh.chunk[i % REC_SLOTS];
+        const int column = lane & 15;
+        float x[REC_TOKENS];
+#pragma unroll
+        for (int t = 0; t < REC_TOKENS; t++) x[t] = t == column ? 1.0f : 0.0f;
+#pragma unroll
+        for (int s_ = 0; s_ < REC_TOKENS - 1; s_++) {
+            const float* below = ch.below + s_ * 20;
+#pragma unroll
+            for (int t4 = (s_ + 1) / 4 * 4; t4 < REC_TOKENS; t4 += 4) {
+                const float4 m = *reinterpret_cast<const float4*>(below + t4);
+                const float f[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+                    if (t4 + r > s_) x[t4 + r] = fmaf(-f[r], x[s_], x[t4 + r]);
+            }
+        }
+        if (lane < REC_TOKENS) {
+#pragma unroll
+            for (int t = 0; t < REC_TOKENS; t += 2) {
+                uint32_t terms[3];
+                three_terms(x[t], x[t + 1], terms[0], terms[1], terms[2]);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    const __nv_bfloat162 two = *reinterpret_cast<const __nv_bfloat162*>(&terms[j]);
+                    ch.solve[j][t * REC_LD + column] = two.x;
+                    ch.solve[j][(t + 1) * REC_LD + column] = two.y;
+                }
+            }
+        }
+    };
+    // the gates of a chunk, asked for a chunk ahead: a lane a token, and then a lane an s
+    const float rate = expf(pp.log_rate[head]), bias = pp.step_bias[head];
+    float raw_a = 0.0f, raw_b = 0.0f;
+    auto ask_gates = [&](int i) {
+        const int t = i * REC_TOKENS + lane;
+        if (lane < REC_TOKENS && t < count) {
+            raw_a = pp.gate_a[(first + t) * pp.ld_gate_a + head];
+            if (DELTA) raw_b = pp.gate_b[(first + t) * pp.ld_gate_b + head];
+        }
+    };
+    auto gates = [&](int i) {
+        RecurrenceChunk& ch = sh.chunk[i % REC_SLOTS];
+        const bool there = lane < REC_TOKENS && i * REC_TOKENS + lane < count;
+        const float step = softplus_f(raw_a + bias), decay = there ? expf(-rate * step) : 1.0f;
+        if (lane < REC_TOKENS) ch.strength[lane] = there ? (DELTA ? sigmoid_f(raw_b) : step) : 0.0f;
+        if (i + 1 < chunks) ask_gates(i + 1);
+        float run = 1.0f;
+#pragma unroll
+        for (int t = 0; t < REC_TOKENS; t++) {
+            const float a = __shfl_sync(0xffffffffu, decay, t);
+            if (lane == REC_TOKENS || t > lane) run *= a;
+            if (t >= lane) ch.rest[t * 17 + lane] = run;
+            if (lane == REC_TOKENS) ch.until[t] = run;
+        }
+    };
+
+    if (warp >= 4 && warp < 8)
+        for (int i = 0; i < 3; i++) bring(i);
+    if (warp == 9) ask_gates(0);
+    // chunk i's gates are made three rounds before it is walked, its pairs two, its T one
+    for (int i = -3; i < chunks; i++) {
+        if (warp < 4) {
+            if (i >= 0) walk(i);
+        } else if (warp < 8) {
+            if (i >= -2 && i + 2 < chunks) pairs(i + 2);
+        } else if (warp == 8) {
+            if (DELTA && i >= -1 && i + 1 < chunks) solve(i + 1);
+        } else if (i + 3 < chunks) gates(i + 3);
+        __syncthreads();
+    }
+    if (warp < 4 && pp.writes) {
+#pragma unroll
+        for (int j = 0; j < TILES; j++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int d = warp * QUARTER + j * 8 + 2 * tq + (e & 1), c = col0 + g + 8 * (e >> 1);
+                if (d < dim && c < vdim) S[(long)d * vdim + c] = s[j][e];
+            }
+    }
+}
+
+// Portions of bfloat16 rows in whole 16-byte pieces; the delta rule with normed keys (what bounds T).  The walk above takes 250 ns
+// a token, a chunk of 16 here 1.7 us and its first three rounds of preparation as long as one chunk more: from some 16 tokens an entry on.
+static bool recurrence_chunks_take(const RecurrenceParams& pp, int n_items, int n_tokens) {
+    auto on_16 = [](const void* x, long ld) { return ((reinterpret_cast<uintptr_t>(x) | (uintptr_t)(ld * 2)) & 15) == 0; };
+    return !pp.channel_decay && n_tokens >= 32 + 2 * n_items && pp.dim % 8 == 0 && pp.dim > 32 && pp.dim <= 128 && pp.vdim % 8 == 0 &&
+           (!pp.delta || pp.unit_norm) && on_16(pp.q, pp.ld_q) && on_16(pp.k, pp.ld_k) && on_16(pp.v, pp.ld_v);
+}
+
+template <int DIM, bool DELTA>
+static int launch_recurrence_chunks(const RecurrenceParams& pp, int n_items, cudaStream_t s) {
+    const int shared = (int)sizeof(RecurrenceShared<DIM>);
+    if (cudaFuncSetAttribute(recurrence_chunks_kernel<DIM, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, shared) != cudaSuccess)
+        return fail("linear_recurrence: the chunks' shared memory was refused");
+    const dim3 grid(n_items, pp.heads, (pp.vdim + 15) / 16);
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, recurrence_chunks_kernel<DIM, DELTA>, grid, dim3(320), shared, s, pp);
+    return check_launch("recurrence_chunks_kernel");
+}
+
 template <typename T, int DPT, int LANES, int TOK, int CPT>
 static int launch_recurrence(const RecurrenceParams& pp, int n_items, cudaStream_t s) {
     if (pp.channel_decay) return launch_recurrence_as<T, DPT, LANES, TOK, CPT, true>(pp, n_items, s);
@@ -1475,6 +1845,10 @@ extern "C" int mllm_hybrid_linear_recurrence(const RecurrenceParams* params, int
     if (pp.channel_decay && pp.skip != nullptr) return fail("linear_recurrence: a decay per key channel goes with no skip");
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == DT_F32) return pick_recurrence<float>(pp, n_items, n_tokens, s);
+    if (dtype == DT_BF16 && recurrence_chunks_take(pp, n_items, n_tokens)) {
+        if (pp.dim <= 64) return pp.delta ? launch_recurrence_chunks<64, true>(pp, n_items, s) : launch_recurrence_chunks<64, false>(pp, n_items, s);
+        return pp.delta ? launch_recurrence_chunks<128, true>(pp, n_items, s) : launch_recurrence_chunks<128, false>(pp, n_items, s);
+    }
     if (dtype == DT_BF16) return pick_recurrence<bf16>(pp, n_items, n_tokens, s);
     return fail("linear_recurrence: unknown dtype");
 }

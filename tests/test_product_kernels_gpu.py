@@ -212,3 +212,40 @@ def test_latent_attention_in_tensor_core_tiles(heads, rank, rot, window, gated, 
                                tiles=dev(np.array(tiles, dtype=np.int32)), n_tiles=len(tiles), window=window, gate=gate)
     # queries and weights keep all 24 bits and sums are 32-bit; a result of 16 bits is rounded once
     np.testing.assert_allclose(f64(got), f64(want), rtol=2 ** -8 if out_dtype == torch.bfloat16 else 2e-5, atol=3e-5)
+
+
+# keys that fill a row and that end inside a 32-entry quarter, values that end inside a block's 16 columns; portions of one token, a chunk,
+# a chunk and one, more than the rows' ring holds
+@pytest.mark.parametrize("heads, qk_heads, dim, vdim, delta", [(2, 1, 40, 8, True), (3, 3, 64, 24, False), (4, 2, 128, 40, True), (2, 1, 96, 16, False)])
+def test_recurrence_in_chunks_of_tokens(heads, qk_heads, dim, vdim, delta):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(dim + vdim)
+    log_rate, bias, skip = (rng.normal(m, 1, heads).astype(np.float32).astype(np.float64) for m in (-1, 0, 0))
+    state = dev(rng.normal(0, 0.3, (5, heads * dim * vdim)), torch.float32)
+    slots, S = [3, 0, 4, 1], f64(state).reshape(5, heads, dim, vdim)
+    for counts in ([17, 1, 32, 0], [129, 16, 1, 3]):
+        n = sum(counts)
+        q, k, v = (dev(rng.normal(size=(n, size + 8)), torch.bfloat16)[:, :size] for size in (qk_heads * dim, qk_heads * dim, heads * vdim))
+        gate_a, gate_b = dev(rng.normal(0, 2, (n, heads)), torch.float32), dev(rng.normal(0, 3, (n, heads)), torch.float32)
+        expected, t = np.zeros((n, heads, vdim)), 0
+        for slot, count in zip(slots, counts):
+            for t in range(t, t + count):
+                for head in range(heads):
+                    g = head // (heads // qk_heads)
+                    qt, kt, vt = f64(q)[t, g * dim:(g + 1) * dim], f64(k)[t, g * dim:(g + 1) * dim], f64(v)[t, head * vdim:(head + 1) * vdim]
+                    step = np.log1p(np.exp(f64(gate_a)[t, head] + bias[head]))
+                    a, b = np.exp(-np.exp(log_rate[head]) * step), step
+                    if delta:
+                        qt, kt, b = qt / np.sqrt(qt @ qt + 1e-6) * 0.5, kt / np.sqrt(kt @ kt + 1e-6), 1 / (1 + np.exp(-f64(gate_b)[t, head]))
+                    S[slot, head] *= a
+                    S[slot, head] += np.outer(kt, b * (vt - (S[slot, head].T @ kt if delta else 0)))
+                    expected[t, head] = S[slot, head].T @ qt + (0 if delta else skip[head] * vt)
+            t += count > 0
+        out = torch.full((n, heads * vdim), float("nan"), device="cuda")
+        offsets = np.cumsum([0] + counts[:-1])
+        ops.linear_recurrence(out, q, k, v, gate_a, gate_b if delta else None, dev(log_rate, torch.float32), dev(bias, torch.float32), state,
+                              dev(np.array(slots, np.int32)), dev(offsets.astype(np.int32)), dev(np.array(counts, np.int32)), heads, qk_heads, dim,
+                              vdim, delta, unit_norm=delta, q_scale=0.5 if delta else 1.0, skip=None if delta else dev(skip, torch.float32))
+        # sums of some hundred products of 32-bit numbers: their rounding follows the largest values that went into them
+        np.testing.assert_allclose(f64(out), expected.reshape(n, -1), rtol=0, atol=4e-6 * max(1.0, np.abs(expected).max()))
+        np.testing.assert_allclose(f64(state).reshape(S.shape), S, rtol=0, atol=4e-6 * max(1.0, np.abs(S).max()))
