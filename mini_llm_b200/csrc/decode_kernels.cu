@@ -17,7 +17,7 @@
 //                   states go to scratch memory and the CTA that finishes
 //                   last for its (token, head) merges them in chunk order, so
 //                   the result does not depend on which CTA came last.
-#include "common.cuh"
+#include "mma_tiles.cuh"
 
 MLLM_DEFINE_ERROR_API(mllm_decode)
 
@@ -264,8 +264,13 @@ __device__ __forceinline__ void cp_async_16(void* smem, const void* global) {
 // passed), then the window's; chunks are ranges of these numbers, so a chunk is full whatever lies between.
 // FULL: keys and values have D entries; else key rows have `dim` and value rows `vdim` entries (multiples of 8 up
 // to D; scratch keeps its stride D), and a lane past a row's end copies nothing and holds zeros.
-template <int D, bool FULL>       // head size: 16, 32, 64, 128 or 256
-__global__ void __launch_bounds__(128)
+// A tile of 16 keys goes through m16n8k16 products: keys times the query (which stands in all eight columns), then values, turned, times the
+// weights, which enter as three bfloat16 terms in three columns and so keep all 24 bits; a tile's product is added with a rounded FMA.
+// What bounds it: few keys a pair, the chain of position, block table, keys and merge; many, the copies' way from HBM.  One lane a key's
+// 16 bytes with FMAs took 50 instructions a key and pair and was bound by their issue (60 % of all cycles); now some 13.  Heads of 64, before
+// and now: 64 x 12 pairs of 110 keys 11.2 -> 8.0 us, 24 x 16 of 112 to 778 22.3 -> 15.5, 64 x 25 of 264 31.1 -> 24.4, 2 x 12 of 1,000 13.6 -> 7.9.
+template <int D, bool FULL, int WARPS, int STAGES>       // head size: 16, 32, 64, 128 or 256
+__global__ void __launch_bounds__(WARPS * 32)
 split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restrict__ q, long ld_q,
                        const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
                        const int* __restrict__ block_table, int max_blocks, const int* __restrict__ positions,
@@ -274,14 +279,13 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
                        int gate_wide, const float* __restrict__ sink, const float* __restrict__ slopes, int chunk, int max_chunks, float* __restrict__ part_acc,
                        float* __restrict__ part_ml, int* __restrict__ counters) {
     if (FULL) dim = vdim = D;
-    constexpr int LPK = D / 8;             // lanes per key: each lane owns 8 of the head's dimensions
-    constexpr int KPW = 32 / LPK;          // keys per warp per step
+    constexpr int LD = D + 8, STEPS = D / 16;              // rows of a tile an odd number of 16 bytes apart: no bank twice
     dependents_may_start();
     wait_for_earlier_kernels();
     const int t = blockIdx.x, h = blockIdx.y, c = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int sub = lane % LPK, group = lane / LPK;
-    const int p = positions[t];
+    const int g = lane >> 2, tq = lane & 3;
+    const int p = positions[t], item = token_item[t];          // (asked for together: one wait for both)
     // the first key seen: the window's, and with a mask of blocks of positions the first of the query's block
     int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
     if (block > 0) lo = max(lo, p - p % block);
@@ -292,129 +296,166 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     const int c_last = (n_seen - 1) / chunk;
     if (c > c_last) return;
     const int begin = c * chunk, end = min(n_seen, begin + chunk) - 1;             // key numbers, inclusive
-    const int* bt = block_table + (long)token_item[t] * max_blocks;
+    const int* bt = block_table + (long)item * max_blocks;
     const int hk = h / (n_heads / n_kv_heads);
     const long k_width = (long)n_kv_heads * dim, v_width = (long)n_kv_heads * vdim;
-    const bool has_key = FULL || sub * 8 < dim, has_value = FULL || sub * 8 < vdim;
 
-    float qf[8], acc[8];
-    uint4 q8 = make_uint4(0u, 0u, 0u, 0u);
-    if (has_key) q8 = *reinterpret_cast<const uint4*>(q + (long)t * ld_q + (long)h * dim + sub * 8);
-    unpack8(q8, qf);
+    // The query stands in all eight columns of the second operand, so that every lane has the scores of its two keys.
+    uint32_t qb[STEPS][2];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int d = k * 16 + u * 8 + 2 * tq;
+            qb[k][u] = FULL || d < dim ? *reinterpret_cast<const uint32_t*>(q + (long)t * ld_q + (long)h * dim + d) : 0u;
+        }
     // scores are kept in units of log2(e): exp(x) = 2^(x log2 e) costs one instruction then
     const float scale_log2 = scale * 1.4426950408889634f;
     // a cap on the scores, cap * tanh(score / cap), in the same units (cap <= 0: none)
     const float cap_log2 = cap * 1.4426950408889634f, inv_cap_log2 = cap > 0.0f ? 1.0f / cap_log2 : 0.0f;
     // a bias by distance, taken off the (capped) score, in the same units
     const float slope_log2 = slopes != nullptr ? slopes[h] * 1.4426950408889634f : 0.0f;
+    float m = -INFINITY, l = 0.0f, acc[STEPS][4];        // m in log2 units; l: of this lane's keys
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        qf[i] *= scale_log2;
-        acc[i] = 0.0f;
-    }
-    float m = -INFINITY, l = 0.0f;       // m in log2 units
-    // Every lane of the warp runs the same trips (the shuffles need all of them); a lane
-    // whose key lies past the end copies nothing and skips the update.  A trip brings two
-    // keys and values per lane; RING trips are in flight per warp (cp.async into a ring in
-    // shared memory that each lane reads back itself), so that a trip's latency (block table,
-    // then the page) is paid once per chunk and not once per trip.
-    constexpr int RING = 4;
-    __shared__ uint4 ring[RING][2][2][128];       // [trip in flight][key of the lane][K, V][thread]
-    const int first_key = begin + warp * KPW + group;
-    const int trips = (end - (begin + warp * KPW)) / (8 * KPW) + 1;      // <= 0: nothing for this warp
+    for (int j = 0; j < STEPS; j++) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.0f;
+    // A warp's tiles are 16 keys each, every WARPS-th of the chunk; STAGES - 1 are on their way while one is worked on, and
+    // where the next one's keys lie is asked for a tile before its copies (lane l mod 16 has key l).
+    extern __shared__ uint4 split_shared[];
+    bf16* ring = reinterpret_cast<bf16*>(split_shared) + warp * (STAGES * 2 * 16 * LD);
+    const int first_key = begin + warp * 16, tiles = (end - first_key) / (WARPS * 16) + (end >= first_key);
     // pages of a power of two are the rule: shift and mask instead of a division per key
     const int page_shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;
-    const long k_offset = (long)hk * dim + sub * 8, v_offset = (long)hk * vdim + sub * 8;
-    auto issue = [&](int trip) {
-        if (trip < trips) {
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int number = first_key + trip * 8 * KPW + u * 4 * KPW;
-                if (number <= end) {
-                    const int j = number < n_kept ? number : number + gap;
-                    const int block = page_shift >= 0 ? j >> page_shift : j / page_size;
-                    const int within = page_shift >= 0 ? j & (page_size - 1) : j % page_size;
-                    const long slot = (long)bt[block] * page_size + within;
-                    if (has_key) cp_async_16(&ring[trip % RING][u][0][threadIdx.x], k_pages + slot * k_width + k_offset);
-                    if (has_value) cp_async_16(&ring[trip % RING][u][1][threadIdx.x], v_pages + slot * v_width + v_offset);
-                }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    const bf16* k_head = k_pages + (long)hk * dim;
+    const bf16* v_head = v_pages + (long)hk * vdim;
+    long row = -1;
+    auto find = [&](int i) {
+        const int number = first_key + i * (WARPS * 16) + (lane & 15);
+        const int j = number < n_kept ? number : number + gap;
+        const int block = page_shift >= 0 ? j >> page_shift : j / page_size;
+        const int within = page_shift >= 0 ? j & (page_size - 1) : j % page_size;
+        row = number <= end ? ((long)bt[block] * page_size + within) * (FULL ? k_width : 1) : -1;
     };
-    for (int i = 0; i < RING - 1; i++) issue(i);
-    for (int trip = 0; trip < trips; trip++) {
-        issue(trip + RING - 1);
-        asm volatile("cp.async.wait_group %0;" ::"n"(RING - 1) : "memory");
-        // the two keys of the trip share one rescaling of the running sums
-        float sc[2], vf[2][8];
+    auto issue = [&](int i) {
+        if (i < tiles) {
+            bf16* kt = ring + (i % STAGES) * (2 * 16 * LD);
+#pragma unroll
+            for (int u = 0; u < STEPS; u++) {
+                const int key = (lane + 32 * u) / (D / 8), d = (lane + 32 * u) % (D / 8) * 8;
+                const long at = __shfl_sync(0xffffffffu, row, key);
+                const bool k_there = at >= 0 && (FULL || d < dim), v_there = at >= 0 && (FULL || d < vdim);
+                copy_16(kt + key * LD + d, k_there ? k_head + (FULL ? at : at * k_width) + d : k_head, k_there);
+                copy_16(kt + (16 + key) * LD + d, v_there ? v_head + (FULL ? at : at * v_width) + d : v_head, v_there);
+            }
+            find(i + 1);
+        }
+        copies_end();
+    };
+    if (tiles > 0) find(0);
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; i++) issue(i);
+    for (int i = 0; i < tiles; i++) {
+        issue(i + STAGES - 1);
+        copies_landed<STAGES - 1>();
+        __syncwarp();
+        const bf16* kt = ring + (i % STAGES) * (2 * 16 * LD);
+        const bf16* vt = kt + 16 * LD;
+        float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int k = 0; k < STEPS; k++) {
+            uint32_t a[4];
+            load_blocks(a, kt + (lane & 15) * LD + k * 16 + (lane >> 4) * 8);
+            mma_added(c, a, qb[k][0], qb[k][1]);
+        }
+        float x[2];                                       // keys g and g + 8
 #pragma unroll
         for (int u = 0; u < 2; u++) {
-            const int number = first_key + trip * 8 * KPW + u * 4 * KPW;
-            const bool valid = number <= end;
-            float kf[8];
-            unpack8(has_key ? ring[trip % RING][u][0][threadIdx.x] : make_uint4(0u, 0u, 0u, 0u), kf);
-            unpack8(has_value ? ring[trip % RING][u][1][threadIdx.x] : make_uint4(0u, 0u, 0u, 0u), vf[u]);
-            float dot = 0.0f;
-#pragma unroll
-            for (int i = 0; i < 8; i++) dot = fmaf(qf[i], kf[i], dot);
-#pragma unroll
-            for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            if (cap > 0.0f) dot = cap_log2 * tanhf(dot * inv_cap_log2);
-            dot = fmaf(-slope_log2, (float)(p - (number < n_kept ? number : number + gap)), dot);
-            sc[u] = valid ? dot : -INFINITY;          // what an absent key left in the ring is never used
-            if (!valid) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) vf[u][i] = 0.0f;
-            }
+            const int number = first_key + i * (WARPS * 16) + g + 8 * u;
+            x[u] = c[2 * u] * scale_log2;
+            if (cap > 0.0f) x[u] = cap_log2 * tanhf(x[u] * inv_cap_log2);
+            if (slopes != nullptr) x[u] = fmaf(-slope_log2, (float)(p - (number < n_kept ? number : number + gap)), x[u]);
+            if (number > end) x[u] = -INFINITY;
         }
-        const float m_new = fmaxf(m, fmaxf(sc[0], sc[1]));
-        if (m_new != -INFINITY) {
-            const float corr = exp2f(m - m_new), e0 = exp2f(sc[0] - m_new), e1 = exp2f(sc[1] - m_new);
-            l = fmaf(l, corr, e0 + e1);
+        float m_new = fmaxf(x[0], x[1]);
 #pragma unroll
-            for (int i = 0; i < 8; i++) acc[i] = fmaf(acc[i], corr, fmaf(e0, vf[0][i], e1 * vf[1][i]));
-            m = m_new;
+        for (int o = 4; o < 32; o <<= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, o));
+        m_new = fmaxf(m_new, m);
+        const float from = m_new == -INFINITY ? 0.0f : m_new;
+        const float corr = exp2f(m - from);
+        x[0] = exp2f(x[0] - from), x[1] = exp2f(x[1] - from);
+        l = fmaf(l, corr, x[0] + x[1]);
+        m = m_new;
+        // the weights, 16 keys in the rows, their three bfloat16 terms (all 24 bits) in the first three columns
+        uint32_t low[3], high[3];
+        three_terms(__shfl_sync(0xffffffffu, x[0], 8 * tq), __shfl_sync(0xffffffffu, x[0], 8 * tq + 4), low[0], low[1], low[2]);
+        three_terms(__shfl_sync(0xffffffffu, x[1], 8 * tq), __shfl_sync(0xffffffffu, x[1], 8 * tq + 4), high[0], high[1], high[2]);
+        const uint32_t b0 = g == 0 ? low[0] : (g == 1 ? low[1] : (g == 2 ? low[2] : 0u));
+        const uint32_t b1 = g == 0 ? high[0] : (g == 1 ? high[1] : (g == 2 ? high[2] : 0u));
+#pragma unroll
+        for (int j = 0; j < STEPS; j++) {
+            uint32_t a[4];
+            float y[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            load_blocks_turned(a, vt + ((lane & 7) + ((lane >> 4) & 1) * 8) * LD + j * 16 + ((lane >> 3) & 1) * 8);
+            mma_tile(y, a, b0, b1);
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[j][e] = fmaf(acc[j][e], corr, y[e]);       // (rounded: what a tile adds is cut off)
         }
+        __syncwarp();                                     // the tile is copied over in the next round
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    copies_landed<0>();
 
-    // merge the key groups of a warp, then the four warps, always in the same order
-    __shared__ float sm_m[4][KPW];
-    __shared__ float sm_l[4][KPW];
-    __shared__ float sm_acc[4][KPW][D];
-    if (sub == 0) {
-        sm_m[warp][group] = m;
-        sm_l[warp][group] = l;
-    }
+    // a lane's keys into the warp's sum, the terms' columns (of lanes tq 0 and 1) into one, then the warps through shared
+    // memory, always in the same order
 #pragma unroll
-    for (int i = 0; i < 8; i++) sm_acc[warp][group][sub * 8 + i] = acc[i];
+    for (int o = 4; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    __syncthreads();                                  // the tiles are used up: what follows lies in their memory
+    float (*sm_acc)[D] = reinterpret_cast<float (*)[D]>(split_shared);
+    float* sm_m = &sm_acc[WARPS][0];
+    float* sm_l = sm_m + WARPS;
+    float* sm_top = sm_l + WARPS;
+    float* sm_sum = sm_top + WARPS;
+    float* weight = sm_sum + WARPS;                   // [threads]
+    float* spread = weight + WARPS * 32;              // [threads]
+    if (lane == 0) sm_m[warp] = m, sm_l[warp] = l;
+#pragma unroll
+    for (int j = 0; j < STEPS; j++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            float value = tq == 0 ? acc[j][2 * u] + acc[j][2 * u + 1] : acc[j][2 * u];
+            value += __shfl_xor_sync(0xffffffffu, value, 1);
+            if (tq == 0) sm_acc[warp][j * 16 + u * 8 + g] = value;
+        }
     __syncthreads();
-    float big = -INFINITY;
-    for (int w = 0; w < 4; w++)
-        for (int g = 0; g < KPW; g++) big = fmaxf(big, sm_m[w][g]);
-    const long cell = (((long)t * n_heads + h) * max_chunks + c);
-    for (int d = threadIdx.x; d < vdim; d += 128) {
+    float top = -INFINITY, total = 0.0f, share[WARPS];
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) top = fmaxf(top, sm_m[w]);
+    const float from = top == -INFINITY ? 0.0f : top;
+#pragma unroll
+    for (int w = 0; w < WARPS; w++) share[w] = exp2f(sm_m[w] - from), total = fmaf(sm_l[w], share[w], total);
+    auto sum_of = [&](int d) {
         float o = 0.0f;
-        for (int w = 0; w < 4; w++)
-            for (int g = 0; g < KPW; g++) {
-                float mg = sm_m[w][g];
-                if (mg != -INFINITY) o += sm_acc[w][g][d] * exp2f(mg - big);
-            }
-        part_acc[cell * D + d] = o;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) o = fmaf(sm_acc[w][d], share[w], o);
+        return o;
+    };
+    // a sink: one more term exp(sink[h]) in the denominator, with no key and no value (scores are in units of log2 e)
+    const float sink_log2 = sink != nullptr ? sink[h] * 1.4426950408889634f : -INFINITY;
+    // a gate per (token, head), or per entry of the head's result, opens it by its sigmoid
+    auto open = [&](int d) {
+        return gate != nullptr ? 1.0f / (1.0f + __expf(-gate[(long)t * ld_gate + (gate_wide ? h * vdim + d : h)])) : 1.0f;
+    };
+    if (c_last == 0) {                               // one chunk: nothing to merge with
+        const float above = fmaxf(top, sink_log2);
+        const float shrink = exp2f(top - above), denom = total * shrink + (sink != nullptr ? exp2f(sink_log2 - above) : 0.0f);
+        for (int d = threadIdx.x; d < vdim; d += WARPS * 32)
+            out[(long)t * ld_out + (long)h * vdim + d] = __float2bfloat16_rn(sum_of(d) * shrink / denom * open(d));
+        return;
     }
-    if (threadIdx.x == 0) {
-        float total = 0.0f;
-        for (int w = 0; w < 4; w++)
-            for (int g = 0; g < KPW; g++) {
-                float mg = sm_m[w][g];
-                if (mg != -INFINITY) total += sm_l[w][g] * exp2f(mg - big);
-            }
-        part_ml[cell * 2] = big;
-        part_ml[cell * 2 + 1] = total;
-    }
+    const long cell = (((long)t * n_heads + h) * max_chunks + c);
+    for (int d = threadIdx.x; d < vdim; d += WARPS * 32) part_acc[cell * D + d] = sum_of(d);
+    if (threadIdx.x == 0) part_ml[cell * 2] = top, part_ml[cell * 2 + 1] = total;
 
-    // the CTA that arrives last for this (token, head) merges the chunks
+    // the CTA that arrives last for this (token, head) merges the chunks: as many threads share an entry of the result as
+    // there are, each with every so many chunks, and what a thread reads is asked for eight chunks at a time
     __shared__ int is_last;
     __threadfence();
     __syncthreads();
@@ -426,22 +467,54 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     __syncthreads();
     if (!is_last) return;
     __threadfence();
+    constexpr int THREADS = WARPS * 32, SPREAD = D >= THREADS ? 1 : THREADS / D, ENTRIES = D > THREADS ? D / THREADS : 1, BATCH = THREADS;
     const long first = ((long)t * n_heads + h) * max_chunks;
-    float top = -INFINITY;
-    for (int cc = 0; cc <= c_last; cc++) top = fmaxf(top, __ldcg(part_ml + (first + cc) * 2));
-    // a sink: one more term exp(sink[h]) in the denominator, with no key and no value (scores are in units of log2 e)
-    const float sink_log2 = sink != nullptr ? sink[h] * 1.4426950408889634f : -INFINITY;
-    top = fmaxf(top, sink_log2);
-    float denom = sink != nullptr ? exp2f(sink_log2 - top) : 0.0f;
-    for (int cc = 0; cc <= c_last; cc++)
-        denom += __ldcg(part_ml + (first + cc) * 2 + 1) * exp2f(__ldcg(part_ml + (first + cc) * 2) - top);
-    for (int d = threadIdx.x; d < vdim; d += 128) {
-        // a gate per (token, head), or per entry of the head's result, opens it by its sigmoid
-        const float open = gate != nullptr ? 1.0f / (1.0f + __expf(-gate[(long)t * ld_gate + (gate_wide ? h * vdim + d : h)])) : 1.0f;
-        float o = 0.0f;
-        for (int cc = 0; cc <= c_last; cc++)
-            o += __ldcg(part_acc + (first + cc) * D + d) * exp2f(__ldcg(part_ml + (first + cc) * 2) - top);
-        out[(long)t * ld_out + (long)h * vdim + d] = __float2bfloat16_rn(o / denom * open);
+    const int d0 = threadIdx.x % (D < THREADS ? D : THREADS), turn = threadIdx.x / (D < THREADS ? D : THREADS);
+    float o[ENTRIES], denom = 0.0f;
+#pragma unroll
+    for (int e = 0; e < ENTRIES; e++) o[e] = 0.0f;
+    top = sink_log2;
+    if (sink != nullptr) denom = 1.0f;
+    for (int base = 0; base <= c_last; base += BATCH) {
+        const int mine = base + threadIdx.x, here = min(BATCH, c_last + 1 - base);
+        const float m_part = mine <= c_last ? __ldcg(part_ml + (first + mine) * 2) : -INFINITY;
+        const float l_part = mine <= c_last ? __ldcg(part_ml + (first + mine) * 2 + 1) : 0.0f;
+        float big = warp_max(m_part);
+        if (lane == 0) sm_top[warp] = big;
+        __syncthreads();
+        big = top;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) big = fmaxf(big, sm_top[w]);
+        const float over = big == -INFINITY ? 0.0f : big;
+        const float w = exp2f(m_part - over), sum = warp_sum(l_part * w), shrink = exp2f(top - over);
+        weight[threadIdx.x] = w;
+        if (lane == 0) sm_sum[warp] = sum;
+        __syncthreads();
+        denom *= shrink;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) denom += sm_sum[w];
+        top = big;
+#pragma unroll
+        for (int e = 0; e < ENTRIES; e++) {
+            o[e] *= shrink;
+#pragma unroll 8
+            for (int cc = turn; cc < here; cc += SPREAD) o[e] = fmaf(__ldcg(part_acc + (first + base + cc) * D + d0 + e * THREADS), weight[cc], o[e]);
+        }
+        __syncthreads();
+    }
+    if (SPREAD > 1) {
+        spread[threadIdx.x] = o[0];
+        __syncthreads();
+        if (turn > 0) return;
+        float x = 0.0f;
+#pragma unroll
+        for (int r = 0; r < SPREAD; r++) x += spread[r * D + d0];
+        o[0] = x;
+    }
+#pragma unroll
+    for (int e = 0; e < ENTRIES; e++) {
+        const int d = d0 + e * THREADS;
+        if (d < vdim) out[(long)t * ld_out + (long)h * vdim + d] = __float2bfloat16_rn(o[e] / denom * open(d));
     }
 }
 
@@ -481,12 +554,28 @@ extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const vo
     const long share = (1184 + pairs - 1) / pairs;
     if (max_chunks > share && max_chunks > 4) max_chunks = (int)(share > 4 ? share : 4);
     dim3 grid(n_tokens, n_heads, max_chunks);
-#define LAUNCH_SPLIT(D, FULL)                                                                                        \
-    launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL>, grid, dim3(128), 0, s, (bf16*)out, ld_out, \
-                  (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks,         \
-                  positions, token_item, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep, \
-                  gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters)
-#define PICK_SPLIT(D) do { if (full) LAUNCH_SPLIT(D, true); else LAUNCH_SPLIT(D, false); } while (0)
+    // Stages of a warp's ring: three where a wave of blocks holds the launch all the same, else two, of which six blocks of
+    // heads of 64 fit an SM.  At heads of 64, three against two: 24 x 16 pairs of 112 to 778 keys 15.1 against 16.2 us, 64 x 12 of 1,000 38.9
+    // against 50.4; 64 x 12 of 110 (five blocks an SM are needed for one wave) 10.9 and 8.0.
+    const bool deep = pairs * max_chunks <= 592 && size <= 64;
+#define LAUNCH_SPLIT(D, FULL, STAGES)                                                                                    \
+    do {                                                                                                                 \
+        constexpr int ring = 4 * STAGES * 2 * 16 * (D + 8) * 2;                                                          \
+        if (ring > 48 * 1024 && cudaFuncSetAttribute(split_attention_kernel<D, FULL, 4, STAGES>,                         \
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, ring) != cudaSuccess)  \
+            return fail("split_attention: the ring's shared memory was refused");                                        \
+        launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL, 4, STAGES>, grid, dim3(128), ring, s, (bf16*)out, ld_out, \
+                      (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks,         \
+                      positions, token_item, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep, \
+                      gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters);           \
+    } while (0)
+#define PICK_SPLIT(D)                                                             \
+    do {                                                                          \
+        if (full && deep) LAUNCH_SPLIT(D, true, 3);                               \
+        else if (full) LAUNCH_SPLIT(D, true, 2);                                  \
+        else if (deep) LAUNCH_SPLIT(D, false, 3);                                 \
+        else LAUNCH_SPLIT(D, false, 2);                                           \
+    } while (0)
     switch (size) {
     case 16: PICK_SPLIT(16); break;
     case 32: PICK_SPLIT(32); break;

@@ -22,6 +22,13 @@ SKINNY_MAX_ROWS = 16          # up to here a product streams the weights once th
 SPLIT_ATTENTION_MAX_ROWS = 64 # up to here attention runs one CTA per (token, head, chunk of keys)
 
 
+def split_attention_chunk(pairs):
+    """Keys of a CTA: few when there are few (token, head) pairs, so that the chunks still fill the GPU; from some 200 on a
+    second chunk costs more than it saves (heads of 64: 24 pairs of 1,000 keys 13.8, 10.2, 8.3, 8.0 us in 1, 2, 4, 8 chunks; 320 of 512
+    12.3 and 17.7 in 1 and 2; 384 of 112 to 778 15.1 and 20.0)."""
+    return 128 if pairs < 64 else (256 if pairs < 128 else (512 if pairs < 256 else 1024))
+
+
 class DeferredNorm:
     """A norm that has not run yet: ``rows`` (or all rows) of the fp32 ``x``.
 
@@ -141,7 +148,7 @@ class Kernels:
             # single tokens: each token's keys in chunks over many CTAs, merged by the last to arrive
             # (its exponentials, weights and sums are 32-bit, which this attention asks for)
             pairs = n * n_heads
-            span = 64 if pairs < 64 else (128 if pairs < 128 else (256 if pairs < 256 else 512))
+            span = split_attention_chunk(pairs)
             reach = cache.block_table.shape[1] * cache.page_size
             if window:
                 reach = min(reach, window + keep)              # the most keys a token sees
@@ -485,18 +492,18 @@ class Kernels:
         self.launches += 1
         n = q.shape[0]
         if (not self.plain_only and n <= SPLIT_ATTENTION_MAX_ROWS and head_size in ops.SPLIT_ATTENTION_HEAD_SIZES):
-            # chunk of keys per CTA: small when there are few (token, head) pairs, so that the
-            # chunks still fill the GPU
             pairs = n * n_heads
-            chunk = 64 if pairs < 64 else (128 if pairs < 128 else (256 if pairs < 256 else 512))
             reach = cache.block_table.shape[1] * cache.page_size
-            max_chunks = -(-reach // chunk)
             acc, ml, counters = self._scratch(ctx, SPLIT_ATTENTION_MAX_ROWS * n_heads, -(-reach // 64), head_size)
             # query heads that share a key/value head go through the tensor-core tiles together,
-            # reading the keys once; with one query head per key/value head the SIMT kernel is
+            # reading the keys once; with one query head per key/value head every pair by itself is
             # as fast or faster (measured at 9 to 64 requests of 12 heads)
             grouped = n_heads // n_kv_heads >= 2 and ops.group_attention_takes(q, n_heads, n_kv_heads, head_size)
             run = ops.group_attention if grouped else ops.split_attention
+            chunk = split_attention_chunk(pairs)
+            if grouped:
+                chunk = 64 if pairs < 64 else (128 if pairs < 128 else (256 if pairs < 256 else 512))
+            max_chunks = -(-reach // chunk)
             self.chose("attention", "group_attention" if grouped else "split_attention", n, n_heads, head_size)
             return run(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                        n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, max_chunks, acc, ml,

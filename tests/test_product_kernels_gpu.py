@@ -249,3 +249,22 @@ def test_recurrence_in_chunks_of_tokens(heads, qk_heads, dim, vdim, delta):
         # sums of some hundred products of 32-bit numbers: their rounding follows the largest values that went into them
         np.testing.assert_allclose(f64(out), expected.reshape(n, -1), rtol=0, atol=4e-6 * max(1.0, np.abs(expected).max()))
         np.testing.assert_allclose(f64(state).reshape(S.shape), S, rtol=0, atol=4e-6 * max(1.0, np.abs(S).max()))
+
+
+# keys that end at a tile's, a round's and a chunk's edges; few pairs (three stages) and more than a wave (two)
+@pytest.mark.parametrize("head", [16, 64, 128, 256])
+@pytest.mark.parametrize("times, chunk", [(1, 64), (1, 1024), (20, 1024)])
+def test_split_attention_at_the_edges_of_its_tiles(head, times, chunk):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(head)
+    lengths, heads, page = [1, 15, 16, 17, 63, 64, 65, 129] * times, 4, 16
+    k_pages, v_pages, table, positions, items, dense = paged_case(rng, lengths, [1] * len(lengths), heads, heads, head, page, torch.bfloat16)
+    dense = [(f64(dev(k, torch.bfloat16)), f64(dev(v, torch.bfloat16))) for k, v in dense]
+    q = dev(rng.normal(size=(len(lengths), heads * head)), torch.bfloat16)
+    max_chunks = -(-table.shape[1] * page // chunk)
+    scratch, out = split_scratch(len(lengths), heads, max_chunks, head), torch.full_like(q, float("nan"))
+    expected = attention_expected(f64(q), dense, f64(positions).astype(int), f64(items).astype(int), heads, heads, head, head ** -0.5, 0)
+    ops.split_attention(out, q, k_pages, v_pages, table, positions, items, heads, heads, head, page, head ** -0.5, 0, chunk, max_chunks, *scratch)
+    # weights and sums are 32-bit; the result is rounded to 8 bits once
+    np.testing.assert_allclose(f64(out), expected, rtol=2 ** -8, atol=1e-5)
+    assert int(scratch[2].abs().sum()) == 0
