@@ -63,6 +63,8 @@ class DeferredNorm:
 
 class Kernels:
     FUSED_NORM_KINDS = ("layer_norm",)    # what the few-row product kernel can apply on the way in
+    FUSED_NORM_ROWS = 1                   # and of how many rows (the head of one wanted row): every block norms all of them, and
+                                          # a norm kernel ahead costs less (4096 x 1024, 8 rows: 8.6 against 11.8 us, 16: 9.4 against 17.4)
 
     def __init__(self, act_dtype: torch.dtype, plain_only: bool = False):
         self.act_dtype = act_dtype
@@ -406,7 +408,7 @@ class Kernels:
         fast = w.shape[0] >= 16                  # (a product narrower than a tile's smallest box goes to the plain kernel)
         skinny = self._skinny(m, k, w.shape[0])
         deferred = isinstance(a, DeferredNorm)
-        if deferred and not (skinny and a.kind in self.FUSED_NORM_KINDS):
+        if deferred and not (skinny and m <= self.FUSED_NORM_ROWS and a.kind in self.FUSED_NORM_KINDS):
             a, deferred = a.materialize(ctx), False      # no kernel here norms this kind on the way in: the norm runs first
         if skinny:
             self.chose("linear", "skinny_linear", m, w.shape[0], k)
@@ -458,19 +460,15 @@ class Kernels:
         the cache pages (if this entry writes its cache); returns the queries [T, q_width]."""
         m, k = a.shape
         skinny = cache.writes and self._skinny(m, k)
-        deferred = isinstance(a, DeferredNorm)
-        if deferred and not (skinny and a.kind in self.FUSED_NORM_KINDS):
-            a, deferred = a.materialize(ctx), False
+        if isinstance(a, DeferredNorm):
+            a = a.materialize(ctx)
         if skinny:
             q = ctx.buffer("q", (m, q_width), ctx.act_dtype)
             scatter = (cache.k_pages, cache.v_pages, ctx.positions, ctx.token_item, cache.block_table,
                        cache.page_size, q_width, kv_width)
             self.launches += 1
             self.chose("qkv", "skinny_linear", m, w.shape[0], k)
-            if deferred:
-                ops.skinny_linear(q, a.x, w, bias, "store", norm=(a.gamma, a.beta, a.eps, a.rows), scatter=scatter)
-            else:
-                ops.skinny_linear(q, a, w, bias, "store", scatter=scatter)
+            ops.skinny_linear(q, a, w, bias, "store", scatter=scatter)
             return q
         if cache.writes and not self.plain_only and ops.gemm_qkv_takes(a, w, q_width, kv_width):
             q = ctx.buffer("q", (m, q_width), ctx.act_dtype)

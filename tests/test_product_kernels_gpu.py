@@ -268,3 +268,26 @@ def test_split_attention_at_the_edges_of_its_tiles(head, times, chunk):
     # weights and sums are 32-bit; the result is rounded to 8 bits once
     np.testing.assert_allclose(f64(out), expected, rtol=2 ** -8, atol=1e-5)
     assert int(scratch[2].abs().sum()) == 0
+
+
+# rows of one and two tiles; features that end inside a tile, K shared by four, eight and sixteen warps and no multiple of a warp's share
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n, k", [(5, 8), (24, 72), (1000, 2056), (3072, 768), (130, 4104)])
+def test_few_row_products_at_the_edges_of_their_tiles(m, n, k):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(m + n + k)
+    x, w = dev(rng.normal(size=(m, k)), torch.bfloat16), dev(rng.normal(size=(n, k)) / math.sqrt(k), torch.bfloat16)
+    bias, out = dev(rng.normal(size=n), torch.float32), torch.full((m, n), float("nan"), device="cuda")
+    ops.skinny_linear(out, x, w, bias, "store")
+    np.testing.assert_allclose(f64(out), f64(x) @ f64(w).T + f64(bias), rtol=0, atol=2e-5)      # 32-bit sums of products of size 1 in all
+
+
+@pytest.mark.parametrize("m, heads, n, k", [(1, 12, 64, 256), (16, 3, 256, 72), (9, 5, 20, 8)])
+def test_few_row_products_per_head(m, heads, n, k):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(n + k)
+    a, w = dev(rng.normal(size=(m, heads * k + 8)), torch.bfloat16)[:, 8:], dev(rng.normal(size=(heads, n, k)) / math.sqrt(k), torch.bfloat16)
+    out = torch.full((m, heads * n), float("nan"), device="cuda")
+    assert ops.skinny_heads_takes(a, w, k)
+    ops.skinny_heads(out, a, w, heads, k, n)
+    np.testing.assert_allclose(f64(out).reshape(m, heads, n), np.einsum("mhk,hnk->mhn", f64(a).reshape(m, heads, k), f64(w)), rtol=0, atol=2e-5)
