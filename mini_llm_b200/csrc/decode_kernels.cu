@@ -277,15 +277,19 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
                        const int* __restrict__ token_item, int n_heads, int n_kv_heads, int dim, int vdim, int page_size,
                        float scale, float cap, int window, int block, int keep, const float* __restrict__ gate, long ld_gate,
                        int gate_wide, const float* __restrict__ sink, const float* __restrict__ slopes, int chunk, int max_chunks, float* __restrict__ part_acc,
-                       float* __restrict__ part_ml, int* __restrict__ counters) {
+                       float* __restrict__ part_ml, int* __restrict__ counters, const int* records) {
     if (FULL) dim = vdim = D;
     constexpr int LD = D + 8, STEPS = D / 16;              // rows of a tile an odd number of 16 bytes apart: no bank twice
     dependents_may_start();
     wait_for_earlier_kernels();
-    const int t = blockIdx.x, h = blockIdx.y, c = blockIdx.z;
+    const int h = blockIdx.y, c = blockIdx.z;
+    const long pair = (long)blockIdx.x * n_heads + h;          // whose scratch this is
+    // (a record of the step's work list: entry, row, rows, position)
+    const int* record = records + (long)blockIdx.x * 8;
+    const int t = records != nullptr ? record[1] : blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3;
-    const int p = positions[t], item = token_item[t];          // (asked for together: one wait for both)
+    const int p = records != nullptr ? record[3] : positions[t], item = records != nullptr ? record[0] : token_item[t];
     // the first key seen: the window's, and with a mask of blocks of positions the first of the query's block
     int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
     if (block > 0) lo = max(lo, p - p % block);
@@ -450,7 +454,7 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
             out[(long)t * ld_out + (long)h * vdim + d] = __float2bfloat16_rn(sum_of(d) * shrink / denom * open(d));
         return;
     }
-    const long cell = (((long)t * n_heads + h) * max_chunks + c);
+    const long cell = pair * max_chunks + c;
     for (int d = threadIdx.x; d < vdim; d += WARPS * 32) part_acc[cell * D + d] = sum_of(d);
     if (threadIdx.x == 0) part_ml[cell * 2] = top, part_ml[cell * 2 + 1] = total;
 
@@ -460,15 +464,15 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ticket = atomicAdd(&counters[t * n_heads + h], 1);
+        int ticket = atomicAdd(&counters[pair], 1);
         is_last = (ticket == c_last);
-        if (is_last) counters[t * n_heads + h] = 0;       // ready for the next launch
+        if (is_last) counters[pair] = 0;       // ready for the next launch
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
     constexpr int THREADS = WARPS * 32, SPREAD = D >= THREADS ? 1 : THREADS / D, ENTRIES = D > THREADS ? D / THREADS : 1, BATCH = THREADS;
-    const long first = ((long)t * n_heads + h) * max_chunks;
+    const long first = pair * max_chunks;
     const int d0 = threadIdx.x % (D < THREADS ? D : THREADS), turn = threadIdx.x / (D < THREADS ? D : THREADS);
     float o[ENTRIES], denom = 0.0f;
 #pragma unroll
@@ -526,13 +530,15 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
 // The widest form: key rows of `dim` and value rows of `vdim` entries (equal and one of 16, 32, 64, 128, 256, or
 // any multiples of 8 up to 256; the scratch's rows then have the least of those sizes that holds both), and the keys
 // below `keep` stay visible behind a window.  max_chunks * chunk covers the most keys a token of the step sees.
-extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,
+// (with `records`, 8 numbers each: the single tokens that n_tokens records of a step's work list name,
+// entry, row, rows, position first; scratch is theirs in the list's order)
+extern "C" int mllm_decode_split_attention_records(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,
                                                 const void* v_pages, const int* block_table, int max_blocks,
                                                 const int* positions, const int* token_item, int n_tokens, int n_heads,
                                                 int n_kv_heads, int dim, int vdim, int page_size, float scale, float cap,
                                                 int window, int block, int keep, const float* gate, long ld_gate,
                                                 int gate_wide, const float* sink, const float* slopes, int chunk, int max_chunks, float* part_acc,
-                                                float* part_ml, int* counters, void* stream) {
+                                                float* part_ml, int* counters, const int* records, void* stream) {
     if (n_tokens <= 0) return 0;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
         return fail("split_attention: heads must be a multiple of key/value heads");
@@ -567,7 +573,7 @@ extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const vo
         launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL, 4, STAGES>, grid, dim3(128), ring, s, (bf16*)out, ld_out, \
                       (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks,         \
                       positions, token_item, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep, \
-                      gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters);           \
+                      gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters, records);  \
     } while (0)
 #define PICK_SPLIT(D)                                                             \
     do {                                                                          \
@@ -586,6 +592,19 @@ extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const vo
 #undef PICK_SPLIT
 #undef LAUNCH_SPLIT
     return check_launch("split_attention_kernel");
+}
+
+extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,
+                                                const void* v_pages, const int* block_table, int max_blocks,
+                                                const int* positions, const int* token_item, int n_tokens, int n_heads,
+                                                int n_kv_heads, int dim, int vdim, int page_size, float scale, float cap,
+                                                int window, int block, int keep, const float* gate, long ld_gate,
+                                                int gate_wide, const float* sink, const float* slopes, int chunk, int max_chunks, float* part_acc,
+                                                float* part_ml, int* counters, void* stream) {
+    return mllm_decode_split_attention_records(out, ld_out, q, ld_q, k_pages, v_pages, block_table, max_blocks, positions, token_item,
+                                               n_tokens, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep,
+                                               gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters,
+                                               nullptr, stream);
 }
 
 extern "C" int mllm_decode_split_attention_sink(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,

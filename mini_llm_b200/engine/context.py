@@ -202,6 +202,7 @@ class StepContext:
         self.dump = None              # a list: the model appends the residual stream after every run entry
         self.att_tiles = None         # device work list (tiles of up to 128 tokens of one entry), or None
         self.n_att_tiles = 0          # records (CTAs) of the work list
+        self.n_att_singles = 0        # the last ones of them: tokens that stand alone beside prompt portions
         self.n_split_tiles = 0        # tiles among them that come in several parts
         self.att_parts = 1            # most parts of a tile
         self.att_units = False        # the work list holds units of up to 256 tokens (two tiles) instead of tiles

@@ -303,12 +303,20 @@ class Engine:
         heads = self.model.attention_unit_heads
         units = heads > 0 and 2 * sum(n for n in ctx.item_counts if n > ops.ATTENTION_TILE) >= n_tokens
         if not self.model.wants_attention_tiles or (decode_only and n_items <= SPLIT_ATTENTION_MAX_ROWS):
-            tiles, n_split, most_parts, units = [], 0, 1, False
-        elif units:
-            tiles, n_split, most_parts = ops.attention_units(ctx.item_offsets, ctx.item_counts, ctx.item_starts, heads,
-                                                             self._n_sms)
+            tiles, singles, n_split, most_parts, units = [], [], 0, 1, False
         else:
-            tiles, n_split, most_parts = ops.attention_tiles(ctx.item_offsets, ctx.item_counts, ctx.item_starts)
+            # Tokens that stand alone beside the portions: in the tiles each is a row of a tile by itself, which walks the request's
+            # keys as the whole tile would.  From a wave of (token, head) pairs on the decode attention takes them, in a launch of
+            # its own (25 heads, 63 lone tokens of some 264 keys beside portions of 512: 74 us a layer in units of two tiles, 26 + 25 this way).
+            alone = [i for i, n in enumerate(ctx.item_counts) if n == 1]
+            if not (heads > 0 and len(alone) <= SPLIT_ATTENTION_MAX_ROWS and len(alone) * heads >= self._n_sms and n_tokens > len(alone)):
+                alone = []
+            counts = [0 if n == 1 and alone else n for n in ctx.item_counts]
+            if units:
+                tiles, n_split, most_parts = ops.attention_units(ctx.item_offsets, counts, ctx.item_starts, heads, self._n_sms)
+            else:
+                tiles, n_split, most_parts = ops.attention_tiles(ctx.item_offsets, counts, ctx.item_starts)
+            singles = [(i, ctx.item_offsets[i], 1, ctx.item_starts[i], 0, 1, 0, ctx.item_starts[i] // ops.ATTENTION_TILE + 1) for i in alone]
         temperature = top_p = seeds = counters = None
         if sampling is not None:
             temperature = np.array([s.temperature for s in sampling], dtype=np.float32)
@@ -355,7 +363,9 @@ class Engine:
                     counters = np.concatenate([counters, np.zeros(more, dtype=np.int32)])
                 n_want = want_filled
             if tiles and extra:
-                tiles = tiles + [(n_items, n_tokens, 1, 0, 0, 1, 0, 1)] * (-len(tiles) % 4)
+                filler = [(n_items, n_tokens, 1, 0, 0, 1, 0, 1)]
+                tiles = tiles + filler * (-len(tiles) % 4)
+                singles = singles + filler * (-len(singles) % 8)
             # the filler is one more entry, in the slot beyond the last request's (state of fixed
             # size is kept there for nobody); the entries after it have no tokens
             more = items_filled - n_items
@@ -365,7 +375,7 @@ class Engine:
             item_start = np.concatenate([item_start, np.zeros(more, dtype=np.int32)])
             n_tokens, n_items = filled, items_filled
         arrays = {"token_ids": token_ids, "positions": positions, "token_item": token_item, "want_rows": want_rows,
-                  "want_slots": want_slots, "att_tiles": np.array(tiles, dtype=np.int32), "item_slot": item_slot,
+                  "want_slots": want_slots, "att_tiles": np.array(tiles + singles, dtype=np.int32), "item_slot": item_slot,
                   "item_offset": item_offset, "item_count": item_count, "item_start": item_start}
         for index, table in tables.items():
             arrays[("block_table", index)] = table
@@ -388,7 +398,8 @@ class Engine:
         ctx.decode_only = decode_only
         ctx.fused = fused
         ctx.dump = [] if dump_hidden else None
-        ctx.att_tiles, ctx.n_att_tiles = (views["att_tiles"] if tiles else None), len(tiles)
+        ctx.att_tiles, ctx.n_att_tiles = (views["att_tiles"] if tiles else None), len(tiles) + len(singles)
+        ctx.n_att_singles = len(singles)
         ctx.n_split_tiles, ctx.att_parts, ctx.att_units = n_split, most_parts, units
         for view in self.storage.paged_views():
             view.block_table = views[("block_table", view.group)]
@@ -491,7 +502,7 @@ class Engine:
             self._graphs.clear()                      # a buffer moved: captured addresses are stale
             self._graph_stamp = stamp
         # (how many units come in parts is data; that some do decides whether the kernel gets scratch)
-        key = (ctx.n_tokens, ctx.n_items, ctx.n_want, ctx.n_att_tiles, ctx.att_parts > 1, ctx.att_units,
+        key = (ctx.n_tokens, ctx.n_items, ctx.n_want, ctx.n_att_tiles, ctx.n_att_singles, ctx.att_parts > 1, ctx.att_units,
                sample_views is not None, self._any_nucleus, ctx.any_previous, self.control.parity)
         held = self._graphs.get(key)
         # A shape runs eagerly the first time (every buffer it needs gets allocated) and is

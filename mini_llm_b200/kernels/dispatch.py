@@ -517,16 +517,26 @@ class Kernels:
                 most = max(ctx.n_split_tiles * n_heads, 8 * n_heads, 256)
                 # (cells of a unit's 256 rows, also for the kernel with tiles of 128: one size, no regrowth)
                 scratch = self._attention_scratch(ctx.device, most, ops.ATTENTION_MAX_PARTS * ops.ATTENTION_UNIT * (head_size + 4))
+            n_tiles = ctx.n_att_tiles - ctx.n_att_singles
+            if ctx.n_att_singles:
+                # the list's last records: tokens that stand alone, a row of a tile each if they stayed in the tiles
+                self.launches += 1
+                chunk = split_attention_chunk(ctx.n_att_singles * n_heads)
+                reach = cache.block_table.shape[1] * cache.page_size
+                acc, ml, counters = self._scratch(ctx, SPLIT_ATTENTION_MAX_ROWS * n_heads, -(-reach // 64), head_size)
+                ops.split_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
+                                    n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, -(-reach // chunk), acc, ml,
+                                    counters, records=ctx.att_tiles[8 * n_tiles:], n_records=ctx.n_att_singles)
             if ctx.att_units:
                 self.chose("attention", "attention_two_tiles", n, n_heads, head_size)
                 return ops.attention_prefill_two_tiles(out, q, cache.k_pages, cache.v_pages, cache.block_table,
-                                                       ctx.att_tiles, ctx.n_att_tiles, n_heads, n_kv_heads, head_size,
+                                                       ctx.att_tiles, n_tiles, n_heads, n_kv_heads, head_size,
                                                        cache.page_size, scale, window, self.status(ctx.device),
                                                        self.attention_work(ctx.device), scratch, ctx.n_split_tiles,
                                                        ops.ATTENTION_MAX_PARTS if ctx.att_parts > 1 else 1)
             self.chose("attention", "attention_tcgen05", n, n_heads, head_size)
             return ops.attention_prefill(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.att_tiles,
-                                         ctx.n_att_tiles, n_heads, n_kv_heads, head_size, cache.page_size, scale,
+                                         n_tiles, n_heads, n_kv_heads, head_size, cache.page_size, scale,
                                          window, self.status(ctx.device), self.attention_work(ctx.device), scratch,
                                          ctx.n_split_tiles,
                                          ops.ATTENTION_MAX_PARTS if ctx.att_parts > 1 else 1)

@@ -229,8 +229,8 @@ class _SkinnyParams(ctypes.Structure):
 
 
 _skinny = Function("decode", "mllm_decode_skinny_linear", [ctypes.POINTER(_SkinnyParams), P])
-_split_attention = Function("decode", "mllm_decode_split_attention_kept",
-                            [P, L, P, L, P, P, P, I, P, P, I, I, I, I, I, I, F, F, I, I, I, P, L, I, P, P, I, I, P, P, P, P])
+_split_attention = Function("decode", "mllm_decode_split_attention_records",
+                            [P, L, P, L, P, P, P, I, P, P, I, I, I, I, I, I, F, F, I, I, I, P, L, I, P, P, I, I, P, P, P, P, P])
 
 SKINNY_MAX_SMEM = 200 * 1024
 SPLIT_ATTENTION_HEAD_SIZES = (16, 32, 64, 128, 256)
@@ -341,7 +341,7 @@ def skinny_heads(out, a, w, heads, a_head, o_head):
 
 def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item, n_heads, n_kv_heads, head_size,
                     page_size, scale, window, chunk, max_chunks, part_acc, part_ml, counters, cap=0.0, block=0, gate=None, sink=None,
-                    value_size=None, keep=0, slopes=None, gate_wide=False):
+                    value_size=None, keep=0, slopes=None, gate_wide=False, records=None, n_records=0):
     """Causal attention over the paged cache for few tokens: one CTA per (token, head, chunk
     of ``chunk`` keys); needs fp32 scratch ``part_acc`` [T*H*max_chunks*D], ``part_ml``
     [T*H*max_chunks*2] and zeroed int32 ``counters`` [T*H] (left zero).  ``cap`` > 0: the scores
@@ -352,7 +352,9 @@ def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item
     key's position) comes off the (capped) score.
     ``value_size``: entries of a value where they are not ``head_size`` (then both are multiples of 8 up to 256 and the
     scratch is sized for ``split_attention_row``).  ``keep``: the first ``keep`` keys stay visible behind the window.
-    ``max_chunks`` chunks must cover the most keys a token may see.  Scores, weights and sums are 32-bit."""
+    ``max_chunks`` chunks must cover the most keys a token may see.  Scores, weights and sums are 32-bit.
+    ``records``: only the rows that ``n_records`` device int32 records of 8 name, single tokens of the step's work list (entry, row,
+    rows, position ...); T is then their number."""
     _check(out, "split_attention.out", torch.bfloat16, 2)
     _check(q, "split_attention.q", torch.bfloat16, 2)
     _check(k_pages, "split_attention.k_pages", torch.bfloat16)
@@ -361,14 +363,18 @@ def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item
     _check(part_acc, "split_attention.part_acc", torch.float32)
     _check(part_ml, "split_attention.part_ml", torch.float32)
     _check(counters, "split_attention.counters", torch.int32)
-    n = q.shape[0]
+    n = q.shape[0] if records is None else int(n_records)
     cells = n * n_heads * max_chunks
     vdim = head_size if value_size is None else int(value_size)
     row = split_attention_row(head_size, vdim)
     if row is None or (value_size is None and row != head_size):
         raise KernelError(f"split_attention does not take head size {head_size}" + (f" with values of {vdim}" if value_size is not None else ""))
-    if q.shape[1] != n_heads * head_size or out.shape != (n, n_heads * vdim):
+    if q.shape[1] != n_heads * head_size or out.shape != (q.shape[0], n_heads * vdim):
         raise KernelError("split_attention: q / out do not have heads * head_size columns")
+    if records is not None:
+        _check(records, "split_attention.records", torch.int32)
+        if not records.is_contiguous() or records.numel() < 8 * n:
+            raise KernelError("split_attention: records are 8 contiguous numbers each")
     if part_acc.numel() < cells * row or part_ml.numel() < cells * 2 or counters.numel() < n * n_heads:
         raise KernelError("split_attention: scratch too small")
     reach = page_size * block_table.shape[1]
@@ -376,14 +382,14 @@ def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item
         raise KernelError("split_attention: the chunks do not cover the longest block table (or the window)")
     if keep < 0 or (keep and block):
         raise KernelError("split_attention: kept first keys go with a window, not with blocks of positions")
-    _check_gate(gate, n, n_heads * (vdim if gate_wide else 1), "split_attention")
+    _check_gate(gate, q.shape[0], n_heads * (vdim if gate_wide else 1), "split_attention")
     _check_per_head(sink, n_heads, "split_attention.sink")
     _check_per_head(slopes, n_heads, "split_attention.slopes")
     _split_attention(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(),
                      block_table.data_ptr(), block_table.shape[1], positions.data_ptr(), token_item.data_ptr(), n,
                      n_heads, n_kv_heads, head_size, vdim, page_size, float(scale), float(cap or 0.0), int(window or 0), int(block or 0),
                      int(keep), _ptr(gate), gate.stride(0) if gate is not None else 0, int(bool(gate_wide)), _ptr(sink), _ptr(slopes), int(chunk), int(max_chunks), part_acc.data_ptr(),
-                     part_ml.data_ptr(), counters.data_ptr(), _stream())
+                     part_ml.data_ptr(), counters.data_ptr(), _ptr(records), _stream())
     return out
 
 

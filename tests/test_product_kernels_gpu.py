@@ -291,3 +291,26 @@ def test_few_row_products_per_head(m, heads, n, k):
     assert ops.skinny_heads_takes(a, w, k)
     ops.skinny_heads(out, a, w, heads, k, n)
     np.testing.assert_allclose(f64(out).reshape(m, heads, n), np.einsum("mhk,hnk->mhn", f64(a).reshape(m, heads, k), f64(w)), rtol=0, atol=2e-5)
+
+
+@pytest.mark.parametrize("heads, kv_heads, window", [(4, 4, 0), (6, 2, 30)])
+def test_split_attention_of_the_tokens_a_work_list_names(heads, kv_heads, window):
+    """Lone tokens beside a portion, by their records at an odd place of the list, one of them twice; the portion's rows stay as they are."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(heads)
+    lengths, new, head, page = [40, 1, 300, 77, 2], [1, 1, 90, 1, 1], 64, 16
+    k_pages, v_pages, table, positions, items, dense = paged_case(rng, lengths, new, heads, kv_heads, head, page, torch.bfloat16)
+    dense = [(f64(dev(k, torch.bfloat16)), f64(dev(v, torch.bfloat16))) for k, v in dense]
+    q = dev(rng.normal(size=(sum(new), heads * head)), torch.bfloat16)
+    offsets = np.cumsum([0] + new[:-1])
+    alone = [3, 0, 4, 1, 3]
+    records = [(9, 9, 9, 9, 9, 9, 9, 9)] + [(i, offsets[i], 1, lengths[i] - 1, 0, 1, 0, 1) for i in alone]
+    expected = attention_expected(f64(q), dense, f64(positions).astype(int), f64(items).astype(int), heads, kv_heads, head, head ** -0.5, window)
+    for chunk in (32, 1024):
+        max_chunks = -(-table.shape[1] * page // chunk)
+        out, scratch = torch.full_like(q, 7.0), split_scratch(len(alone), heads, max_chunks, head)
+        ops.split_attention(out, q, k_pages, v_pages, table, positions, items, heads, kv_heads, head, page, head ** -0.5, window, chunk, max_chunks,
+                            *scratch, records=dev(np.array(records, np.int32)).reshape(-1)[8:], n_records=len(alone))
+        rows = sorted({int(offsets[i]) for i in alone})
+        np.testing.assert_allclose(f64(out)[rows], expected[rows], rtol=2 ** -8, atol=1e-5)      # rounded to 8 bits once
+        assert (np.delete(f64(out), rows, axis=0) == 7.0).all()
