@@ -1428,6 +1428,87 @@ static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStr
     return check_launch("linear_recurrence_kernel");
 }
 
+// ---- few tokens an entry ---------------------------------------------------------------------------
+// Keys of up to 128 entries.  One token's update reads and writes the state once (0.3 us of HBM time for an entry of six heads of
+// 128 x 128), so what it takes is the way there and back: a block takes 32 columns of a head, a lane a column and a warp 16 rows,
+// all asked for at once and kept in registers, and both sums over the old state meet in shared memory once.  Staging the
+// state and 16 tokens' places as the walk above does took 10.3 us for two entries (11.4 for one with a decay a channel); here 4.4 and 4.3.
+template <typename T, bool CHANNEL>
+__global__ void __launch_bounds__(256) recurrence_few_kernel(RecurrenceParams pp) {
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    constexpr int ROWS = 16, WARPS = 8;
+    __shared__ float ks[ROWS * WARPS], qs[ROWS * WARPS], gs[CHANNEL ? ROWS * WARPS : 1], sums[3][4], part_k[WARPS][32], part_q[WARPS][32];
+    const int item = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int count = pp.item_count[item];
+    if (count <= 0) return;
+    const long first = pp.item_offset[item];
+    const int dim = pp.dim, vdim = pp.vdim, col = blockIdx.z * 32 + lane;
+    const long qk_at = (long)(head / (pp.heads / pp.qk_heads)) * dim;
+    float* S = pp.state + (long)pp.item_slot[item] * pp.state_stride + (long)head * dim * vdim;
+    float s[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        const int d = warp * ROWS + r;
+        s[r] = d < dim && col < vdim ? S[(long)d * vdim + col] : 0.0f;
+    }
+    const float rate = expf(pp.log_rate[head]), skip = pp.skip != nullptr ? pp.skip[head] : 0.0f;
+    const float bias = CHANNEL ? (tid < dim ? pp.step_bias[(long)head * dim + tid] : 0.0f) : pp.step_bias[head];
+    for (int i = 0; i < count; i++) {
+        const long t = first + i;
+        const float value = col < vdim ? to_f32(((const T*)pp.v)[t * pp.ld_v + (long)head * vdim + col]) : 0.0f;
+        float a = 1.0f, b = pp.delta ? sigmoid_f(pp.gate_b[t * pp.ld_gate_b + head]) : 0.0f;
+        if (!CHANNEL) {
+            const float step = softplus_f(pp.gate_a[t * pp.ld_gate_a + head] + bias);
+            a = expf(-rate * step);
+            if (!pp.delta) b = step;
+        }
+        if (tid < ROWS * WARPS) {
+            const float k = tid < dim ? to_f32(((const T*)pp.k)[t * pp.ld_k + qk_at + tid]) : 0.0f;
+            const float q = tid < dim ? to_f32(((const T*)pp.q)[t * pp.ld_q + qk_at + tid]) : 0.0f;
+            if (CHANNEL) gs[tid] = tid < dim ? expf(-rate * softplus_f(pp.gate_a[t * pp.ld_gate_a + (long)head * dim + tid] + bias)) : 1.0f;
+            ks[tid] = k, qs[tid] = q;
+            const float kk = warp_sum(k * k), qq = warp_sum(q * q), kq = warp_sum(k * q);
+            if (lane == 0) sums[0][warp] = kk, sums[1][warp] = qq, sums[2][warp] = kq;
+        }
+        __syncthreads();
+        const float kk = (sums[0][0] + sums[0][1]) + (sums[0][2] + sums[0][3]), qq = (sums[1][0] + sums[1][1]) + (sums[1][2] + sums[1][3]);
+        const float fk = pp.unit_norm ? 1.0f / sqrtf(kk + 1e-6f) : 1.0f, fq = pp.unit_norm ? pp.q_scale / sqrtf(qq + 1e-6f) : pp.q_scale;
+        const float both = ((sums[2][0] + sums[2][1]) + (sums[2][2] + sums[2][3])) * fk * fq;
+        float dk[2] = {0.0f, 0.0f}, dq[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) {
+            const int d = warp * ROWS + r;
+            if (CHANNEL) s[r] *= gs[d];
+            dk[r & 1] = fmaf(s[r], ks[d], dk[r & 1]), dq[r & 1] = fmaf(s[r], qs[d], dq[r & 1]);
+        }
+        part_k[warp][lane] = dk[0] + dk[1], part_q[warp][lane] = dq[0] + dq[1];
+        __syncthreads();
+        float sum_k = 0.0f, sum_q = 0.0f;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) sum_k += part_k[w][lane], sum_q += part_q[w][lane];
+        const float u = pp.delta ? b * (value - a * sum_k * fk) : b * value;
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) s[r] = fmaf(ks[warp * ROWS + r] * fk, u, a * s[r]);
+        if (warp == 0 && col < vdim) pp.out[t * pp.ld_out + (long)head * vdim + col] = fmaf(u, both, a * sum_q * fq) + skip * value;
+        if (i + 1 < count) __syncthreads();
+    }
+    if (!pp.writes) return;
+#pragma unroll
+    for (int r = 0; r < ROWS; r++) {
+        const int d = warp * ROWS + r;
+        if (d < dim && col < vdim) S[(long)d * vdim + col] = s[r];
+    }
+}
+
+template <typename T>
+static int launch_recurrence_few(const RecurrenceParams& pp, int n_items, cudaStream_t s) {
+    const dim3 grid(n_items, pp.heads, (pp.vdim + 31) / 32);
+    if (pp.channel_decay) launch_kernel(g_dependent_launch != 0, recurrence_few_kernel<T, true>, grid, dim3(256), 0, s, pp);
+    else launch_kernel(g_dependent_launch != 0, recurrence_few_kernel<T, false>, grid, dim3(256), 0, s, pp);
+    return check_launch("recurrence_few_kernel");
+}
+
 // ---- prompt portions, 16 tokens at a time --------------------------------------------------------
 // bfloat16 rows, one decay per head.  The walk above is a chain of one token after the other; over a chunk of 16 tokens the
 // same sums are products of small matrices.  With S the state before the chunk, G(t) the product of the decays up to token t, R(t, s) that of
@@ -1805,16 +1886,12 @@ static int launch_recurrence(const RecurrenceParams& pp, int n_items, cudaStream
 }
 
 // A column of the state lies in the registers of 4 to 32 lanes of a warp.  Prompt portions: eight
-// rows a lane up to a key size of 256 (short sums).  Steps of few tokens per entry: as many rows a
-// lane as registers hold, so that the blocks, each of which pays the same chain of loads for its
-// one token, are few.
+// rows a lane up to a key size of 256 (short sums).  Steps of few tokens per entry have a kernel of their own.
 template <typename T>
 static int pick_recurrence(const RecurrenceParams& pp, int n_items, int n_tokens, cudaStream_t s) {
     if (pp.dim <= 32) return launch_recurrence<T, 8, 4, 16, 1>(pp, n_items, s);
-    if (n_tokens <= 4 * n_items) {
-        if (pp.dim <= 64) return launch_recurrence<T, 16, 4, 16, 1>(pp, n_items, s);
-        if (pp.dim <= 128) return launch_recurrence<T, 32, 4, 16, 1>(pp, n_items, s);
-    } else if (pp.dim <= 128) {
+    if (pp.dim <= 128 && n_tokens <= 4 * n_items) return launch_recurrence_few<T>(pp, n_items, s);
+    if (pp.dim <= 128) {
         // Prompt portions.  The walk from token to token is a chain of dependent sums and exchanges
         // between lanes; a thread takes two columns, whose chains run in one another's gaps, or four
         // where two would leave the busy entries' blocks more than one an SM (entries of a step that

@@ -218,12 +218,21 @@ def test_latent_attention_in_tensor_core_tiles(heads, rank, rot, window, gated, 
 # a chunk and one, more than the rows' ring holds
 @pytest.mark.parametrize("heads, qk_heads, dim, vdim, delta", [(2, 1, 40, 8, True), (3, 3, 64, 24, False), (4, 2, 128, 40, True), (2, 1, 96, 16, False)])
 def test_recurrence_in_chunks_of_tokens(heads, qk_heads, dim, vdim, delta):
+    recurrence_case(heads, qk_heads, dim, vdim, delta, ([17, 1, 32, 0], [129, 16, 1, 3]))
+
+
+@pytest.mark.parametrize("heads, qk_heads, dim, vdim, delta", [(2, 1, 33, 33, True), (4, 2, 128, 32, False), (3, 3, 128, 65, True)])
+def test_recurrence_of_few_tokens(heads, qk_heads, dim, vdim, delta):
+    recurrence_case(heads, qk_heads, dim, vdim, delta, ([1, 0, 1, 1], [3, 1, 0, 2]))
+
+
+def recurrence_case(heads, qk_heads, dim, vdim, delta, portions):
     from mini_llm_b200.kernels import ops
     rng = np.random.default_rng(dim + vdim)
     log_rate, bias, skip = (rng.normal(m, 1, heads).astype(np.float32).astype(np.float64) for m in (-1, 0, 0))
     state = dev(rng.normal(0, 0.3, (5, heads * dim * vdim)), torch.float32)
     slots, S = [3, 0, 4, 1], f64(state).reshape(5, heads, dim, vdim)
-    for counts in ([17, 1, 32, 0], [129, 16, 1, 3]):
+    for counts in portions:
         n = sum(counts)
         q, k, v = (dev(rng.normal(size=(n, size + 8)), torch.bfloat16)[:, :size] for size in (qk_heads * dim, qk_heads * dim, heads * vdim))
         gate_a, gate_b = dev(rng.normal(0, 2, (n, heads)), torch.float32), dev(rng.normal(0, 3, (n, heads)), torch.float32)
