@@ -2303,22 +2303,23 @@ expert_down_kernel(float* __restrict__ hidden, long ld_hidden, const T* __restri
 // Now 11.9 + 13.4 us, and two tokens of eight choices 7.3 + 11.1 (in a step, one kernel after the other).
 constexpr int EXPERT_TILE_TOKENS = 31, EXPERT_TABLES = 64, EXPERT_UNITS = 64, EXPERT_UNIT_K = 256;
 
-// The pairs that chose expert e, in their order, by one warp; returns how many.
-__device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, int e, int* list, int* place) {
+// The pairs that chose expert e, in their order, by one warp: the list gets those from number `begin` on, 32 at most, and `place`
+// (if there is one) a pair's place in it, -1 for those that found none.  Returns how many chose the expert in all: more than 32
+// only where a token names an expert more than once, as the router does for a token whose scores are no numbers.
+__device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, int e, int begin, int* list, int* place) {
     const int lane = threadIdx.x & 31;
     int count = 0;
     for (int first = 0; first < n_pairs; first += 32) {
         const int pair = first + lane;
         const bool mine = pair < n_pairs && choice[pair] == e;
         const unsigned all = __ballot_sync(0xffffffffu, mine);
-        const int at = count + __popc(all & ((1u << lane) - 1u));
-        if (mine && at < 32) {
-            list[at] = pair;
-            if (place != nullptr) place[pair] = at;
-        }
+        const int at = count + __popc(all & ((1u << lane) - 1u)) - begin;
+        const bool listed = at >= 0 && at < 32;
+        if (mine && listed) list[at] = pair;
+        if (mine && place != nullptr) place[pair] = listed ? at : -1;
         count += __popc(all);
     }
-    return min(count, 32);
+    return count;
 }
 
 // A block: 16 inner features of an expert, in two tiles of 8 whose K four warps share.
@@ -2329,7 +2330,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
                        int width, int pairs, int n_tokens, float limit, float shared_limit, float alpha, int n_experts) {
     constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
     constexpr int AHEAD = 4;
-    __shared__ int list[32], found;
+    __shared__ int list[32], found;                          // (32 pairs at a time)
     __shared__ float sums[2][8][16][9];                      // [gate, up][warp][row][feature]
     const int e = blockIdx.y, inner = __ldg(inner_of + e);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
@@ -2359,12 +2360,17 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
     x = behind_the_wait(x);
     in_weight = behind_the_wait(in_weight);
     if (warp == 0) {
-        const int count = pairs_of_expert(choice, n_tokens * pairs, e, list, nullptr);
+        const int count = pairs_of_expert(choice, n_tokens * pairs, e, 0, list, nullptr);
         if (lane == 0) found = count;
     }
     __syncthreads();
     const int count = found;
     for (int m0 = 0; m0 < count; m0 += 16) {
+        if (m0 > 0 && m0 % 32 == 0) {                        // (every thread left the list before the barrier that ended the last tile)
+            if (warp == 0) pairs_of_expert(choice, n_tokens * pairs, e, m0, list, nullptr);
+            __syncthreads();
+        }
+        const int* listed = list + m0 % 32;
         if (m0 > 0 || !early)
 #pragma unroll
             for (int i = 0; i < AHEAD; i++) weights(i, begin + i);
@@ -2374,7 +2380,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             const bool there = m0 + r * 8 + g < count;
-            const int pair = there ? list[m0 + r * 8 + g] : 0;
+            const int pair = there ? listed[r * 8 + g] : 0;
             xr[r] = there ? reinterpret_cast<const uint4*>(x + (long)(pair / pairs) * ld_x) : nullptr;
             scale[r] = there ? in_weight[pair] : 1.0f;
         }
@@ -2423,7 +2429,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
                 if (GATED) a += sums[0][(f >> 3) * 4 + s][r][f & 7];
                 b += sums[1][(f >> 3) * 4 + s][r][f & 7];
             }
-            act[(long)list[m0 + r] * ld_act + f_block + f] =
+            act[(long)listed[r] * ld_act + f_block + f] =
                 __float2bfloat16_rn(expert_form<FORM>(a, b, e == n_experts ? shared_limit : limit, alpha));
         }
         __syncthreads();
@@ -2450,8 +2456,8 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
     out_weight = behind_the_wait(out_weight);
     x = behind_the_wait(x);
     for (int e = warp; e < n_tables; e += 16) {
-        const int count = pairs_of_expert(choice, n_pairs, e, list[e], place);
-        if (lane == 0) count_of[e] = count;
+        const int count = pairs_of_expert(choice, n_pairs, e, 0, list[e], place);
+        if (lane == 0) count_of[e] = min(count, 32);
     }
     __syncthreads();
     if (warp == 0) {
@@ -2529,7 +2535,15 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
         float total = 0.0f;
         for (int k = 0; k < pairs; k++) {
             const int pair = t * pairs + k, e = choice[pair];
-            if (e < 0) continue;
+            if (e < 0 || e >= n_tables) continue;
+            if (place[pair] < 0) {                           // beyond an expert's 32 (a token that named it more than once): by itself
+                const bf16* row = act + (long)pair * ld_act;
+                const bf16* w = reinterpret_cast<const bf16*>(__ldg(down_of + e)) + (long)c * ld_down;
+                float z = 0.0f;
+                for (int f = 0; f < __ldg(inner_of + e); f++) z = fmaf(to_f32(row[f]), to_f32(w[f]), z);
+                total = fmaf(out_weight[pair], z, total);
+                continue;
+            }
             const int last = unit_k > 0 ? first_unit[e] + (__ldg(inner_of + e) + EXPERT_UNIT_K - 1) / EXPERT_UNIT_K : first_unit[e] + 1;
             float z = 0.0f;
             for (int u = first_unit[e]; u < last; u++) z += down_shared[(u * 32 + place[pair]) * 8 + i % 8];

@@ -1464,7 +1464,8 @@ def experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_
     g' = min(g, limit) and u' = clamp(u, -limit, limit); expert ``n_experts`` (the shared one) has ``shared_limit``.  ``act`` [T * pairs, max_inner] is scratch.  A pair whose choice is negative has no
     expert; with ``identity_weight`` [T] identity_weight[t] * x[t] joins the sum.  ``assign``: ``hidden`` is set
     to the sum instead of added to.  ``tiles``: the pairs go through the tensor cores expert by expert (``expert_tiles_take``;
-    the caller says with it that every inner size is a multiple of 8 and that no token chose an expert twice)."""
+    the caller says with it that every inner size is a multiple of 8; an expert's pairs beyond 32, which there are only where a
+    token named it more than once, are summed one by one)."""
     _check(hidden, "experts.hidden", torch.float32, 2)
     _check(x, "experts.x", None, 2)
     _check(act, "experts.act", x.dtype, 2)
