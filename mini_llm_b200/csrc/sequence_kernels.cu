@@ -1474,9 +1474,11 @@ extern "C" int mllm_sequence_latent_attention_tiled(const LatentTiledParams* par
 // all 32-bit, read at the start of the entry's tokens and written back at their end.
 // One block per (entry, head, slice of VS value columns); a lane has one column of S in shared memory and a warp an eighth of
 // its rows, and the block walks the entry's tokens in order; q and k of the next token are fetched into the other half of a double
-// buffer meanwhile.  Every slice keeps n and m for itself; the last slice, whose block is the last to start, writes them back.
+// buffer meanwhile.  Every slice keeps n and m for itself.  In memory a head's slices share them, and blocks start and read in no
+// promised order: the slices of a head are one cluster, and the block that writes them back waits until all have read.
 // A token's update is short (the state read and written once); one warp that walked all rows of its columns took 16.7 us
-// for 8 entries of 4 heads and 6 slices and 10.7 of 12 heads and 2, eight warps 7.8 and 4.5.
+// for 8 entries of 4 heads and 6 slices and 10.7 of 12 heads and 2, eight warps 7.8 and 4.5.  (The wait for the readers: 8 entries of
+// 4 heads and 6 slices 6.3 us without it, 6.8 as a cluster, 8.2 with a counter in memory as below.)
 // ---------------------------------------------------------------------------
 struct MemoryScanParams {
     float* out; long ld_out;                      // [T, heads * vdim], 32-bit
@@ -1490,19 +1492,21 @@ struct MemoryScanParams {
     int heads, dim, vdim;
     float q_scale, gate_cap;
     int silu, writes;
+    int* readers;                                 // memory_chunk_kernel: [entries * heads], zero before and after
 };
 
 constexpr int SCAN_WARPS = 8;
 
+// (slices first_slice .. of the values; writes_shared: this launch's first slice writes n and m back)
 template <typename T, int VS>
 __global__ void __launch_bounds__(SCAN_WARPS * 32)
-memory_scan_kernel(MemoryScanParams p) {
+memory_scan_kernel(MemoryScanParams p, int first_slice, int writes_shared) {
     dependents_may_start();
     wait_for_earlier_kernels();
     extern __shared__ float shared[];
-    const int item = blockIdx.x, head = blockIdx.y, v0 = blockIdx.z * VS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int item = blockIdx.x, head = blockIdx.y, v0 = (first_slice + blockIdx.z) * VS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int count = p.item_count[item];
-    if (count <= 0) return;
+    if (count <= 0) return;                  // (every block of the cluster)
     const int dim = p.dim, vdim = p.vdim, heads = p.heads;
     const int each = (dim + SCAN_WARPS - 1) / SCAN_WARPS, begin = min(dim, warp * each), end = min(dim, begin + each);      // the warp's rows
     const bool gated = p.gates != nullptr;
@@ -1523,6 +1527,7 @@ memory_scan_kernel(MemoryScanParams p) {
     if (gated) {
         for (int d = tid; d < dim; d += SCAN_WARPS * 32) nvec[d] = n_held[d];
         m = *m_held;
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     }
     const long first = p.item_offset[item];
     const T* q = (const T*)p.q + (long)head * dim;
@@ -1592,13 +1597,28 @@ memory_scan_kernel(MemoryScanParams p) {
         }
         if (i + 1 < count) fetch(row + 1, qk + ((i + 1) & 1) * 2 * dim);
     }
+    if (gated) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");        // every slice has read n and m
     if (!p.writes) return;
     if (active)
 #pragma unroll 8
         for (int d = begin; d < end; d++) S_held[(long)d * vdim + column] = S[d * VS + lane];
-    if (gated && blockIdx.z == gridDim.z - 1) {
+    if (gated && writes_shared && blockIdx.z == 0) {
         for (int d = tid; d < dim; d += SCAN_WARPS * 32) n_held[d] = nvec[d];
         if (tid == 0) *m_held = m;
+    }
+}
+
+// In the gated form the slices of a head are a cluster, of which there are eight blocks at most: values of more than 256
+// entries take more launches, of which only the last one, behind all others' reads, writes n and m.
+template <typename T>
+static void launch_memory_scan(const MemoryScanParams& p, int n_items, size_t shared, cudaStream_t s) {
+    const bool gated = p.gates != nullptr;
+    const int slices = (p.vdim + 31) / 32, most = gated ? 8 : slices;
+    if (shared > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+    for (int first = 0; first < slices; first += most) {
+        const int here = slices - first < most ? slices - first : most;
+        launch_kernel_in_clusters(AFTER_THE_KERNELS_AHEAD, gated && here > 1 ? dim3(1, 1, here) : dim3(0, 1, 1), memory_scan_kernel<T, 32>,
+                                  dim3(n_items, p.heads, here), dim3(SCAN_WARPS * 32), shared, s, p, first, (int)(first + here == slices));
     }
 }
 
@@ -1611,13 +1631,10 @@ extern "C" int mllm_sequence_memory_scan(const MemoryScanParams* params, int n_i
     const size_t total = shared + (SCAN_WARPS * VS + 2 * SCAN_WARPS) * sizeof(float);
     if (shared > 200 * 1024) return fail("memory_scan: the key size is too large for one slice of the state in shared memory");
     cudaStream_t s = (cudaStream_t)stream;
-    dim3 grid(n_items, p.heads, (p.vdim + VS - 1) / VS);
     if (dtype == DT_F32) {
-        if (total > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<float, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)total);
-        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_scan_kernel<float, VS>, dim3(grid), dim3(SCAN_WARPS * 32), total, s, p);
+        launch_memory_scan<float>(p, n_items, total, s);
     } else if (dtype == DT_BF16) {
-        if (total > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<bf16, VS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)total);
-        launch_kernel(AFTER_THE_KERNELS_AHEAD, memory_scan_kernel<bf16, VS>, dim3(grid), dim3(SCAN_WARPS * 32), total, s, p);
+        launch_memory_scan<bf16>(p, n_items, total, s);
     } else {
         return fail("memory_scan: unknown dtype");
     }
@@ -1637,7 +1654,20 @@ extern "C" int mllm_sequence_memory_scan(const MemoryScanParams* params, int n_i
 // n_t . q_t = carried weight_t (n_before . q_t) + sum_s A[t, s].  One block per (entry, head,
 // slice of 32 value columns).  Results differ from the token-by-token kernel by rounding only
 // (other order of the sums); decays, gates and state stay 32-bit.
+// The n and m that a head's slices share in memory: a slice that has read them takes a ticket, and the one with the last ticket,
+// behind which nobody reads them, writes them back.  (63 entries of two tokens, 6 slices: 98 us, as a cluster 161.)
 // ---------------------------------------------------------------------------
+// By one thread of a block, behind a barrier that follows its threads' reads: whether all other slices have read, too.
+__device__ __forceinline__ bool was_last_to_read(const MemoryScanParams& p, int item, int head) {
+    if (gridDim.z == 1) return true;
+    int* readers = p.readers + (long)item * p.heads + head;
+    __threadfence();
+    const bool last = atomicAdd(readers, 1) == (int)gridDim.z - 1;
+    if (last) *readers = 0;                       // (every slice has its ticket)
+    __threadfence();
+    return last;
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256)
 memory_chunk_kernel(MemoryScanParams p) {
@@ -1665,6 +1695,8 @@ memory_chunk_kernel(MemoryScanParams p) {
     float* nq = wt + C;                   // [C]      n_before . q_t
     float* dl = nq + C;                   // [C]      weight[last, s]
     float* pw = dl + C;                   // [C + 1]  powers of a fixed decay
+    bool last_reader = false;             // (of the first thread)
+    __shared__ bool writes_vector;
     float* held = p.state + (long)p.item_slot[item] * p.state_stride;
     float* S_held = held + (long)head * dim * vdim;
     float* n_held = held + (long)heads * dim * vdim + (long)head * dim;
@@ -1727,6 +1759,7 @@ memory_chunk_kernel(MemoryScanParams p) {
         const int n = min(C, count - done), last = n - 1;
         const long row0 = first + done;
         __syncthreads();                  // the chunk before is done with everything
+        if (done == 0 && gated && p.writes && tid == 0) last_reader = was_last_to_read(p, item, head);
         if (vectors) {
 #pragma unroll
             for (int e = 0; e < MAXV; e++) {
@@ -1910,7 +1943,10 @@ memory_chunk_kernel(MemoryScanParams p) {
         const int d = i / VS, c = v0 + (i % VS);
         if (d < dim && c < vdim) S_held[(long)d * vdim + c] = S[i];
     }
-    if (gated && blockIdx.z == 0) {
+    if (!gated) return;
+    if (tid == 0) writes_vector = last_reader;
+    __syncthreads();
+    if (writes_vector) {
         for (int d = tid; d < dim; d += 256) n_held[d] = nv[d];
         if (tid == 0) *m_held = m_before;
     }
@@ -1928,6 +1964,7 @@ extern "C" int mllm_sequence_memory_chunk(const MemoryScanParams* params, int n_
     MemoryScanParams p = *params;
     if (n_items <= 0) return 0;
     if (p.heads <= 0 || p.heads > 65535 || p.dim <= 0 || p.vdim <= 0) return fail("memory_chunk: bad sizes");
+    if (p.gates != nullptr && p.writes && p.vdim > 32 && p.readers == nullptr) return fail("memory_chunk: slices that share a vector need their counters");
     const size_t shared = memory_chunk_shared_bytes(p.dim);
     if (shared > 200 * 1024) return fail("memory_chunk: the key size is too large for a chunk in shared memory");
     cudaStream_t s = (cudaStream_t)stream;

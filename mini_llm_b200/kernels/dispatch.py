@@ -77,6 +77,7 @@ class Kernels:
         self._status = None          # device word the tensor-core kernels report a timed-out wait in
         self._att_scratch = None
         self._att_work = None
+        self._memory_readers = None
 
     # ---- operations without a fast variant --------------------------------------------------
     def keep_tokens(self, kept, slots, tokens):
@@ -303,12 +304,22 @@ class Kernels:
             # long portions: the chunks side by side (their sums, a scan over their states, their outputs)
             passes = self._memory_scratch(ctx.device, ops.memory_passes_scratch(q.shape[0], ctx.n_items, heads, dim, vdim))
             self.launches += 3 if "gates" in how else 2
+        elif "gates" in how and chunked:
+            how["readers"] = self._memory_counters(ctx.device, ctx.n_items * heads)
+        elif "gates" in how:
+            self.launches += (vdim - 1) // 256           # (eight slices of 32 values a launch)
         self.chose("memory_scan", "memory_passes" if passes else ("memory_chunk" if chunked else "memory_scan"),
                    q.shape[0], heads, dim, vdim)
         return ops.memory_scan(out, q, k, v, state, ctx.item_slot, ctx.item_offset, ctx.item_count, heads, dim, vdim,
                                writes=writes, chunked=chunked, passes=passes, **how)
 
     MEMORY_PASSES_TOKENS = 128     # from here on a step's chunks are worth four launches
+
+    def _memory_counters(self, device, count):
+        if self._memory_readers is None or self._memory_readers.numel() < count:
+            self._memory_readers = torch.zeros(max(count, 1024), dtype=torch.int32, device=device)
+            self.scratch_generation += 1
+        return self._memory_readers
 
     def _memory_scratch(self, device, floats):
         held = getattr(self, "_memory_passes", None)
@@ -445,6 +456,8 @@ class Kernels:
             self._att_work.zero_()
         if self._split_scratch is not None:
             self._split_scratch[2].zero_()
+        if self._memory_readers is not None:
+            self._memory_readers.zero_()
         if self._sample_scratch is not None:
             self._sample_scratch[2].zero_()
 

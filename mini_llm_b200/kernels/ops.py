@@ -1120,7 +1120,7 @@ class _MemoryScanParams(ctypes.Structure):
     _fields_ = [("out", P), ("ld_out", L), ("q", P), ("k", P), ("v", P), ("ld_q", L), ("ld_k", L), ("ld_v", L),
                 ("gates", P), ("ld_gates", L), ("gate_bias", P), ("decay", P), ("state", P), ("state_stride", L),
                 ("item_slot", P), ("item_offset", P), ("item_count", P), ("heads", I), ("dim", I), ("vdim", I),
-                ("q_scale", F), ("gate_cap", F), ("silu", I), ("writes", I)]
+                ("q_scale", F), ("gate_cap", F), ("silu", I), ("writes", I), ("readers", P)]
 
 
 _memory_scan = Function("sequence", "mllm_sequence_memory_scan", [ctypes.POINTER(_MemoryScanParams), I, I, P])
@@ -1155,7 +1155,7 @@ def memory_state_floats(heads, dim, vdim, gated) -> int:
 
 
 def memory_scan(out, q, k, v, state, item_slot, item_offset, item_count, heads, dim, vdim, q_scale=1.0, silu=False,
-                gates=None, gate_bias=None, gate_cap=0.0, decay=None, writes=True, chunked=False, passes=None):
+                gates=None, gate_bias=None, gate_cap=0.0, decay=None, writes=True, chunked=False, passes=None, readers=None):
     """The matrix-memory recurrence over each entry's tokens, in order:
     S <- a S + b k v^T, out = S^T q, with a fixed decay per head (``decay`` [heads]; a = decay,
     b = 1) or with ``gates`` [T, 2 * heads] (fp32: input gates then forget gates, ``gate_bias``
@@ -1166,7 +1166,8 @@ def memory_scan(out, q, k, v, state, item_slot, item_offset, item_count, heads, 
     another order); without, every token is a step of its own (single decoded tokens).
     ``passes``: three fp32 scratch tensors of ``memory_passes_scratch`` floats: the chunks are then
     taken side by side (their own sums, a scan over the chunks' states, their outputs) instead of
-    one after the other."""
+    one after the other.  ``readers``: int32 [entries * heads], zeros (left zero), in which the gated form counts with
+    ``chunked``; made here where the caller keeps none."""
     _check(out, "memory_scan.out", torch.float32, 2)
     for name, t in (("q", q), ("k", k), ("v", v)):
         _check(t, f"memory_scan.{name}", q.dtype, 2)
@@ -1212,6 +1213,13 @@ def memory_scan(out, q, k, v, state, item_slot, item_offset, item_count, heads, 
         both.max_chunks, both.n_items = n // 32 + n_items, n_items
         _memory_passes(ctypes.byref(both), dtype_code(q.dtype), _stream())
         return out
+    if gated and writes and chunked and vdim > 32:
+        if readers is None:
+            readers = torch.zeros(item_count.shape[0] * heads, dtype=torch.int32, device=q.device)
+        _check(readers, "memory_scan.readers", torch.int32, 1)
+        if readers.shape[0] < item_count.shape[0] * heads:
+            raise KernelError("memory_scan: too few counters")
+        params.readers = readers.data_ptr()
     (_memory_chunk if chunked else _memory_scan)(ctypes.byref(params), item_count.shape[0], dtype_code(q.dtype), _stream())
     return out
 

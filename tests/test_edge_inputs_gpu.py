@@ -72,3 +72,60 @@ def test_an_expert_named_more_than_once_by_its_tokens():
                     ld_down=experts * inner, tiles=tiles)
         # an activation's rounding is 2^-9 of it, 6 x 136 of them go into a sum of size 6
         np.testing.assert_allclose(f64(hidden), expected, rtol=0, atol=2e-2, err_msg=f"tiles={tiles}")
+
+
+def sigmoid_log(x):
+    return -np.logaddexp(0.0, -x)
+
+
+# six slices of the values and more blocks than the GPU holds at once; slices that take two launches; one slice
+@pytest.mark.parametrize("entries, heads, dim, vdim", [(63, 4, 96, 192), (5, 2, 40, 300), (9, 3, 16, 20)])
+@pytest.mark.parametrize("chunked", [False, True])
+@pytest.mark.parametrize("writes", [True, False])
+def test_gated_memories_of_more_entries_than_are_resident(entries, heads, dim, vdim, chunked, writes):
+    """The vector and the maximum that a head's slices share are read by every slice and written by one."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(entries + vdim)
+    cap, scale = 15.0, dim ** -0.5
+    bias = rng.normal(size=2 * heads).astype(np.float32)
+    state = dev(rng.normal(0, 0.5, (entries + 2, ops.memory_state_floats(heads, dim, vdim, True))), torch.float32)
+    slots = rng.permutation(entries + 2)[:entries]
+    held = f64(state)
+    S = held[slots, :heads * dim * vdim].reshape(entries, heads, dim, vdim)
+    n = held[slots, heads * dim * vdim:heads * dim * (vdim + 1)].reshape(entries, heads, dim)
+    m = held[slots, heads * dim * (vdim + 1):heads * dim * (vdim + 1) + heads]
+    for most in (1, 2, 3):
+        counts = rng.integers(0, most + 1, entries)
+        counts[:3] = (most, 0, 1)
+        offsets, total = np.cumsum(counts) - counts, int(counts.sum())
+        q, k, v = (dev(rng.normal(size=(total, heads * size)), torch.bfloat16) for size in (dim, dim, vdim))
+        gates = dev(rng.normal(0, 3, (total, 2 * heads)), torch.float32)
+        before, readers = state.clone(), torch.zeros(entries * heads + 1, dtype=torch.int32, device="cuda")
+        expected = np.zeros((total, heads, vdim))
+        S1, n1, m1 = S.copy(), n.copy(), m.copy()
+        for t in range(most):
+            e = np.flatnonzero(counts > t)
+            at = offsets[e] + t
+            qt, kt, vt = (f64(x)[at].reshape(len(e), heads, -1) for x in (q, k, v))
+            raw = f64(gates)[at] + bias
+            li, lf = cap * np.tanh(raw[:, :heads] / cap), sigmoid_log(cap * np.tanh(raw[:, heads:] / cap))
+            new = np.maximum(lf + m1[e], li)
+            a, b = np.exp(lf + m1[e] - new)[..., None], np.exp(li - new)[..., None]
+            S1[e] = a[..., None] * S1[e] + b[..., None] * kt[..., None] * vt[:, :, None]
+            n1[e], m1[e] = a * n1[e] + b * kt, new
+            qt = qt * scale
+            below = np.maximum(np.abs((n1[e] * qt).sum(-1)), np.exp(-new)) + 1e-6
+            expected[at] = np.einsum("ehdv,ehd->ehv", S1[e], qt) / below[..., None]
+        out = torch.full((total, heads * vdim), math.nan, device="cuda")
+        ops.memory_scan(out, q, k, v, state, dev(slots.astype(np.int32)), dev(offsets.astype(np.int32)), dev(counts.astype(np.int32)), heads, dim,
+                        vdim, q_scale=scale, gates=gates, gate_bias=dev(bias), gate_cap=cap, writes=writes, chunked=chunked,
+                        readers=readers if most > 1 else None)
+        assert int(readers.abs().sum()) == 0
+        # a state's entries below 10 and sums of `dim` products of them in 32 bits; the quotient's divisor is 0.01 or more here
+        np.testing.assert_allclose(f64(out), expected.reshape(total, -1), rtol=2e-5, atol=2e-5 * max(1.0, np.abs(expected).max()))
+        if writes:
+            S, n, m = S1, n1, m1
+            both = np.concatenate([S.reshape(entries, -1), n.reshape(entries, -1), m], 1)
+            np.testing.assert_allclose(f64(state)[slots], both, rtol=0, atol=5e-5)
+        else:
+            assert torch.equal(state, before)
