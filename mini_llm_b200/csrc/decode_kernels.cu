@@ -72,7 +72,7 @@ __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
 template <int ROWS, int WARPS>     // rows of x of a tile: 8 (half of the tensor core's) or 16
 __global__ void __launch_bounds__(WARPS * 32)
 skinny_linear_kernel(const SkinnyParams p, int split) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];             // normed rows [ROWS][K], if there is a norm; the sums otherwise
+    extern __shared__ __align__(16) unsigned char smem_raw[];             // the sums, then, if there is a norm, normed rows [ROWS or M][K]
     constexpr int AHEAD = 8, STEP = ROWS == 8 ? 8 : 4, STRIDE = ROWS + 1;  // (partial sums: [warp][feature][row])
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int m0 = blockIdx.y * ROWS;
@@ -204,7 +204,8 @@ static int g_smem_optin = -1;
 template <int ROWS, int WARPS>
 static int launch_skinny(const SkinnyParams& p, int split, cudaStream_t s) {
     const size_t sums = sizeof(float) * WARPS * 8 * (ROWS + 1);
-    const size_t smem = sums + (p.gamma != nullptr ? (size_t)ROWS * p.K * sizeof(bf16) : 0);
+    // (normed rows: those there are, so that one row may be as long as the sizes that are taken say)
+    const size_t smem = sums + (p.gamma != nullptr ? (size_t)(p.M < ROWS ? p.M : ROWS) * p.K * sizeof(bf16) : 0);
     if (g_smem_optin < 0) {
         int dev = 0;
         cudaGetDevice(&dev);

@@ -129,3 +129,20 @@ def test_gated_memories_of_more_entries_than_are_resident(entries, heads, dim, v
             np.testing.assert_allclose(f64(state)[slots], both, rtol=0, atol=5e-5)
         else:
             assert torch.equal(state, before)
+
+
+@pytest.mark.parametrize("m, k", [(1, 102400), (1, 14344), (2, 51200), (8, 12800), (16, 6400), (3, 25600)])
+def test_norms_inside_few_row_products_of_the_longest_rows_they_take(m, k):
+    from mini_llm_b200.kernels import ops
+    assert ops.skinny_linear_takes(m, k)
+    rng = np.random.default_rng(k)
+    n = 24
+    x, w = dev(rng.normal(2.0, 3.0, (m + 2, k)), torch.float32), dev(rng.normal(size=(n, k)) / math.sqrt(k), torch.bfloat16)
+    gain, shift = dev(rng.uniform(0.5, 1.5, k), torch.float32), dev(rng.normal(0, 0.1, k), torch.float32)
+    rows, out = rng.permutation(m + 2)[:m], torch.full((m, n), math.nan, device="cuda")
+    ops.skinny_linear(out, x, w, None, "store", norm=(gain, shift, 1e-5, dev(rows.astype(np.int32))))
+    c = f64(x)[rows] - f64(x)[rows].mean(-1, keepdims=True)
+    normed = c / np.sqrt((c * c).mean(-1, keepdims=True) + 1e-5) * f64(gain) + f64(shift)
+    # an entry of the normed row is rounded by 2^-9 of itself at most; over k products of size 1 / sqrt(k) that walks to 2^-9, of
+    # which no sum here is more than four times off
+    np.testing.assert_allclose(f64(out), normed @ f64(w).T, rtol=0, atol=8e-3)
