@@ -63,8 +63,10 @@ class DeferredNorm:
 
 class Kernels:
     FUSED_NORM_KINDS = ("layer_norm",)    # what the few-row product kernel can apply on the way in
-    FUSED_NORM_ROWS = 1                   # and of how many rows (the head of one wanted row): every block norms all of them, and
-                                          # a norm kernel ahead costs less (4096 x 1024, 8 rows: 8.6 against 11.8 us, 16: 9.4 against 17.4)
+    FUSED_NORM_ROWS = 2                   # and of how many rows: every block norms all of them, so from three on a norm kernel ahead costs
+                                          # less (2,304 x 768: 1 row 5.4 us against 7.1, 2 rows 6.6 against 7.3, 4 rows 7.9 against 7.3)
+    FUSED_NORM_FEATURES = 8192            # and of fewer features than this: a vocabulary's many blocks all norm (1 x 50,257 x 768: 21.5
+                                          # against 16.4 us, 1 x 6,400 x 1,600: 9.3 against 9.8)
 
     def __init__(self, act_dtype: torch.dtype, plain_only: bool = False):
         self.act_dtype = act_dtype
@@ -411,6 +413,9 @@ class Kernels:
         rows = 2 if n >= 8192 and k % 8 == 0 else (SKINNY_MAX_ROWS if k <= 4096 else 8)
         return not self.plain_only and m <= rows and ops.skinny_linear_takes(m, k)
 
+    def _norm_inside(self, a, w) -> bool:
+        return a.kind in self.FUSED_NORM_KINDS and a.shape[0] <= self.FUSED_NORM_ROWS and w.shape[0] < self.FUSED_NORM_FEATURES
+
     def linear(self, ctx, out, a, w, bias=None, epilogue="store"):
         """out = epilogue(a @ w.T + bias).  ``a``: an activation tensor or a ``DeferredNorm``."""
         m, k = a.shape
@@ -419,7 +424,7 @@ class Kernels:
         fast = w.shape[0] >= 16                  # (a product narrower than a tile's smallest box goes to the plain kernel)
         skinny = self._skinny(m, k, w.shape[0])
         deferred = isinstance(a, DeferredNorm)
-        if deferred and not (skinny and m <= self.FUSED_NORM_ROWS and a.kind in self.FUSED_NORM_KINDS):
+        if deferred and not (skinny and self._norm_inside(a, w)):
             a, deferred = a.materialize(ctx), False      # no kernel here norms this kind on the way in: the norm runs first
         if skinny:
             self.chose("linear", "skinny_linear", m, w.shape[0], k)
@@ -473,15 +478,19 @@ class Kernels:
         the cache pages (if this entry writes its cache); returns the queries [T, q_width]."""
         m, k = a.shape
         skinny = cache.writes and self._skinny(m, k)
-        if isinstance(a, DeferredNorm):
-            a = a.materialize(ctx)
+        deferred = isinstance(a, DeferredNorm)
+        if deferred and not (skinny and self._norm_inside(a, w)):
+            a, deferred = a.materialize(ctx), False
         if skinny:
             q = ctx.buffer("q", (m, q_width), ctx.act_dtype)
             scatter = (cache.k_pages, cache.v_pages, ctx.positions, ctx.token_item, cache.block_table,
                        cache.page_size, q_width, kv_width)
             self.launches += 1
             self.chose("qkv", "skinny_linear", m, w.shape[0], k)
-            ops.skinny_linear(q, a, w, bias, "store", scatter=scatter)
+            if deferred:
+                ops.skinny_linear(q, a.x, w, bias, "store", norm=(a.gamma, a.beta, a.eps, a.rows), scatter=scatter)
+            else:
+                ops.skinny_linear(q, a, w, bias, "store", scatter=scatter)
             return q
         if cache.writes and not self.plain_only and ops.gemm_qkv_takes(a, w, q_width, kv_width):
             q = ctx.buffer("q", (m, q_width), ctx.act_dtype)
