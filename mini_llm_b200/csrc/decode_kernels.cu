@@ -70,7 +70,7 @@ __device__ __forceinline__ void unpack8(const uint4& v, float* f) {
 // Replayed back to back, against a warp a feature that unpacked x from shared memory for every one: 8 x 768 x 768 5.6 -> 2.2 us,
 // 8 x 768 x 3072 13.3 -> 4.2, 16 x 3072 x 768 12.8 -> 3.6, 1 x 50257 x 768 19.2 -> 17.1 (floor 11.9).
 template <int ROWS, int WARPS, bool NORM>     // rows of x of a tile: 8 (half of the tensor core's) or 16
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 3 : (ROWS == 8 ? 2 : 1))
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 skinny_linear_kernel(const SkinnyParams p, int split) {
     extern __shared__ __align__(16) unsigned char smem_raw[];             // the sums, then, if there is a norm, normed rows [ROWS or M][K]
     constexpr int AHEAD = 8, STEP = ROWS == 8 ? 8 : 4, STRIDE = ROWS + 1;  // (partial sums: [warp][feature][row])
@@ -169,7 +169,9 @@ skinny_linear_kernel(const SkinnyParams p, int split) {
         residual_mine = residual(n_mine, m_mine);
     }
 
-    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    // Every product of 16 entries of K is added by a rounded addition, in turn to one of four sums: left in the tensor cores'
+    // accumulators, whose sums are cut off, the error against 64 bits was up to ten times that of rounded FMAs.
+    float sums_of[4][4] = {};
     const bool low_there = g < m_count, high_there = ROWS > 8 && g + 8 < m_count;
     const uint4* x_low = reinterpret_cast<const uint4*>(x + (long)g * ldx);
     const uint4* x_high = reinterpret_cast<const uint4*>(x + (long)(g + 8) * ldx);
@@ -190,11 +192,15 @@ skinny_linear_kernel(const SkinnyParams p, int split) {
                 const uint4 w = wv[half + i];
                 const int c = (first + AHEAD + half + i) * 4 + tq;
                 wv[half + i] = first + AHEAD + half + i < end && c < pieces ? __ldg(w_row + c) : none;
-                mma_bf16_16816(acc[0], acc[1], acc[2], acc[3], xl[i].x, xh[i].x, xl[i].y, xh[i].y, w.x, w.y);
-                mma_bf16_16816(acc[0], acc[1], acc[2], acc[3], xl[i].z, xh[i].z, xl[i].w, xh[i].w, w.z, w.w);
+                const uint32_t first_half[4] = {xl[i].x, xh[i].x, xl[i].y, xh[i].y}, second_half[4] = {xl[i].z, xh[i].z, xl[i].w, xh[i].w};
+                mma_added(sums_of[2 * (i & 1)], first_half, w.x, w.y);
+                mma_added(sums_of[2 * (i & 1) + 1], second_half, w.z, w.w);
             }
         }
     }
+    float acc[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) acc[e] = (sums_of[0][e] + sums_of[1][e]) + (sums_of[2][e] + sums_of[3][e]);
     float* sums = partial + (warp * 8 + 2 * tq) * STRIDE + g;
     sums[0] = acc[0];
     sums[STRIDE] = acc[1];
@@ -257,14 +263,14 @@ static int launch_skinny(const SkinnyParams& p, int split, cudaStream_t s) {
                     "skinny_linear_kernel");
 }
 
-// Warps that share a tile's K: all eight of a block while the tiles' blocks run side by side (three an SM), fewer where the
-// features alone bring enough warps (a vocabulary: one warp a tile); sixteen for a long K of few features, so that each
-// warp's share is asked for ahead as a whole.
+// Warps that share a tile's K: all eight of a block while the tiles' blocks run side by side (two an SM), fewer where the
+// features alone bring enough warps (a vocabulary: one warp a tile; with eight it took 25.3 us in place of 14.3, as every block's
+// sums meet); sixteen for a long K of few features, so that each warp's share is asked for ahead as a whole.
 template <int ROWS, bool NORM>
 static int launch_skinny_rows(const SkinnyParams& p, cudaStream_t s) {
     const long tiles = (long)((p.N + 7) / 8) * p.batch;
-    if (p.K > 2048 && tiles <= 296) return launch_skinny<ROWS, 16, NORM>(p, 16, s);
-    return launch_skinny<ROWS, 8, NORM>(p, tiles <= 444 ? 8 : tiles <= 888 ? 4 : tiles <= 1776 ? 2 : 1, s);
+    if (p.K > 2048 && tiles <= 148) return launch_skinny<ROWS, 16, NORM>(p, 16, s);
+    return launch_skinny<ROWS, 8, NORM>(p, tiles <= 296 ? 8 : tiles <= 592 ? 4 : tiles <= 1184 ? 2 : 1, s);
 }
 
 extern "C" int mllm_decode_skinny_linear(const SkinnyParams* params, void* stream) {

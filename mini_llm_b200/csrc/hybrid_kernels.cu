@@ -2324,7 +2324,7 @@ __device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, i
 
 // A block: 16 inner features of an expert, in two tiles of 8 whose K four warps share.
 template <int FORM>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long ld_x, const int* choice, const float* in_weight,
                        const long long* __restrict__ gate_of, const long long* __restrict__ up_of, const int* __restrict__ inner_of,
                        int width, int pairs, int n_tokens, float limit, float shared_limit, float alpha, int n_experts) {
@@ -2408,11 +2408,12 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
                         for (int k = 0; k < 4; k++) two[k] = __floats2bfloat162_rn(scale[r] * y[2 * k], scale[r] * y[2 * k + 1]);
                         xv[i][r] = *reinterpret_cast<const uint4*>(two);
                     }
-                mma_bf16_16816(zu[0], zu[1], zu[2], zu[3], xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y, u.x, u.y);
-                mma_bf16_16816(zu[0], zu[1], zu[2], zu[3], xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w, u.z, u.w);
+                const uint32_t first_half[4] = {xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y}, second_half[4] = {xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w};
+                mma_added(zu, first_half, u.x, u.y);
+                mma_added(zu, second_half, u.z, u.w);
                 if (GATED) {
-                    mma_bf16_16816(zg[0], zg[1], zg[2], zg[3], xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y, v.x, v.y);
-                    mma_bf16_16816(zg[0], zg[1], zg[2], zg[3], xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w, v.z, v.w);
+                    mma_added(zg, first_half, v.x, v.y);
+                    mma_added(zg, second_half, v.z, v.w);
                 }
             }
         }
@@ -2519,8 +2520,10 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
                 }
 #pragma unroll
                 for (int i = 0; i < BLOCKS; i++) {
-                    mma_bf16_16816(z[0], z[1], z[2], z[3], av[i][0].x, av[i][1].x, av[i][0].y, av[i][1].y, wv[i].x, wv[i].y);
-                    mma_bf16_16816(z[0], z[1], z[2], z[3], av[i][0].z, av[i][1].z, av[i][0].w, av[i][1].w, wv[i].z, wv[i].w);
+                    const uint32_t first_half[4] = {av[i][0].x, av[i][1].x, av[i][0].y, av[i][1].y};
+                    const uint32_t second_half[4] = {av[i][0].z, av[i][1].z, av[i][0].w, av[i][1].w};
+                    mma_added(z, first_half, wv[i].x, wv[i].y);
+                    mma_added(z, second_half, wv[i].z, wv[i].w);
                 }
             }
             float* mine = down_shared + (unit * 32 + m0 + g) * 8 + 2 * tq;

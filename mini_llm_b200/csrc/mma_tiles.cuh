@@ -55,8 +55,10 @@ __device__ __forceinline__ void terms_of(uint32_t (&a)[3][4], const float (&x)[4
 // A tile's sum is cut off at 24 bits when it is added to what the accumulators held: over a long row of products that adds up.
 // The product by itself, added with a rounded addition, keeps a sum as near as a chain of FMAs does.
 __device__ __forceinline__ void mma_added(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    float x[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    mma_tile(x, a, b0, b1);
+    float x[4];
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%10, %10, %10, %10};"
+        : "=f"(x[0]), "=f"(x[1]), "=f"(x[2]), "=f"(x[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 #pragma unroll
     for (int e = 0; e < 4; e++) c[e] += x[e];
 }

@@ -146,3 +146,38 @@ def test_norms_inside_few_row_products_of_the_longest_rows_they_take(m, k):
     # an entry of the normed row is rounded by 2^-9 of itself at most; over k products of size 1 / sqrt(k) that walks to 2^-9, of
     # which no sum here is more than four times off
     np.testing.assert_allclose(f64(out), normed @ f64(w).T, rtol=0, atol=8e-3)
+
+
+@pytest.mark.parametrize("m, n, k", [(2, 16384, 3072), (8, 24, 4096), (8, 768, 768), (16, 3072, 768)])
+def test_few_row_products_of_one_sign(m, n, k):
+    """Sums that only grow: what is cut off them instead of rounded would add up."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(n)
+    x, w = dev(rng.uniform(size=(m, k)), torch.bfloat16), dev(rng.uniform(size=(n, k)), torch.bfloat16)
+    out, heads = torch.empty(m, n, device="cuda"), torch.empty(m, n, device="cuda")
+    ops.skinny_linear(out, x, w, None, "store")
+    ops.skinny_heads(heads, x, w[None].contiguous(), 1, k, n)
+    want = (x.double() @ w.double().T)
+    # 16 entries' product is cut off by 2^-24 of itself at most, their additions and the last rounding are off by as much of what is
+    # summed, up or down: some 2^-23 of a result together (as one chain in the tensor cores 1.1e-7 to 5e-6)
+    for got in (out, heads):
+        assert float((got.double() - want).norm() / want.norm()) < 1.0e-7
+
+
+def test_expert_tiles_of_one_sign():
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(0)
+    tokens, experts, inner, width = 16, 4, 768, 64
+    total = experts * inner
+    gates, ups, downs = (dev(rng.uniform(0.0, 0.1, s), torch.bfloat16) for s in ((total, width), (total, width), (width, total)))
+    at = lambda matrix, step: torch.tensor([matrix.data_ptr() + 2 * step * e * inner for e in range(experts)], dtype=torch.int64, device="cuda")
+    chosen = np.stack([rng.permutation(experts)[:2] for _ in range(tokens)]).astype(np.int32)
+    x, ones = dev(rng.uniform(size=(tokens, width)), torch.bfloat16), torch.ones(tokens * 2, device="cuda")
+    hidden, act = torch.zeros(tokens, width, device="cuda"), torch.empty(tokens * 2, inner, dtype=torch.bfloat16, device="cuda")
+    ops.experts(hidden, act, x, dev(chosen.reshape(-1)), ones, ones, at(gates, width), at(ups, width), at(downs, 1), dev(np.full(experts, inner, np.int32)),
+                inner, 2, ld_down=total, tiles=True)
+    want = np.zeros((tokens, width))
+    for t in range(tokens):
+        for j, e in enumerate(chosen[t]):
+            want[t] += f64(downs)[:, e * inner:(e + 1) * inner] @ f64(act)[2 * t + j]
+    assert np.linalg.norm(f64(hidden) - want) / np.linalg.norm(want) < 1.0e-7          # (as above; 2.5e-7 as chains of 256)
