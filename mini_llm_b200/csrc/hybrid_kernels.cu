@@ -2723,7 +2723,7 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
         const bf16* xb = (const bf16*)x;
         bf16* ab = (bf16*)act;
 #define UP_TILES(FORM)                                                                                                           \
-    launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_up_tiles_kernel<FORM>, tiles, dim3(256), 0, s, ab, ld_act, xb, ld_x, choice, in_weight, \
+    launch_kernel(g_dependent_launch != 0, expert_up_tiles_kernel<FORM>, tiles, dim3(256), 0, s, ab, ld_act, xb, ld_x, choice, in_weight, \
                   gate_of, up_of, inner_of, width, pairs, n_tokens, limit, shared_limit, alpha, n_experts)
         if (form == EXPERT_GATED_SILU) UP_TILES(EXPERT_GATED_SILU);
         else if (form == EXPERT_RELU_SQUARED) UP_TILES(EXPERT_RELU_SQUARED);

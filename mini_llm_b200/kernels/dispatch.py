@@ -181,10 +181,16 @@ class Kernels:
         return ops.route(x, router, shared_gate, top, choice, in_weight, out_weight, **how)
 
     def experts(self, hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
-                ld_down=None, assign=False, identity_weight=None, eights=False, **form):
-        """``eights``: every expert's inner size is a multiple of 8."""
+                ld_down=None, assign=False, identity_weight=None, eights=False, features=0, **form):
+        """``eights``: every expert's inner size is a multiple of 8; ``features``: inner features of all experts of a token.
+        Pair by pair a block has 32 features of a pair, and an expert's weights are read once a pair: as fast as the tiles, which
+        find every expert's pairs first, or faster, while those blocks fit the GPU at once (592, four an SM).  Only one or two
+        tokens, whose blocks are few, go through the tiles all the same.  A layer of 8 experts of 768, two and a shared one of
+        1,536 a token, norm and router with it, at 1, 4, 8, 16 tokens: tiles 22.4, 28.9, 29.9, 31.2 us, pairs 27.0, 27.3, 33.1, 44.3; 16 experts of 512, two and a shared one of
+        512, at 2, 12, 16, 31: tiles 21.4, 31.5, 31.8, 38.9, pairs 22.4, 24.5, 33.6, 44.8."""
         self.launches += 2
-        tiles = eights and not self.plain_only and ld_down is not None and ops.expert_tiles_take(x, act, inner_of.shape[0], ld_down)
+        tiles = (eights and not self.plain_only and ld_down is not None and ops.expert_tiles_take(x, act, inner_of.shape[0], ld_down)
+                 and (x.shape[0] <= 2 or x.shape[0] * features > 592 * 32))
         self.chose("experts", "expert_tiles" if tiles else "expert_pairs", x.shape[0], max_inner, x.shape[1])
         return ops.experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
                            ld_down, assign, identity_weight, tiles=tiles, **form)

@@ -169,7 +169,8 @@ class RoutedExperts(FeedForward):
         act = ctx.buffer("expert_act", (n * self.pairs, self.max_inner), ctx.act_dtype)
         k.experts(hidden, act, x, choice, in_weight, out_weight, self.gate_of, self.up_of, self.down_of, self.inner_of,
                   self.max_inner, self.pairs, ld_down=self.total, assign=assign, identity_weight=identity,
-                  n_experts=self.n_experts, eights=self.eights, **self.form_constants)
+                  n_experts=self.n_experts, eights=self.eights, features=self.top * self.inner + (self.shared_inner or 0),
+                  **self.form_constants)
 
     def compute(self, ctx, x):
         out = ctx.buffer("mlp_out", (x.shape[0], self.width), torch.float32)
