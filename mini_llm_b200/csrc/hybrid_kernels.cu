@@ -2730,12 +2730,6 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
         else UP_TILES(EXPERT_CLAMPED_GLU);
 #undef UP_TILES
         const size_t bytes = sizeof(float) * EXPERT_UNITS * 32 * 8 + sizeof(int) * (size_t)n_tokens * pairs;
-        static bool configured = false;
-        if (!configured) {
-            if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
-                return fail("experts: cannot raise the shared memory limit");
-            configured = true;
-        }
         if (bytes > 128 * 1024) return fail("experts: too many pairs for the tiles");
         launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_down_tiles_kernel, dim3((width + 7) / 8), dim3(512), bytes, s, hidden, ld_hidden,
                       (const bf16*)act, ld_act, choice, out_weight, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, assign, xb,
@@ -2780,6 +2774,9 @@ __global__ void scaled_add_kernel(float* __restrict__ x, const float* __restrict
 }
 
 extern "C" int mllm_hybrid_scaled_add(float* x, const float* u, float a, const float* v, float b, long n, int assign, void* stream) {
+        // (at every launch, as the limit is a device's own)
+        if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
+            return fail("experts: cannot raise the shared memory limit");
     if (n <= 0) return 0;
     long blocks = (n + 255) / 256;
     if (blocks > 4096) blocks = 4096;
