@@ -181,3 +181,31 @@ def test_expert_tiles_of_one_sign():
         for j, e in enumerate(chosen[t]):
             want[t] += f64(downs)[:, e * inner:(e + 1) * inner] @ f64(act)[2 * t + j]
     assert np.linalg.norm(f64(hidden) - want) / np.linalg.norm(want) < 1.0e-7          # (as above; 2.5e-7 as chains of 256)
+
+
+# tokens that stand alone beside a portion (few tokens a block) and a prompt whose blocks fill the GPU (as many as fit)
+@pytest.mark.parametrize("lengths, new, heads, kv_heads, window", [
+    ([90 + 7 * i for i in range(20)] + [60], [1] * 20 + [60], 12, 4, 0), ([700], [700], 12, 4, 0), ([200] * 9 + [33, 2], [1] * 9 + [33, 2], 4, 4, 64)])
+def test_capped_attention_of_tokens_that_stand_alone_beside_portions(lengths, new, heads, kv_heads, window):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(len(new))
+    dim, page = 64, 16
+    table, (k_pages, v_pages) = pages_of(rng, lengths, page, kv_heads, (dim, dim))
+    positions = dev(np.concatenate([np.arange(l - m, l) for l, m in zip(lengths, new)]).astype(np.int32))
+    items, n = dev(np.repeat(np.arange(len(new)), new).astype(np.int32)), sum(new)
+    q = dev(rng.normal(size=(n, heads * dim)), torch.bfloat16)
+    want, got = (torch.full((n, heads * dim), math.nan, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for out, tiled in ((want, False), (got, True)):
+        ops.capped_attention(out, q, k_pages, v_pages, table.cuda(), positions, items, heads, kv_heads, dim, dim, page, dim ** -0.5, cap=20.0,
+                             window=window, tiled=tiled)
+    # both keep scores, weights and sums in 32 bits, so they may differ by the last rounding to 8 bits: 2^-8 of values below 4
+    np.testing.assert_allclose(f64(got), f64(want), rtol=2 ** -7, atol=2 ** -10)
+
+
+def pages_of(rng, lengths, page, heads, size):
+    blocks = [-(-n // page) for n in lengths]
+    table = torch.zeros(len(lengths), max(blocks), dtype=torch.int32)
+    order = rng.permutation(sum(blocks))
+    for i, count in enumerate(blocks):
+        table[i, :count] = torch.tensor(order[sum(blocks[:i]):sum(blocks[:i]) + count])
+    return table, [dev(rng.normal(size=(sum(blocks), page, heads, s)), torch.bfloat16) for s in size]
