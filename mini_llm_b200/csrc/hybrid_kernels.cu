@@ -1434,7 +1434,7 @@ static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStr
     return check_launch("linear_recurrence_kernel");
 }
 
-// ---- few tokens an entry ---------------------------------------------------------------------------
+// ---- one token an entry ----------------------------------------------------------------------------
 // Keys of up to 128 entries.  One token's update reads and writes the state once (0.3 us of HBM time for an entry of six heads of
 // 128 x 128), so what it takes is the way there and back: a block takes 32 columns of a head, a lane a column and a warp 16 rows,
 // all asked for at once and kept in registers, and both sums over the old state meet in shared memory once.  Staging the
@@ -1892,12 +1892,19 @@ static int launch_recurrence(const RecurrenceParams& pp, int n_items, cudaStream
 }
 
 // A column of the state lies in the registers of 4 to 32 lanes of a warp.  Prompt portions: eight
-// rows a lane up to a key size of 256 (short sums).  Steps of few tokens per entry have a kernel of their own.
+// rows a lane up to a key size of 256 (short sums).  Steps of few tokens per entry: as many rows a
+// lane as registers hold, so that the blocks, each of which pays the same chain of loads for its
+// few tokens, are few.  Steps of one token an entry (or two more in all) have a kernel of their own, which asks for a token's
+// values when the one before is done: beside them an entry of many tokens would wait for each (63 entries of one token and one of 95, 6 heads of
+// 128 x 128: 155 us, 80 on the walk; one entry of four, heads of 64 x 64: 7.8 and 5.9).
 template <typename T>
 static int pick_recurrence(const RecurrenceParams& pp, int n_items, int n_tokens, cudaStream_t s) {
     if (pp.dim <= 32) return launch_recurrence<T, 8, 4, 16, 1>(pp, n_items, s);
-    if (pp.dim <= 128 && n_tokens <= 4 * n_items) return launch_recurrence_few<T>(pp, n_items, s);
-    if (pp.dim <= 128) {
+    if (pp.dim <= 128 && n_tokens <= n_items + 2) return launch_recurrence_few<T>(pp, n_items, s);
+    if (n_tokens <= 4 * n_items) {
+        if (pp.dim <= 64) return launch_recurrence<T, 16, 4, 16, 1>(pp, n_items, s);
+        if (pp.dim <= 128) return launch_recurrence<T, 32, 4, 16, 1>(pp, n_items, s);
+    } else if (pp.dim <= 128) {
         // Prompt portions.  The walk from token to token is a chain of dependent sums and exchanges
         // between lanes; a thread takes two columns, whose chains run in one another's gaps, or four
         // where two would leave the busy entries' blocks more than one an SM (entries of a step that

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from test_kernels_gpu import dev, f64
+from test_product_kernels_gpu import recurrence_case
 
 pytestmark = pytest.mark.gpu
 
@@ -209,3 +210,9 @@ def pages_of(rng, lengths, page, heads, size):
     for i, count in enumerate(blocks):
         table[i, :count] = torch.tensor(order[sum(blocks[:i]):sum(blocks[:i]) + count])
     return table, [dev(rng.normal(size=(sum(blocks), page, heads, s)), torch.bfloat16) for s in size]
+
+
+# portions of some tokens beside tokens that stand alone: more than the kernel for one token an entry takes, fewer than the chunks'
+@pytest.mark.parametrize("heads, qk_heads, dim, vdim, delta", [(2, 1, 64, 24, True), (4, 2, 128, 33, True), (3, 3, 40, 65, False)])
+def test_recurrence_of_uneven_entries(heads, qk_heads, dim, vdim, delta):
+    recurrence_case(heads, qk_heads, dim, vdim, delta, ([1, 1, 11, 1], [2, 2, 1, 3], [1, 3, 1, 1]))
