@@ -429,8 +429,8 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
         m = m_new;
         // the weights, 16 keys in the rows, their three bfloat16 terms (all 24 bits) in the first three columns
         uint32_t low[3], high[3];
-        three_terms(__shfl_sync(0xffffffffu, x[0], 8 * tq), __shfl_sync(0xffffffffu, x[0], 8 * tq + 4), low[0], low[1], low[2]);
-        three_terms(__shfl_sync(0xffffffffu, x[1], 8 * tq), __shfl_sync(0xffffffffu, x[1], 8 * tq + 4), high[0], high[1], high[2]);
+        three_weight_terms(__shfl_sync(0xffffffffu, x[0], 8 * tq), __shfl_sync(0xffffffffu, x[0], 8 * tq + 4), low[0], low[1], low[2]);
+        three_weight_terms(__shfl_sync(0xffffffffu, x[1], 8 * tq), __shfl_sync(0xffffffffu, x[1], 8 * tq + 4), high[0], high[1], high[2]);
         const uint32_t b0 = g == 0 ? low[0] : (g == 1 ? low[1] : (g == 2 ? low[2] : 0u));
         const uint32_t b1 = g == 0 ? high[0] : (g == 1 ? high[1] : (g == 2 ? high[2] : 0u));
 #pragma unroll

@@ -905,7 +905,7 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
                 }
                 uint32_t a[2][3][4];
 #pragma unroll
-                for (int k = 0; k < 2; k++) terms_of(a[k], s[2 * k], s[2 * k + 1]);
+                for (int k = 0; k < 2; k++) weight_terms_of(a[k], s[2 * k], s[2 * k + 1]);
 #pragma unroll
                 for (int j = 0; j < VALUE / 8; j += 2) {
                     uint32_t b[2][4];
@@ -1552,13 +1552,13 @@ template <int DIM> struct RecurrenceShared {
 
 __device__ __forceinline__ void barrier_of_128(int id) { asm volatile("bar.sync %0, 128;" ::"r"(id) : "memory"); }
 
-// c = a b, both 32-bit as three terms; the products whose terms are together below 2^-24 of the largest are left out.
+// c = a b, both 32-bit as three terms; the product of the two smallest, 2^-28 of the largest at most, is left out.
 __device__ __forceinline__ void mma_terms(float (&c)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][4], int half) {
     c[0] = c[1] = c[2] = c[3] = 0.0f;
 #pragma unroll
-    for (int order = 2; order >= 1; order--)
+    for (int order = 3; order >= 1; order--)
 #pragma unroll
-        for (int i = 0; i <= order; i++) mma_tile(c, a[i], half ? b[order - i][2] : b[order - i][0], half ? b[order - i][3] : b[order - i][1]);
+        for (int i = order == 3 ? 1 : 0; i <= order && i < 3; i++) mma_tile(c, a[i], half ? b[order - i][2] : b[order - i][0], half ? b[order - i][3] : b[order - i][1]);
     mma_added(c, a[0], half ? b[0][2] : b[0][0], half ? b[0][3] : b[0][1]);
 }
 
@@ -1590,6 +1590,29 @@ __global__ void __launch_bounds__(320, 1) recurrence_chunks_kernel(RecurrencePar
             }
     }
     const float skip = pp.skip != nullptr ? pp.skip[head] : 0.0f;
+    // y(t) = the sum over s <= t of L(t, s) x(s), one product after the other: where an x is no finite number, the zeros that
+    // the tensor cores take in place of the L(t, s) of later tokens would carry it into earlier ones.
+    auto lower_product = [&](const bf16 (&terms)[3][REC_TOKENS * REC_LD], const float (&x)[2][4], float (&y)[2][4]) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) y[e / 4][e % 4] = 0.0f;
+#pragma unroll
+        for (int s_ = 0; s_ < REC_TOKENS; s_++) {
+            const int from = g * 4 + s_ % 8 / 2;
+            const float left = __shfl_sync(0xffffffffu, x[s_ / 8][s_ % 2], from), right = __shfl_sync(0xffffffffu, x[s_ / 8][2 + s_ % 2], from);
+#pragma unroll
+            for (int e = 0; e < 8; e++) {
+                const int t = e / 4 * 8 + 2 * tq + (e & 1), at = t * REC_LD + s_;
+                const float l = to_f32(terms[0][at]) + (to_f32(terms[1][at]) + to_f32(terms[2][at]));
+                if (s_ <= t) y[e / 4][e % 4] = fmaf(l, (e & 2) ? right : left, y[e / 4][e % 4]);
+            }
+        }
+    };
+    auto all_finite = [&](const float (&x)[2][4]) {
+        bool finite = true;
+#pragma unroll
+        for (int e = 0; e < 8; e++) finite = finite && fabsf(x[e / 4][e % 4]) < INFINITY;
+        return __all_sync(0xffffffffu, finite) != 0;
+    };
     auto walk = [&](int i) {
         const RecurrenceRows<DIM>& rows = sh.rows[i % REC_ROW_SLOTS];
         const RecurrenceChunk& ch = sh.chunk[i % REC_SLOTS];
@@ -1638,6 +1661,7 @@ __global__ void __launch_bounds__(320, 1) recurrence_chunks_kernel(RecurrencePar
             for (int term = 0; term < 3; term++) load_blocks(b[term], ch.solve[term] + ((lane & 7) + ((lane >> 4) & 1) * 8) * REC_LD + ((lane >> 3) & 1) * 8);
             mma_terms(u[0], a, b, 0);
             mma_terms(u[1], a, b, 1);
+            if (!all_finite(r)) lower_product(ch.solve, r, u);
         } else {
 #pragma unroll
             for (int j = 0; j < 2; j++)
@@ -1672,6 +1696,12 @@ __global__ void __launch_bounds__(320, 1) recurrence_chunks_kernel(RecurrencePar
             for (int term = 0; term < 3; term++) load_blocks(b[term], ch.read[term] + ((lane & 7) + ((lane >> 4) & 1) * 8) * REC_LD + ((lane >> 3) & 1) * 8);
             float o[4];
             mma_terms(o, a, b, warp);
+            if (!all_finite(u)) {
+                float y[2][4];
+                lower_product(ch.read, u, y);
+#pragma unroll
+                for (int e = 0; e < 4; e++) o[e] = warp == 0 ? y[0][e] : y[1][e];
+            }
             const float4 x = sh.sums[0][2 + warp][lane], y = sh.sums[1][2 + warp][lane], z = sh.sums[2][2 + warp][lane], w = sh.sums[3][2 + warp][lane];
             const float old[4] = {(x.x + y.x) + (z.x + w.x), (x.y + y.y) + (z.y + w.y), (x.z + y.z) + (z.z + w.z), (x.w + y.w) + (z.w + w.w)};
 #pragma unroll
@@ -2744,6 +2774,9 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
 #undef UP_TILES
         const size_t bytes = sizeof(float) * EXPERT_UNITS * 32 * 8 + sizeof(int) * (size_t)n_tokens * pairs;
         if (bytes > 128 * 1024) return fail("experts: too many pairs for the tiles");
+        // (at every launch, as the limit is a device's own)
+        if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
+            return fail("experts: cannot raise the shared memory limit");
         launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_down_tiles_kernel, dim3((width + 7) / 8), dim3(512), bytes, s, hidden, ld_hidden,
                       (const bf16*)act, ld_act, choice, out_weight, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, assign, xb,
                       ld_x, identity_weight);
@@ -2787,9 +2820,6 @@ __global__ void scaled_add_kernel(float* __restrict__ x, const float* __restrict
 }
 
 extern "C" int mllm_hybrid_scaled_add(float* x, const float* u, float a, const float* v, float b, long n, int assign, void* stream) {
-        // (at every launch, as the limit is a device's own)
-        if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
-            return fail("experts: cannot raise the shared memory limit");
     if (n <= 0) return 0;
     long blocks = (n + 255) / 256;
     if (blocks > 4096) blocks = 4096;

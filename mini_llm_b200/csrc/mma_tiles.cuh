@@ -33,15 +33,29 @@ template <int LEFT> __device__ __forceinline__ void copies_landed() { asm volati
 
 // Two 32-bit numbers as three pairs of bfloat16 whose sums they are: 8 bits of the significand a term, all 24 in three.  A
 // product of such an operand with a bfloat16 one is three products with 32-bit sums, and rounds where those sums do.
+// The terms are cut off, not rounded, so that they have the number's sign, and a term is 2^-126 rather than zero where the number
+// is not: times an infinity all three are the infinity that the number times it is (with a rounded term of the other sign, or
+// a zero, their sum would be no number), and times anything else 2^-126 is nothing beside the first term.
+__device__ __forceinline__ uint32_t upper_halves(float low, float high) { return __byte_perm(__float_as_uint(low), __float_as_uint(high), 0x7632); }
+__device__ __forceinline__ float upper_half(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
 __device__ __forceinline__ void three_terms(float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
-    __nv_bfloat162 t = __floats2bfloat162_rn(x, y);
-    first = *reinterpret_cast<uint32_t*>(&t);
-    x -= __low2float(t), y -= __high2float(t);
-    t = __floats2bfloat162_rn(x, y);
-    second = *reinterpret_cast<uint32_t*>(&t);
-    x -= __low2float(t), y -= __high2float(t);
-    t = __floats2bfloat162_rn(x, y);
-    third = *reinterpret_cast<uint32_t*>(&t);
+    constexpr float LEAST = 1.1754943508222875e-38f;                      // 2^-126
+    const float least_x = fminf(fabsf(x), LEAST), least_y = fminf(fabsf(y), LEAST);
+    first = upper_halves(x, y);
+    // (of an infinity nothing is left that is a number: fmaxf takes the other)
+    const float x2 = x - upper_half(x), y2 = y - upper_half(y);
+    second = upper_halves(copysignf(fmaxf(fabsf(upper_half(x2)), least_x), x), copysignf(fmaxf(fabsf(upper_half(y2)), least_y), y));
+    const float x3 = x2 - upper_half(x2), y3 = y2 - upper_half(y2);
+    third = upper_halves(copysignf(fmaxf(fabsf(x3), least_x), x), copysignf(fmaxf(fabsf(y3), least_y), y));
+}
+// The same for numbers that are not negative (an attention's weights).
+__device__ __forceinline__ void three_weight_terms(float x, float y, uint32_t& first, uint32_t& second, uint32_t& third) {
+    constexpr float LEAST = 1.1754943508222875e-38f;
+    const float least_x = fminf(x, LEAST), least_y = fminf(y, LEAST);
+    first = upper_halves(x, y);
+    const float x2 = x - upper_half(x), y2 = y - upper_half(y);
+    second = upper_halves(fmaxf(upper_half(x2), least_x), fmaxf(upper_half(y2), least_y));
+    third = upper_halves(fmaxf(x2 - upper_half(x2), least_x), fmaxf(y2 - upper_half(y2), least_y));
 }
 
 // The accumulators of two tiles, 16 rows by 16, as the first operand of the next product.
@@ -61,6 +75,13 @@ __device__ __forceinline__ void mma_added(float (&c)[4], const uint32_t (&a)[4],
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 #pragma unroll
     for (int e = 0; e < 4; e++) c[e] += x[e];
+}
+
+__device__ __forceinline__ void weight_terms_of(uint32_t (&a)[3][4], const float (&x)[4], const float (&y)[4]) {
+    three_weight_terms(x[0], x[1], a[0][0], a[1][0], a[2][0]);
+    three_weight_terms(x[2], x[3], a[0][1], a[1][1], a[2][1]);
+    three_weight_terms(y[0], y[1], a[0][2], a[1][2], a[2][2]);
+    three_weight_terms(y[2], y[3], a[0][3], a[1][3], a[2][3]);
 }
 
 // x = the weights of 16 rows and 32 keys, as three terms, times two tiles of eight value columns: the small terms first.

@@ -1286,7 +1286,7 @@ latent_attention_mma_kernel(LatentTiledParams p) {
             const bf16* v_at = kt + ((lane & 7) + ((lane >> 3) & 1) * 8) * ld + ((lane >> 4) & 1) * 8;
             uint32_t a[2][3][4];
 #pragma unroll
-            for (int k = 0; k < 2; k++) terms_of(a[k], s[2 * k], s[2 * k + 1]);
+            for (int k = 0; k < 2; k++) weight_terms_of(a[k], s[2 * k], s[2 * k + 1]);
 #pragma unroll
             for (int j = 0; j < RANK / 8; j += 2) {
                 uint32_t b[2][4];

@@ -216,3 +216,110 @@ def pages_of(rng, lengths, page, heads, size):
 @pytest.mark.parametrize("heads, qk_heads, dim, vdim, delta", [(2, 1, 64, 24, True), (4, 2, 128, 33, True), (3, 3, 40, 65, False)])
 def test_recurrence_of_uneven_entries(heads, qk_heads, dim, vdim, delta):
     recurrence_case(heads, qk_heads, dim, vdim, delta, ([1, 1, 11, 1], [2, 2, 1, 3], [1, 3, 1, 1]))
+
+
+def cell(pages, table, entry, position):
+    return pages[int(table[entry, position // pages.shape[1]]), position % pages.shape[1]]
+
+
+@pytest.mark.parametrize("dim", [64, 128])
+def test_infinite_cached_values_in_tiled_attention(dim):
+    """An infinite value makes its column infinite where its key is seen, and a key that is infinitely far away weighs nothing."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(dim)
+    heads, kv_heads, page, lengths = 4, 2, 16, [100, 70]
+    table, (k_pages, v_pages) = pages_of(rng, lengths, page, kv_heads, (dim, dim))
+    cell(v_pages, table, 0, 3)[1, 5] = math.inf
+    cell(v_pages, table, 0, 40)[0, 9] = -math.inf
+    cell(v_pages, table, 1, 20)[1, 7] = math.inf
+    cell(k_pages, table, 1, 2)[0, 1] = -math.inf                  # (queries are positive there: the score is -infinity)
+    new = [50, 45]
+    positions = dev(np.concatenate([np.arange(l - m, l) for l, m in zip(lengths, new)]).astype(np.int32))
+    items, n = dev(np.repeat(np.arange(2), new).astype(np.int32)), sum(new)
+    q = dev(rng.normal(size=(n, heads * dim)), torch.bfloat16)
+    q.view(n, heads, dim)[:, :, 1].abs_()
+    tiled, split = (torch.full((n, heads * dim), math.nan, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    common = (k_pages, v_pages, table.cuda(), positions, items, heads, kv_heads, dim)
+    ops.capped_attention(tiled, q, *common, dim, page, dim ** -0.5, tiled=True)
+    scratch = (torch.empty(n * heads * 4 * dim, device="cuda"), torch.empty(n * heads * 8, device="cuda"),
+               torch.zeros(n * heads, dtype=torch.int32, device="cuda"))
+    ops.split_attention(split, q, *common, page, dim ** -0.5, 0, 64, -(-table.shape[1] * page // 64), *scratch)
+    want = np.zeros((n, heads, dim))
+    for t, (entry, position) in enumerate(zip(f64(items).astype(int), f64(positions).astype(int))):
+        k, v = (np.stack([f64(cell(pages, table, entry, j)) for j in range(position + 1)]) for pages in (k_pages, v_pages))
+        for h in range(heads):
+            scores = k[:, h // 2] @ f64(q)[t, h * dim:(h + 1) * dim] * dim ** -0.5
+            weights = np.exp(scores - scores.max())
+            want[t, h] = (weights[:, None] / weights.sum() * v[:, h // 2]).sum(0)
+    assert (want[:50, 2:, 5] == math.inf).all() and (want[:50, :2, 9] == -math.inf).all() and (want[50:, 2:, 7] == math.inf).all()
+    assert np.isinf(want).sum() == (50 + 50 + 45) * 2 and not np.isnan(want).any()
+    for got in (tiled, split):                                    # (rounded to 8 bits once)
+        np.testing.assert_allclose(f64(got).reshape(n, heads, dim), want, rtol=2 ** -8, atol=1e-5)
+
+
+@pytest.mark.parametrize("rank", [128, 256])
+def test_infinite_cached_rows_in_tiled_latent_attention(rank):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(rank)
+    heads, rot, page, lengths, new = 3, 32, 16, [90], [30]
+    row = rank + rot
+    table, (pages,) = pages_of(rng, lengths, page, 1, (row,))
+    cell(pages, table, 0, 11)[0, rank + 2] = -math.inf            # (in the part that is no value)
+    positions, items = dev(np.arange(60, 90).astype(np.int32)), torch.zeros(30, dtype=torch.int32, device="cuda")
+    q = dev(rng.normal(size=(30, heads * row)), torch.float32)
+    q.view(30, heads, row)[:, :, rank + 2] = 0.5                  # (one significant bit: its second and third terms are nothing)
+    want, got = torch.full((30, heads * rank), math.nan, device="cuda"), torch.full((30, heads * rank), math.nan, device="cuda")
+    ops.latent_attention_plain(want, q, pages, table.cuda(), positions, items, heads, rank, rot, page, 0.1)
+    tiles, _, _ = ops.attention_tiles([0], new, [60])
+    ops.latent_attention_tiled(got, q, pages, table.cuda(), positions, items, heads, rank, rot, page, 0.1,
+                               tiles=dev(np.array(tiles, dtype=np.int32)), n_tiles=len(tiles))
+    assert np.isfinite(f64(want)).all()
+    np.testing.assert_allclose(f64(got), f64(want), rtol=2e-5, atol=3e-5)        # 32-bit sums on both sides
+
+
+@pytest.mark.parametrize("delta", [True, False])
+@pytest.mark.parametrize("where", ["value", "key", "state", "nan"])
+def test_numbers_that_are_not_finite_in_recurrences_over_portions(delta, where):
+    """They reach the tokens behind them, as token by token, and none before."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(5)
+    heads, dim, vdim, counts, bad = 2, 64, 24, [70, 33], 37
+    n = sum(counts)
+    q, k = (dev(np.abs(rng.normal(size=(n, heads * dim))) + 0.1, torch.bfloat16) for _ in range(2))
+    v = dev(rng.normal(size=(n, heads * vdim)), torch.bfloat16)
+    gate_a, gate_b = dev(rng.normal(size=(n, heads)), torch.float32), dev(rng.normal(size=(n, heads)), torch.float32)
+    state = dev(np.abs(rng.normal(0, 0.3, (2, heads * dim * vdim))), torch.float32)
+    if where == "value":
+        v[bad, vdim + 3] = math.inf
+    elif where == "nan":
+        v[bad, vdim + 3] = math.nan
+    elif where == "key":
+        k[bad, dim + 1] = math.nan
+    else:
+        state.view(2, heads, dim, vdim)[0, 1, 6, 3] = math.inf
+    S, expected, t = f64(state).reshape(2, heads, dim, vdim), np.zeros((n, heads, vdim)), 0
+    with np.errstate(all="ignore"):
+        for entry, count in enumerate(counts):
+            for t in range(t, t + count):
+                for h in range(heads):
+                    qt, kt, vt = f64(q)[t, h * dim:(h + 1) * dim], f64(k)[t, h * dim:(h + 1) * dim], f64(v)[t, h * vdim:(h + 1) * vdim]
+                    step = np.log1p(np.exp(f64(gate_a)[t, h]))
+                    a, b = np.exp(-step), step
+                    if delta:
+                        qt, kt, b = qt / np.sqrt(qt @ qt + 1e-6), kt / np.sqrt(kt @ kt + 1e-6), 1 / (1 + np.exp(-f64(gate_b)[t, h]))
+                    old = a * S[entry, h]
+                    S[entry, h] = old + kt[:, None] * (b * (vt - ((old * kt[:, None]).sum(0) if delta else 0)))[None]
+                    expected[t, h] = (S[entry, h] * qt[:, None]).sum(0) + 0.0 * vt           # (no skip: a factor of zero)
+            t += 1
+    zeros, out = torch.zeros(heads, device="cuda"), torch.full((n, heads * vdim), math.nan, device="cuda")
+    ints = lambda x: dev(np.array(x, np.int32))
+    ops.linear_recurrence(out, q, k, v, gate_a, gate_b if delta else None, zeros, zeros, state, ints([0, 1]), ints([0, 70]), ints(counts), heads, heads,
+                          dim, vdim, delta, unit_norm=delta)
+    got = f64(out).reshape(n, heads, vdim)
+    assert np.isfinite(got[:bad if where != "state" else 0]).all() and np.isfinite(got[70:]).all() and np.isfinite(got[:, 0]).all()
+    assert not np.isfinite(got[bad:70, 1, 3]).any()
+    sound = np.isfinite(expected)
+    np.testing.assert_array_equal(np.isfinite(got), sound)
+    if not delta and where in ("value", "state"):
+        np.testing.assert_array_equal(got[~sound], expected[~sound])          # infinities, as all keys and queries are positive
+    np.testing.assert_allclose(got[sound], expected[sound], rtol=0, atol=4e-6 * max(1.0, np.abs(expected[sound]).max()))
