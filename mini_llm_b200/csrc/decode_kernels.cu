@@ -45,19 +45,10 @@ struct SkinnyParams {
     const int* block_table;
     int max_blocks, page_size, q_width, kv_width;
     // a batch of products of one shape (no norm, no scatter): product b reads x + b * x_step and w + b * w_step and
-    // writes out + b * out_step (elements); batch 1: one product
+    // writes out + b * out_step (elements); batch 0 or 1: one product
     int batch;
     long x_step, w_step, out_step;
 };
-
-__device__ __forceinline__ void unpack8(const uint4& v, float* f) {
-    const uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        f[2 * i] = __uint_as_float(u[i] << 16);
-        f[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
-    }
-}
 
 // A tile is 8 output features by up to 16 rows of x on mma.sync m16n8k16 (the rows of x are the tile's rows: with a handful of
 // tokens a tcgen05 tile of 128 rows would be padding and its way through tensor memory longer than the product).  What bounds such a
@@ -274,12 +265,13 @@ static int launch_skinny_rows(const SkinnyParams& p, cudaStream_t s) {
 }
 
 extern "C" int mllm_decode_skinny_linear(const SkinnyParams* params, void* stream) {
-    const SkinnyParams& p = *params;
+    SkinnyParams p = *params;
+    if (p.batch == 0) p.batch = 1;
     if (p.M <= 0 || p.N <= 0) return 0;
     if (p.K <= 0 || p.K % 8 != 0) return fail("skinny_linear: K must be a positive multiple of 8");
     if (p.gamma == nullptr && p.ldx % 8 != 0) return fail("skinny_linear: the row stride of x must be a multiple of 8");
     if (p.epilogue == EPI_ADD && p.k_pages != nullptr) return fail("skinny_linear: no scatter with the residual sum");
-    if (p.batch < 1 || p.batch > 65535) return fail("skinny_linear: a batch has 1 to 65535 products");
+    if (p.batch < 0 || p.batch > 65535) return fail("skinny_linear: a batch has up to 65535 products");
     if (p.batch > 1 && (p.gamma != nullptr || p.k_pages != nullptr || p.x_step % 8 != 0 || p.w_step % 8 != 0))
         return fail("skinny_linear: a batch takes no norm and no scatter, and its products start on 16-byte boundaries");
     cudaStream_t s = (cudaStream_t)stream;

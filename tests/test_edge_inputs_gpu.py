@@ -323,3 +323,16 @@ def test_numbers_that_are_not_finite_in_recurrences_over_portions(delta, where):
     if not delta and where in ("value", "state"):
         np.testing.assert_array_equal(got[~sound], expected[~sound])          # infinities, as all keys and queries are positive
     np.testing.assert_allclose(got[sound], expected[sound], rtol=0, atol=4e-6 * max(1.0, np.abs(expected[sound]).max()))
+
+
+def test_one_product_by_its_sizes_alone():
+    """A caller of the kernel library that knows of no batches leaves that field zero."""
+    import ctypes
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(0)
+    x, w, out = dev(rng.normal(size=(3, 64)), torch.bfloat16), dev(rng.normal(size=(40, 64)) / 8, torch.bfloat16), torch.empty(3, 40, device="cuda")
+    params = ops._SkinnyParams()
+    params.out, params.x, params.w, params.M, params.N, params.K = out.data_ptr(), x.data_ptr(), w.data_ptr(), 3, 40, 64
+    params.ldx, params.ldo, params.epilogue, params.out_f32 = 64, 40, ops.EPILOGUES["store"], 1
+    ops._skinny(ctypes.byref(params), ops._stream())
+    np.testing.assert_allclose(f64(out), f64(x) @ f64(w).T, rtol=0, atol=2e-6)
