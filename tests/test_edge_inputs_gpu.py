@@ -325,6 +325,73 @@ def test_numbers_that_are_not_finite_in_recurrences_over_portions(delta, where):
     np.testing.assert_allclose(got[sound], expected[sound], rtol=0, atol=4e-6 * max(1.0, np.abs(expected[sound]).max()))
 
 
+# groups of one and of many quads, widths that end inside a warp, the widest row a block takes
+@pytest.mark.parametrize("width, groups", [(96, 3), (768, 4), (20, 5), (4096, 1), (1036, 7)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_norm_and_four_taps_in_one_step(width, groups, dtype):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(width)
+    tokens, slots = 5, np.array([6, 0, 3, 1, 5], np.int32)
+    x, gain, w = (dev(v, torch.float32) for v in (rng.normal(0, 2, (tokens, width)), rng.uniform(0.5, 1.5, width), rng.normal(0, 0.5, (width, 4))))
+    state = dev(rng.normal(size=(7, 3, width)), torch.float32)
+    items, before = dev(np.array([4, 2, 0, 1, 3], np.int32)), f64(state)
+    mine = slots[f64(items).astype(int)]
+    kept, out = state.clone(), torch.full((tokens, width), math.nan, dtype=dtype, device="cuda")
+    ops.norm_taps_step(out, x, gain, groups, 1e-5, w, kept, items, dev(slots), writes=False)
+    assert torch.equal(kept, state)
+    again = torch.empty_like(out)
+    ops.norm_taps_step(again, x, gain, groups, 1e-5, w, state, items, dev(slots))
+    assert torch.equal(again, out)
+    moved = f64(state)
+    pieces = f64(x).reshape(tokens, groups, -1)
+    normed = (pieces / np.sqrt((pieces ** 2).mean(-1, keepdims=True) + 1e-5)).reshape(tokens, width) * f64(gain)
+    rounding = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-6
+    np.testing.assert_allclose(moved[mine, 2], normed, rtol=rounding, atol=1e-6)             # (rounded as an activation)
+    np.testing.assert_array_equal(moved[mine, :2], before[mine, 1:])
+    np.testing.assert_array_equal(moved[[2, 4]], before[[2, 4]])
+    taps = f64(w)
+    expected = moved[mine, 2] * (1 + taps[:, 3]) + sum(before[mine, j] * taps[:, j] for j in range(3))
+    np.testing.assert_allclose(f64(out), expected, rtol=rounding, atol=4e-6)                 # five 32-bit products of values below 8
+
+
+@pytest.mark.parametrize("width, identity, bias, silu", [(8, True, False, False), (24, False, True, True), (1288, False, False, True), (1536, True, True, False)])
+@pytest.mark.parametrize("dtype, counts", [(torch.bfloat16, [1, 7, 4, 0, 13, 2, 3]), (torch.bfloat16, None), (torch.float32, None)])
+def test_filters_of_four_taps(width, identity, bias, silu, dtype, counts):
+    """Portions that begin and end inside a thread's run of four tokens, from a state and moving it on; and steps of single tokens."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(width)
+    single = counts is None
+    counts = [1] * 6 if single else counts
+    n, entries = sum(counts), len(counts)
+    slots, starts, offsets = rng.permutation(entries + 2)[:entries], rng.integers(0, 9, entries), np.cumsum(counts) - counts
+    wide, into = dev(rng.normal(size=(n, width + 16)), dtype), torch.full((n, width + 8), math.nan, dtype=dtype, device="cuda")
+    h, out = wide[:, 8:8 + width], into[:, 8:]
+    w, state = dev(rng.normal(0, 0.5, (width, 4)), torch.float32), dev(rng.normal(size=(entries + 2, 3, width)), torch.float32)
+    b = dev(rng.normal(size=width), torch.float32) if bias else None
+    items = np.repeat(np.arange(entries), counts)
+    positions = np.concatenate([np.arange(s, s + c) for s, c in zip(starts, counts)])
+    ints = lambda values: dev(np.asarray(values).astype(np.int32))
+    before, expected, after = f64(state), np.zeros((n, width)), f64(state)
+    for entry, (slot, offset, count) in enumerate(zip(slots, offsets, counts)):
+        rows = np.concatenate([before[slot], f64(h)[offset:offset + count]])
+        for t in range(count):
+            y = (rows[t:t + 4] * f64(w).T).sum(0) + (rows[t + 3] if identity else 0) + (f64(b) if bias else 0)
+            expected[offset + t] = y / (1 + np.exp(-y)) if silu else y
+        after[slot] = rows[-3:]
+    kept = state.clone()
+    for moving, writes in ((kept, False), (state, True)):
+        if single and not writes:
+            continue                                                         # (a step of single tokens that writes nothing is a portion's)
+        ops.causal_taps(out, h, w, moving, ints(positions), ints(items), ints(slots), ints(starts), ints(offsets), ints(counts), writes, identity, b, silu,
+                        single_tokens=single)
+        # five 32-bit products of values below 4, rounded once
+        np.testing.assert_allclose(f64(out), expected, rtol=2 ** -8 if dtype == torch.bfloat16 else 2e-6, atol=4e-6)
+    if not single:
+        np.testing.assert_array_equal(f64(kept), before)
+    np.testing.assert_array_equal(f64(state), after)
+    assert torch.isnan(into[:, :8]).all()
+
+
 def test_one_product_by_its_sizes_alone():
     """A caller of the kernel library that knows of no batches leaves that field zero."""
     import ctypes
