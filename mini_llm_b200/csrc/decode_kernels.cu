@@ -58,8 +58,9 @@ struct SkinnyParams {
 //     ended (no kernel of a step writes weights), x, bias and residual right behind that wait;
 //   - both operands come straight into registers, 16 bytes a lane: the entries of a block of 32 of K are taken in the order
 //     0-1, 8-9, 16-17, 24-25 | 2-3, ... by both, so that a lane's piece of 8 feeds two products.
-// Replayed back to back, against a warp a feature that unpacked x from shared memory for every one: 8 x 768 x 768 5.6 -> 2.2 us,
-// 8 x 768 x 3072 13.3 -> 4.2, 16 x 3072 x 768 12.8 -> 3.6, 1 x 50257 x 768 19.2 -> 17.1 (floor 11.9).
+// Replayed back to back, against a warp a feature that unpacked x from shared memory for every one: 8 x 768 x 768 3.8 -> 2.3 us,
+// 8 x 768 x 3072 7.7 -> 3.0, 16 x 3072 x 768 10.8 -> 3.9, 1 x 50257 x 768 15.2 -> 14.2 (floor 11.9).  Errors against 64 bits (operands
+// of one sign in brackets): 6.6e-8 (3.6e-8) -> 7.3e-8 (5.0e-8) at K = 768, 1.1e-7 (3.9e-8) -> 9.7e-8 (5.0e-8) at 6,400.
 template <int ROWS, int WARPS, bool NORM>     // rows of x of a tile: 8 (half of the tensor core's) or 16
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 skinny_linear_kernel(const SkinnyParams p, int split) {
@@ -91,7 +92,7 @@ skinny_linear_kernel(const SkinnyParams p, int split) {
     if (NORM) {
         // The rows are normed on the way in, into shared memory: as many warps share a row as there are, whose first KEPT entries a
         // thread stay in registers through both sums.  One row of 768
-        // with 2,304 features took 8.7 us with a warp a row, 5.4 so.
+        // with 2,304 features took 8.7 us with a warp a row, 4.1 so.
         constexpr int KEPT = 4;
         bf16* xs = reinterpret_cast<bf16*>(smem_raw + sizeof(float) * (WARPS * 8 * STRIDE));
         const float* src = behind_the_wait(reinterpret_cast<const float*>(p.x));

@@ -757,8 +757,8 @@ capped_attention_block_kernel(T* __restrict__ out, long ld_out, const T* __restr
 // with all 64 keys left a scheduler one warp, whose products, exponentials and exchanges then stood one behind the other).  Scores are products of bfloat16 operands with 32-bit sums; the weights stay 32-bit: each goes into the
 // second product as three bfloat16 terms, which hold all 24 bits of it, against the values as they are.  Maxima, sums,
 // weights and results are 32-bit in the rows' threads, four threads a row; cap, slopes, masks, sink and gate as above.
-// The products no longer bound it: a tile of 16 x 64 takes 128 of them (KEY 64, VALUE 64) against 32,768 FMAs of the
-// register tiles, and the exponentials and masks stand beside them.
+// The products no longer bound it: a tile of 16 x 64 takes 128 of them (KEY 64, VALUE 64, three terms a weight) against 131,072 FMAs,
+// 4,096 instructions of a warp, on register tiles, and the exponentials and masks stand beside them.
 // Three prompts of 640, 1,200 and 2,048 tokens (12 heads over 4, sizes 64, capped): 480 us a launch on register tiles, 175 here (four warps 210).
 // A tile's product is added with a rounded FMA: left in the tensor cores' accumulators, whose sums are cut off, the error against 64 bits
 // was twice the register tiles'; so it is two thirds of theirs.
@@ -1074,7 +1074,7 @@ static int launch_capped_attention(bool tiled, void* out, long ld_out, const voi
     if constexpr (sizeof(T) == 2) {
         if (capped_mma_takes(q, ld_q, k_pages, v_pages, dim, vdim)) {
             // A block walks the keys of every request among its tokens, one request behind the other: fewer tokens a block while the
-            // blocks are no more than the SMs, or tokens that stand alone beside a short portion wait for one another (20 of 600
+            // blocks are no more than half the SMs, or tokens that stand alone beside a short portion wait for one another (20 of 600
             // keys beside a portion of 60, 12 heads over 4: 631 us with 21 tokens a block, 78 with 2; a prompt of 300 23.1 and 22.0).
             const int group = n_heads / n_kv_heads, heads_per_block = group < 64 ? group : 64;
             const int head_blocks = n_kv_heads * ((group + heads_per_block - 1) / heads_per_block);
@@ -1529,8 +1529,10 @@ static int launch_recurrence_few(const RecurrenceParams& pp, int n_items, cudaSt
 // every sum are 32-bit: 32-bit operands enter a product as three bfloat16 terms that hold all their bits, the rows are bfloat16 as they
 // come and their norms are factors of the sums.  T is bounded: with |k| = 1 and b <= 1 every factor of the recurrence shrinks.
 // What bounds it: issue slots (4,900 warp instructions a chunk, a quarter of them splitting operands) and the chain from S to S.  Two portions of
-// 1,024 tokens, 6 heads of 128 x 128: 513 us a launch token by token, 114 here; 24 heads of 128 x 64 without the delta rule 662 and 94.
-// Errors against 64 bits (relative, 1,000 + 777 tokens): 2.83e-7 token by token, 2.43e-7 here; without the delta rule 1.0e-7 and 8.3e-8.
+// 1,024 tokens, 6 heads of 128 x 128: 513 us a launch token by token, 107 here; 24 heads of 128 x 64 without the delta rule, whose
+// 192 blocks take two passes over the SMs, 662 and 173 (6 such heads 88).
+// Errors against 64 bits (relative): 1,000 + 777 tokens 2.83e-7 token by token, 2.43e-7 here, without the delta rule 1.0e-7 and 8.3e-8; 1,000
+// tokens under faster decays 1.29e-7 and 1.43e-7, without the delta rule 1.06e-7 and 1.19e-7.
 constexpr int REC_TOKENS = 16, REC_ROW_SLOTS = 6, REC_SLOTS = 4, REC_LD = 24;     // (rows of 16 terms, 48 bytes apart: no bank twice)
 
 template <int DIM> struct RecurrenceRows {
@@ -2342,8 +2344,8 @@ expert_down_kernel(float* __restrict__ hidden, long ld_hidden, const T* __restri
 // Up to EXPERT_TILE_TOKENS tokens, bfloat16, inner sizes and the width multiples of 8: the pairs of one expert are the rows of
 // mma.sync tiles (m16n8k16, as the few-row products), so that an expert's weights cross the chip once however many tokens
 // chose it, and the sums are the tensor cores'.  A block a pair read them once a pair and spent its time unpacking: 16 tokens of 8 experts of
-// 768 and a shared one of 1,536 at a width of 768 took 23.4 + 14.7 us (floor 5.4 at measured copy bandwidth).
-// Now 11.9 + 13.4 us, and two tokens of eight choices 7.3 + 11.1 (in a step, one kernel after the other).
+// 768 and a shared one of 1,536 at a width of 768 took 23.4 + 14.7 us (floor 5.4 at measured copy bandwidth), in tiles 12 + 13; where fewer
+// tokens are as fast or faster pair by pair, the dispatcher sends them there.  Weights are asked for ahead of the wait for the kernels ahead.
 constexpr int EXPERT_TILE_TOKENS = 31, EXPERT_TABLES = 64, EXPERT_UNITS = 64, EXPERT_UNIT_K = 256;
 
 // The pairs that chose expert e, in their order, by one warp: the list gets those from number `begin` on, 32 at most, and `place`

@@ -240,7 +240,7 @@ causal_taps_single_kernel(T* __restrict__ out, long ld_out, const T* __restrict_
     held[2L * width] = mine;
 }
 
-// Four taps, bfloat16 rows on 16-byte boundaries, prompt portions: a thread takes eight channels of four tokens one behind
+// Four taps, bfloat16 rows on 16-byte boundaries, prompt portions (launched behind the kernels ahead, as many blocks as it has): a thread takes eight channels of four tokens one behind
 // the other, so that a row is read seven times for four results (four times for one) and 16 bytes at a time.  Two
 // bytes a load, four rows a result: 2,048 tokens of 1,280 to 1,536 channels 25 us against 15.
 constexpr int TAPS_RUN = 4;

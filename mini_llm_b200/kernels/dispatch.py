@@ -63,10 +63,11 @@ class DeferredNorm:
 
 class Kernels:
     FUSED_NORM_KINDS = ("layer_norm",)    # what the few-row product kernel can apply on the way in
-    FUSED_NORM_ROWS = 2                   # and of how many rows: every block norms all of them, so from three on a norm kernel ahead costs
-                                          # less (2,304 x 768: 1 row 5.4 us against 7.1, 2 rows 6.6 against 7.3, 4 rows 7.9 against 7.3)
+    FUSED_NORM_ROWS = 2                   # and of how many rows: every block norms all of them, so that a norm kernel ahead costs less
+                                          # where they are long (2,304 x 768: 1 row 4.1 us against 7.1, 2 rows 4.9 against 7.2; 4 rows of
+                                          # 1,600: 10.0 against 7.9)
     FUSED_NORM_FEATURES = 8192            # and of fewer features than this: a vocabulary's many blocks all norm (1 x 50,257 x 768: 21.5
-                                          # against 16.4 us, 1 x 6,400 x 1,600: 9.3 against 9.8)
+                                          # against 18.3 us, 1 x 6,400 x 1,600: 9.3 against 10.5)
 
     def __init__(self, act_dtype: torch.dtype, plain_only: bool = False):
         self.act_dtype = act_dtype
