@@ -914,8 +914,10 @@ capped_attention_mma_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, 
                     for (int k = 0; k < 2; k++)
                         load_blocks_turned(b[k], vt + (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LDV + j * 8 + ((lane >> 4) & 1) * 8);
                     weighted_rows(x, a, b);
+                    // (a row of another request keeps what it has: its weights of zero would carry a value that is no finite number into it)
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
+                        if (my_item[e >> 1] != item) continue;
                         o[j][e] = fmaf(o[j][e], corr[e >> 1], x[0][e]);
                         o[j + 1][e] = fmaf(o[j + 1][e], corr[e >> 1], x[1][e]);
                     }

@@ -257,6 +257,26 @@ def test_infinite_cached_values_in_tiled_attention(dim):
         np.testing.assert_allclose(f64(got).reshape(n, heads, dim), want, rtol=2 ** -8, atol=1e-5)
 
 
+@pytest.mark.parametrize("new", [[8, 20, 40], [3, 5, 300], [1, 1, 1, 1, 1, 35]])
+def test_cached_values_that_are_no_numbers_stay_with_their_request(new):
+    """Requests that share a tile of queries: what is wrong in the second one's cache is not seen by the others."""
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(len(new))
+    heads, dim, page, lengths = 16, 64, 16, [m + 30 for m in new]         # (16 heads: eight tokens a block and more)
+    table, (k_pages, v_pages) = pages_of(rng, lengths, page, heads, (dim, dim))
+    positions = dev(np.concatenate([np.arange(l - m, l) for l, m in zip(lengths, new)]).astype(np.int32))
+    items, n = np.repeat(np.arange(len(new)), new), sum(new)
+    q = dev(rng.normal(size=(n, heads * dim)), torch.bfloat16)
+    healthy, beside = (torch.full((n, heads * dim), math.nan, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    for out in (healthy, beside):
+        ops.capped_attention(out, q, k_pages, v_pages, table.cuda(), positions, dev(items.astype(np.int32)), heads, heads, dim, dim, page,
+                             dim ** -0.5, tiled=True)
+        for j in range(lengths[1]):                               # (for the second pass)
+            cell(v_pages, table, 1, j)[:] = math.nan if j % 2 else math.inf
+    assert np.isfinite(f64(healthy)).all() and np.isnan(f64(beside)[items == 1]).all()
+    np.testing.assert_array_equal(f64(beside)[items != 1], f64(healthy)[items != 1])
+
+
 @pytest.mark.parametrize("rank", [128, 256])
 def test_infinite_cached_rows_in_tiled_latent_attention(rank):
     from mini_llm_b200.kernels import ops
