@@ -60,7 +60,7 @@ struct SkinnyParams {
 //     0-1, 8-9, 16-17, 24-25 | 2-3, ... by both, so that a lane's piece of 8 feeds two products.
 // Replayed back to back, against a warp a feature that unpacked x from shared memory for every one: 8 x 768 x 768 3.8 -> 2.3 us,
 // 8 x 768 x 3072 7.7 -> 3.0, 16 x 3072 x 768 10.8 -> 3.9, 1 x 50257 x 768 15.2 -> 14.2 (floor 11.9).  Errors against 64 bits (operands
-// of one sign in brackets): 6.6e-8 (3.6e-8) -> 7.3e-8 (5.0e-8) at K = 768, 1.1e-7 (3.9e-8) -> 9.7e-8 (5.0e-8) at 6,400.
+// of one sign in brackets): 6.6e-8 (3.6e-8) -> 7.4e-8 (5.0e-8) at K = 768, 1.1e-7 (3.9e-8) -> 9.7e-8 (5.0e-8) at 6,400.
 template <int ROWS, int WARPS, bool NORM>     // rows of x of a tile: 8 (half of the tensor core's) or 16
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
 skinny_linear_kernel(const SkinnyParams p, int split) {
