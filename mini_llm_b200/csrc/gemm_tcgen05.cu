@@ -10,12 +10,13 @@
 // (engine/src/matrixmult.cu:7-34, engine/src/linear.cu:9-18,
 // engine/src/transformer_block.cu:153-202).
 //
-// Two kernels:
+// Three kernels:
 //   rows     (more than 64 tokens) tiles of 128 tokens x BN output features, walked by
 //            persistent CTAs with two accumulators, so that a tile's epilogue runs under the
 //            next tile's products; the fused query/key/value product scatters keys and values
 //            straight into the cache pages.
-//   swapped  (up to 64 tokens) the 128 tile rows are rows of W (output features), the BN
+//   narrow   (up to 64 tokens) mma.sync tiles of 16 to 48 features: narrow_products.cuh.
+//   swapped  (up to 64 tokens, where the narrow tiles are not) the 128 tile rows are rows of W (output features), the BN
 //            columns are tokens: a 128-row token tile would be mostly padding.  When such a
 //            product has few tiles, each is shared along K by a cluster of CTAs.
 //
@@ -1316,6 +1317,8 @@ int launch_rows_split(const CUtensorMap& a, const CUtensorMap& b, const CUtensor
 
 }  // namespace
 
+#include "narrow_products.cuh"
+
 // The SM count of the current device (asked once per device).
 static int sm_count() {
     static int counts[64] = {0};
@@ -1432,7 +1435,14 @@ static int gemm_bf16(void* out, const void* x, const void* w, const float* bias,
     }
     CUtensorMap map_x, map_w;
     const int sms = sm_count();
-    // Which kernel: up to 64 tokens the one with swapped operands.  It also takes products of up
+    // (A forced code 8000 + a plan: narrow tiles, see narrow_plan.)
+    if (forced_bn >= 8000) return launch_narrow_plan(p, forced_bn - 8000, x, ldx, w, s);
+    // Up to 64 tokens the narrow tiles, where neither K nor the features are so many that 128 x 64 tiles fill the SMs.  Replayed back to
+    // back over weights larger than L2, swapped tiles and narrow ones: 24 x 2304 x 768 4.97 and 3.05 us, 64 x 768 x 768 5.73 and 3.37,
+    // 64 x 3072 x 768 7.57 and 5.64, 64 x 768 x 3072 6.24 and 5.77, 64 x 4800 x 1600 11.8 and 11.6 (within a step of GPT-2 XL 13.8 and 11.5);
+    // 24 x 1600 x 6400 8.79 and 8.68, but 32 x 1600 x 6400 8.72 and 9.15, 64 x 50257 x 768 21.4 and 58.9.
+    if (forced_bn == 0 && M <= 64 && N < 16384 && (M <= 24 || K <= 4096)) return launch_narrow_plan(p, narrow_plan(M, N, K, sms), x, ldx, w, s);
+    // Which kernel: up to 64 tokens, behind the narrow tiles, the one with swapped operands.  It also takes products of up
     // to 512 tokens with a long K and few output features (the feed-forward's second product in
     // steps of prompt portions): there the persistent kernel is one chain of K / 64 dependent
     // blocks on few CTAs (17 us at 768 x 3072 whatever the tokens), and tiles of 128 tokens
@@ -1532,7 +1542,7 @@ extern "C" int mllm_gemm_bf16_tile(void* out, const void* x, const void* w, cons
                                    long ldx, long ldo, int epilogue, int out_f32, int* status, int tile_width,
                                    unsigned long long* timeline, void* stream) {
     // 1000 + width: on a pair of CTAs; 2000 + width: two issuing threads (the launcher refuses what it has not)
-    if (tile_width <= 0 || (tile_width >= 3000 && tile_width < 5000) || (tile_width > 5256 && tile_width < 7002) || tile_width > 7104)
+    if (tile_width <= 0 || (tile_width >= 3000 && tile_width < 5000) || (tile_width > 5256 && tile_width < 7002) || (tile_width > 7104 && tile_width < 8011) || tile_width > 8134)
         return fail("gemm: the tile width is 64, 96, 128, 192 or 256");
     return gemm_bf16(out, x, w, bias, M, N, K, ldx, ldo, epilogue, out_f32, status, nullptr, stream, tile_width, timeline);
 }

@@ -323,3 +323,28 @@ def test_split_attention_of_the_tokens_a_work_list_names(heads, kv_heads, window
         rows = sorted({int(offsets[i]) for i in alone})
         np.testing.assert_allclose(f64(out)[rows], expected[rows], rtol=2 ** -8, atol=1e-5)      # rounded to 8 bits once
         assert (np.delete(f64(out), rows, axis=0) == 7.0).all()
+
+
+# tokens: an eighth's edges, every number of token tiles, shared by one and two blocks; features: less than a tile, its edges; K: one
+# 16-byte piece, less than a block of 32 a warp, shares that end inside one, a cluster's shares of unequal length
+@pytest.mark.parametrize("m", [1, 16, 17, 24, 25, 33, 48, 49, 64])
+@pytest.mark.parametrize("n, k", [(16, 8), (50, 264), (768, 768), (100, 2056)])
+@pytest.mark.parametrize("epilogue", ["add", "store", "gelu_tanh"])
+def test_narrow_products(m, n, k, epilogue):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(m * 7 + n + k)
+    a = dev(rng.normal(size=(m, k + 8)), torch.bfloat16)[:, 8:]
+    w, bias = dev(rng.normal(size=(n, k)) / math.sqrt(k), torch.bfloat16), dev(rng.normal(size=n), torch.float32)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    acc = f64(a) @ f64(w).T + f64(bias)
+    for shares in (0, 100):
+        for tiles in (10, 20, 30):
+            for blocks in (1, 2, 4):
+                out = torch.full((m + 1, n + 4), 0.5, dtype=torch.bfloat16 if epilogue == "gelu_tanh" else torch.float32, device="cuda")
+                ops.gemm_bf16_tile(out[:m, :n], a, w, bias, epilogue, status, 8000 + shares + tiles + blocks)
+                expected = {"add": 0.5 + acc, "store": acc, "gelu_tanh": plain.gelu_tanh(acc)}[epilogue]
+                # sums: 2,056 terms whose sizes add up to 30, each cut off at 2^-23 of them, and with gelu a result rounded to
+                # 8 bits and a tanh of 2^-11, of values up to 6
+                np.testing.assert_allclose(f64(out)[:m, :n], expected, rtol=0, atol=2e-5 if epilogue != "gelu_tanh" else 0.03)
+                assert bool((out[m] == 0.5).all()) and bool((out[:m, n:] == 0.5).all())
+    assert int(status) == 0
