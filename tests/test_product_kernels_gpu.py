@@ -348,3 +348,40 @@ def test_narrow_products(m, n, k, epilogue):
                 np.testing.assert_allclose(f64(out)[:m, :n], expected, rtol=0, atol=2e-5 if epilogue != "gelu_tanh" else 0.03)
                 assert bool((out[m] == 0.5).all()) and bool((out[:m, n:] == 0.5).all())
     assert int(status) == 0
+
+
+# widths: a ring that holds all of K, rows whose end is no block of 32 of K, K shared by two and by four warps; tokens: of which nearly
+# every expert has one and hardly any, tiles of 8, 16 and 32 pairs, more than fit shared memory beside the weights
+@pytest.mark.parametrize("tokens, experts, top, inner, width", [(1, 24, 1, 40, 768), (2, 8, 2, 136, 776), (16, 3, 2, 264, 1000), (31, 2, 2, 72, 1032),
+                                                                (9, 4, 2, 80, 2056), (31, 5, 1, 48, 4096), (3, 40, 2, 64, 2048)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, gated):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(tokens + width)
+    total = experts * inner
+    ups = dev(rng.normal(size=((2 if gated else 1) * total, width)) / math.sqrt(width), torch.bfloat16)
+    downs = dev(rng.normal(size=(width, total)) / math.sqrt(inner), torch.bfloat16)
+    x = dev(rng.normal(size=(tokens, width)), torch.bfloat16)
+    chosen = np.stack([rng.permutation(experts)[:top] for _ in range(tokens)]).astype(np.int32)
+    weights = rng.uniform(0.5, 1.5, size=(tokens, top)).astype(np.float32)
+    table = lambda matrix, first, step: torch.tensor([matrix.data_ptr() + 2 * (first + e * step) for e in range(experts)], dtype=torch.int64, device="cuda")
+    act = torch.full((tokens * top, inner), math.nan, dtype=torch.bfloat16, device="cuda")
+    hidden = dev(rng.normal(size=(tokens, width)), torch.float32)
+    expected = f64(hidden)
+    up, down, rows = f64(ups)[-total:], f64(downs), f64(x)
+    for t in range(tokens):
+        for k, e in enumerate(chosen[t]):
+            at = slice(e * inner, (e + 1) * inner)
+            u = up[at] @ rows[t]
+            if gated:
+                g = f64(ups)[at] @ rows[t]
+                u = g / (1.0 + np.exp(-g)) * u
+            else:
+                u = np.maximum(u, 0.0) ** 2
+            expected[t] += weights[t, k] * (down[:, at] @ f64(dev(u, torch.bfloat16)))
+    ops.experts(hidden, act, x, dev(chosen.reshape(-1)), dev(np.ones(tokens * top), torch.float32), dev(weights.reshape(-1), torch.float32),
+                table(ups, 0, inner * width) if gated else None, table(ups, (total if gated else 0) * width, inner * width), table(downs, 0, inner),
+                dev(np.full(experts, inner, np.int32)), inner, top, ld_down=total, tiles=True, n_experts=experts)
+    # of the activations, of size 1, one in some thousands rounds the other way (2^-8 of it): far below 1e-3 of the sums
+    assert np.linalg.norm(f64(hidden) - expected) <= 1e-3 * np.linalg.norm(expected)
+    assert np.abs(f64(hidden) - expected).max() <= 0.03
