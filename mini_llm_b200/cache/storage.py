@@ -16,6 +16,7 @@ from __future__ import annotations
 
 import torch
 
+from ..kernels import ops
 from ..parts.spec import FixedState, PagedKV
 
 _STATE_DTYPES = {"float32": torch.float32, "bfloat16": torch.bfloat16, "int32": torch.int32}
@@ -78,6 +79,7 @@ class CacheStorage:
         self.device = device
         self.max_items = int(max_items)
         self.poison = poison
+        self._state_table = None              # where every state of fixed size lies, for the kernel that empties a slot
         self.spare_page = True                # every pool has a page past its last (index n_pages)
         self.keys, self.values, self.states, self.block_tables = {}, {}, {}, {}
         for group in manager.groups:
@@ -174,8 +176,12 @@ class CacheStorage:
 
     def reset_slot(self, slot: int) -> None:
         """Fixed-size state starts at zero for a new request."""
-        for state in self.states.values():
-            state[:, slot].zero_()
+        if not self.states:
+            return
+        if self._state_table is None:
+            self._state_table = torch.tensor([[s.data_ptr(), s.shape[0], s.stride(0) * s.element_size(), s.stride(1) * s.element_size()]
+                                              for s in self.states.values()], dtype=torch.int64, device=self.device)
+        ops.zero_slot(self._state_table, slot)
 
     def bytes(self) -> int:
         total = 0

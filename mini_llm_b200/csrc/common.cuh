@@ -147,7 +147,8 @@ template <typename T> __device__ __forceinline__ T* behind_the_wait(T* p) {
 // A kernel of few long blocks is launched the second way: as a dependent its blocks go to whatever SMs have room while other
 // kernels' waiting blocks hold the rest, several to an SM, and stay there (per launch within a replayed step, early against
 // not: a gated delta rule over two prompts of 1,000 tokens 680 against 513 us, latent attention of one token in 32 parts 23.5 against
-// 12.4, a 32-bit product of 240 x 768 x 768 73 against 41).
+// 12.4, a 32-bit product of 240 x 768 x 768 73 against 41).  A step's first kernels are, too: those behind them may read the step's
+// arrays, which the very first one brings, ahead of their waits.
 constexpr bool AFTER_THE_KERNELS_AHEAD = false;
 
 // (cluster: the CTAs of a thread block cluster, or x = 0 for a launch without clusters)

@@ -56,10 +56,10 @@ extern "C" int mllm_plain_embed(float* out, const int* ids, const int* positions
     cudaStream_t s = (cudaStream_t)stream;
     int threads = width >= 256 ? 256 : 64;
     if (table_dtype == DT_F32)
-        launch_kernel(g_dependent_launch != 0, embed_kernel<float>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, embed_kernel<float>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,
                       (const float*)table, (const float*)position_table, width, scale);
     else if (table_dtype == DT_BF16)
-        launch_kernel(g_dependent_launch != 0, embed_kernel<bf16>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,
+        launch_kernel(AFTER_THE_KERNELS_AHEAD, embed_kernel<bf16>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,
                       (const bf16*)table, (const bf16*)position_table, width, scale);
     else
         return fail("embed: unknown table dtype");

@@ -445,14 +445,79 @@ extern "C" int mllm_sampling_sample_rows(int* out, const float* logits, long ld,
 // single-sequence greedy loop on the device in the same spirit
 // (engine/src/gpt2_gpu_greedy.cu:80-119).
 // ---------------------------------------------------------------------------
-__global__ void keep_tokens_kernel(int* __restrict__ kept, const int* __restrict__ slots,
-                                   const int* __restrict__ tokens, int n, int n_kept) {
+// `ids` and `status_copy`, where given, lie in pinned host memory, two steps' worth: the draws and the kernels' status word go to the part that
+// `turn` (of the step's control block) names, so that no copy engine stands between this step and the next (two copies of a few bytes
+// behind a step took 14 us of the GPU's time).
+__global__ void keep_tokens_kernel(int* __restrict__ kept, const int* __restrict__ slots, const int* __restrict__ tokens, int n,
+                                   int n_kept, int* ids, long ids_step, int* status_copy, const int* turn, const int* status) {
     dependents_may_start();
     wait_for_earlier_kernels();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
-    const int slot = slots[r];
-    if (slot >= 0 && slot < n_kept) kept[slot] = tokens[r];
+    const int slot = slots[r], token = tokens[r];
+    if (slot >= 0 && slot < n_kept) kept[slot] = token;
+    if (ids != nullptr) {
+        const int which = *turn & 1;
+        ids[which * ids_step + r] = token;
+        if (r == 0) status_copy[which] = *status;
+    }
+}
+
+// The step's arrays from pinned host memory into the control block on the device: the host fills the parts of a ring in turn, and
+// `steps[0]` counts the steps that were taken from it.  In a captured step this is the first kernel, so that a step's arrays come in behind the
+// step before without a copy engine between the two (a copy of 20 KB took 23 us from the kernel before to the one after).
+// What bounds it is one trip over PCIe: a thread asks for its four pieces together.  The kernels behind it read the step's arrays
+// ahead of their waits (they count as memory that no kernel writes), so the next one is launched when this one has ended: neither does it let
+// dependents start, nor are the kernels that may follow it (token embeddings, resolve_tokens) launched as dependents.
+__global__ void __launch_bounds__(256) control_kernel(uint4* control, const uint4* ring, long ring_step, int ring_parts, int* steps, int pieces) {
+    wait_for_earlier_kernels();
+    __shared__ int taken;
+    if (threadIdx.x == 0) taken = *reinterpret_cast<volatile int*>(steps);
+    __syncthreads();
+    const uint4* from = ring + (long)(taken % ring_parts) * ring_step;
+    constexpr int EACH = 4;
+    for (int first = blockIdx.x * 256 * EACH; first < pieces; first += gridDim.x * 256 * EACH) {
+        uint4 v[EACH];
+#pragma unroll
+        for (int i = 0; i < EACH; i++) {
+            const int at = first + i * 256 + threadIdx.x;
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (at < pieces)
+                asm volatile("ld.volatile.global.v4.u32 {%0, %1, %2, %3}, [%4];"
+                             : "=r"(v[i].x), "=r"(v[i].y), "=r"(v[i].z), "=r"(v[i].w) : "l"(from + at) : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < EACH; i++) {
+            const int at = first + i * 256 + threadIdx.x;
+            if (at < pieces) control[at] = v[i];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        // the last block to end counts the step: every block has read the count by then
+        __threadfence();
+        if (atomicAdd(steps + 1, 1) == (int)gridDim.x - 1) {
+            steps[1] = 0;
+            steps[0] = (taken + 1) % ring_parts;
+        }
+    }
+}
+
+// What a request's slot holds of every state of fixed size becomes zero: one launch for all of them.  tables[4 * s ..]: state s's first
+// byte, its run entries, the bytes from one entry to the next, the bytes of a slot.
+__global__ void __launch_bounds__(256) zero_slot_kernel(const long long* __restrict__ tables, int slot) {
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    const long long* table = tables + 4 * blockIdx.y;
+    const long long entries = table[1], step = table[2], bytes = table[3];
+    char* base = reinterpret_cast<char*>(table[0]) + slot * bytes;
+    const int unit = (table[0] | step | bytes) % 16 == 0 ? 16 : 1;
+    const long long per_entry = bytes / unit;
+    for (long long i = blockIdx.x * 256 + threadIdx.x; i < entries * per_entry; i += (long long)gridDim.x * 256) {
+        char* at = base + i / per_entry * step + i % per_entry * unit;
+        if (unit == 16) *reinterpret_cast<uint4*>(at) = make_uint4(0u, 0u, 0u, 0u);
+        else *at = 0;
+    }
 }
 
 __global__ void resolve_tokens_kernel(int* __restrict__ ids, const int* __restrict__ kept, int n, int n_kept) {
@@ -466,17 +531,46 @@ __global__ void resolve_tokens_kernel(int* __restrict__ ids, const int* __restri
     ids[t] = slot < n_kept ? kept[slot] : 0;
 }
 
-extern "C" int mllm_sampling_keep_tokens(int* kept, const int* slots, const int* tokens, int n, int n_kept,
-                                         void* stream) {
+// (ids null: nothing goes to the host)
+extern "C" int mllm_sampling_keep_tokens(int* kept, const int* slots, const int* tokens, int n, int n_kept, int* ids, long ids_step,
+                                         int* status_copy, const int* turn, const int* status, void* stream) {
     if (n <= 0) return 0;
+    if (ids != nullptr && (status_copy == nullptr || turn == nullptr || status == nullptr)) return fail("keep_tokens: the way to the host is incomplete");
     return launched(launch_kernel(g_dependent_launch != 0, keep_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0,
-                                  (cudaStream_t)stream, kept, slots, tokens, n, n_kept),
+                                  (cudaStream_t)stream, kept, slots, tokens, n, n_kept, ids, ids_step, status_copy, turn, status),
                     "keep_tokens_kernel");
+}
+
+// The device's address of pinned host memory, or null.
+extern "C" int mllm_sampling_device_address(void* host, void** device) {
+    if (cudaHostGetDevicePointer(device, host, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return fail("the host memory is not pinned");
+    }
+    return 0;
+}
+
+// ring_step and bytes are multiples of 16; steps: two ints, zero at first.
+extern "C" int mllm_sampling_control(void* control, const void* ring, long ring_step, int ring_parts, int* steps, long bytes, void* stream) {
+    if (bytes <= 0) return 0;
+    if (bytes % 16 != 0 || ring_step % 16 != 0 || bytes > ring_step || ring_parts < 1 || (reinterpret_cast<uintptr_t>(control) & 15) != 0 ||
+        (reinterpret_cast<uintptr_t>(ring) & 15) != 0)
+        return fail("control: whole pieces of 16 bytes of a part of the ring");
+    const long pieces = bytes / 16, blocks = (pieces + 1023) / 1024;
+    return launched(launch_kernel(g_dependent_launch != 0, control_kernel, dim3((unsigned)(blocks < 64 ? blocks : 64)), dim3(256), 0, (cudaStream_t)stream,
+                                  (uint4*)control, (const uint4*)ring, ring_step / 16, ring_parts, steps, (int)pieces),
+                    "control_kernel");
+}
+
+extern "C" int mllm_sampling_zero_slot(const long long* tables, int n_states, int slot, void* stream) {
+    if (n_states <= 0) return 0;
+    return launched(launch_kernel(g_dependent_launch != 0, zero_slot_kernel, dim3(64, n_states), dim3(256), 0, (cudaStream_t)stream, tables, slot),
+                    "zero_slot_kernel");
 }
 
 extern "C" int mllm_sampling_resolve_tokens(int* ids, const int* kept, int n, int n_kept, void* stream) {
     if (n <= 0) return 0;
-    return launched(launch_kernel(g_dependent_launch != 0, resolve_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0,
+    return launched(launch_kernel(AFTER_THE_KERNELS_AHEAD, resolve_tokens_kernel, dim3((n + 127) / 128), dim3(128), 0,
                                   (cudaStream_t)stream, ids, kept, n, n_kept),
                     "resolve_tokens_kernel");
 }

@@ -73,7 +73,7 @@ extern "C" int mllm_token_pair_embed(float* out, const int* ids, const int* posi
     const bool vec = width % 4 == 0 && (((unsigned long long)out | (unsigned long long)table | (unsigned long long)pairs) & 15ull) == 0;
     const int threads = width >= 1024 ? 256 : 64;
 #define RUN(T, VEC)                                                                                                              \
-    launch_kernel(g_dependent_launch != 0, pair_embed_kernel<T, VEC>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,   \
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, pair_embed_kernel<T, VEC>, dim3(n_tokens), dim3(threads), 0, s, out, ids, positions,   \
                   token_item, item_slot, item_offset, item_count, (const T*)table, (const T*)pairs, state, (long long)buckets,    \
                   (long long)mul_prev, (long long)mul_cur, width, scale)
     if (dtype == DT_F32) { if (vec) RUN(float, true); else RUN(float, false); }

@@ -13,6 +13,8 @@ from __future__ import annotations
 import numpy as np
 import torch
 
+from ..kernels import ops
+
 
 class Workspace:
     """Named scratch tensors, reused across layers and steps.  A buffer is
@@ -49,7 +51,10 @@ class ControlBlock:
     of step k still read theirs, so no copy stands between two steps' kernels; a step's kernels
     wait for their copy, and a copy waits for the kernels that read the buffer it overwrites
     (``consumed`` records them).  Other steps keep to the first buffer (their kernels are
-    replayed from graphs with fixed addresses) and copy in the order of the compute stream."""
+    replayed from graphs with fixed addresses): the host fills the parts of a ring in turn, and a step's
+    first kernel (``take``) brings the part whose turn it is, which it counts on the device, into the buffer."""
+
+    RING = 3                                  # parts: the host fills one while two steps are on their way
 
     def __init__(self, device, groups):
         self.device = device
@@ -57,11 +62,12 @@ class ControlBlock:
         self.capacity = 0
         self.device_buffers = [None, None]
         self.copy_stream = torch.cuda.Stream(device=device)
-        self._host = []
         self._layouts = {}
+        self._host_views = {}
         self.parity = 0
         self.generation = 0
         self.last_upload_bytes = 0            # bytes of the last step's host-to-device copy
+        self.done = None                      # the event behind the last step's kernels (``consumed``)
 
     @staticmethod
     def tile_ints(n_tokens: int, n_items: int) -> int:
@@ -72,8 +78,8 @@ class ControlBlock:
     def _layout(self, n_tokens: int, n_items: int):
         """Offsets (in int32 units) as a function of the step's sizes only, so
         that steps of equal sizes find their arrays at equal addresses."""
-        offsets = {}
-        cursor = 0
+        offsets = {"turn": 0}                     # the step's number modulo two: where its draws go on the host
+        cursor = 4
         for name in ("token_ids", "positions", "token_item", "want_rows", "want_slots", "counters", "temperature",
                      "top_p"):
             offsets[name] = cursor
@@ -96,69 +102,124 @@ class ControlBlock:
         if size <= self.capacity:
             return
         torch.cuda.synchronize(self.device)      # nothing may still read or fill the old buffers
-        self.capacity = max(size, 2 * self.capacity, 4096)
+        self.capacity = (max(size, 2 * self.capacity, 4096) + 3) // 4 * 4
         self.device_buffers = [torch.zeros(self.capacity, dtype=torch.int32, device=self.device) for _ in range(2)]
         self._host = [torch.zeros(self.capacity, dtype=torch.int32).pin_memory() for _ in range(2)]
         self._host_np = [h.numpy() for h in self._host]
         self._copied = [torch.cuda.Event(), torch.cuda.Event()]       # the copy out of host buffer t is done
         self._copied_once = [False, False]
         self._host_turn = 0
-        self._consumed = [torch.cuda.Event(), torch.cuda.Event()]     # the kernels that read device buffer p are done
-        self._in_use = [False, False]
+        self._consumed_by = [torch.cuda.Event(), torch.cuda.Event()]
+        self._consumed = [None, None]        # the event behind the kernels that read device buffer p, once there are any
+        self._ring = torch.zeros(self.RING * self.capacity, dtype=torch.int32).pin_memory()
+        self._ring_np = self._ring.numpy()
+        self._ring_address = ops.device_address(self._ring)
+        self._ring_done = [torch.cuda.Event() for _ in range(self.RING)]      # the step that took part r is done
+        self._ring_used = [False] * self.RING
+        self._ring_turn, self._ring_open = 0, False
+        self._steps = torch.zeros(2, dtype=torch.int32, device=self.device)
         self._layouts = {}                   # (parity, tokens, entries) -> (offsets, size, device views)
+        self._host_views = {}                # (ring or not, part, tokens, entries) -> host views
         self.generation += 1
 
-    def upload(self, arrays: dict, n_tokens: int, n_items: int, alternate: bool = True):
-        """``arrays``: name -> numpy array (int32, or float32/int64 viewed as
-        int32).  Returns name -> device view (of this step's buffer).  ``alternate=False``
-        keeps to the first buffer: steps whose kernels are replayed from a captured graph
-        (fixed addresses) use that, and wait for the step before them."""
+    def begin(self, n_tokens: int, n_items: int, alternate: bool = True):
+        """The arrays of a step of these sizes: (host views to fill, device views).  ``send`` follows."""
         self.parity = (self.parity ^ 1) if alternate else 0
-        parity = self.parity
-        key = (parity, n_tokens, n_items)
+        key = (self.parity, n_tokens, n_items)
         held = self._layouts.get(key)
         if held is None:
             offsets, size = self._layout(n_tokens, n_items)
+            size = (size + 3) // 4 * 4
             self._ensure(size)               # may drop every cached layout
-            held = self._layouts[key] = (offsets, size, self._views(self.device_buffers[parity], offsets, n_tokens, n_items))
+            held = self._layouts[key] = (offsets, size, self._views(self.device_buffers[self.parity], offsets, n_tokens, n_items))
         offsets, size, views = held
+        self._size = size
         self.last_upload_bytes = 4 * size
-        # host side: two pinned buffers in turn; the copy that last read this one must be done
-        self._host_turn ^= 1
-        turn = self._host_turn
-        if self._copied_once[turn]:
-            self._copied[turn].synchronize()
-        host_np = self._host_np[turn]
-        for name, values in arrays.items():
-            flat = np.ascontiguousarray(values).reshape(-1).view(np.int32)
-            start = offsets[name]
-            host_np[start:start + flat.size] = flat
-        compute = torch.cuda.current_stream(self.device)
         if alternate:
-            # beside the kernels of the step before; behind the kernels that last read this buffer
-            with torch.cuda.stream(self.copy_stream):
-                if self._in_use[parity]:
-                    self.copy_stream.wait_event(self._consumed[parity])
-                self.device_buffers[parity][:size].copy_(self._host[turn][:size], non_blocking=True)
-                self._copied[turn].record(self.copy_stream)
-            compute.wait_event(self._copied[turn])
+            # two pinned buffers in turn; the copy that last read this one must be done
+            self._host_turn ^= 1
+            part = self._host_turn
+            if self._copied_once[part]:
+                self._copied[part].synchronize()
         else:
-            # in the order of the compute stream: behind everything that read the buffer
-            self.device_buffers[parity][:size].copy_(self._host[turn][:size], non_blocking=True)
-            self._copied[turn].record(compute)
-        self._copied_once[turn] = True
-        return views
+            if self._ring_open:
+                # a step was begun and did not get behind its kernels: whether they took its part is not known
+                torch.cuda.synchronize(self.device)
+                self._steps.zero_()
+                torch.cuda.synchronize(self.device)
+                self._ring_turn = 0
+            part = self._ring_turn
+            self._ring_open = True
+            if self._ring_used[part]:
+                self._ring_done[part].synchronize()
+        host_key = (alternate, part, n_tokens, n_items)
+        host = self._host_views.get(host_key)
+        if host is None:
+            if len(self._host_views) >= 512:
+                self._host_views.clear()
+            memory = self._host_np[part] if alternate else self._ring_np[part * self.capacity:(part + 1) * self.capacity]
+            host = self._host_views[host_key] = self._array_views(memory, offsets, n_tokens, n_items)
+        return host, views
 
-    def consumed(self) -> None:
+    def send(self, alternate: bool = True) -> None:
+        """The filled arrays are on their way (the alternating steps' copy), or ready to be taken (``take``)."""
+        if not alternate:
+            return
+        turn, parity, size = self._host_turn, self.parity, self._size
+        # beside the kernels of the step before; behind the kernels that last read this buffer
+        with torch.cuda.stream(self.copy_stream):
+            if self._consumed[parity] is not None:
+                self.copy_stream.wait_event(self._consumed[parity])
+            self.device_buffers[parity][:size].copy_(self._host[turn][:size], non_blocking=True)
+            self._copied[turn].record(self.copy_stream)
+        torch.cuda.current_stream(self.device).wait_event(self._copied[turn])
+        self._copied_once[turn] = True
+
+    def take(self) -> None:
+        """Launch the kernel that brings the step's arrays into the device buffer (the step's upload, which the count of the
+        model's kernels leaves out as it left out the copy)."""
+        ops.control(self.device_buffers[0], self._ring_address, self.capacity, self.RING, self._steps, self._size)
+
+    def consumed(self, alternate: bool) -> None:
         """Call after the step's kernels are enqueued: its buffer may be overwritten once they
         are done."""
-        self._consumed[self.parity].record(torch.cuda.current_stream(self.device))
-        self._in_use[self.parity] = True
+        compute = torch.cuda.current_stream(self.device)
+        if alternate:
+            self.done = self._consumed_by[self.parity]
+        else:
+            part = self._ring_turn
+            self.done = self._ring_done[part]
+            self._ring_used[part] = True
+            self._ring_turn, self._ring_open = (part + 1) % self.RING, False
+        self.done.record(compute)
+        self._consumed[self.parity] = self.done
+
+    def _array_views(self, memory, offsets, n_tokens: int, n_items: int):
+        """The same as ``_views``, of the host's memory, as arrays of the types that are written."""
+        views = {}
+        for name, start in offsets.items():
+            if name == "turn":
+                views[name] = memory[start:start + 1]
+            elif name == "seeds":
+                views[name] = memory[start:start + 2 * n_tokens].view(np.uint64)
+            elif name in ("temperature", "top_p"):
+                views[name] = memory[start:start + n_tokens].view(np.float32)
+            elif name == "att_tiles":
+                views[name] = memory[start:start + self.tile_ints(n_tokens, n_items)].reshape(-1, 8)
+            elif isinstance(name, tuple):
+                views[name] = memory[start:start + n_items * dict(self.groups)[name[1]]].reshape(n_items, -1)
+            elif name.startswith("item_"):
+                views[name] = memory[start:start + n_items]
+            else:
+                views[name] = memory[start:start + n_tokens]
+        return views
 
     def _views(self, buffer, offsets, n_tokens: int, n_items: int):
         views = {}
         for name, start in offsets.items():
-            if name == "seeds":
+            if name == "turn":
+                views[name] = buffer[start:start + 1]
+            elif name == "seeds":
                 views[name] = buffer[start:start + 2 * n_tokens].view(torch.int64)
             elif name in ("temperature", "top_p"):
                 views[name] = buffer[start:start + n_tokens].view(torch.float32)

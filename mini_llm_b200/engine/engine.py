@@ -14,6 +14,7 @@ of its input before it launches anything, and a refused step changes nothing.
 
 from __future__ import annotations
 
+import itertools
 import sys
 from dataclasses import dataclass, field
 
@@ -104,7 +105,9 @@ class Engine:
         self._sampled = None
         self.kept_tokens = torch.zeros(self.max_requests, dtype=torch.int32, device=self.device)
         self._kept_valid = set()              # slots whose entry of kept_tokens is a sampled token
-        self._readback = [None, None]         # per step parity: (pinned host buffer, rows, event)
+        self._readback = [None, None]         # per step parity: (pinned host memory, rows, event)
+        self._ids_beside, self._copied_beside = [None, None], [torch.cuda.Event(), torch.cuda.Event()]
+        self._make_ids_pinned(self.max_tokens_per_step + 8)
         self._turn = 0
         self._alternated = False              # whether the last step took its arrays from the alternating buffers
         self._readback_stream = torch.cuda.Stream(device=self.device)    # sampled ids go to the host beside the next step
@@ -120,8 +123,14 @@ class Engine:
             print(f"[mini_llm_b200] decode steps run part by part, not as one kernel: {self.fused_reason}",
                   file=sys.stderr, flush=True)
         self._status_pinned = torch.zeros(2, dtype=torch.int32).pin_memory()   # per step parity: the kernels' status word
+        self._status_address = ops.device_address(self._status_pinned)
         self._status_host = self._status_pinned.numpy()
         self.hidden_dump = None               # set by step(dump_hidden=True): the residual stream after every run entry
+
+    def _make_ids_pinned(self, rows: int) -> None:
+        """Room on the host for the draws of two steps of up to ``rows`` rows, which a step's last kernel writes."""
+        self._ids_pinned = torch.zeros((2, rows), dtype=torch.int32).pin_memory()
+        self._ids_address = ops.device_address(self._ids_pinned)
 
     # ---- requests ---------------------------------------------------------------------------
     def open_request(self) -> int | None:
@@ -150,13 +159,16 @@ class Engine:
         return self.cache.length(slot)
 
     # ---- the step ---------------------------------------------------------------------------
-    def _validate(self, entries) -> None:
+    def _validate(self, entries) -> list:
+        """Raises ``StepError``, or returns every entry's token ids as an array (None for a decoding request's one token)."""
         if not entries:
             raise StepError("a step needs at least one entry")
         seen = set()
         vocab = self.spec.vocab_size
         total = 0
+        every = []
         for index, entry in enumerate(entries):
+            ids = None
             if not self.cache.is_open(entry.slot):
                 raise StepError(f"entry {index}: slot {entry.slot} holds no request")
             if entry.slot in seen:
@@ -189,6 +201,7 @@ class Engine:
                     bad = next((t for t in entry.tokens if not 0 <= int(t) < vocab), None)
                     raise StepError(f"entry {index}: token id {bad} is outside the vocabulary [0, {vocab}) "
                                     f"(PREVIOUS may only be an entry's first token)")
+            every.append(ids)
             have = self.cache.length(entry.slot)
             if have + n > self.max_positions:
                 raise StepError(f"entry {index}: {have} cached + {n} new tokens exceed the {self.max_positions} "
@@ -199,6 +212,7 @@ class Engine:
         if total > self.max_tokens_per_step:
             raise StepError(f"the step brings {total} tokens, more than the {self.max_tokens_per_step} "
                             f"this engine takes in one step (max_tokens_per_step)")
+        return every
 
     def _reserve(self, entries) -> None:
         cache = self.cache
@@ -229,13 +243,13 @@ class Engine:
         outputs of ``gpt2_gpu_forward_last``, engine/src/gpt2_gpu.cu:224-250).  A step
         that fails after its check (out of pages, a kernel that reports an error) leaves
         every request as it was."""
-        self._validate(entries)
+        ids = self._validate(entries)
         n_want = sum(len(e.want) for e in entries)
         if sampling is not None and len(sampling) != n_want:
             raise StepError(f"{len(sampling)} sampling parameters for {n_want} wanted rows")
         self._reserve(entries)
         try:
-            return self._step_reserved(entries, sampling, n_want, dump_hidden)
+            return self._step_reserved(entries, ids, sampling, n_want, dump_hidden)
         except BaseException:
             # nothing was committed: the pages this step reserved go back, and every request
             # is as long as it was (what the step may have stored lies past that length)
@@ -243,60 +257,22 @@ class Engine:
                 self.cache.unreserve(entry.slot)
             raise
 
-    def _step_reserved(self, entries, sampling, n_want, dump_hidden):
-        n_tokens = sum(len(e.tokens) for e in entries)
-        n_items = len(entries)
-        any_previous = False
+    def _step_reserved(self, entries, ids, sampling, n_want, dump_hidden):
+        n_real = n_tokens = sum(len(e.tokens) for e in entries)
+        n_real_items = n_items = len(entries)
+        n_real_want = n_want
         ctx = self.ctx
         cache_length = self.cache.length
-        if n_tokens == n_items and all(type(e.tokens[0]) is int and len(e.want) <= 1 for e in entries):
-            # single tokens only (a decode step): the arrays straight from lists, no slices per entry
-            slots = [e.slot for e in entries]
-            starts = [cache_length(slot) for slot in slots]
-            firsts = [e.tokens[0] for e in entries]
-            any_previous = PREVIOUS in firsts
-            if any_previous:
-                firsts = [-1 - slot if t == PREVIOUS else t for t, slot in zip(firsts, slots)]
-            token_ids = np.array(firsts, dtype=np.int32)
-            positions = np.array(starts, dtype=np.int32)
-            token_item = np.arange(n_items, dtype=np.int32)
-            wanted = [(index, e.slot) for index, e in enumerate(entries) if e.want]
-            want_rows = np.array([index for index, _ in wanted], dtype=np.int32)
-            want_slots = np.array([slot for _, slot in wanted], dtype=np.int32)
-            ctx.item_slots, ctx.item_starts = slots, starts
+        decode_only = n_tokens == n_items
+        slots = ctx.item_slots = [e.slot for e in entries]
+        starts = ctx.item_starts = [cache_length(slot) for slot in slots]
+        if decode_only:
             ctx.item_counts, ctx.item_offsets = [1] * n_items, list(range(n_items))
         else:
-            token_ids = np.empty(n_tokens, dtype=np.int32)
-            positions = np.empty(n_tokens, dtype=np.int32)
-            token_item = np.empty(n_tokens, dtype=np.int32)
-            want_rows = np.empty(n_want, dtype=np.int32)
-            want_slots = np.full(n_want, -1, dtype=np.int32)      # the entry's last wanted row is kept for its slot
-            ctx.item_slots, ctx.item_starts, ctx.item_counts, ctx.item_offsets = [], [], [], []
-            row = 0
-            w = 0
-            for index, entry in enumerate(entries):
-                n = len(entry.tokens)
-                start = cache_length(entry.slot)
-                token_ids[row:row + n] = entry.tokens
-                if token_ids[row] == PREVIOUS:
-                    token_ids[row] = -1 - entry.slot
-                    any_previous = True
-                positions[row:row + n] = np.arange(start, start + n, dtype=np.int32)
-                token_item[row:row + n] = index
-                for place in entry.want:
-                    want_rows[w] = row + int(place)
-                    w += 1
-                if entry.want:
-                    want_slots[w - 1] = entry.slot
-                ctx.item_slots.append(entry.slot)
-                ctx.item_starts.append(start)
-                ctx.item_counts.append(n)
-                ctx.item_offsets.append(row)
-                row += n
-        tables = {group.index: group.table[ctx.item_slots] for group in self.cache.groups if group.paged}
+            ctx.item_counts = [len(e.tokens) for e in entries]
+            ctx.item_offsets = list(itertools.accumulate(ctx.item_counts, initial=0))[:-1]
         # A step of single tokens of few requests goes to the decode attention, which takes no
         # work list: none is made for it.
-        decode_only = n_tokens == n_items
         # Where most of the step's tokens lie in portions longer than a tile, the list is made of
         # units of two tiles (measured: 21 against 28.5 us for two prompts of 1,024 tokens of
         # twelve heads, 36 against 30 us for sixteen portions of 128 tokens).
@@ -317,20 +293,9 @@ class Engine:
             else:
                 tiles, n_split, most_parts = ops.attention_tiles(ctx.item_offsets, counts, ctx.item_starts)
             singles = [(i, ctx.item_offsets[i], 1, ctx.item_starts[i], 0, 1, 0, ctx.item_starts[i] // ops.ATTENTION_TILE + 1) for i in alone]
-        temperature = top_p = seeds = counters = None
-        if sampling is not None:
-            temperature = np.array([s.temperature for s in sampling], dtype=np.float32)
-            top_p = np.array([s.top_p for s in sampling], dtype=np.float32)
-            seeds = np.array([s.seed & 0xFFFFFFFFFFFFFFFF for s in sampling], dtype=np.uint64)
-            counters = np.array([s.counter for s in sampling], dtype=np.int32)
-        # the entries as the device sees them: slot, first row, rows, first position
-        item_slot = np.array(ctx.item_slots, dtype=np.int32)
-        item_offset = np.array(ctx.item_offsets, dtype=np.int32)
-        item_count = np.array(ctx.item_counts, dtype=np.int32)
-        item_start = np.array(ctx.item_starts, dtype=np.int32)
-        n_real_want = n_want
-        if (not decode_only and not dump_hidden and self.cuda_graphs and self.model.graph_safe
-                and n_want <= n_tokens and self._can_pad):
+        padded = (not decode_only and not dump_hidden and self.cuda_graphs and self.model.graph_safe
+                  and n_want <= n_tokens and self._can_pad)
+        if padded:
             # Steps with prompt portions come in endless shapes, and a captured graph serves one
             # shape.  So such a step is filled up to a round shape: tokens of a request that does
             # not exist (id 0 at position 0; its block table names the spare page that every
@@ -341,53 +306,87 @@ class Engine:
             # filler's first row, if there is one).  Rows never mix, so the real rows' results
             # are what they would be alone; steps of one round shape replay one graph.
             step = 64 if n_tokens < 512 else 128
-            filled = -(-n_tokens // step) * step
-            extra = filled - n_tokens                     # (none, if the step is round already)
-            token_ids = np.concatenate([token_ids, np.zeros(extra, dtype=np.int32)])
-            positions = np.concatenate([positions, np.zeros(extra, dtype=np.int32)])
-            token_item = np.concatenate([token_item, np.full(extra, n_items, dtype=np.int32)])
-            items_filled = -(-(n_items + 1) // 8) * 8
-            for group in self.cache.groups:
-                if group.paged:
-                    spare = np.full((items_filled - n_items, group.max_blocks), group.pool.n_pages, dtype=np.int32)
-                    tables[group.index] = np.concatenate([tables[group.index], spare])
-            if n_want > 0:
-                want_filled = -(-n_want // 8) * 8
-                more = want_filled - n_want
-                want_rows = np.concatenate([want_rows, np.full(more, n_tokens if extra else 0, dtype=np.int32)])
-                want_slots = np.concatenate([want_slots, np.full(more, -1, dtype=np.int32)])
-                if sampling is not None:
-                    temperature = np.concatenate([temperature, np.zeros(more, dtype=np.float32)])
-                    top_p = np.concatenate([top_p, np.ones(more, dtype=np.float32)])
-                    seeds = np.concatenate([seeds, np.zeros(more, dtype=np.uint64)])
-                    counters = np.concatenate([counters, np.zeros(more, dtype=np.int32)])
-                n_want = want_filled
-            if tiles and extra:
-                filler = [(n_items, n_tokens, 1, 0, 0, 1, 0, 1)]
+            n_tokens = -(-n_real // step) * step          # (no filler, if the step is round already)
+            n_items = -(-(n_real_items + 1) // 8) * 8
+            n_want = -(-n_want // 8) * 8
+            if tiles and n_tokens > n_real:
+                filler = [(n_real_items, n_real, 1, 0, 0, 1, 0, 1)]
                 tiles = tiles + filler * (-len(tiles) % 4)
                 singles = singles + filler * (-len(singles) % 8)
-            # the filler is one more entry, in the slot beyond the last request's (state of fixed
-            # size is kept there for nobody); the entries after it have no tokens
-            more = items_filled - n_items
-            item_slot = np.concatenate([item_slot, np.full(more, self.max_requests, dtype=np.int32)])
-            item_offset = np.concatenate([item_offset, np.full(more, n_tokens, dtype=np.int32)])
-            item_count = np.concatenate([item_count, np.array([extra] + [0] * (more - 1), dtype=np.int32)])
-            item_start = np.concatenate([item_start, np.zeros(more, dtype=np.int32)])
-            n_tokens, n_items = filled, items_filled
-        arrays = {"token_ids": token_ids, "positions": positions, "token_item": token_item, "want_rows": want_rows,
-                  "want_slots": want_slots, "att_tiles": np.array(tiles + singles, dtype=np.int32), "item_slot": item_slot,
-                  "item_offset": item_offset, "item_count": item_count, "item_start": item_start}
-        for index, table in tables.items():
-            arrays[("block_table", index)] = table
-        if sampling is not None:
-            arrays.update(temperature=temperature, top_p=top_p, seeds=seeds, counters=counters)
         # the one-kernel decode step takes its arrays from alternating buffers, so that the next
         # step's copy runs beside it; captured graphs have their addresses fixed
         fused = (self.fused is not None and not dump_hidden and n_want <= n_tokens
                  and self.fused.takes_sizes(n_tokens, decode_only))
         alternate = fused
         # a place may be wanted twice: the per-row arrays have room for the larger count
-        views = self.control.upload(arrays, max(n_tokens, n_want), n_items, alternate)
+        if n_want > self._ids_pinned.shape[1]:
+            torch.cuda.synchronize(self.device)           # no step on its way may still write the old memory
+            self._make_ids_pinned(2 * n_want)
+            self._graphs.clear()
+        host, views = self.control.begin(max(n_tokens, n_want), n_items, alternate)
+        self._turn ^= 1                       # the slot of the readback ring this step fills
+        host["turn"][0] = self._turn
+        token_ids, want_rows, want_slots = host["token_ids"], host["want_rows"], host["want_slots"]
+        if decode_only and all(len(e.want) <= 1 for e in entries):
+            # single tokens: the arrays straight from lists
+            token_ids[:n_real] = [e.tokens[0] for e in entries]
+            host["positions"][:n_real] = starts
+            host["token_item"][:n_real] = range(n_items)
+            wanted = [(index, e.slot) for index, e in enumerate(entries) if e.want]
+            if wanted:
+                want_rows[:n_real_want] = [index for index, _ in wanted]
+                want_slots[:n_real_want] = [slot for _, slot in wanted]
+            any_previous = any(e.tokens[0] == PREVIOUS for e in entries)
+            if any_previous:
+                for row, entry in enumerate(entries):
+                    if entry.tokens[0] == PREVIOUS:
+                        token_ids[row] = -1 - entry.slot
+        else:
+            positions, token_item = host["positions"], host["token_item"]
+            want_slots[:n_real_want] = -1                 # the entry's last wanted row is kept for its slot
+            any_previous = False
+            w = 0
+            for index, entry in enumerate(entries):
+                row, n, start = ctx.item_offsets[index], ctx.item_counts[index], starts[index]
+                token_ids[row:row + n] = entry.tokens if ids[index] is None else ids[index]
+                if token_ids[row] == PREVIOUS:
+                    token_ids[row] = -1 - entry.slot
+                    any_previous = True
+                positions[row:row + n] = np.arange(start, start + n, dtype=np.int32)
+                token_item[row:row + n] = index
+                for place in entry.want:
+                    want_rows[w] = row + int(place)
+                    w += 1
+                if entry.want:
+                    want_slots[w - 1] = entry.slot
+        # the entries as the device sees them: slot, first row, rows, first position
+        for name, values in (("item_slot", slots), ("item_offset", ctx.item_offsets), ("item_count", ctx.item_counts), ("item_start", starts)):
+            host[name][:n_real_items] = values
+        for group in self.cache.groups:
+            if group.paged:
+                table = host[("block_table", group.index)]
+                table[:n_real_items] = group.table[slots]
+                table[n_real_items:] = group.pool.n_pages          # (the filler's: the spare page)
+        if tiles or singles:
+            host["att_tiles"][:len(tiles) + len(singles)] = tiles + singles
+        if sampling is not None and n_want > 0:
+            temperature, top_p, seeds, counters = (host[name] for name in ("temperature", "top_p", "seeds", "counters"))
+            temperature[:n_real_want] = [s.temperature for s in sampling]
+            top_p[:n_real_want] = [s.top_p for s in sampling]
+            seeds[:n_real_want] = [s.seed & 0xFFFFFFFFFFFFFFFF for s in sampling]
+            counters[:n_real_want] = [s.counter for s in sampling]
+            temperature[n_real_want:n_want], top_p[n_real_want:n_want] = 0.0, 1.0
+            seeds[n_real_want:n_want], counters[n_real_want:n_want] = 0, 0
+        if padded:
+            token_ids[n_real:n_tokens], host["positions"][n_real:n_tokens] = 0, 0
+            host["token_item"][n_real:n_tokens] = n_real_items
+            want_rows[n_real_want:n_want], want_slots[n_real_want:n_want] = n_real if n_tokens > n_real else 0, -1
+            # the filler is one more entry, in the slot beyond the last request's (state of fixed
+            # size is kept there for nobody); the entries after it have no tokens
+            host["item_slot"][n_real_items:], host["item_offset"][n_real_items:] = self.max_requests, n_real
+            host["item_count"][n_real_items:], host["item_start"][n_real_items:] = 0, 0
+            host["item_count"][n_real_items] = n_tokens - n_real
+        self.control.send(alternate)
 
         ctx.n_tokens, ctx.n_items, ctx.n_want = n_tokens, n_items, n_want
         ctx.token_ids, ctx.positions = views["token_ids"][:n_tokens], views["positions"][:n_tokens]
@@ -397,6 +396,8 @@ class Engine:
         ctx.any_previous = any_previous
         ctx.decode_only = decode_only
         ctx.fused = fused
+        ctx.in_ring = not alternate
+        ctx.turn = views["turn"]
         ctx.dump = [] if dump_hidden else None
         ctx.att_tiles, ctx.n_att_tiles = (views["att_tiles"] if tiles else None), len(tiles) + len(singles)
         ctx.n_att_singles = len(singles)
@@ -411,7 +412,6 @@ class Engine:
         if sampling is not None and n_want > 0:
             sample_views = (views["temperature"][:n_want], views["top_p"][:n_want], views["seeds"][:n_want],
                             views["counters"][:n_want])
-        self._turn ^= 1                       # the slot of the readback ring this step fills
         compute = torch.cuda.current_stream(self.device)
         # This step's kernels write their sampled ids where an earlier step left its own: that
         # step's copy to the host must be done.  Two steps that alternate use different buffers,
@@ -423,7 +423,7 @@ class Engine:
         self._alternated = alternate
         logits = self._run(ctx, sample_views)
         self.hidden_dump = ctx.dump
-        self.control.consumed()
+        self.control.consumed(alternate)
         for entry in entries:
             self.cache.commit(entry.slot, len(entry.tokens))
         self.steps += 1
@@ -431,27 +431,23 @@ class Engine:
         if logits is not None and logits.shape[0] != n_want:
             logits = logits[:n_want]
         if self._sampled is not None:
-            # the sampled ids start for the host right behind the step's kernels; for the steps
-            # that alternate on a stream of their own, so that the next step's kernels do not
-            # queue behind the copy
-            held = self._readback[self._turn]
-            if held is None or held[0].shape[0] < n_want:
-                held = (torch.empty(max(n_want, 64), dtype=torch.int32).pin_memory(), 0, torch.cuda.Event())
-            # with them comes the word in which a kernel reports a wait that ran out, so that
-            # no token of a failed step is ever handed on
-            status = self.kernels.status(self.device)
+            # the sampled ids start for the host right behind the step's kernels, with the word in which a kernel reports a wait
+            # that ran out, so that no token of a failed step is ever handed on
             if alternate:
+                # on a stream of their own, so that the next step's kernels do not queue behind the copy
+                if self._ids_beside[self._turn] is None or self._ids_beside[self._turn].shape[0] < n_want:
+                    self._ids_beside[self._turn] = torch.empty(max(n_want, 64), dtype=torch.int32).pin_memory()
+                held = (self._ids_beside[self._turn], n_want, self._copied_beside[self._turn])
                 done = self._sampled_events[self._turn]
                 done.record(compute)
                 with torch.cuda.stream(self._readback_stream):
                     self._readback_stream.wait_event(done)
                     held[0][:n_want].copy_(self._sampled[:n_want], non_blocking=True)
-                    self._status_pinned[self._turn:self._turn + 1].copy_(status, non_blocking=True)
+                    self._status_pinned[self._turn:self._turn + 1].copy_(self.kernels.status(self.device), non_blocking=True)
                     held[2].record(self._readback_stream)
             else:
-                held[0][:n_want].copy_(self._sampled[:n_want], non_blocking=True)
-                self._status_pinned[self._turn:self._turn + 1].copy_(status, non_blocking=True)
-                held[2].record(compute)
+                # the last kernel wrote them to pinned memory itself
+                held = (self._ids_pinned[self._turn], n_want, self.control.done)
             self._readback[self._turn] = (held[0], n_want, held[2])
             for entry in entries:
                 if entry.want:
@@ -466,6 +462,8 @@ class Engine:
             return self._forward_on_stream(ctx, sample_views)
 
     def _forward_on_stream(self, ctx, sample_views):
+        if ctx.in_ring:
+            self.control.take()
         if ctx.any_previous:
             self.kernels.resolve_tokens(ctx.token_ids, self.kept_tokens)
         logits = self.model.forward(ctx, self.storage.views)
@@ -473,7 +471,9 @@ class Engine:
         if sample_views is not None and logits is not None:
             out = self.workspace.get(f"sampled{self.control.parity}", (ctx.n_want,), torch.int32)
             self.kernels.sample_rows(out, logits, *sample_views, any_nucleus=self._any_nucleus)
-            self.kernels.keep_tokens(self.kept_tokens, ctx.want_slots, out)
+            self.kernels.keep_tokens(self.kept_tokens, ctx.want_slots, out,
+                                     (self._ids_address, self._ids_pinned.shape[1], self._status_address, ctx.turn,
+                                      self.kernels.status(self.device)))
             self._sampled = out
         return logits
 
@@ -503,7 +503,7 @@ class Engine:
             self._graph_stamp = stamp
         # (how many units come in parts is data; that some do decides whether the kernel gets scratch)
         key = (ctx.n_tokens, ctx.n_items, ctx.n_want, ctx.n_att_tiles, ctx.n_att_singles, ctx.att_parts > 1, ctx.att_units,
-               sample_views is not None, self._any_nucleus, ctx.any_previous, self.control.parity)
+               sample_views is not None, self._any_nucleus, ctx.any_previous, self.control.parity, ctx.in_ring)
         held = self._graphs.get(key)
         # A shape runs eagerly the first time (every buffer it needs gets allocated) and is
         # captured when it comes back: a capture costs about as much as two eager steps of a

@@ -83,9 +83,9 @@ class Kernels:
         self._memory_readers = None
 
     # ---- operations without a fast variant --------------------------------------------------
-    def keep_tokens(self, kept, slots, tokens):
+    def keep_tokens(self, kept, slots, tokens, to_host=None):
         self.launches += 1
-        return ops.keep_tokens(kept, slots, tokens)
+        return ops.keep_tokens(kept, slots, tokens, to_host)
 
     def resolve_tokens(self, token_ids, kept):
         self.launches += 1

@@ -818,20 +818,58 @@ def layernorm_warp(out, x, gamma, beta, eps, rows=None):
     return out
 
 
-_keep_tokens = Function("sampling", "mllm_sampling_keep_tokens", [P, P, P, I, I, P])
+_keep_tokens = Function("sampling", "mllm_sampling_keep_tokens", [P, P, P, I, I, P, L, P, P, P, P])
+_control = Function("sampling", "mllm_sampling_control", [P, P, L, I, P, L, P])
+_zero_slot = Function("sampling", "mllm_sampling_zero_slot", [P, I, I, P])
+_device_address = Function("sampling", "mllm_sampling_device_address", [P, ctypes.POINTER(ctypes.c_void_p)])
 _resolve_tokens = Function("sampling", "mllm_sampling_resolve_tokens", [P, P, I, I, P])
 
 
-def keep_tokens(kept, slots, tokens):
-    """kept[slots[r]] = tokens[r] for every row r with slots[r] >= 0 (all int32, on the device)."""
+def keep_tokens(kept, slots, tokens, to_host=None):
+    """kept[slots[r]] = tokens[r] for every row r with slots[r] >= 0 (all int32, on the device).  ``to_host``: (device address of
+    pinned ids [2, step], step, device address of two pinned status words, turn, status): the tokens and the status word also go to
+    the part of them that the device int32 ``turn`` names."""
     _check(kept, "keep_tokens.kept", torch.int32, 1)
     _check(slots, "keep_tokens.slots", torch.int32, 1)
     _check(tokens, "keep_tokens.tokens", torch.int32, 1)
     n = tokens.shape[0]
     if slots.shape[0] < n:
         raise KernelError("keep_tokens: fewer slots than tokens")
-    _keep_tokens(kept.data_ptr(), slots.data_ptr(), tokens.data_ptr(), n, kept.shape[0], _stream())
+    if to_host is None:
+        _keep_tokens(kept.data_ptr(), slots.data_ptr(), tokens.data_ptr(), n, kept.shape[0], None, 0, None, None, None, _stream())
+        return kept
+    ids, step, status_copy, turn, status = to_host
+    _check(turn, "keep_tokens.turn", torch.int32, 1)
+    _check(status, "keep_tokens.status", torch.int32, 1)
+    if n > step:
+        raise KernelError("keep_tokens: more tokens than the pinned memory holds")
+    _keep_tokens(kept.data_ptr(), slots.data_ptr(), tokens.data_ptr(), n, kept.shape[0], ids, step, status_copy, turn.data_ptr(),
+                 status.data_ptr(), _stream())
     return kept
+
+
+def device_address(pinned) -> int:
+    """Where the device finds a pinned host tensor."""
+    found = ctypes.c_void_p()
+    _device_address(pinned.data_ptr(), ctypes.byref(found))
+    return found.value
+
+
+def control(block, ring_address, ring_step, ring_parts, steps, n_ints):
+    """block[:n_ints] = the part of a ring of ``ring_parts`` in pinned host memory, ``ring_step`` ints apart, that ``steps[0]`` names
+    (device int32 [2], zero at first); counts the step there.  n_ints and ring_step are multiples of 4."""
+    _check(block, "control.block", torch.int32, 1)
+    _check(steps, "control.steps", torch.int32, 1)
+    if block.shape[0] < n_ints or steps.shape[0] < 2:
+        raise KernelError("control: the block or the counters are too short")
+    _control(block.data_ptr(), ring_address, 4 * int(ring_step), int(ring_parts), steps.data_ptr(), 4 * int(n_ints), _stream())
+
+
+def zero_slot(tables, slot):
+    """Zeroes slot ``slot`` of every state that ``tables`` (device int64 [n, 4]: first byte, run entries, bytes between entries,
+    bytes of a slot) names."""
+    _check(tables, "zero_slot.tables", torch.int64, 2)
+    _zero_slot(tables.data_ptr(), tables.shape[0], int(slot), _stream())
 
 
 def resolve_tokens(token_ids, kept):

@@ -385,3 +385,37 @@ def test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, ga
     # of the activations, of size 1, one in some thousands rounds the other way (2^-8 of it): far below 1e-3 of the sums
     assert np.linalg.norm(f64(hidden) - expected) <= 1e-3 * np.linalg.norm(expected)
     assert np.abs(f64(hidden) - expected).max() <= 0.03
+
+
+@pytest.mark.parametrize("ints", [4, 1020, 4096, 4100, 70000])       # a piece, a thread's, a block's and all blocks' edges
+def test_control_block_from_the_ring(ints):
+    from mini_llm_b200.kernels import ops
+    parts, step = 3, ints + 8
+    ring = torch.arange(parts * step, dtype=torch.int32).pin_memory()
+    steps, block = torch.zeros(2, dtype=torch.int32, device="cuda"), torch.empty(ints + 4, dtype=torch.int32, device="cuda")
+    for taken in range(5):
+        block.fill_(-1)
+        ops.control(block, ops.device_address(ring), step, parts, steps, ints)
+        start = taken % parts * step
+        assert bool((block[:ints].cpu() == ring[start:start + ints]).all()) and bool((block[ints:] == -1).all())
+        assert steps.tolist() == [(taken + 1) % parts, 0]
+
+
+def test_an_emptied_slot_and_draws_on_the_host():
+    from mini_llm_b200.kernels import ops
+    states = [torch.ones(3, 5, 8, 16, device="cuda"), torch.ones(1, 5, 7, dtype=torch.bfloat16, device="cuda"), torch.ones(2, 5, 3, dtype=torch.int32, device="cuda")]
+    table = torch.tensor([[s.data_ptr(), s.shape[0], s.stride(0) * s.element_size(), s.stride(1) * s.element_size()] for s in states],
+                         dtype=torch.int64, device="cuda")
+    for slot in (4, 0):
+        ops.zero_slot(table, slot)
+    for s in states:
+        assert bool((s[:, [0, 4]] == 0).all()) and bool((s[:, 1:4] == 1).all())
+    ids, words = torch.full((2, 200), -1, dtype=torch.int32).pin_memory(), torch.zeros(2, dtype=torch.int32).pin_memory()
+    kept, status = torch.zeros(4, dtype=torch.int32, device="cuda"), torch.tensor([7], dtype=torch.int32, device="cuda")
+    slots, tokens = dev(np.arange(130) % 9 - 4, torch.int32), dev(np.arange(130) + 50, torch.int32)
+    for turn in (0, 1):
+        ops.keep_tokens(kept, slots, tokens + turn, (ops.device_address(ids), 200, ops.device_address(words), dev([turn], torch.int32), status))
+    torch.cuda.synchronize()
+    for turn in (0, 1):
+        assert ids[turn].tolist() == [50 + turn + r for r in range(130)] + [-1] * 70
+    assert words.tolist() == [7, 7]
