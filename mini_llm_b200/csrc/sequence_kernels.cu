@@ -541,10 +541,12 @@ __global__ void latent_prepare_kernel(T* __restrict__ pages, float* __restrict__
                                       const int* __restrict__ token_item, const int* __restrict__ block_table,
                                       int max_blocks, int page_size, int rank, int rot, int rot_dims, int heads, int dim,
                                       float eps, int writes, int layout) {
-    dependents_may_start();
-    wait_for_earlier_kernels();
-    __shared__ float scratch[33];
+    // What the projections ahead do not write is done ahead of the wait for them: the angles, the row's place, the gains.
+    // (Behind it every load is asked for before any is used: 5.9 us in a decode step of 8 tokens when all of it followed the wait.)
+    constexpr int HELD = 4;
+    __shared__ float slots[32];
     extern __shared__ float turn[];                  // cos[rot_dims / 2], sin[rot_dims / 2]
+    dependents_may_start();
     const int t = blockIdx.x;
     const int p = positions[t];
     const int half = rot_dims / 2;
@@ -563,38 +565,73 @@ __global__ void latent_prepare_kernel(T* __restrict__ pages, float* __restrict__
         i = e < half ? e : e - half, partner = e < half ? e + half : e - half;
         return e >= half;
     };
+    auto turned = [&](int e, float v, float other) {
+        if (e >= 2 * half) return v;
+        int i, partner;
+        const bool second = pair_of(e, i, partner);
+        const float c = turn[i], s = turn[half + i];
+        return second ? v * c + other * s : v * c - other * s;
+    };
+    auto partner_of = [&](int e) {
+        int i, partner = e;
+        if (e < 2 * half) pair_of(e, i, partner);
+        return partner;
+    };
+    T* row = pages;
+    float gains[HELD];
     if (writes) {
-        const float* mine = down + (long)t * ld_down;
-        float sq = 0.0f;
-        for (int d = threadIdx.x; d < rank; d += blockDim.x) sq = fmaf(mine[d], mine[d], sq);
-        const float inv = 1.0f / sqrtf(block_sum(sq, scratch) / (float)rank + eps);      // (its barriers also publish turn[])
         const int page = block_table[(long)token_item[t] * max_blocks + p / page_size];
-        T* row = pages + ((long)page * page_size + (p % page_size)) * (rank + rot);
-        for (int d = threadIdx.x; d < rank; d += blockDim.x) row[d] = from_f32<T>(mine[d] * inv * gain[d]);
-        for (int e = threadIdx.x; e < rot; e += blockDim.x) {
-            float v = mine[rank + e];
-            if (e < 2 * half) {
-                int i, partner;
-                const bool second = pair_of(e, i, partner);
-                const float c = turn[i], s = turn[half + i];
-                v = second ? v * c + mine[rank + partner] * s : v * c - mine[rank + partner] * s;
-            }
-            row[rank + e] = from_f32<T>(v);
+        row += ((long)page * page_size + (p % page_size)) * (rank + rot);
+#pragma unroll
+        for (int i = 0; i < HELD; i++) {
+            const int d = threadIdx.x + i * blockDim.x;
+            gains[i] = d < rank ? gain[d] : 0.0f;
         }
+    }
+    wait_for_earlier_kernels();
+    q = behind_the_wait(q) + (long)t * ld_q + dim;
+    const int per_head = heads * rot, entries = max(rot, 1);
+    float qv[HELD], qo[HELD];
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+        const int u = threadIdx.x + i * blockDim.x;
+        const T* from = q + (long)(u / entries) * (dim + rot);
+        qv[i] = u < per_head ? to_f32(from[u % entries]) : 0.0f;
+        qo[i] = u < per_head ? to_f32(from[partner_of(u % entries)]) : 0.0f;
+    }
+    if (writes) {
+        const float* mine = behind_the_wait(down) + (long)t * ld_down;
+        float held[HELD], sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < HELD; i++) {
+            const int d = threadIdx.x + i * blockDim.x;
+            held[i] = d < rank ? mine[d] : 0.0f;
+            sq = fmaf(held[i], held[i], sq);
+        }
+        for (int d = threadIdx.x + HELD * blockDim.x; d < rank; d += blockDim.x) sq = fmaf(mine[d], mine[d], sq);
+        const int e = threadIdx.x;
+        const float v = e < rot ? mine[rank + e] : 0.0f, other = e < rot ? mine[rank + partner_of(e)] : 0.0f;
+        const float inv = 1.0f / sqrtf(block_sum_once(sq, slots) / (float)rank + eps);      // (its barrier also publishes turn[])
+#pragma unroll
+        for (int i = 0; i < HELD; i++) {
+            const int d = threadIdx.x + i * blockDim.x;
+            if (d < rank) row[d] = from_f32<T>(held[i] * inv * gains[i]);
+        }
+        for (int d = threadIdx.x + HELD * blockDim.x; d < rank; d += blockDim.x) row[d] = from_f32<T>(mine[d] * inv * gain[d]);
+        if (e < rot) row[rank + e] = from_f32<T>(turned(e, v, other));
+        for (int u = e + blockDim.x; u < rot; u += blockDim.x) row[rank + u] = from_f32<T>(turned(u, mine[rank + u], mine[rank + partner_of(u)]));
     } else {
         __syncthreads();                             // publishes turn[]
     }
-    for (int u = threadIdx.x; u < heads * rot; u += blockDim.x) {
-        const int head = u / rot, e = u % rot;
-        const T* from = q + (long)t * ld_q + (long)head * (dim + rot) + dim;
-        float v = to_f32(from[e]);
-        if (e < 2 * half) {
-            int i, partner;
-            const bool second = pair_of(e, i, partner);
-            const float c = turn[i], s = turn[half + i];
-            v = second ? v * c + to_f32(from[partner]) * s : v * c - to_f32(from[partner]) * s;
-        }
-        q_eff[((long)t * heads + head) * (rank + rot) + rank + e] = v;
+    float* to = q_eff + (long)t * heads * (rank + rot) + rank;
+#pragma unroll
+    for (int i = 0; i < HELD; i++) {
+        const int u = threadIdx.x + i * blockDim.x;
+        if (u < per_head) to[(long)(u / entries) * (rank + rot) + u % entries] = turned(u % entries, qv[i], qo[i]);
+    }
+    for (int u = threadIdx.x + HELD * blockDim.x; u < per_head; u += blockDim.x) {
+        const T* from = q + (long)(u / entries) * (dim + rot);
+        to[(long)(u / entries) * (rank + rot) + u % entries] = turned(u % entries, to_f32(from[u % entries]), to_f32(from[partner_of(u % entries)]));
     }
 }
 
@@ -882,6 +919,7 @@ struct LatentTiledParams {
     int window;                    // a query sees the last `window` positions only (<= 0: all)
     const float* gate;             // [T, >= heads] (rows ld_gate apart) or null: head h's result times sigmoid(gate[t, h])
     long ld_gate;
+    int rows_ahead;                // single tokens: of the cached rows only the tokens' own are written by kernels that may still run
 };
 
 template <typename T> struct Chunk4;
@@ -1367,6 +1405,241 @@ static int launch_latent_mma(const LatentTiledParams& p, int n_units, cudaStream
     return check_launch("latent_attention_mma_kernel");
 }
 
+// ---------------------------------------------------------------------------
+// Single tokens over a latent of 128 or 256 entries, bfloat16 rows, up to 16 heads, on tensor-core tiles: the heads are the 16 rows.  The
+// `parts` blocks of a cluster take a share of a token's cached rows each, 32 at a time, and merge through each other's shared memory,
+// every block the heads' sums of its share of the columns, in the order of the parts.  For a tile the warps share the rows' entries (two
+// groups of 16 keys, four quarters of the entries), then the columns of the weighted sum; queries and weights enter as three
+// bfloat16 terms, as for prompt portions.  What bounds it is a chain of latencies, so with `rows_ahead` all cached rows but the token's own
+// are asked for ahead of the wait for the kernels ahead (within a step only that one row is written, and no kernel of a step starts before the
+// step before has ended; position and block table come with the step's arrays).
+// One token of 512, 8 of up to 266, 3 of up to 900, 40 of up to 100 cached rows, 12 heads over 256 + 32: 7.0, 8.7, 8.7, 11.7 us back to back, where
+// FMAs with up to 32 blocks a token and a merge in a kernel of its own took 14.5, 15.6, 15.4, 20.7.  Errors against 64 bits 4.5e-7 -> 1.7e-7.
+// ---------------------------------------------------------------------------
+constexpr int LATENT_STEP_KEYS = 32;
+template <int RANK> struct LatentStep {
+    static constexpr int LDP = LATENT_STEP_KEYS + 8, LDS = LATENT_STEP_KEYS + 4, LDO = RANK + 4;
+    static constexpr size_t SCORES = 4 * 16 * LDS * 4, WEIGHTS = 3 * 16 * LDP * 2, STATES = 3 * 16 * 4;
+    static size_t bytes(int row_width) {
+        const size_t operands = (size_t)(3 * 16 + 2 * LATENT_STEP_KEYS) * (row_width + 8) * 2, sums = (size_t)16 * LDO * 4;
+        return SCORES + WEIGHTS + STATES + (operands > sums ? operands : sums);
+    }
+};
+
+__device__ __forceinline__ float load_of_block(const float* mine, int rank) {
+    uint32_t at;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+    return v;
+}
+
+template <int RANK>
+__global__ void __launch_bounds__(256)
+latent_step_kernel(LatentTiledParams p) {
+    using L = LatentStep<RANK>;
+    constexpr int KEYS = LATENT_STEP_KEYS, LDP = L::LDP, LDS = L::LDS, LDO = L::LDO, PAIRS = RANK / 128;      // PAIRS: of column tiles a warp
+    extern __shared__ __align__(16) unsigned char step_shared[];
+    const int row_width = p.rank + p.rot, ld = row_width + 8, pieces = row_width / 8;                          // (an odd number of 16 bytes)
+    float* scores = reinterpret_cast<float*>(step_shared);                        // [quarter][16][LDS]
+    bf16* weights = reinterpret_cast<bf16*>(step_shared + L::SCORES);             // [term][16][LDP]
+    float* factor = reinterpret_cast<float*>(step_shared + L::SCORES + L::WEIGHTS);       // [16], then the rows' maxima and sums
+    float *maxima = factor + 16, *totals = factor + 32;
+    bf16* q_terms = reinterpret_cast<bf16*>(step_shared + L::SCORES + L::WEIGHTS + L::STATES);       // [term][16][ld]
+    bf16* tiles = q_terms + 3 * 16 * ld;                                          // [2][KEYS][ld]
+    float* sums = reinterpret_cast<float*>(q_terms);                              // over both, at the end: [16][LDO]
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+    const int t = blockIdx.x, part = blockIdx.z, parts = gridDim.z;
+    dependents_may_start();
+    const int position = p.positions[t];
+    const int* bt = p.block_table + (long)p.token_item[t] * p.max_blocks;
+    const int first_key = p.window > 0 ? max(0, position - p.window + 1) : 0, n_keys = position + 1 - first_key;
+    const int each = ((n_keys + parts - 1) / parts + KEYS - 1) / KEYS * KEYS, used = (n_keys + each - 1) / each;
+    const int key_begin = min(position + 1, first_key + part * each), key_end = min(position + 1, key_begin + each);
+    // one warp a row; `before`: rows from there on are left out
+    auto ask = [&](int k0, int buffer, int before) {
+        for (int j = warp; j < KEYS; j += 8) {
+            const int key = k0 + j;
+            if (key >= before && key < key_end) continue;
+            const bool there = key < key_end;
+            const bf16* from = reinterpret_cast<const bf16*>(p.pages);
+            if (there) from += ((long)bt[key / p.page_size] * p.page_size + key % p.page_size) * row_width;
+            bf16* to = tiles + (buffer * KEYS + j) * ld;
+            for (int c = lane; c < pieces; c += 32) copy_16(to + c * 8, there ? from + c * 8 : from, there);
+        }
+    };
+    if (p.rows_ahead) {
+        ask(key_begin, 0, position);
+        ask(key_begin + KEYS, 1, position);
+    }
+    wait_for_earlier_kernels();
+    const float* q_eff = behind_the_wait(p.q_eff);
+    if (!p.rows_ahead) {
+        ask(key_begin, 0, position);
+        ask(key_begin + KEYS, 1, position);
+    }
+    {
+        // the token's own row, if it lies in the first two tiles
+        const int j = position - key_begin;
+        if (position < key_end && j < 2 * KEYS && warp == 0) {
+            const bf16* from = reinterpret_cast<const bf16*>(behind_the_wait(p.pages)) +
+                               ((long)bt[position / p.page_size] * p.page_size + position % p.page_size) * row_width;
+            for (int c = lane; c < pieces; c += 32) copy_16(tiles + j * ld + c * 8, from + c * 8, true);
+        }
+        copies_end();
+    }
+    for (int r = warp; r < 16; r += 8)
+        for (int d = lane * 4; d < row_width; d += 128) {
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (r < p.heads) x = *reinterpret_cast<const float4*>(q_eff + ((long)t * p.heads + r) * row_width + d);
+            uint2 terms[3];
+            three_terms(x.x, x.y, terms[0].x, terms[1].x, terms[2].x);
+            three_terms(x.z, x.w, terms[0].y, terms[1].y, terms[2].y);
+#pragma unroll
+            for (int i = 0; i < 3; i++) *reinterpret_cast<uint2*>(q_terms + (i * 16 + r) * ld + d) = terms[i];
+        }
+    const float scale_log2 = p.scale * 1.4426950408889634f;                       // exp(x) = 2^(x log2 e)
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.0f, 0.0f};                     // of rows 2 warp and 2 warp + 1, the same in every lane
+    float o[2 * PAIRS][4];
+#pragma unroll
+    for (int j = 0; j < 2 * PAIRS; j++) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.0f;
+    int buffer = 0;
+    for (int k0 = key_begin; k0 < key_end; k0 += KEYS, buffer ^= 1) {
+        if (k0 < key_begin + 2 * KEYS) copies_landed<0>();
+        else copies_landed<1>();
+        __syncthreads();                                                          // (the queries' terms are written, too)
+        const bf16* kt = tiles + buffer * KEYS * ld;
+        {
+            const int group = warp & 1, quarter = warp >> 1;
+            float s[2][4] = {};
+            const bf16* q_at = q_terms + (lane & 15) * ld + (lane >> 4) * 8;
+            const bf16* k_at = kt + (group * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * ld + ((lane >> 3) & 1) * 8;
+            for (int k = quarter * 16; k < row_width; k += 64) {
+                uint32_t b[4];
+                float x[2][4] = {};
+                load_blocks(b, k_at + k);
+#pragma unroll
+                for (int i = 2; i >= 0; i--) {                                    // the small terms first
+                    uint32_t a[4];
+                    load_blocks(a, q_at + i * 16 * ld + k);
+                    mma_tile(x[0], a, b[0], b[1]);
+                    mma_tile(x[1], a, b[2], b[3]);
+                }
+#pragma unroll
+                for (int e = 0; e < 8; e++) s[e / 4][e % 4] += x[e / 4][e % 4];   // (rounded, not cut off)
+            }
+#pragma unroll
+            for (int e = 0; e < 8; e++)
+                scores[(quarter * 16 + g + ((e >> 1) & 1) * 8) * LDS + group * 16 + (e >> 2) * 8 + 2 * tq + (e & 1)] = s[e / 4][e % 4];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int r = 2 * warp + h;
+            float x = 0.0f;
+#pragma unroll
+            for (int u = 0; u < 4; u++) x += scores[(u * 16 + r) * LDS + lane];
+            x = k0 + lane < key_end ? x * scale_log2 : -INFINITY;
+            const float m_new = fmaxf(m[h], warp_max(x)), from = m_new == -INFINITY ? 0.0f : m_new;
+            const float corr = exp2f(m[h] - from), w = exp2f(x - from);
+            l[h] = l[h] * corr + warp_sum(w);
+            m[h] = m_new;
+            uint32_t terms[3];
+            three_weight_terms(w, w, terms[0], terms[1], terms[2]);
+#pragma unroll
+            for (int i = 0; i < 3; i++) reinterpret_cast<unsigned short*>(weights)[(i * 16 + r) * LDP + lane] = (unsigned short)terms[i];
+            if (lane == 0) factor[r] = corr;
+        }
+        __syncthreads();
+        {
+            uint32_t a[2][3][4];
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+#pragma unroll
+                for (int i = 0; i < 3; i++) load_blocks(a[k][i], weights + (i * 16 + (lane & 15)) * LDP + k * 16 + (lane >> 4) * 8);
+            const float corr[2] = {factor[g], factor[g + 8]};
+            const bf16* v_at = kt + ((lane & 7) + ((lane >> 3) & 1) * 8) * ld + ((lane >> 4) & 1) * 8 + warp * (RANK / 8);
+#pragma unroll
+            for (int j = 0; j < 2 * PAIRS; j += 2) {
+                uint32_t b[2][4];
+                float x[2][4];
+#pragma unroll
+                for (int k = 0; k < 2; k++) load_blocks_turned(b[k], v_at + k * 16 * ld + j * 8);
+                weighted_rows(x, a, b);
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    o[j][e] = fmaf(o[j][e], corr[e >> 1], x[0][e]);
+                    o[j + 1][e] = fmaf(o[j + 1][e], corr[e >> 1], x[1][e]);
+                }
+            }
+        }
+        __syncthreads();                                                          // this tile and the scores are used up
+        if (k0 + 2 * KEYS < key_end) ask(k0 + 2 * KEYS, buffer, position + 1);
+        copies_end();
+    }
+    copies_landed<0>();
+    __syncthreads();                                                              // (no copy still writes where the sums go)
+#pragma unroll
+    for (int j = 0; j < 2 * PAIRS; j++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) sums[(g + (e >> 1) * 8) * LDO + warp * (RANK / 8) + j * 8 + 2 * tq + (e & 1)] = o[j][e];
+    if (lane == 0)
+#pragma unroll
+        for (int h = 0; h < 2; h++) maxima[2 * warp + h] = m[h], totals[2 * warp + h] = l[h];
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int columns = RANK / parts;
+    for (int i = tid; i < p.heads * columns; i += 256) {
+        const int head = i / columns, c = part * columns + i % columns;
+        float big = -INFINITY, total = 0.0f, out = 0.0f;
+        float mz[16], lz[16], oz[16];
+#pragma unroll
+        for (int z = 0; z < 16; z++) {
+            mz[z] = z < used ? load_of_block(maxima + head, z) : -INFINITY;
+            lz[z] = z < used ? load_of_block(totals + head, z) : 0.0f;
+            oz[z] = z < used ? load_of_block(sums + head * LDO + c, z) : 0.0f;
+        }
+#pragma unroll
+        for (int z = 0; z < 16; z++) big = fmaxf(big, mz[z]);
+#pragma unroll
+        for (int z = 0; z < 16; z++) {
+            const float w = mz[z] == -INFINITY ? 0.0f : exp2f(mz[z] - big);
+            total = fmaf(lz[z], w, total);
+            out = fmaf(oz[z], w, out);
+        }
+        out *= (p.gate != nullptr ? gate_open(behind_the_wait(p.gate)[(long)t * p.ld_gate + head]) : 1.0f) / total;
+        const long at = ((long)t * p.heads + head) * RANK + c;
+        if (p.out_bf16) reinterpret_cast<bf16*>(p.out)[at] = __float2bfloat16_rn(out);
+        else reinterpret_cast<float*>(p.out)[at] = out;
+    }
+    // nobody leaves while its shared memory may still be read
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+static bool latent_step_takes(const LatentTiledParams& p, int dtype) {
+    const int row_width = p.rank + p.rot;
+    return dtype == DT_BF16 && p.tiles == nullptr && p.heads <= 16 && (p.rank == 128 || p.rank == 256) && row_width % 16 == 0 && row_width <= 512 &&
+           (reinterpret_cast<uintptr_t>(p.pages) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.q_eff) & 15) == 0;
+}
+
+// Blocks that share a token's rows: 16 while no more than two come to an SM (17 tokens of up to 981 rows, heads of 128: 14.6 us with 8,
+// 11.1 with 16; 80 of up to 1,034: 78, 42 us with 1, 4).
+static int latent_step_parts(int n_tokens) { return n_tokens <= 18 ? 16 : n_tokens <= 37 ? 8 : n_tokens <= 74 ? 4 : n_tokens <= 148 ? 2 : 1; }
+
+template <int RANK>
+static int launch_latent_step(const LatentTiledParams& p, int n_tokens, cudaStream_t s) {
+    const size_t shared = LatentStep<RANK>::bytes(p.rank + p.rot);
+    // (at every launch, as the limits are a device's own)
+    if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess ||
+        cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+        return fail("latent_attention: the steps' shared memory or clusters were refused");
+    const int parts = latent_step_parts(n_tokens);
+    if (launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p) != cudaSuccess) {
+        cudaGetLastError();
+        return fail("latent_attention: the clusters of a step were refused");
+    }
+    return check_launch("latent_step_kernel");
+}
+
 // The parts of a (token, head) into one result, in the order of the parts.
 __global__ void latent_merge_kernel(void* __restrict__ out, int out_bf16, const float* __restrict__ part_out,
                                     const float* __restrict__ part_ml, int parts, int rank, int heads,
@@ -1443,6 +1716,8 @@ extern "C" int mllm_sequence_latent_attention_tiled(const LatentTiledParams* par
         return fail("latent_attention_tiled: parts are for single tokens and need scratch");
     if (latent_mma_takes(p, dtype))
         return p.rank == 128 ? launch_latent_mma<128>(p, n_units, (cudaStream_t)stream) : launch_latent_mma<256>(p, n_units, (cudaStream_t)stream);
+    if (latent_step_takes(p, dtype))
+        return p.rank == 128 ? launch_latent_step<128>(p, n_units, (cudaStream_t)stream) : launch_latent_step<256>(p, n_units, (cudaStream_t)stream);
     const int element_bytes = dtype == DT_F32 ? 4 : 2;
     // prompt portions take 64 keys a block where two such blocks, or one, fit beside the queries
     int keys = 32;

@@ -294,7 +294,7 @@ class Kernels:
                 scratch = self._latent_scratch(ctx.device, n * heads * parts * rank, n * heads * parts * 2) if parts > 1 else None
                 self.launches += 1 if parts > 1 else 0
                 self.chose("latent_attention", "latent_attention_tiled_parts", n, heads, rank + rot)
-                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate)
+                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate, rows_ahead=True)
         self.chose("latent_attention", "latent_attention_plain", n, heads, rank + rot)
         plain_out = out if out.dtype == torch.float32 else ctx.buffer("latent_mixed_32", out.shape, torch.float32)
         ops.latent_attention_plain(plain_out, q_eff, cache.k_pages, cache.block_table, ctx.positions, ctx.token_item,

@@ -419,3 +419,35 @@ def test_an_emptied_slot_and_draws_on_the_host():
     for turn in (0, 1):
         assert ids[turn].tolist() == [50 + turn + r for r in range(130)] + [-1] * 70
     assert words.tolist() == [7, 7]
+
+
+# a cluster's share of the keys: none for most blocks, one tile's edges, two tiles and one more, a ring that is asked for again; windows that
+# cut the first tile; the token's own row in the first, the second and a later tile of its block; all numbers of blocks a cluster has
+@pytest.mark.parametrize("tokens, heads, rank, rot, window", [(1, 12, 256, 32, 0), (3, 16, 256, 64, 70), (5, 3, 128, 0, 0), (19, 5, 128, 48, 0), (40, 12, 256, 32, 33), (90, 2, 128, 16, 0),
+                                                              (150, 1, 128, 32, 200)])
+@pytest.mark.parametrize("ahead", [True, False])
+def test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, ahead):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(tokens + rank)
+    page, row = 16, rank + rot
+    lengths = [(1, 32, 33, 64, 65, 512, 513, 1030, 1500)[i % 9] + i // 9 for i in range(tokens)]
+    blocks = [-(-n // page) for n in lengths]
+    order = rng.permutation(sum(blocks))
+    table = np.full((tokens, max(blocks)), -1, dtype=np.int32)
+    for i, count in enumerate(blocks):
+        table[i, :count] = order[sum(blocks[:i]):sum(blocks[:i]) + count]
+    pages = dev(rng.normal(size=(sum(blocks), page, 1, row)), torch.bfloat16)
+    for i, n in enumerate(lengths):                       # what lies past a request's end must not matter
+        pages[table[i, -(-n // page) - 1], (n - 1) % page + 1:] = math.nan
+    q, gate = dev(rng.normal(size=(tokens, heads * row)) * 0.7, torch.float32), dev(rng.normal(size=(tokens, heads)), torch.float32)
+    common = (q, pages, dev(table, torch.int32), dev(np.array(lengths) - 1, torch.int32), dev(np.arange(tokens), torch.int32), heads, rank, rot, page, 0.1)
+    got = torch.full((tokens, heads * rank), math.nan, device="cuda")
+    scratch = (torch.empty(tokens * heads * 2 * rank, device="cuda"), torch.empty(tokens * heads * 4, device="cuda"))
+    ops.latent_attention_tiled(got, *common, parts=2, scratch=scratch, window=window, gate=gate, rows_ahead=ahead)
+    for i, n in enumerate(lengths):
+        rows = f64(pages[table[i, :blocks[i]]]).reshape(-1, row)[max(0, n - window) if window else 0:n]
+        s = f64(q)[i].reshape(heads, row) @ rows.T * 0.1
+        w = np.exp(s - s.max(axis=1, keepdims=True))
+        want = w / w.sum(axis=1, keepdims=True) @ rows[:, :rank] / (1.0 + np.exp(-f64(gate)[i]))[:, None]
+        # queries and weights keep all 24 bits and sums are 32-bit: scores of up to 8 off by some 2^-21, weights by as much
+        np.testing.assert_allclose(f64(got)[i].reshape(heads, rank), want, rtol=2e-5, atol=1e-5)
