@@ -303,17 +303,17 @@ __device__ __forceinline__ void cp_async_16(void* smem, const void* global) {
 // and now: 64 x 12 pairs of 110 keys 11.2 -> 8.0 us, 24 x 16 of 112 to 778 22.3 -> 15.5, 64 x 25 of 264 31.1 -> 24.4, 2 x 12 of 1,000 13.6 -> 7.9.
 template <int D, bool FULL, int WARPS, int STAGES>       // head size: 16, 32, 64, 128 or 256
 __global__ void __launch_bounds__(WARPS * 32)
-split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restrict__ q, long ld_q,
+split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* q, long ld_q,
                        const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
                        const int* __restrict__ block_table, int max_blocks, const int* __restrict__ positions,
                        const int* __restrict__ token_item, int n_heads, int n_kv_heads, int dim, int vdim, int page_size,
-                       float scale, float cap, int window, int block, int keep, const float* __restrict__ gate, long ld_gate,
+                       float scale, float cap, int window, int block, int keep, const float* gate, long ld_gate,
                        int gate_wide, const float* __restrict__ sink, const float* __restrict__ slopes, int chunk, int max_chunks, float* __restrict__ part_acc,
-                       float* __restrict__ part_ml, int* __restrict__ counters, const int* records) {
+                       float* __restrict__ part_ml, int* __restrict__ counters, const int* records, const int* first_new) {
     if (FULL) dim = vdim = D;
     constexpr int LD = D + 8, STEPS = D / 16;              // rows of a tile an odd number of 16 bytes apart: no bank twice
     dependents_may_start();
-    wait_for_earlier_kernels();
+    if (first_new == nullptr) wait_for_earlier_kernels();
     const int h = blockIdx.y, c = blockIdx.z;
     const long pair = (long)blockIdx.x * n_heads + h;          // whose scratch this is
     // (a record of the step's work list: entry, row, rows, position)
@@ -336,15 +336,9 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     const int hk = h / (n_heads / n_kv_heads);
     const long k_width = (long)n_kv_heads * dim, v_width = (long)n_kv_heads * vdim;
 
-    // The query stands in all eight columns of the second operand, so that every lane has the scores of its two keys.
-    uint32_t qb[STEPS][2];
-#pragma unroll
-    for (int k = 0; k < STEPS; k++)
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int d = k * 16 + u * 8 + 2 * tq;
-            qb[k][u] = FULL || d < dim ? *reinterpret_cast<const uint32_t*>(q + (long)t * ld_q + (long)h * dim + d) : 0u;
-        }
+    // Keys from this position on are written by kernels of the step that may still run (`first_new`, one position an entry; without it
+    // nothing is read ahead of the wait): the first tiles of the others are asked for ahead of the wait.
+    const int limit = first_new != nullptr ? first_new[item] : p + 1;
     // scores are kept in units of log2(e): exp(x) = 2^(x log2 e) costs one instruction then
     const float scale_log2 = scale * 1.4426950408889634f;
     // a cap on the scores, cap * tanh(score / cap), in the same units (cap <= 0: none)
@@ -363,34 +357,70 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
     const int page_shift = (page_size & (page_size - 1)) == 0 ? 31 - __clz(page_size) : -1;
     const bf16* k_head = k_pages + (long)hk * dim;
     const bf16* v_head = v_pages + (long)hk * vdim;
-    long row = -1;
-    auto find = [&](int i) {
+    long row = -1;                                        // (-1: no such key, -2: left for a second look)
+    auto find = [&](int i, int from, int to) {            // positions [from, to)
         const int number = first_key + i * (WARPS * 16) + (lane & 15);
         const int j = number < n_kept ? number : number + gap;
         const int block = page_shift >= 0 ? j >> page_shift : j / page_size;
         const int within = page_shift >= 0 ? j & (page_size - 1) : j % page_size;
-        row = number <= end ? ((long)bt[block] * page_size + within) * (FULL ? k_width : 1) : -1;
+        row = number > end ? (from == 0 ? -1 : -2) : j < from || j >= to ? -2 : ((long)bt[block] * page_size + within) * (FULL ? k_width : 1);
     };
-    auto issue = [&](int i) {
-        if (i < tiles) {
-            bf16* kt = ring + (i % STAGES) * (2 * 16 * LD);
+    auto copy_rows = [&](int i) {
+        bf16* kt = ring + (i % STAGES) * (2 * 16 * LD);
 #pragma unroll
-            for (int u = 0; u < STEPS; u++) {
-                const int key = (lane + 32 * u) / (D / 8), d = (lane + 32 * u) % (D / 8) * 8;
-                const long at = __shfl_sync(0xffffffffu, row, key);
-                const bool k_there = at >= 0 && (FULL || d < dim), v_there = at >= 0 && (FULL || d < vdim);
+        for (int u = 0; u < STEPS; u++) {
+            const int key = (lane + 32 * u) / (D / 8), d = (lane + 32 * u) % (D / 8) * 8;
+            const long at = __shfl_sync(0xffffffffu, row, key);
+            const bool k_there = at >= 0 && (FULL || d < dim), v_there = at >= 0 && (FULL || d < vdim);
+            if (at != -2) {
                 copy_16(kt + key * LD + d, k_there ? k_head + (FULL ? at : at * k_width) + d : k_head, k_there);
                 copy_16(kt + (16 + key) * LD + d, v_there ? v_head + (FULL ? at : at * v_width) + d : v_head, v_there);
             }
-            find(i + 1);
+        }
+    };
+    auto issue = [&](int i, int to) {
+        if (i < tiles) {
+            copy_rows(i);
+            find(i + 1, 0, to);
         }
         copies_end();
     };
-    if (tiles > 0) find(0);
+    const int ahead = first_new != nullptr ? limit : p + 1;
+    if (tiles > 0) find(0, 0, ahead);
 #pragma unroll
-    for (int i = 0; i < STAGES - 1; i++) issue(i);
+    for (int i = 0; i < STAGES - 1; i++) issue(i, ahead);
+    if (first_new != nullptr) {
+        wait_for_earlier_kernels();
+        // the step's own keys among those tiles' (a key below the window that stays visible may be one)
+        bool left = false;
+#pragma unroll
+        for (int i = 0; i < STAGES - 1; i++)
+            if (i < tiles) {
+                find(i, limit, p + 1);
+                if (__any_sync(0xffffffffu, row >= 0)) {
+                    copy_rows(i);
+                    left = true;
+                }
+            }
+        if (left) {
+            copies_end();
+            copies_landed<0>();
+        }
+        if (STAGES - 1 < tiles) find(STAGES - 1, 0, p + 1);
+    }
+    // The query stands in all eight columns of the second operand, so that every lane has the scores of its two keys.
+    q = behind_the_wait(q);
+    uint32_t qb[STEPS][2];
+#pragma unroll
+    for (int k = 0; k < STEPS; k++)
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int d = k * 16 + u * 8 + 2 * tq;
+            qb[k][u] = FULL || d < dim ? *reinterpret_cast<const uint32_t*>(q + (long)t * ld_q + (long)h * dim + d) : 0u;
+        }
+    gate = behind_the_wait(gate);
     for (int i = 0; i < tiles; i++) {
-        issue(i + STAGES - 1);
+        issue(i + STAGES - 1, p + 1);
         copies_landed<STAGES - 1>();
         __syncwarp();
         const bf16* kt = ring + (i % STAGES) * (2 * 16 * LD);
@@ -564,13 +594,15 @@ split_attention_kernel(bf16* __restrict__ out, long ld_out, const bf16* __restri
 // below `keep` stay visible behind a window.  max_chunks * chunk covers the most keys a token of the step sees.
 // (with `records`, 8 numbers each: the single tokens that n_tokens records of a step's work list name,
 // entry, row, rows, position first; scratch is theirs in the list's order)
+// (with `first_new`, a position an entry: kernels that may still run write no key or value before it, so those are read ahead of the wait
+// for them.  Positions, block table and records are read there too: they come with the step's arrays)
 extern "C" int mllm_decode_split_attention_records(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,
                                                 const void* v_pages, const int* block_table, int max_blocks,
                                                 const int* positions, const int* token_item, int n_tokens, int n_heads,
                                                 int n_kv_heads, int dim, int vdim, int page_size, float scale, float cap,
                                                 int window, int block, int keep, const float* gate, long ld_gate,
                                                 int gate_wide, const float* sink, const float* slopes, int chunk, int max_chunks, float* part_acc,
-                                                float* part_ml, int* counters, const int* records, void* stream) {
+                                                float* part_ml, int* counters, const int* records, const int* first_new, void* stream) {
     if (n_tokens <= 0) return 0;
     if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0)
         return fail("split_attention: heads must be a multiple of key/value heads");
@@ -605,7 +637,7 @@ extern "C" int mllm_decode_split_attention_records(void* out, long ld_out, const
         launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL, 4, STAGES>, grid, dim3(128), ring, s, (bf16*)out, ld_out, \
                       (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks,         \
                       positions, token_item, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep, \
-                      gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters, records);  \
+                      gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters, records, first_new); \
     } while (0)
 #define PICK_SPLIT(D)                                                             \
     do {                                                                          \
@@ -636,7 +668,7 @@ extern "C" int mllm_decode_split_attention_kept(void* out, long ld_out, const vo
     return mllm_decode_split_attention_records(out, ld_out, q, ld_q, k_pages, v_pages, block_table, max_blocks, positions, token_item,
                                                n_tokens, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep,
                                                gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters,
-                                               nullptr, stream);
+                                               nullptr, nullptr, stream);
 }
 
 extern "C" int mllm_decode_split_attention_sink(void* out, long ld_out, const void* q, long ld_q, const void* k_pages,

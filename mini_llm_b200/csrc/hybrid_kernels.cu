@@ -43,8 +43,8 @@ __global__ void rotary_store_kernel(T* __restrict__ qkv, long ld, int k_off, int
                                     const int* __restrict__ positions, const int* __restrict__ token_item,
                                     const int* __restrict__ block_table, int max_blocks, int page_size,
                                     T* __restrict__ k_pages, T* __restrict__ v_pages, int writes) {
+    // the angles and the token's place ahead of the wait: they come with the step's arrays
     dependents_may_start();
-    wait_for_earlier_kernels();
     extern __shared__ float turn[];              // [rot_dims / 2][2]: cosine, sine
     const int t = blockIdx.x;
     const int p = positions[t];
@@ -55,13 +55,15 @@ __global__ void rotary_store_kernel(T* __restrict__ qkv, long ld, int k_off, int
         turn[2 * i] = (float)(c * amplitude);
         turn[2 * i + 1] = (float)(s * amplitude);
     }
-    __syncthreads();
-    T* row = qkv + (long)t * ld;
     const int page = block_table[(long)token_item[t] * max_blocks + p / page_size];
     const long slot = (long)page * page_size + (p % page_size);
+    wait_for_earlier_kernels();
+    __syncthreads();
+    T* row = behind_the_wait(qkv) + (long)t * ld;
+    const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;      // (blockIdx.y: a share of the token's row)
     // queries and keys: pairs of the rotated part, then what passes unchanged
     const int pairs_per_head = dim / 2 + (dim & 1);
-    for (int u = threadIdx.x; u < (heads + kv_heads) * pairs_per_head; u += blockDim.x) {
+    for (int u = first; u < (heads + kv_heads) * pairs_per_head; u += step) {
         const int head = u / pairs_per_head, i = u % pairs_per_head;
         const bool is_key = head >= heads;
         T* x = is_key ? row + k_off + (long)(head - heads) * dim : row + (long)head * dim;
@@ -81,7 +83,7 @@ __global__ void rotary_store_kernel(T* __restrict__ qkv, long ld, int k_off, int
         }
     }
     if (writes)
-        for (int c = threadIdx.x; c < kv_heads * vdim; c += blockDim.x)
+        for (int c = first; c < kv_heads * vdim; c += step)
             v_pages[slot * kv_heads * vdim + c] = row[v_off + c];
 }
 
@@ -93,12 +95,16 @@ extern "C" int mllm_hybrid_rotary_store(void* qkv, long ld, int k_off, int v_off
     if (rot_dims < 0 || rot_dims % 2 != 0 || rot_dims > dim) return fail("rotary_store: an even number of at most dim entries is rotated");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t shared = (size_t)(rot_dims + 2) * sizeof(float);
+    // few tokens: a thread a pair (16 heads of 64 by one block of 128 threads are four trips to L2 one after the other, as a
+    // store may be what the next load reads)
+    const int shares = n_tokens <= 64 ? ((heads + kv_heads) * ((dim + 1) / 2) + 127) / 128 : 1;
+    const dim3 grid(n_tokens, shares < 64 ? shares : 64);
     if (dtype == DT_F32)
-        launch_kernel(g_dependent_launch != 0, rotary_store_kernel<float>, dim3(n_tokens), dim3(128), shared, s, (float*)qkv, ld,
+        launch_kernel(g_dependent_launch != 0, rotary_store_kernel<float>, grid, dim3(128), shared, s, (float*)qkv, ld,
                       k_off, v_off, heads, kv_heads, dim, vdim, rot_dims, inv_freq, amplitude, positions, token_item, block_table,
                       max_blocks, page_size, (float*)k_pages, (float*)v_pages, writes);
     else if (dtype == DT_BF16)
-        launch_kernel(g_dependent_launch != 0, rotary_store_kernel<bf16>, dim3(n_tokens), dim3(128), shared, s, (bf16*)qkv, ld,
+        launch_kernel(g_dependent_launch != 0, rotary_store_kernel<bf16>, grid, dim3(128), shared, s, (bf16*)qkv, ld,
                       k_off, v_off, heads, kv_heads, dim, vdim, rot_dims, inv_freq, amplitude, positions, token_item, block_table,
                       max_blocks, page_size, (bf16*)k_pages, (bf16*)v_pages, writes);
     else
@@ -119,13 +125,13 @@ head_norm_store_kernel(T* __restrict__ qkv, long ld, int k_off, int v_off, int h
                        const int* __restrict__ block_table, int max_blocks, int page_size, T* __restrict__ k_pages,
                        T* __restrict__ v_pages, int writes) {
     dependents_may_start();
-    wait_for_earlier_kernels();
     const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int p = positions[t];
-    T* row = qkv + (long)t * ld;
     long slot = 0;
     if (writes) slot = (long)block_table[(long)token_item[t] * max_blocks + p / page_size] * page_size + (p % page_size);
-    for (int head = warp; head < heads + kv_heads; head += 4) {
+    wait_for_earlier_kernels();                      // (the token's place comes with the step's arrays)
+    T* row = behind_the_wait(qkv) + (long)t * ld;
+    for (int head = blockIdx.y * 4 + warp; head < heads + kv_heads; head += gridDim.y * 4) {
         const bool is_key = head >= heads;
         T* x = is_key ? row + k_off + (long)(head - heads) * dim : row + (long)head * dim;
         float sq = 0.0f;
@@ -142,7 +148,7 @@ head_norm_store_kernel(T* __restrict__ qkv, long ld, int k_off, int v_off, int h
         }
     }
     if (writes)
-        for (int c = threadIdx.x; c < kv_heads * vdim; c += blockDim.x) v_pages[slot * kv_heads * vdim + c] = row[v_off + c];
+        for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < kv_heads * vdim; c += gridDim.y * blockDim.x) v_pages[slot * kv_heads * vdim + c] = row[v_off + c];
 }
 
 extern "C" int mllm_hybrid_head_norm_store(void* qkv, long ld, int k_off, int v_off, int heads, int kv_heads, int dim, int vdim,
@@ -152,12 +158,15 @@ extern "C" int mllm_hybrid_head_norm_store(void* qkv, long ld, int k_off, int v_
     if (n_tokens <= 0) return 0;
     if (heads <= 0 || kv_heads <= 0 || dim <= 0 || vdim <= 0) return fail("head_norm_store: sizes must be positive");
     cudaStream_t s = (cudaStream_t)stream;
+    // few tokens: a warp a head (the heads of one token one after the other took 5.9 us in a decode step of one token)
+    const int shares = n_tokens <= 64 ? (heads + kv_heads + 3) / 4 : 1;
+    const dim3 grid(n_tokens, shares < 64 ? shares : 64);
     if (dtype == DT_F32)
-        launch_kernel(g_dependent_launch != 0, head_norm_store_kernel<float>, dim3(n_tokens), dim3(128), 0, s, (float*)qkv, ld, k_off,
+        launch_kernel(g_dependent_launch != 0, head_norm_store_kernel<float>, grid, dim3(128), 0, s, (float*)qkv, ld, k_off,
                       v_off, heads, kv_heads, dim, vdim, eps, positions, token_item, block_table, max_blocks, page_size,
                       (float*)k_pages, (float*)v_pages, writes);
     else if (dtype == DT_BF16)
-        launch_kernel(g_dependent_launch != 0, head_norm_store_kernel<bf16>, dim3(n_tokens), dim3(128), 0, s, (bf16*)qkv, ld, k_off,
+        launch_kernel(g_dependent_launch != 0, head_norm_store_kernel<bf16>, grid, dim3(128), 0, s, (bf16*)qkv, ld, k_off,
                       v_off, heads, kv_heads, dim, vdim, eps, positions, token_item, block_table, max_blocks, page_size,
                       (bf16*)k_pages, (bf16*)v_pages, writes);
     else

@@ -79,8 +79,8 @@ __device__ __forceinline__ void turn_of(int position, double f, float* c, float*
 template <typename T, int G, int TAPS>
 __global__ void __launch_bounds__(G > 1 ? 256 : 1024)
 norm_rotary_store_kernel(NormRotaryParams pp) {
+    // the tokens' places and angles ahead of the wait: they come with the step's arrays
     dependents_may_start();
-    wait_for_earlier_kernels();
     extern __shared__ float shared[];
     __shared__ int tok_pos[G], tok_local[G], tok_slot[G];
     __shared__ long tok_place[G];
@@ -108,6 +108,9 @@ norm_rotary_store_kernel(NormRotaryParams pp) {
     bool interior = TAPS > 0 && n_here == G;
     if (TAPS > 0)
         for (int g = 0; g < n_here; g++) interior = interior && tok_local[g] >= TAPS - 1;
+    for (int i = threadIdx.x; i < half * n_here; i += blockDim.x)
+        turn_of(tok_pos[i / half], pp.inv_freq[i % half], &turn[2 * i], &turn[2 * i + 1]);
+    wait_for_earlier_kernels();
 
     // column c of the block's tokens, filtered
     auto column = [&](int c, float* y) {
@@ -209,8 +212,6 @@ norm_rotary_store_kernel(NormRotaryParams pp) {
             for (int g = 0; g < G; g++)
                 if (g < n_here) v_pages[tok_place[g] * v_row + at] = from_f32<T>(y[g]);
         }
-    for (int i = threadIdx.x; i < half * n_here; i += blockDim.x)
-        turn_of(tok_pos[i / half], pp.inv_freq[i % half], &turn[2 * i], &turn[2 * i + 1]);
     __syncthreads();
     if (n_keys > 0 && pp.v_off == pp.k_off) {
         // values that are the keys as they came in

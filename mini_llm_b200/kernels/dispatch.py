@@ -163,7 +163,7 @@ class Kernels:
             return ops.split_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                                        n_heads, n_kv_heads, dim, cache.page_size, scale, window, span, -(-reach // span), acc,
                                        ml, counters, cap=cap, block=chunk, gate=gate, sink=sink, value_size=vdim, keep=keep, slopes=slopes,
-                                       gate_wide=gate_wide)
+                                       gate_wide=gate_wide, first_new=ctx.item_start)
         tiled = not ctx.decode_only and ops.capped_attention_tiled_takes(dim, vdim, q.dtype)
         self.chose("capped_attention", "capped_attention_tiled" if tiled else "capped_attention_plain", q.shape[0], n_heads, dim, vdim)
         return ops.capped_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
@@ -532,9 +532,10 @@ class Kernels:
                 chunk = 64 if pairs < 64 else (128 if pairs < 128 else (256 if pairs < 256 else 512))
             max_chunks = -(-reach // chunk)
             self.chose("attention", "group_attention" if grouped else "split_attention", n, n_heads, head_size)
+            more = {} if grouped else {"first_new": ctx.item_start}
             return run(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                        n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, max_chunks, acc, ml,
-                       counters)
+                       counters, **more)
         if (not self.plain_only and ctx.att_tiles is not None
                 and ops.attention_prefill_takes(q, head_size, cache.page_size)):
             scratch = None
@@ -555,7 +556,7 @@ class Kernels:
                 acc, ml, counters = self._scratch(ctx, SPLIT_ATTENTION_MAX_ROWS * n_heads, -(-reach // 64), head_size)
                 ops.split_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                                     n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, -(-reach // chunk), acc, ml,
-                                    counters, records=ctx.att_tiles[8 * n_tiles:], n_records=ctx.n_att_singles)
+                                    counters, records=ctx.att_tiles[8 * n_tiles:], n_records=ctx.n_att_singles, first_new=ctx.item_start)
             if ctx.att_units:
                 self.chose("attention", "attention_two_tiles", n, n_heads, head_size)
                 return ops.attention_prefill_two_tiles(out, q, cache.k_pages, cache.v_pages, cache.block_table,

@@ -230,7 +230,7 @@ class _SkinnyParams(ctypes.Structure):
 
 _skinny = Function("decode", "mllm_decode_skinny_linear", [ctypes.POINTER(_SkinnyParams), P])
 _split_attention = Function("decode", "mllm_decode_split_attention_records",
-                            [P, L, P, L, P, P, P, I, P, P, I, I, I, I, I, I, F, F, I, I, I, P, L, I, P, P, I, I, P, P, P, P, P])
+                            [P, L, P, L, P, P, P, I, P, P, I, I, I, I, I, I, F, F, I, I, I, P, L, I, P, P, I, I, P, P, P, P, P, P])
 
 SKINNY_MAX_SMEM = 200 * 1024
 SPLIT_ATTENTION_HEAD_SIZES = (16, 32, 64, 128, 256)
@@ -341,7 +341,7 @@ def skinny_heads(out, a, w, heads, a_head, o_head):
 
 def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item, n_heads, n_kv_heads, head_size,
                     page_size, scale, window, chunk, max_chunks, part_acc, part_ml, counters, cap=0.0, block=0, gate=None, sink=None,
-                    value_size=None, keep=0, slopes=None, gate_wide=False, records=None, n_records=0):
+                    value_size=None, keep=0, slopes=None, gate_wide=False, records=None, n_records=0, first_new=None):
     """Causal attention over the paged cache for few tokens: one CTA per (token, head, chunk
     of ``chunk`` keys); needs fp32 scratch ``part_acc`` [T*H*max_chunks*D], ``part_ml``
     [T*H*max_chunks*2] and zeroed int32 ``counters`` [T*H] (left zero).  ``cap`` > 0: the scores
@@ -354,7 +354,8 @@ def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item
     scratch is sized for ``split_attention_row``).  ``keep``: the first ``keep`` keys stay visible behind the window.
     ``max_chunks`` chunks must cover the most keys a token may see.  Scores, weights and sums are 32-bit.
     ``records``: only the rows that ``n_records`` device int32 records of 8 name, single tokens of the step's work list (entry, row,
-    rows, position ...); T is then their number."""
+    rows, position ...); T is then their number.  ``first_new`` int32 [entries]: kernels that may still run write no key or value of an
+    entry before that position (within a step: its first token's), and the step's arrays are there; those keys are read early."""
     _check(out, "split_attention.out", torch.bfloat16, 2)
     _check(q, "split_attention.q", torch.bfloat16, 2)
     _check(k_pages, "split_attention.k_pages", torch.bfloat16)
@@ -385,11 +386,13 @@ def split_attention(out, q, k_pages, v_pages, block_table, positions, token_item
     _check_gate(gate, q.shape[0], n_heads * (vdim if gate_wide else 1), "split_attention")
     _check_per_head(sink, n_heads, "split_attention.sink")
     _check_per_head(slopes, n_heads, "split_attention.slopes")
+    if first_new is not None:
+        _check(first_new, "split_attention.first_new", torch.int32, 1)
     _split_attention(out.data_ptr(), out.stride(0), q.data_ptr(), q.stride(0), k_pages.data_ptr(), v_pages.data_ptr(),
                      block_table.data_ptr(), block_table.shape[1], positions.data_ptr(), token_item.data_ptr(), n,
                      n_heads, n_kv_heads, head_size, vdim, page_size, float(scale), float(cap or 0.0), int(window or 0), int(block or 0),
                      int(keep), _ptr(gate), gate.stride(0) if gate is not None else 0, int(bool(gate_wide)), _ptr(sink), _ptr(slopes), int(chunk), int(max_chunks), part_acc.data_ptr(),
-                     part_ml.data_ptr(), counters.data_ptr(), _ptr(records), _stream())
+                     part_ml.data_ptr(), counters.data_ptr(), _ptr(records), _ptr(first_new), _stream())
     return out
 
 
