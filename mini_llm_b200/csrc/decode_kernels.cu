@@ -624,36 +624,48 @@ extern "C" int mllm_decode_split_attention_records(void* out, long ld_out, const
     const long share = (1184 + pairs - 1) / pairs;
     if (max_chunks > share && max_chunks > 4) max_chunks = (int)(share > 4 ? share : 4);
     dim3 grid(n_tokens, n_heads, max_chunks);
-    // Stages of a warp's ring: three where a wave of blocks holds the launch all the same, else two, of which six blocks of
-    // heads of 64 fit an SM.  At heads of 64, three against two: 24 x 16 pairs of 112 to 778 keys 15.1 against 16.2 us, 64 x 12 of 1,000 38.9
-    // against 50.4; 64 x 12 of 110 (five blocks an SM are needed for one wave) 10.9 and 8.0.
-    const bool deep = pairs * max_chunks <= 592 && size <= 64;
-#define LAUNCH_SPLIT(D, FULL, STAGES)                                                                                    \
+    // Heads of up to 64: eight warps a block where three such blocks an SM hold the launch, so that a long request's keys are half as many
+    // tiles one after the other; else four warps, with three stages of the ring where a wave of blocks holds the launch all the same, else
+    // two, of which six blocks of heads of 64 fit an SM.  At heads of 64, four warps of three stages against eight: 24 x 16 pairs of 114 to 780
+    // keys 17.4 and 14.0 us, 20 x 12 of 500 11.8 and 9.3, 32 x 12 of 30 to 960 19.6 and 15.1, 3 x 12 of 800 in chunks of 128 6.6 and 6.1; three
+    // stages against two: 24 x 16 pairs of 112 to 778 15.1 and 16.2 us, 64 x 12 of 1,000 38.9 and 50.4; 64 x 12 of 110 (five blocks an SM are
+    // needed for one wave) 10.9 and 8.0.
+    const long blocks = pairs * max_chunks;
+    const bool wide = blocks <= 444 && size <= 64, deep = blocks <= 592 && size <= 64;
+#define LAUNCH_SPLIT(D, FULL, WARPS, STAGES)                                                                             \
     do {                                                                                                                 \
-        constexpr int ring = 4 * STAGES * 2 * 16 * (D + 8) * 2;                                                          \
-        if (ring > 48 * 1024 && cudaFuncSetAttribute(split_attention_kernel<D, FULL, 4, STAGES>,                         \
+        constexpr int ring = WARPS * STAGES * 2 * 16 * (D + 8) * 2;                                                      \
+        if (ring > 48 * 1024 && cudaFuncSetAttribute(split_attention_kernel<D, FULL, WARPS, STAGES>,                     \
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize, ring) != cudaSuccess)  \
             return fail("split_attention: the ring's shared memory was refused");                                        \
-        launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL, 4, STAGES>, grid, dim3(128), ring, s, (bf16*)out, ld_out, \
+        launch_kernel(g_dependent_launch != 0, split_attention_kernel<D, FULL, WARPS, STAGES>, grid, dim3(WARPS * 32), ring, s, (bf16*)out, ld_out, \
                       (const bf16*)q, ld_q, (const bf16*)k_pages, (const bf16*)v_pages, block_table, max_blocks,         \
                       positions, token_item, n_heads, n_kv_heads, dim, vdim, page_size, scale, cap, window, block, keep, \
                       gate, ld_gate, gate_wide, sink, slopes, chunk, max_chunks, part_acc, part_ml, counters, records, first_new); \
     } while (0)
+#define PICK_SPLIT_SMALL(D)                                                       \
+    do {                                                                          \
+        if (full && wide) LAUNCH_SPLIT(D, true, 8, 2);                            \
+        else if (wide) LAUNCH_SPLIT(D, false, 8, 2);                              \
+        else if (full && deep) LAUNCH_SPLIT(D, true, 4, 3);                       \
+        else if (full) LAUNCH_SPLIT(D, true, 4, 2);                               \
+        else if (deep) LAUNCH_SPLIT(D, false, 4, 3);                              \
+        else LAUNCH_SPLIT(D, false, 4, 2);                                        \
+    } while (0)
 #define PICK_SPLIT(D)                                                             \
     do {                                                                          \
-        if (full && deep) LAUNCH_SPLIT(D, true, 3);                               \
-        else if (full) LAUNCH_SPLIT(D, true, 2);                                  \
-        else if (deep) LAUNCH_SPLIT(D, false, 3);                                 \
-        else LAUNCH_SPLIT(D, false, 2);                                           \
+        if (full) LAUNCH_SPLIT(D, true, 4, 2);                                    \
+        else LAUNCH_SPLIT(D, false, 4, 2);                                        \
     } while (0)
     switch (size) {
-    case 16: PICK_SPLIT(16); break;
-    case 32: PICK_SPLIT(32); break;
-    case 64: PICK_SPLIT(64); break;
+    case 16: PICK_SPLIT_SMALL(16); break;
+    case 32: PICK_SPLIT_SMALL(32); break;
+    case 64: PICK_SPLIT_SMALL(64); break;
     case 128: PICK_SPLIT(128); break;
     default: PICK_SPLIT(256); break;
     }
 #undef PICK_SPLIT
+#undef PICK_SPLIT_SMALL
 #undef LAUNCH_SPLIT
     return check_launch("split_attention_kernel");
 }

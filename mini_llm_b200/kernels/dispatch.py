@@ -24,9 +24,9 @@ SPLIT_ATTENTION_MAX_ROWS = 64 # up to here attention runs one CTA per (token, he
 
 def split_attention_chunk(pairs):
     """Keys of a CTA: few when there are few (token, head) pairs, so that the chunks still fill the GPU; from some 200 on a
-    second chunk costs more than it saves (heads of 64: 24 pairs of 1,000 keys 13.8, 10.2, 8.3, 8.0 us in 1, 2, 4, 8 chunks; 320 of 512
-    12.3 and 17.7 in 1 and 2; 384 of 112 to 778 15.1 and 20.0)."""
-    return 128 if pairs < 64 else (256 if pairs < 128 else (512 if pairs < 256 else 1024))
+    second chunk costs more than it saves (heads of 64: 24 pairs of 1,000 keys 10.2, 8.2, 7.0, 6.3 us in 1, 2, 4, 8 chunks; 96 of up to 1,000
+    11.7, 9.7, 7.7; 240 of 500 9.3 and 12.2 in 1 and 2; 384 of 114 to 780 14.0 and 16.9)."""
+    return 128 if pairs < 64 else (256 if pairs < 128 else (512 if pairs <= 222 else 1024))
 
 
 class DeferredNorm:
