@@ -1183,8 +1183,10 @@ extern "C" int mllm_hybrid_capped_attention(void* out, long ld_out, const void* 
 // One block per (entry, head, slice of the value entries): a column of S belongs to LANES threads
 // of one warp, each with DPT rows in registers; both sums over the old column (with k and with q)
 // are taken in one pass, and the read-out follows from them: S_new^T q = a S^T q + u (k . q).
-// The entry's tokens are taken in order, TOK at a time through shared memory; a chunk's rows are
-// asked for into registers while the chunk before it is worked on.
+// The entry's tokens are taken in order, TOK at a time through shared memory, by four warps; four others
+// ask for the chunk after next into registers and prepare the next one (decays, gates, unit vectors) meanwhile.  What bounds it are
+// instructions, some 180 a token for the walk and 2,000 a chunk for what comes before: 700 tokens of 6 heads of 128 x 128 with a decay per
+// channel 319 us when the same four warps did both in turn, 239 so; 2 x 350 163 and 124; 100 tokens in 32 bits 42 and 36.
 // ---------------------------------------------------------------------------
 struct RecurrenceParams {
     float* out; long ld_out;
@@ -1200,7 +1202,7 @@ struct RecurrenceParams {
 };
 
 template <typename T, int DPT, int LANES, int TOK, int CPT, bool CHANNEL>      // CPT: columns of the state a thread takes
-__global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams pp) {
+__global__ void __launch_bounds__(256) linear_recurrence_kernel(RecurrenceParams pp) {
     dependents_may_start();
     wait_for_earlier_kernels();
     constexpr int GROUPS = 128 / LANES;                    // groups of lanes; each takes CPT columns of the state,
@@ -1212,27 +1214,34 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
     constexpr int VPER = (TOK * COLS + 127) / 128;         // values a thread brings
     extern __shared__ float shared[];
     const int dim = pp.dim, vdim = pp.vdim;
-    float* ks = shared;                         // [TOK][ROW]: entry i of a row at (i / DPT) * PAD + i % DPT, zero past dim
-    float* qs = ks + TOK * ROW;                 // [TOK][ROW]
-    float* vs = qs + TOK * ROW;                 // [TOK][COLS]
-    float* as = vs + TOK * COLS;                // [TOK] the step's gate, then the decay
-    float* bs = as + TOK;                       // [TOK] the write gate, then the write strength
-    float* kq = bs + TOK;                       // [TOK] k . q
-    float* gs = kq + TOK;                       // [TOK][ROW] (CHANNEL only): the decay of every key channel, laid out as ks
+    // Four warps take the tokens one by one; four others bring the next chunk meanwhile, into the other of two buffers.
+    constexpr int CHUNK = (CHANNEL ? 3 : 2) * TOK * ROW + TOK * COLS + 3 * TOK;
+    const bool brings = threadIdx.x >= 128;
+    const int tid = threadIdx.x & 127;
+    float *ks, *qs, *vs, *as, *bs, *kq, *gs;
+    auto buffer = [&](int which) {
+        ks = shared + which * CHUNK;            // [TOK][ROW]: entry i of a row at (i / DPT) * PAD + i % DPT, zero past dim
+        qs = ks + TOK * ROW;                    // [TOK][ROW]
+        vs = qs + TOK * ROW;                    // [TOK][COLS]
+        as = vs + TOK * COLS;                   // [TOK] the step's gate, then the decay
+        bs = as + TOK;                          // [TOK] the write gate, then the write strength
+        kq = bs + TOK;                          // [TOK] k . q
+        gs = kq + TOK;                          // [TOK][ROW] (CHANNEL only): the decay of every key channel, laid out as ks
+    };
     constexpr int GPER = CHANNEL ? (TOK * DPT * LANES + 127) / 128 : 1;     // decays a thread brings
     const int item = blockIdx.x, head = blockIdx.y;
     const int count = pp.item_count[item];
     if (count <= 0) return;
     const long first = pp.item_offset[item];
     const int qk_head = head / (pp.heads / pp.qk_heads);
-    const int lane_in = threadIdx.x % LANES, col_local = threadIdx.x / LANES;
+    const int lane_in = tid % LANES, col_local = tid / LANES;
     // this thread's columns: col_local, col_local + GROUPS, ... of the block's COLS
     // this thread's part of its column of the state: rows lane_in * DPT .. + DPT - 1 (zero past dim, and it stays zero)
     float* S = pp.state + (long)pp.item_slot[item] * pp.state_stride + (long)head * dim * vdim;
     // (the block's slice of the state goes through shared memory both ways, so that the global
     // reads and writes run along the rows of S, whatever the lanes' share of a column is)
     float s[CPT][DPT];
-    for (int u = threadIdx.x; u < dim * COLS; u += 128) {
+    for (int u = threadIdx.x; u < dim * COLS; u += 256) {
         const int i = u / COLS, c = blockIdx.z * COLS + u % COLS;
         shared[u] = c < vdim ? S[(long)i * vdim + c] : 0.0f;
     }
@@ -1250,16 +1259,15 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
     const T* q = (const T*)pp.q;
     const T* k = (const T*)pp.k;
     const T* v = (const T*)pp.v;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = tid >> 5, lane = tid & 31;
 
     // What a thread brings of every chunk of TOK tokens: PER entries of one row (the k or the q of one
     // token), VPER values, and (the first threads) a token's gates.  The next chunk is asked for
     // before the current one is worked on, so its way through the memory lies under the sums.
-    const int row = threadIdx.x / TPR, row_sub = threadIdx.x % TPR;
+    const int row = tid / TPR, row_sub = tid % TPR;
     const int row_token = row >> 1;
     const T* row_base = (row & 1) ? q : k;
     const long row_ld = (row & 1) ? pp.ld_q : pp.ld_k;
-    float* row_smem = ((row & 1) ? qs : ks) + row_token * ROW;
     T raw[PER], raw_v[VPER];
     float raw_a = 0.0f, raw_b = 0.0f;
     float raw_g[GPER];
@@ -1269,7 +1277,7 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
     if (CHANNEL) {
 #pragma unroll
         for (int i = 0; i < GPER; i++) {
-            const int d = (threadIdx.x + 128 * i) % (DPT * LANES);
+            const int d = (tid + 128 * i) % (DPT * LANES);
             bias_g[i] = d < dim ? pp.step_bias[(long)head * dim + d] : 0.0f;
         }
     }
@@ -1283,25 +1291,25 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
         }
 #pragma unroll
         for (int i = 0; i < VPER; i++) {
-            const int u = threadIdx.x + 128 * i, tt = u / COLS, c = blockIdx.z * COLS + u % COLS;
+            const int u = tid + 128 * i, tt = u / COLS, c = blockIdx.z * COLS + u % COLS;
             raw_v[i] = (tt < n && c < vdim) ? v[(t0 + tt) * pp.ld_v + (long)head * vdim + c] : from_f32<T>(0.0f);
         }
-        if (threadIdx.x < n) {
-            if (!CHANNEL) raw_a = pp.gate_a[(t0 + threadIdx.x) * pp.ld_gate_a + head];
-            if (pp.delta) raw_b = pp.gate_b[(t0 + threadIdx.x) * pp.ld_gate_b + head];
+        if (tid < n) {
+            if (!CHANNEL) raw_a = pp.gate_a[(t0 + tid) * pp.ld_gate_a + head];
+            if (pp.delta) raw_b = pp.gate_b[(t0 + tid) * pp.ld_gate_b + head];
         }
         if (CHANNEL) {
 #pragma unroll
             for (int i = 0; i < GPER; i++) {
-                const int u = threadIdx.x + 128 * i, tt = u / (DPT * LANES), d = u % (DPT * LANES);
+                const int u = tid + 128 * i, tt = u / (DPT * LANES), d = u % (DPT * LANES);
                 raw_g[i] = (tt < n && d < dim) ? pp.gate_a[(t0 + tt) * pp.ld_gate_a + (long)head * dim + d] : 0.0f;
             }
         }
     };
-    ask(0);
-    for (int start = 0; start < count; start += TOK) {
+    // (the bringing warps alone) the chunk that was asked for, from token `start` on, into the current buffer
+    auto stage = [&](int start) {
         const int n = min(TOK, count - start);
-        __syncthreads();                                      // the chunk before has been read
+        float* row_smem = ((row & 1) ? qs : ks) + row_token * ROW;
 #pragma unroll
         for (int i = 0; i < PER; i++) {
             const int d = row_sub + TPR * i;
@@ -1309,23 +1317,23 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
         }
 #pragma unroll
         for (int i = 0; i < VPER; i++) {
-            const int u = threadIdx.x + 128 * i;
+            const int u = tid + 128 * i;
             if (u < TOK * COLS) vs[u] = to_f32(raw_v[i]);
         }
-        if (threadIdx.x < TOK) {
+        if (tid < TOK) {
             // a thread a token: the step, the decay, the write strength
             const float step = softplus_f(raw_a + bias);
-            as[threadIdx.x] = CHANNEL ? 1.0f : expf(-rate * step);
-            bs[threadIdx.x] = pp.delta ? sigmoid_f(raw_b) : step;
+            as[tid] = CHANNEL ? 1.0f : expf(-rate * step);
+            bs[tid] = pp.delta ? sigmoid_f(raw_b) : step;
         }
         if (CHANNEL) {
 #pragma unroll
             for (int i = 0; i < GPER; i++) {
-                const int u = threadIdx.x + 128 * i, tt = u / (DPT * LANES), d = u % (DPT * LANES);
+                const int u = tid + 128 * i, tt = u / (DPT * LANES), d = u % (DPT * LANES);
                 if (tt < TOK) gs[tt * ROW + (d / DPT) * PAD + d % DPT] = expf(-rate * softplus_f(raw_g[i] + bias_g[i]));
             }
         }
-        __syncthreads();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
         // a warp finishes TOK / 4 tokens: unit vectors if asked, and k . q; the sums of its tokens are
         // taken side by side, so that their exchanges between the lanes lie under one another
         {
@@ -1364,9 +1372,24 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
                 if (lane == 0) kq[tt] = sd[j] * fk * fq;
             }
         }
-        __syncthreads();
-        if (start + TOK < count) ask(start + TOK);
-        for (int tt = 0; tt < n; tt++) {
+    };
+    buffer(0);
+    if (brings) {
+        ask(0);
+        stage(0);
+        if (TOK < count) ask(TOK);
+    }
+    __syncthreads();
+    for (int start = 0, which = 0; start < count; start += TOK, which ^= 1) {
+        const int n = min(TOK, count - start);
+        if (brings) {
+            buffer(which ^ 1);
+            if (start + TOK < count) stage(start + TOK);
+            if (start + 2 * TOK < count) ask(start + 2 * TOK);
+        } else {
+            buffer(which);
+        }
+        for (int tt = 0; tt < (brings ? 0 : n); tt++) {
             const float* kr = ks + tt * ROW + lane_in * PAD;
             const float* qr = qs + tt * ROW + lane_in * PAD;
             float kreg[DPT];
@@ -1415,18 +1438,18 @@ __global__ void __launch_bounds__(128) linear_recurrence_kernel(RecurrenceParams
                     pp.out[(first + start + tt) * pp.ld_out + (long)head * vdim + col] = fmaf(u, both, a * sum_q[c]) + skip * value;
             }
         }
+        __syncthreads();                                      // this chunk has been read, the next one is there
     }
     if (pp.writes) {
-        __syncthreads();
 #pragma unroll
         for (int r = 0; r < DPT; r++) {
             const int i = lane_in * DPT + r;
 #pragma unroll
             for (int c = 0; c < CPT; c++)
-                if (i < dim) shared[i * COLS + col_local + c * GROUPS] = s[c][r];
+                if (i < dim && !brings) shared[i * COLS + col_local + c * GROUPS] = s[c][r];
         }
         __syncthreads();
-        for (int u = threadIdx.x; u < dim * COLS; u += 128) {
+        for (int u = threadIdx.x; u < dim * COLS; u += 256) {
             const int i = u / COLS, c = blockIdx.z * COLS + u % COLS;
             if (c < vdim) S[(long)i * vdim + c] = shared[u];
         }
@@ -1437,13 +1460,13 @@ template <typename T, int DPT, int LANES, int TOK, int CPT, bool CHANNEL>
 static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStream_t s) {
     constexpr int COLS = 128 / LANES * CPT;
     // the staged chunk, or the block's slice of the state on its way in and out, whichever is larger
-    const size_t staged = (size_t)(CHANNEL ? 3 : 2) * TOK * LANES * (DPT + 4) + TOK * COLS + 3 * TOK, slice = (size_t)DPT * LANES * COLS;
+    const size_t staged = 2 * ((size_t)(CHANNEL ? 3 : 2) * TOK * LANES * (DPT + 4) + TOK * COLS + 3 * TOK), slice = (size_t)DPT * LANES * COLS;
     const size_t shared = sizeof(float) * (staged > slice ? staged : slice);
     dim3 grid(n_items, pp.heads, (pp.vdim + COLS - 1) / COLS);
     if (shared > 48 * 1024 &&
         cudaFuncSetAttribute(linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess)
         return fail("linear_recurrence: the staged rows' shared memory was refused");
-    launch_kernel(AFTER_THE_KERNELS_AHEAD, linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, grid, dim3(128), shared, s, pp);
+    launch_kernel(AFTER_THE_KERNELS_AHEAD, linear_recurrence_kernel<T, DPT, LANES, TOK, CPT, CHANNEL>, grid, dim3(256), shared, s, pp);
     return check_launch("linear_recurrence_kernel");
 }
 
