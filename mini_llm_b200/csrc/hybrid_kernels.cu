@@ -1199,6 +1199,7 @@ struct RecurrenceParams {
     float q_scale;
     int delta, unit_norm, writes;
     int channel_decay;
+    int state_ahead;               // recurrence_few_kernel: no kernel that may still run writes the states
 };
 
 template <typename T, int DPT, int LANES, int TOK, int CPT, bool CHANNEL>      // CPT: columns of the state a thread takes
@@ -1478,7 +1479,7 @@ static int launch_recurrence_as(const RecurrenceParams& pp, int n_items, cudaStr
 template <typename T, bool CHANNEL>
 __global__ void __launch_bounds__(256) recurrence_few_kernel(RecurrenceParams pp) {
     dependents_may_start();
-    wait_for_earlier_kernels();
+    if (!pp.state_ahead) wait_for_earlier_kernels();
     constexpr int ROWS = 16, WARPS = 8;
     __shared__ float ks[ROWS * WARPS], qs[ROWS * WARPS], gs[CHANNEL ? ROWS * WARPS : 1], sums[3][4], part_k[WARPS][32], part_q[WARPS][32];
     const int item = blockIdx.x, head = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1496,6 +1497,7 @@ __global__ void __launch_bounds__(256) recurrence_few_kernel(RecurrenceParams pp
     }
     const float rate = expf(pp.log_rate[head]), skip = pp.skip != nullptr ? pp.skip[head] : 0.0f;
     const float bias = CHANNEL ? (tid < dim ? pp.step_bias[(long)head * dim + tid] : 0.0f) : pp.step_bias[head];
+    if (pp.state_ahead) wait_for_earlier_kernels();          // (the state is asked for; what the kernels ahead write follows)
     for (int i = 0; i < count; i++) {
         const long t = first + i;
         const float value = col < vdim ? to_f32(((const T*)pp.v)[t * pp.ld_v + (long)head * vdim + col]) : 0.0f;

@@ -1768,6 +1768,7 @@ struct MemoryScanParams {
     float q_scale, gate_cap;
     int silu, writes;
     int* readers;                                 // memory_chunk_kernel: [entries * heads], zero before and after
+    int state_ahead;                              // memory_scan_kernel: no kernel that may still run writes the states
 };
 
 constexpr int SCAN_WARPS = 8;
@@ -1777,7 +1778,7 @@ template <typename T, int VS>
 __global__ void __launch_bounds__(SCAN_WARPS * 32)
 memory_scan_kernel(MemoryScanParams p, int first_slice, int writes_shared) {
     dependents_may_start();
-    wait_for_earlier_kernels();
+    if (!p.state_ahead) wait_for_earlier_kernels();
     extern __shared__ float shared[];
     const int item = blockIdx.x, head = blockIdx.y, v0 = (first_slice + blockIdx.z) * VS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int count = p.item_count[item];
@@ -1804,6 +1805,7 @@ memory_scan_kernel(MemoryScanParams p, int first_slice, int writes_shared) {
         m = *m_held;
         asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     }
+    if (p.state_ahead) wait_for_earlier_kernels();           // (the state is read; what the kernels ahead write follows)
     const long first = p.item_offset[item];
     const T* q = (const T*)p.q + (long)head * dim;
     const T* k = (const T*)p.k + (long)head * dim;
@@ -1892,7 +1894,7 @@ static void launch_memory_scan(const MemoryScanParams& p, int n_items, size_t sh
     if (shared > 48 * 1024) cudaFuncSetAttribute(memory_scan_kernel<T, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
     for (int first = 0; first < slices; first += most) {
         const int here = slices - first < most ? slices - first : most;
-        launch_kernel_in_clusters(AFTER_THE_KERNELS_AHEAD, gated && here > 1 ? dim3(1, 1, here) : dim3(0, 1, 1), memory_scan_kernel<T, 32>,
+        launch_kernel_in_clusters(p.state_ahead && g_dependent_launch != 0, gated && here > 1 ? dim3(1, 1, here) : dim3(0, 1, 1), memory_scan_kernel<T, 32>,
                                   dim3(n_items, p.heads, here), dim3(SCAN_WARPS * 32), shared, s, p, first, (int)(first + here == slices));
     }
 }

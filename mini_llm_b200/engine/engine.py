@@ -101,6 +101,8 @@ class Engine:
         self.workspace = Workspace(self.device, min_rows=min(self.max_tokens_per_step, 256))
         self.control = ControlBlock(self.device, self.cache.groups)
         self.ctx = StepContext(self.kernels, self.workspace, self.dtype, self.device)
+        # (a step's first kernel is launched behind the step before, and the second one behind the first)
+        self.ctx.steps_apart = True
         self.steps = 0
         self._sampled = None
         self.kept_tokens = torch.zeros(self.max_requests, dtype=torch.int32, device=self.device)

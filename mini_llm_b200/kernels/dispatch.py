@@ -163,7 +163,7 @@ class Kernels:
             return ops.split_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                                        n_heads, n_kv_heads, dim, cache.page_size, scale, window, span, -(-reach // span), acc,
                                        ml, counters, cap=cap, block=chunk, gate=gate, sink=sink, value_size=vdim, keep=keep, slopes=slopes,
-                                       gate_wide=gate_wide, first_new=ctx.item_start)
+                                       gate_wide=gate_wide, first_new=ctx.item_start if ctx.steps_apart else None)
         tiled = not ctx.decode_only and ops.capped_attention_tiled_takes(dim, vdim, q.dtype)
         self.chose("capped_attention", "capped_attention_tiled" if tiled else "capped_attention_plain", q.shape[0], n_heads, dim, vdim)
         return ops.capped_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
@@ -175,7 +175,7 @@ class Kernels:
         self.launches += 1
         return ops.linear_recurrence(out, q, k, v, gate_a, gate_b, log_rate, step_bias, state, ctx.item_slot, ctx.item_offset,
                                      ctx.item_count, heads, qk_heads, dim, vdim, delta, unit_norm, q_scale, skip, writes,
-                                     channel_decay)
+                                     channel_decay, ctx.steps_apart)
 
     def route(self, x, router, shared_gate, top, choice, in_weight, out_weight, **how):
         self.launches += 1
@@ -294,7 +294,7 @@ class Kernels:
                 scratch = self._latent_scratch(ctx.device, n * heads * parts * rank, n * heads * parts * 2) if parts > 1 else None
                 self.launches += 1 if parts > 1 else 0
                 self.chose("latent_attention", "latent_attention_tiled_parts", n, heads, rank + rot)
-                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate, rows_ahead=True)
+                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate, rows_ahead=ctx.steps_apart)
         self.chose("latent_attention", "latent_attention_plain", n, heads, rank + rot)
         plain_out = out if out.dtype == torch.float32 else ctx.buffer("latent_mixed_32", out.shape, torch.float32)
         ops.latent_attention_plain(plain_out, q_eff, cache.k_pages, cache.block_table, ctx.positions, ctx.token_item,
@@ -320,7 +320,7 @@ class Kernels:
         self.chose("memory_scan", "memory_passes" if passes else ("memory_chunk" if chunked else "memory_scan"),
                    q.shape[0], heads, dim, vdim)
         return ops.memory_scan(out, q, k, v, state, ctx.item_slot, ctx.item_offset, ctx.item_count, heads, dim, vdim,
-                               writes=writes, chunked=chunked, passes=passes, **how)
+                               writes=writes, chunked=chunked, passes=passes, state_ahead=ctx.steps_apart, **how)
 
     MEMORY_PASSES_TOKENS = 128     # from here on a step's chunks are worth four launches
 
@@ -532,7 +532,7 @@ class Kernels:
                 chunk = 64 if pairs < 64 else (128 if pairs < 128 else (256 if pairs < 256 else 512))
             max_chunks = -(-reach // chunk)
             self.chose("attention", "group_attention" if grouped else "split_attention", n, n_heads, head_size)
-            more = {} if grouped else {"first_new": ctx.item_start}
+            more = {} if grouped else {"first_new": ctx.item_start if ctx.steps_apart else None}
             return run(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                        n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, max_chunks, acc, ml,
                        counters, **more)
@@ -556,7 +556,7 @@ class Kernels:
                 acc, ml, counters = self._scratch(ctx, SPLIT_ATTENTION_MAX_ROWS * n_heads, -(-reach // 64), head_size)
                 ops.split_attention(out, q, cache.k_pages, cache.v_pages, cache.block_table, ctx.positions, ctx.token_item,
                                     n_heads, n_kv_heads, head_size, cache.page_size, scale, window, chunk, -(-reach // chunk), acc, ml,
-                                    counters, records=ctx.att_tiles[8 * n_tiles:], n_records=ctx.n_att_singles, first_new=ctx.item_start)
+                                    counters, records=ctx.att_tiles[8 * n_tiles:], n_records=ctx.n_att_singles, first_new=ctx.item_start if ctx.steps_apart else None)
             if ctx.att_units:
                 self.chose("attention", "attention_two_tiles", n, n_heads, head_size)
                 return ops.attention_prefill_two_tiles(out, q, cache.k_pages, cache.v_pages, cache.block_table,

@@ -1165,7 +1165,7 @@ class _MemoryScanParams(ctypes.Structure):
     _fields_ = [("out", P), ("ld_out", L), ("q", P), ("k", P), ("v", P), ("ld_q", L), ("ld_k", L), ("ld_v", L),
                 ("gates", P), ("ld_gates", L), ("gate_bias", P), ("decay", P), ("state", P), ("state_stride", L),
                 ("item_slot", P), ("item_offset", P), ("item_count", P), ("heads", I), ("dim", I), ("vdim", I),
-                ("q_scale", F), ("gate_cap", F), ("silu", I), ("writes", I), ("readers", P)]
+                ("q_scale", F), ("gate_cap", F), ("silu", I), ("writes", I), ("readers", P), ("state_ahead", I)]
 
 
 _memory_scan = Function("sequence", "mllm_sequence_memory_scan", [ctypes.POINTER(_MemoryScanParams), I, I, P])
@@ -1200,7 +1200,8 @@ def memory_state_floats(heads, dim, vdim, gated) -> int:
 
 
 def memory_scan(out, q, k, v, state, item_slot, item_offset, item_count, heads, dim, vdim, q_scale=1.0, silu=False,
-                gates=None, gate_bias=None, gate_cap=0.0, decay=None, writes=True, chunked=False, passes=None, readers=None):
+                gates=None, gate_bias=None, gate_cap=0.0, decay=None, writes=True, chunked=False, passes=None, readers=None,
+                state_ahead=False):
     """The matrix-memory recurrence over each entry's tokens, in order:
     S <- a S + b k v^T, out = S^T q, with a fixed decay per head (``decay`` [heads]; a = decay,
     b = 1) or with ``gates`` [T, 2 * heads] (fp32: input gates then forget gates, ``gate_bias``
@@ -1243,6 +1244,7 @@ def memory_scan(out, q, k, v, state, item_slot, item_offset, item_count, heads, 
     params.heads, params.dim, params.vdim = heads, dim, vdim
     params.q_scale, params.gate_cap = float(q_scale), float(gate_cap)
     params.silu, params.writes = int(bool(silu)), int(bool(writes))
+    params.state_ahead = int(bool(state_ahead))         # (no kernel that may still run writes the states: they are read early)
     if (chunked or passes is not None) and not memory_chunk_takes(dim):
         raise KernelError(f"memory_scan: the chunked kernels do not take a key size of {dim}")
     if passes is not None:
@@ -1393,14 +1395,15 @@ class _RecurrenceParams(ctypes.Structure):
                 ("gate_a", P), ("gate_b", P), ("ld_gate_a", L), ("ld_gate_b", L), ("log_rate", P), ("step_bias", P),
                 ("skip", P), ("state", P), ("state_stride", L), ("item_slot", P), ("item_offset", P), ("item_count", P),
                 ("heads", I), ("qk_heads", I), ("dim", I), ("vdim", I), ("q_scale", F), ("delta", I), ("unit_norm", I),
-                ("writes", I), ("channel_decay", I)]
+                ("writes", I), ("channel_decay", I), ("state_ahead", I)]
 
 
 _linear_recurrence = Function("hybrid", "mllm_hybrid_linear_recurrence", [ctypes.POINTER(_RecurrenceParams), I, I, I, P])
 
 
 def linear_recurrence(out, q, k, v, gate_a, gate_b, log_rate, step_bias, state, item_slot, item_offset, item_count, heads,
-                      qk_heads, dim, vdim, delta, unit_norm=False, q_scale=1.0, skip=None, writes=True, channel_decay=False):
+                      qk_heads, dim, vdim, delta, unit_norm=False, q_scale=1.0, skip=None, writes=True, channel_decay=False,
+                      state_ahead=False):
     """Per entry, its tokens in order, per head with the state S [dim, vdim] (fp32, in ``state``
     [slots, heads * dim * vdim]): step = softplus(gate_a[t, h] + step_bias[h]), a = exp(-exp(log_rate[h]) * step);
     without ``delta``: u = step * v; with: u = sigmoid(gate_b[t, h]) * (v - (a S)^T k); S <- a S + k u^T;
@@ -1441,6 +1444,7 @@ def linear_recurrence(out, q, k, v, gate_a, gate_b, log_rate, step_bias, state, 
     params.heads, params.qk_heads, params.dim, params.vdim = heads, qk_heads, dim, vdim
     params.q_scale, params.delta, params.unit_norm, params.writes = float(q_scale), int(bool(delta)), int(bool(unit_norm)), int(bool(writes))
     params.channel_decay = int(bool(channel_decay))
+    params.state_ahead = int(bool(state_ahead))         # (no kernel that may still run writes the states: they are read early)
     _linear_recurrence(ctypes.byref(params), item_count.shape[0], n, dtype_code(q.dtype), _stream())
     return out
 
