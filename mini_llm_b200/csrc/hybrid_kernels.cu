@@ -2396,10 +2396,10 @@ expert_down_kernel(float* __restrict__ hidden, long ld_hidden, const T* __restri
 // (m16n8k16) together, so that an expert's weights cross the chip once however many tokens chose it, and the sums are the tensor
 // cores', every product added by a rounded addition.  What bounds the two kernels are the weights' way from HBM (35 MB at 8 experts of 768 and a shared one of
 // 1,536 with a width of 768: 5.4 us) and the chain of choice, lists, operands and sums behind the router.  So all of a block's
-// weights are asked for at once, ahead of the wait for the kernels ahead where a quarter of the experts will have a token, and the
-// first kernel's idle lanes bring the second one's into L2.  Both kernels, 1, 7, 16, 31 tokens of such experts, replayed back to back: 17.0,
-// 19.0, 21.2, 27.9 us (16.1, 25.1, 27.0, 33.8 with weights in registers, 16 features a block whose K four warps shared, and a plan of the second kernel behind the
-// wait); in a decode step of 16 requests 17.8 us a layer where it was 25.4.
+// weights are asked for at once, ahead of the wait for the kernels ahead where the tokens choose half as many experts as there are, and the
+// first kernel's idle lanes bring the second one's into L2.  Both kernels, 1, 2, 7, 16, 31 tokens of such experts, replayed back to back:
+// 14.7, 17.7, 18.8, 20.8, 26.5 us (16.0, 21.2, 24.8, 26.9, 34.2 by the kernels for wide rows below); in a decode step of 16 requests 17.8 us a
+// layer where it was 25.4.
 constexpr int EXPERT_TILE_TOKENS = 31, EXPERT_TABLES = 64, EXPERT_UNITS = 64, EXPERT_UNIT_K = 256;
 
 // The pairs that chose expert e, in their order, by one warp: the list gets those from number `begin` on, 32 at most, and `place`
@@ -2421,10 +2421,11 @@ __device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, i
     return count;
 }
 
-// Whether the weights of all experts are asked for ahead of the wait, before their tokens are known: where a quarter of the experts or more
-// will have one.  (What is read in vain costs less than the wait for what is not: the router's kernel runs meanwhile.)
+// Whether the weights of all experts are asked for ahead of the wait, before their tokens are known: where the tokens choose half as many
+// experts as there are or more.  (What is read in vain costs less than the wait for what is not: the router's kernel runs meanwhile.  One
+// token of 8 experts, two and a shared one: 15.4 us behind the wait, 16.7 ahead; two: 18.4 and 17.7.)
 __device__ __forceinline__ bool experts_ahead(int n_tokens, int pairs, int n_experts) {
-    return n_tokens * (pairs > 1 ? pairs - 1 : 1) * 4 >= n_experts;
+    return n_tokens * (pairs > 1 ? pairs - 1 : 1) * 2 >= n_experts;
 }
 
 // By one warp, two experts a lane: where the parts of the experts that `has` names begin, expert e's `parts_of(e)` of them, in
@@ -2462,8 +2463,7 @@ __device__ __forceinline__ int expert_of_part(const int* first_part, int n_table
 
 // A warp: eight inner features of an expert with a gate (16 without): its tile's 16 rows are the gates and the ups of the same features,
 // so that a lane holds both of a result; the tile's columns are pairs, eight at a time.  The weights lie in a ring of the lane's own
-// in shared memory (`depth` blocks of 32 of K: all of them at a width of 768), the tokens beside them where they fit.  Where the rows are
-// long, `share` warps side by side take a share of K each and the first one adds their sums in order.
+// in shared memory (`depth` blocks of 32 of K: all of them at a width of 768), the tokens beside them where they fit.
 constexpr int EXPERT_UP_WARPS = 8, EXPERT_UP_SHARED = 224 * 1024, EXPERT_UP_BLOCK = EXPERT_UP_WARPS * 2 * 32 * 16;     // (bytes of a block of 32 of K)
 constexpr int EXPERT_UP_STATIC = (EXPERT_UP_WARPS * 32 + EXPERT_TABLES + 1) * 4 + EXPERT_TABLES * 28 + 64;
 
@@ -2472,7 +2472,7 @@ __global__ void __launch_bounds__(EXPERT_UP_WARPS * 32, 1)
 expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long ld_x, const int* choice, const float* in_weight,
                        const long long* __restrict__ gate_of, const long long* __restrict__ up_of, const long long* __restrict__ down_of,
                        const int* __restrict__ inner_of, int n_tables, long ld_down, int width, int pairs, int n_tokens, float limit,
-                       float shared_limit, float alpha, int n_experts, int depth, int share) {
+                       float shared_limit, float alpha, int n_experts, int depth) {
     const int held_tokens = HELD ? n_tokens : 0;
     constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
     constexpr int FEATURES = GATED ? 8 : 16, THREADS = EXPERT_UP_WARPS * 32;
@@ -2485,10 +2485,8 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
     unsigned char* held = up_shared + (size_t)depth * EXPERT_UP_BLOCK;
     int* chosen = reinterpret_cast<int*>(held + (size_t)held_tokens * ld_held);
     float* scales = reinterpret_cast<float*>(chosen + n_pairs);
-    float* shared_sums = scales + n_pairs;                                    // [warp][16][lane] where K is shared
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int half = depth / 2;
-    const int each = (all + share - 1) / share, begin = warp % share * each, end = min(all, begin + each);      // this warp's blocks of 32 of K
     dependents_may_start();
     for (int e = threadIdx.x; e < n_tables; e += THREADS) {
         inner_here[e] = __ldg(inner_of + e);
@@ -2512,27 +2510,26 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
     };
     auto ask = [&](int which, int first) {                                    // half the ring: blocks of K from `first` on
         for (int i = 0; i < half; i++) {
-            const bool there = first + i < end && (first + i) * 4 + tq < pieces;
+            const bool there = first + i < all && (first + i) * 4 + tq < pieces;
             uint4* to = ring + (size_t)(which * half + i) * 2 * THREADS + threadIdx.x;
-            if (first + i < end) {
+            if (first + i < all) {
                 copy_16(to, there ? low + (first + i) * 32 : low - tq * 8, there);
                 copy_16(to + THREADS, there ? high + (first + i) * 32 : high - tq * 8, there);
             }
         }
         copies_end();
     };
-    const int teams = EXPERT_UP_WARPS / share;
-    const int walker = warp / share * gridDim.x + blockIdx.x, walkers = teams * gridDim.x;       // neighbouring parts on different SMs
+    const int walker = warp * gridDim.x + blockIdx.x, walkers = EXPERT_UP_WARPS * gridDim.x;     // neighbouring parts on different SMs
     auto begin_part = [&](int part, int& e, int& f0) {
         e = expert_of_part(first_part, n_tables, part);
         f0 = (part - first_part[e]) * FEATURES;
         rows_of(e, f0);
-        ask(0, begin);
-        ask(1, begin + half);
+        ask(0, 0);
+        ask(1, half);
     };
     // the other kernel's weights come into L2 meanwhile, an expert's piece of a row at a time
     auto down_ahead = [&](auto has) {
-        for (int i = warp * gridDim.x + blockIdx.x; i < n_tables * width; i += EXPERT_UP_WARPS * gridDim.x) {
+        for (int i = walker; i < n_tables * width; i += walkers) {
             const int e = i / width;
             if (!has(e)) continue;
             const char* row = reinterpret_cast<const char*>(down_here[e]) + (long)(i - e * width) * ld_down * 2;
@@ -2592,10 +2589,10 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
         for (int t = 0; t < TILES; t++)
 #pragma unroll
             for (int i = 0; i < 16; i++) sums[t][i / 4][i % 4] = 0.0f;
-        for (int first = begin, which = 0; first < end; first += half, which ^= 1) {
+        for (int first = 0, which = 0; first < all; first += half, which ^= 1) {
             copies_landed<1>();
             const uint4* mine = ring + (size_t)which * half * 2 * THREADS + threadIdx.x;
-            const int here_blocks = min(half, end - first);
+            const int here_blocks = min(half, all - first);
             // four blocks of K at a time: their loads do not wait on one another
             for (int i = 0; i < here_blocks; i += 4) {
                 uint4 a[4], b[4], v[4][TILES];
@@ -2637,23 +2634,6 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
         for (int t = 0; t < TILES; t++)
 #pragma unroll
             for (int i = 0; i < 4; i++) z[t][i & 1][i >> 1] = (sums[t][0][i] + sums[t][1][i]) + (sums[t][2][i] + sums[t][3][i]);
-        if (share > 1) {
-            // (the warps of a team are at the same part and pairs)
-            float* mine = shared_sums + warp * 16 * 32 + lane;
-#pragma unroll
-            for (int t = 0; t < TILES; t++)
-#pragma unroll
-                for (int i = 0; i < 4; i++) mine[(t * 4 + i) * 32] = z[t][i & 1][i >> 1];
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / share), "r"(share * 32) : "memory");
-            if (warp % share == 0)
-                for (int o = 1; o < share; o++)
-#pragma unroll
-                    for (int t = 0; t < TILES; t++)
-#pragma unroll
-                        for (int i = 0; i < 4; i++) z[t][i & 1][i >> 1] += mine[o * 16 * 32 + (t * 4 + i) * 32];
-            asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / share), "r"(share * 32) : "memory");
-            if (warp % share != 0) return;
-        }
         const int inner = inner_here[e];
         const float most = e == n_experts ? shared_limit : limit;
 #pragma unroll
@@ -2683,8 +2663,8 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
             __syncwarp();
             const int here = min(32, count - m0);
             if (m0 > 0) {
-                ask(0, begin);
-                ask(1, begin + half);
+                ask(0, 0);
+                ask(1, half);
             }
             if (here > 0 && here <= 8) multiply(std::integral_constant<int, 1>(), here, e, f0, list);
             else if (here > 8 && here <= 16) multiply(std::integral_constant<int, 2>(), here, e, f0, list);
@@ -2843,6 +2823,245 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
         if (identity_weight != nullptr) total = fmaf(behind_the_wait(identity_weight)[t], to_f32(x[(long)t * ld_x + c]), total);
         float* h = hidden + (long)t * ld_hidden + c;
         *h = assign ? total : (i == (int)threadIdx.x ? hidden_mine : *h) + total;
+    }
+}
+
+// Rows wider than the second kernel above has blocks for at once (eight columns each, one an SM): the same by more and smaller blocks, weights
+// in registers, two and more of them an SM.  8 experts of 1,024, two a token, 16 tokens, these kernels against those: width 1,024 25.3
+// and 23.2 us, 1,280 29.3 and 32.3, 2,048 34.5 and 43.1.
+// A block: 16 inner features of an expert, in two tiles of 8 whose K four warps share.
+template <int FORM>
+__global__ void __launch_bounds__(256, 2)
+expert_up_blocks_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long ld_x, const int* choice, const float* in_weight,
+                       const long long* __restrict__ gate_of, const long long* __restrict__ up_of, const int* __restrict__ inner_of,
+                       int width, int pairs, int n_tokens, float limit, float shared_limit, float alpha, int n_experts) {
+    constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
+    constexpr int AHEAD = 4;
+    __shared__ int list[32], found;                          // (32 pairs at a time)
+    __shared__ float sums[2][8][16][9];                      // [gate, up][warp][row][feature]
+    const int e = blockIdx.y, inner = __ldg(inner_of + e);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int f_block = blockIdx.x * 16, f0 = f_block + (warp >> 2) * 8;
+    dependents_may_start();
+    if (f_block >= inner) return;
+    const int pieces = width / 8, all = (width + 31) / 32, each = (all + 3) / 4;
+    const int begin = (warp & 3) * each, end = f0 < inner ? min(all, begin + each) : begin;
+    const long row = (long)min(f0 + g, inner - 1) * pieces;
+    const uint4* up = reinterpret_cast<const uint4*>(__ldg(up_of + e)) + row;
+    const uint4* gate = GATED ? reinterpret_cast<const uint4*>(__ldg(gate_of + e)) + row : up;
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    uint4 wu[AHEAD], wg[AHEAD];
+    auto weights = [&](int i, int block) {
+        const int c = block * 4 + tq;
+        const bool there = block < end && c < pieces;
+        wu[i] = there ? __ldg(up + c) : none;
+        if (GATED) wg[i] = there ? __ldg(gate + c) : none;
+    };
+    // (ahead of the wait only where nearly every expert will have a token: a step of one reads four of eight)
+    const bool early = n_tokens * (pairs > 1 ? pairs - 1 : 1) >= n_experts;
+    if (early)
+#pragma unroll
+        for (int i = 0; i < AHEAD; i++) weights(i, begin + i);
+    wait_for_earlier_kernels();
+    choice = behind_the_wait(choice);
+    x = behind_the_wait(x);
+    in_weight = behind_the_wait(in_weight);
+    if (warp == 0) {
+        const int count = pairs_of_expert(choice, n_tokens * pairs, e, 0, list, nullptr);
+        if (lane == 0) found = count;
+    }
+    __syncthreads();
+    const int count = found;
+    for (int m0 = 0; m0 < count; m0 += 16) {
+        if (m0 > 0 && m0 % 32 == 0) {                        // (every thread left the list before the barrier that ended the last tile)
+            if (warp == 0) pairs_of_expert(choice, n_tokens * pairs, e, m0, list, nullptr);
+            __syncthreads();
+        }
+        const int* listed = list + m0 % 32;
+        if (m0 > 0 || !early)
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++) weights(i, begin + i);
+        // rows g and g + 8 of the tile: the tokens of two pairs and the weight their entries get
+        const uint4* xr[2];
+        float scale[2];
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            const bool there = m0 + r * 8 + g < count;
+            const int pair = there ? listed[r * 8 + g] : 0;
+            xr[r] = there ? reinterpret_cast<const uint4*>(x + (long)(pair / pairs) * ld_x) : nullptr;
+            scale[r] = there ? in_weight[pair] : 1.0f;
+        }
+        float zg[4] = {0.0f, 0.0f, 0.0f, 0.0f}, zu[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        for (int first = begin; first < end; first += AHEAD) {
+            uint4 xv[AHEAD][2];
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++)
+#pragma unroll
+                for (int r = 0; r < 2; r++) {
+                    const int c = (first + i) * 4 + tq;
+                    xv[i][r] = xr[r] != nullptr && first + i < end && c < pieces ? xr[r][c] : none;
+                }
+#pragma unroll
+            for (int i = 0; i < AHEAD; i++) {
+                const uint4 u = wu[i], v = GATED ? wg[i] : none;
+                weights(i, first + AHEAD + i);
+#pragma unroll
+                for (int r = 0; r < 2; r++)
+                    if (scale[r] != 1.0f) {                  // the input's weight, rounded as an activation
+                        float y[8];
+                        Vec16<bf16>::unpack(xv[i][r], y);
+                        __nv_bfloat162 two[4];
+#pragma unroll
+                        for (int k = 0; k < 4; k++) two[k] = __floats2bfloat162_rn(scale[r] * y[2 * k], scale[r] * y[2 * k + 1]);
+                        xv[i][r] = *reinterpret_cast<const uint4*>(two);
+                    }
+                const uint32_t first_half[4] = {xv[i][0].x, xv[i][1].x, xv[i][0].y, xv[i][1].y}, second_half[4] = {xv[i][0].z, xv[i][1].z, xv[i][0].w, xv[i][1].w};
+                mma_added(zu, first_half, u.x, u.y);
+                mma_added(zu, second_half, u.z, u.w);
+                if (GATED) {
+                    mma_added(zg, first_half, v.x, v.y);
+                    mma_added(zg, second_half, v.z, v.w);
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            sums[1][warp][g + (i >> 1) * 8][2 * tq + (i & 1)] = zu[i];
+            if (GATED) sums[0][warp][g + (i >> 1) * 8][2 * tq + (i & 1)] = zg[i];
+        }
+        __syncthreads();
+        const int f = threadIdx.x & 15, r = threadIdx.x >> 4;
+        if (m0 + r < count && f_block + f < inner) {
+            float a = 0.0f, b = 0.0f;
+            for (int s = 0; s < 4; s++) {
+                if (GATED) a += sums[0][(f >> 3) * 4 + s][r][f & 7];
+                b += sums[1][(f >> 3) * 4 + s][r][f & 7];
+            }
+            act[(long)listed[r] * ld_act + f_block + f] =
+                __float2bfloat16_rn(expert_form<FORM>(a, b, e == n_experts ? shared_limit : limit, alpha));
+        }
+        __syncthreads();
+    }
+}
+
+// A block: eight columns of the sum, all tokens.  A unit is an expert's pairs and EXPERT_UNIT_K of its inner size (all of it
+// where the chosen experts would bring more units than there is room for); sixteen warps take the units in turn, and a
+// token's column adds its pairs' units in their order.
+__global__ void __launch_bounds__(512)
+expert_down_blocks_kernel(float* hidden, long ld_hidden, const bf16* act, long ld_act, const int* choice, const float* out_weight,
+                         const long long* __restrict__ down_of, const int* __restrict__ inner_of, int n_tables, long ld_down,
+                         int width, int pairs, int n_tokens, int assign, const bf16* x, long ld_x, const float* identity_weight) {
+    constexpr int BLOCKS = EXPERT_UNIT_K / 32;
+    __shared__ int list[EXPERT_TABLES][32], count_of[EXPERT_TABLES], first_unit[EXPERT_TABLES + 1], unit_k;
+    extern __shared__ float down_shared[];                   // [units][32 rows][8 columns], then the pairs' places as ints
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int c0 = blockIdx.x * 8, n_pairs = n_tokens * pairs;
+    int* place = reinterpret_cast<int*>(down_shared + EXPERT_UNITS * 32 * 8);
+    dependents_may_start();
+    wait_for_earlier_kernels();
+    choice = behind_the_wait(choice);
+    act = behind_the_wait(act);
+    out_weight = behind_the_wait(out_weight);
+    x = behind_the_wait(x);
+    for (int e = warp; e < n_tables; e += 16) {
+        const int count = pairs_of_expert(choice, n_pairs, e, 0, list[e], place);
+        if (lane == 0) count_of[e] = min(count, 32);
+    }
+    __syncthreads();
+    if (warp == 0) {
+        // how many units every expert has, and where they begin: two experts a lane
+        int size = EXPERT_UNIT_K, total = 0;
+        for (int attempt = 0; attempt < 2; attempt++) {
+            int mine[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int e = 2 * lane + h;
+                mine[h] = e < n_tables && count_of[e] > 0 ? (attempt == 0 ? (__ldg(inner_of + e) + EXPERT_UNIT_K - 1) / EXPERT_UNIT_K : 1) : 0;
+            }
+            int sum = mine[0] + mine[1];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int before = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += before;
+            }
+            total = __shfl_sync(0xffffffffu, sum, 31);
+            const int start = sum - mine[0] - mine[1];
+            if (2 * lane < n_tables) first_unit[2 * lane] = start;
+            if (2 * lane + 1 < n_tables) first_unit[2 * lane + 1] = start + mine[0];
+            size = attempt == 0 ? EXPERT_UNIT_K : 0;
+            if (total <= EXPERT_UNITS) break;
+        }
+        if (lane == 0) {
+            first_unit[n_tables] = total;
+            unit_k = size;
+        }
+    }
+    __syncthreads();
+    const int units = first_unit[n_tables];
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+    for (int unit = warp; unit < units; unit += 16) {
+        int e = 0;                                           // the last expert that begins at or before this unit and has units
+        for (int first = 0; first < n_tables; first += 32) {
+            const int at = first + lane;
+            const unsigned here = __ballot_sync(0xffffffffu, at < n_tables && count_of[at] > 0 && first_unit[at] <= unit);
+            if (here != 0u) e = first + 31 - __clz(here);
+        }
+        const int inner = __ldg(inner_of + e), count = count_of[e];
+        const int k_first = unit_k > 0 ? (unit - first_unit[e]) * unit_k : 0, k_end = unit_k > 0 ? min(inner, k_first + unit_k) : inner;
+        const uint4* w = reinterpret_cast<const uint4*>(reinterpret_cast<const bf16*>(__ldg(down_of + e)) + (long)min(c0 + g, width - 1) * ld_down);
+        for (int m0 = 0; m0 < count; m0 += 16) {
+            const uint4* ar[2];
+#pragma unroll
+            for (int r = 0; r < 2; r++)
+                ar[r] = m0 + r * 8 + g < count ? reinterpret_cast<const uint4*>(act + (long)list[e][m0 + r * 8 + g] * ld_act) : nullptr;
+            float z[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (int k0 = k_first; k0 < k_end; k0 += EXPERT_UNIT_K) {
+                uint4 wv[BLOCKS], av[BLOCKS][2];
+#pragma unroll
+                for (int i = 0; i < BLOCKS; i++) {
+                    const int c = k0 / 8 + i * 4 + tq;
+                    const bool there = c * 8 < k_end;
+                    wv[i] = there ? __ldg(w + c) : none;
+#pragma unroll
+                    for (int r = 0; r < 2; r++) av[i][r] = there && ar[r] != nullptr ? ar[r][c] : none;
+                }
+#pragma unroll
+                for (int i = 0; i < BLOCKS; i++) {
+                    const uint32_t first_half[4] = {av[i][0].x, av[i][1].x, av[i][0].y, av[i][1].y};
+                    const uint32_t second_half[4] = {av[i][0].z, av[i][1].z, av[i][0].w, av[i][1].w};
+                    mma_added(z, first_half, wv[i].x, wv[i].y);
+                    mma_added(z, second_half, wv[i].z, wv[i].w);
+                }
+            }
+            float* mine = down_shared + (unit * 32 + m0 + g) * 8 + 2 * tq;
+            mine[0] = z[0], mine[1] = z[1];
+            mine[64] = z[2], mine[65] = z[3];
+        }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n_tokens * 8; i += 512) {
+        const int t = i / 8, c = c0 + i % 8;
+        if (c >= width) continue;
+        float total = 0.0f;
+        for (int k = 0; k < pairs; k++) {
+            const int pair = t * pairs + k, e = choice[pair];
+            if (e < 0 || e >= n_tables) continue;
+            if (place[pair] < 0) {                           // beyond an expert's 32 (a token that named it more than once): by itself
+                const bf16* row = act + (long)pair * ld_act;
+                const bf16* w = reinterpret_cast<const bf16*>(__ldg(down_of + e)) + (long)c * ld_down;
+                float z = 0.0f;
+                for (int f = 0; f < __ldg(inner_of + e); f++) z = fmaf(to_f32(row[f]), to_f32(w[f]), z);
+                total = fmaf(out_weight[pair], z, total);
+                continue;
+            }
+            const int last = unit_k > 0 ? first_unit[e] + (__ldg(inner_of + e) + EXPERT_UNIT_K - 1) / EXPERT_UNIT_K : first_unit[e] + 1;
+            float z = 0.0f;
+            for (int u = first_unit[e]; u < last; u++) z += down_shared[(u * 32 + place[pair]) * 8 + i % 8];
+            total = fmaf(out_weight[pair], z, total);
+        }
+        if (identity_weight != nullptr) total = fmaf(behind_the_wait(identity_weight)[t], to_f32(x[(long)t * ld_x + c]), total);
+        float* h = hidden + (long)t * ld_hidden + c;
+        *h = assign ? total : *h + total;
     }
 }
 
@@ -3011,15 +3230,30 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
         if (n_pairs > 16384) return fail("experts: too many pairs for the tiles");
         const bf16* xb = (const bf16*)x;
         bf16* ab = (bf16*)act;
+        if ((width + 7) / 8 > sm_count()) {
+            const dim3 tiles((max_inner + 15) / 16, n_tables);
+#define UP_BLOCKS(FORM)                                                                                                          \
+    launch_kernel(g_dependent_launch != 0, expert_up_blocks_kernel<FORM>, tiles, dim3(256), 0, s, ab, ld_act, xb, ld_x, choice, in_weight, \
+                  gate_of, up_of, inner_of, width, pairs, n_tokens, limit, shared_limit, alpha, n_experts)
+            if (form == EXPERT_GATED_SILU) UP_BLOCKS(EXPERT_GATED_SILU);
+            else if (form == EXPERT_RELU_SQUARED) UP_BLOCKS(EXPERT_RELU_SQUARED);
+            else UP_BLOCKS(EXPERT_CLAMPED_GLU);
+#undef UP_BLOCKS
+            // (at every launch, as the limit is a device's own)
+            if (cudaFuncSetAttribute(expert_down_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
+                return fail("experts: cannot raise the shared memory limit");
+            launch_kernel(AFTER_THE_KERNELS_AHEAD, expert_down_blocks_kernel, dim3((width + 7) / 8), dim3(512),
+                          sizeof(float) * EXPERT_UNITS * 32 * 8 + sizeof(int) * n_pairs, s, hidden, ld_hidden, (const bf16*)act, ld_act, choice,
+                          out_weight, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, assign, xb, ld_x, identity_weight);
+            return check_launch("expert blocks");
+        }
         // the first kernel's shared memory: the pairs' choices and weights, then the tokens if they leave half of it, then the ring of weights
         const size_t room = EXPERT_UP_SHARED - EXPERT_UP_STATIC, chosen_bytes = n_pairs * 8;
         const size_t token_bytes = (size_t)n_tokens * (width * 2 + (width % 64 == 0 ? 64 : 16));
-        const int share = width <= 1024 ? 1 : width <= 2048 ? 2 : 4;        // (4 tokens, 4 experts of 1,024, a width of 4,096: 48 us by one warp)
-        const size_t sums_bytes = share > 1 ? EXPERT_UP_WARPS * 16 * 32 * 4 : 0;
         const int held_tokens = chosen_bytes + token_bytes <= room / 2 ? n_tokens : 0;
-        const size_t beside = chosen_bytes + (held_tokens > 0 ? token_bytes : 0) + sums_bytes;
+        const size_t beside = chosen_bytes + (held_tokens > 0 ? token_bytes : 0);
         int depth = (int)((room - beside) / EXPERT_UP_BLOCK) / 2 * 2;
-        const int blocks_of_k = ((width + 31) / 32 + share - 1) / share;
+        const int blocks_of_k = (width + 31) / 32;
         if (depth > (blocks_of_k + 1) / 2 * 2) depth = (blocks_of_k + 1) / 2 * 2;
         const size_t up_bytes = (size_t)depth * EXPERT_UP_BLOCK + beside;
         const dim3 walkers(sm_count());
@@ -3030,7 +3264,7 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
             return fail("experts: cannot raise the shared memory limit");                                                        \
         launch_kernel(g_dependent_launch != 0, expert_up_tiles_kernel<FORM, HELD>, walkers, dim3(EXPERT_UP_WARPS * 32), up_bytes, s, ab, ld_act, xb, ld_x, \
                       choice, in_weight, gate_of, up_of, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, limit, shared_limit, alpha, \
-                      n_experts, depth, share);                                                                                       \
+                      n_experts, depth);                                                                                       \
     } while (0)
 #define UP_TILES(FORM)                                  \
     do {                                                \
