@@ -187,8 +187,8 @@ class Kernels:
         Pair by pair a block has 32 features of a pair, and an expert's weights are read once a pair: as fast as the tiles, which
         find every expert's pairs first, or faster, while those blocks fit the GPU at once (592, four an SM).  Only one or two
         tokens, whose blocks are few, go through the tiles all the same.  A layer of 8 experts of 768, two and a shared one of
-        1,536 a token, at 1, 4, 7, 16 tokens: tiles 14.7, 18.4, 18.8, 20.8 us, pairs 20.6, 21.8, 26.1, 38.1; 16 experts of 512, two and a shared one of
-        512, at 3, 8, 13, 31: tiles 19.3, 20.7, 21.7, 27.2, pairs 17.2, 18.2, 25.0, 37.8."""
+        1,536 a token, at 1, 4, 7, 16 tokens: tiles 14.7, 18.3, 18.7, 20.8 us, pairs 20.5, 21.6, 25.9, 37.8; 16 experts of 512, two and a shared one of
+        512, at 3, 8, 13, 31: tiles 16.6, 20.6, 21.8, 27.0, pairs 16.9, 18.1, 24.7, 37.5."""
         self.launches += 2
         tiles = (eights and not self.plain_only and ld_down is not None and ops.expert_tiles_take(x, act, inner_of.shape[0], ld_down)
                  and (x.shape[0] <= 2 or x.shape[0] * features > 592 * 32))
