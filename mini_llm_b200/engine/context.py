@@ -123,33 +123,30 @@ class ControlBlock:
         self.generation += 1
 
     def begin(self, n_tokens: int, n_items: int, alternate: bool = True):
-        """The arrays of a step of these sizes: (host views to fill, device views).  ``send`` follows."""
-        self.parity = (self.parity ^ 1) if alternate else 0
-        key = (self.parity, n_tokens, n_items)
+        """The arrays of a step of these sizes: (host views to fill, device views).  ``send`` follows; until then nothing has
+        changed: a step that is given up while its arrays are filled leaves no trace, and the next one begins where it did."""
+        parity = (self.parity ^ 1) if alternate else 0
+        key = (parity, n_tokens, n_items)
         held = self._layouts.get(key)
         if held is None:
             offsets, size = self._layout(n_tokens, n_items)
             size = (size + 3) // 4 * 4
             self._ensure(size)               # may drop every cached layout
-            held = self._layouts[key] = (offsets, size, self._views(self.device_buffers[self.parity], offsets, n_tokens, n_items))
+            held = self._layouts[key] = (offsets, size, self._views(self.device_buffers[parity], offsets, n_tokens, n_items))
         offsets, size, views = held
-        self._size = size
-        self.last_upload_bytes = 4 * size
         if alternate:
             # two pinned buffers in turn; the copy that last read this one must be done
-            self._host_turn ^= 1
-            part = self._host_turn
+            part = self._host_turn ^ 1
             if self._copied_once[part]:
                 self._copied[part].synchronize()
         else:
             if self._ring_open:
-                # a step was begun and did not get behind its kernels: whether they took its part is not known
+                # a step was sent and did not get behind its kernels: whether they took its part is not known
                 torch.cuda.synchronize(self.device)
                 self._steps.zero_()
                 torch.cuda.synchronize(self.device)
-                self._ring_turn = 0
+                self._ring_turn, self._ring_open = 0, False
             part = self._ring_turn
-            self._ring_open = True
             if self._ring_used[part]:
                 self._ring_done[part].synchronize()
         host_key = (alternate, part, n_tokens, n_items)
@@ -159,13 +156,18 @@ class ControlBlock:
                 self._host_views.clear()
             memory = self._host_np[part] if alternate else self._ring_np[part * self.capacity:(part + 1) * self.capacity]
             host = self._host_views[host_key] = self._array_views(memory, offsets, n_tokens, n_items)
+        self._begun = (parity, part, size)
         return host, views
 
     def send(self, alternate: bool = True) -> None:
         """The filled arrays are on their way (the alternating steps' copy), or ready to be taken (``take``)."""
+        parity, turn, size = self._begun
+        self.parity, self._size = parity, size
+        self.last_upload_bytes = 4 * size
         if not alternate:
+            self._ring_open = True
             return
-        turn, parity, size = self._host_turn, self.parity, self._size
+        self._host_turn = turn
         # beside the kernels of the step before; behind the kernels that last read this buffer
         with torch.cuda.stream(self.copy_stream):
             if self._consumed[parity] is not None:

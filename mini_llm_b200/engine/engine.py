@@ -326,8 +326,8 @@ class Engine:
             self._make_ids_pinned(2 * n_want)
             self._graphs.clear()
         host, views = self.control.begin(max(n_tokens, n_want), n_items, alternate)
-        self._turn ^= 1                       # the slot of the readback ring this step fills
-        host["turn"][0] = self._turn
+        turn = self._turn ^ 1                 # the slot of the readback ring this step fills, once it is on its way
+        host["turn"][0] = turn
         token_ids, want_rows, want_slots = host["token_ids"], host["want_rows"], host["want_slots"]
         if decode_only and all(len(e.want) <= 1 for e in entries):
             # single tokens: the arrays straight from lists
@@ -418,12 +418,13 @@ class Engine:
         # This step's kernels write their sampled ids where an earlier step left its own: that
         # step's copy to the host must be done.  Two steps that alternate use different buffers,
         # so the second need not wait for the first one's copy (it runs beside it).
-        for slot in (self._turn, self._turn ^ 1):
-            beside = slot != self._turn and alternate and self._alternated
+        for slot in (turn, turn ^ 1):
+            beside = slot != turn and alternate and self._alternated
             if self._readback[slot] is not None and not beside:
                 compute.wait_event(self._readback[slot][2])
-        self._alternated = alternate
+        self._alternated = False              # (behind a step that fails in here the next one waits for every copy)
         logits = self._run(ctx, sample_views)
+        self._turn, self._alternated = turn, alternate
         self.hidden_dump = ctx.dump
         self.control.consumed(alternate)
         for entry in entries:

@@ -327,6 +327,49 @@ def test_a_step_over_the_token_limit_is_refused_and_a_failed_step_changes_nothin
     engine.cache.check()
 
 
+@pytest.mark.parametrize("one_kernel", [True, False])
+def test_a_step_given_up_on_the_host_leaves_the_draws_and_the_turns(folder_d, one_kernel):
+    """A step whose arrays cannot be filled (a counter and a seed that do not fit) is given up before anything was sent: the draws
+    of the last two steps are still to be had, and nothing has to be waited for.  One that fails after its arrays were sent, before or
+    behind the kernel that takes them, leaves them too.  The steps after it draw what they draw without it."""
+    from mini_llm_b200.engine import Engine, SamplingParams, StepEntry
+    tokens = random_tokens(12, 40, TINY_D["vocab_size"])
+    draw = lambda counter, seed=5: [SamplingParams(0.9, 1.0, seed, counter)] * 2
+
+    def injected(*_, **__):
+        raise RuntimeError("injected")
+
+    drawn = {}
+    for refusals in (False, True):
+        engine = Engine(folder_d, dtype="bfloat16", page_size=16, cache_tokens=1024, max_requests=2, fused_decode=one_kernel)
+        assert (engine.fused is not None) == one_kernel
+        a, b = engine.open_request(), engine.open_request()
+        step = lambda i, sampling: engine.step([StepEntry(s, [tokens[20 + i]], [0]) for s in (a, b)], sampling)
+        engine.step([StepEntry(a, tokens[:20], []), StepEntry(b, tokens[3:20], [])])
+        drawn[refusals] = []
+        for i in range(16):
+            step(i, draw(i))
+            if refusals and i > 0:
+                if i % 4 < 2:
+                    with pytest.raises((OverflowError, TypeError)):
+                        step(i, draw(2 ** 31) if i % 2 else draw(0, seed=None))
+                    assert not engine.control._ring_open
+                elif not one_kernel:
+                    owner, name = (engine.control, "take") if i % 4 == 2 else (engine.model, "forward")
+                    real, cuda_graphs = getattr(owner, name), engine.cuda_graphs
+                    setattr(owner, name, injected)
+                    engine.cuda_graphs = False
+                    with pytest.raises(RuntimeError, match="injected"):
+                        step(i, draw(0))
+                    setattr(owner, name, real)
+                    engine.cuda_graphs = cuda_graphs
+                assert engine.sampled_tokens(1) == drawn[refusals][-1]
+            drawn[refusals].append(engine.sampled_tokens())
+        engine.check_status()
+        engine.cache.check()
+    assert drawn[True] == drawn[False] and len({tuple(d) for d in drawn[False]}) > 4
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_a_place_may_be_wanted_twice(folder_d, dtype):
     from mini_llm_b200.engine import Engine, StepEntry
