@@ -1408,6 +1408,24 @@ static int rows_split_code(int M, int N, int K, int sms, int width, bool scatter
     return best;
 }
 
+// The narrow tiles' plan for a product, or 0 where it goes to the kernels behind them.  Up to 64 tokens the narrow tiles are ahead while their
+// blocks fit the SMs at once; in a second round a block's way in and out and its sums over the warps come on top, where the swapped tiles
+// of more features, several CTAs an SM, still run at their loop's speed.  Replayed back to back over weights larger than L2, swapped tiles
+// and narrow ones: in one round 64 x 768 x 768 6.6 and 3.4 us, 64 x 3072 x 768 7.4 and 5.4, 64 x 6144 x 768 10.0 and 8.9, 64 x 6144 x 2048 13.9 and
+// 13.7, 24 x 8192 x 4096 17.6 and 15.4, 64 x 3072 x 4096 12.2 and 12.9; in more 32 x 8192 x 1024 9.0 and 9.7, 64 x 4096 x 2048 10.1 and 13.2,
+// 64 x 8192 x 2048 15.0 and 24.4, 64 x 12288 x 4096 28.6 and 41.5 (one the other way: 48 x 8192 x 512, 8.5 and 8.0).  Up to 16 tokens a second
+// round costs little: 12 x 16000 x 768 9.6 and 8.6 (64 x 50257 x 768 21.4 and 58.9).  From more than 4,096 of K on the loop over it, with x's way from
+// L2, is what counts, and from 17 tokens on it is the longer one, but for blocks that share neither K nor tokens: 24 x 8192 x 6400 23.7 and 22.9,
+// 24 x 4096 x 8192 16.9 and 16.8, 24 x 4096 x 11008 21.2 and 22.5; shared 24 x 1600 x 6400 9.2 and 10.7 (16 tokens 8.9 and 8.3).
+extern "C" int mllm_gemm_narrow_plan(int M, int N, int K, int sms) {
+    if (M > 64 || N >= 16384 || (M > 24 && K > 4096) || (M > 16 && K > 8192)) return 0;
+    int rounds = 1;
+    const int plan = narrow_plan(M, N, K, sms, &rounds);
+    if (M <= 16) return plan;
+    const bool shared = plan >= 100 || plan % 10 > 1;
+    return rounds == 1 && !(shared && K > 4096) ? plan : 0;
+}
+
 static int gemm_bf16(void* out, const void* x, const void* w, const float* bias, int M, int N, int K, long ldx, long ldo,
                      int epilogue, int out_f32, int* status, const GemmScatter* scatter, void* stream, int forced_bn,
                      unsigned long long* timeline = nullptr) {
@@ -1437,11 +1455,8 @@ static int gemm_bf16(void* out, const void* x, const void* w, const float* bias,
     const int sms = sm_count();
     // (A forced code 8000 + a plan: narrow tiles, see narrow_plan.)
     if (forced_bn >= 8000) return launch_narrow_plan(p, forced_bn - 8000, x, ldx, w, s);
-    // Up to 64 tokens the narrow tiles, where neither K nor the features are so many that 128 x 64 tiles fill the SMs.  Replayed back to
-    // back over weights larger than L2, swapped tiles and narrow ones: 24 x 2304 x 768 4.97 and 3.05 us, 64 x 768 x 768 5.73 and 3.37,
-    // 64 x 3072 x 768 7.57 and 5.64, 64 x 768 x 3072 6.24 and 5.77, 64 x 4800 x 1600 11.8 and 11.6 (within a step of GPT-2 XL 13.8 and 11.5);
-    // 24 x 1600 x 6400 8.79 and 8.68, but 32 x 1600 x 6400 8.72 and 9.15, 64 x 50257 x 768 21.4 and 58.9.
-    if (forced_bn == 0 && M <= 64 && N < 16384 && (M <= 24 || K <= 4096)) return launch_narrow_plan(p, narrow_plan(M, N, K, sms), x, ldx, w, s);
+    const int narrow = forced_bn == 0 ? mllm_gemm_narrow_plan(M, N, K, sms) : 0;
+    if (narrow != 0) return launch_narrow_plan(p, narrow, x, ldx, w, s);
     // Which kernel: up to 64 tokens, behind the narrow tiles, the one with swapped operands.  It also takes products of up
     // to 512 tokens with a long K and few output features (the feed-forward's second product in
     // steps of prompt portions): there the persistent kernel is one chain of K / 64 dependent

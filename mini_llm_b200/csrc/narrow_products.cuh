@@ -173,10 +173,10 @@ int launch_narrow(const GemmParams& p, const bf16* x, long ldx, const bf16* w, c
 
 // How a product is split: tiles of 16 features a block, blocks that share K, and blocks that share the tokens, as
 // 100 * (blocks - 1) + 10 * tiles + blocks; the plan with the least expected time, in us.  Fitted to products of 12 to 64 tokens, 768 to
-// 6,400 features and 768 to 6,400 of K: a block's way in and out, its loop over K (x's way from L2, then the products), blocks that
+// 6,400 features and 768 to 6,400 of K, and its rounds of blocks: a block's way in and out, its loop over K (x's way from L2, then the products), blocks that
 // wait for others to end, a cluster's exchange, and the weights' way from HBM.
 static int narrow_token_tiles(int M) { return M <= 16 ? 2 : M <= 24 ? 3 : M <= 32 ? 4 : M <= 48 ? 6 : 8; }
-int narrow_plan(int M, int N, int K, int sms) {
+int narrow_plan(int M, int N, int K, int sms, int* rounds_of_plan) {
     int best = 11;
     double least = -1.0;
     for (int shares = 1; shares <= (M > 16 ? 2 : 1); shares++)
@@ -193,6 +193,7 @@ int narrow_plan(int M, int N, int K, int sms) {
                 if (least < 0.0 || cost < least) {
                     least = cost;
                     best = 100 * (shares - 1) + 10 * ft + splits;
+                    *rounds_of_plan = (int)waves;
                 }
             }
     return best;

@@ -1,0 +1,22 @@
+"""Which kernel a launcher takes, where the launcher decides by sizes alone (host code of the kernel libraries, no device)."""
+import ctypes
+
+import pytest
+
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def narrow_plan():
+    from mini_llm_b200.kernels import build
+    return ctypes.CDLL(build.library_path("gemm")).mllm_gemm_narrow_plan
+
+
+# measured (us, swapped tiles and narrow ones): the faster kernel is the one that runs
+@pytest.mark.parametrize("m, n, k, swapped, narrow", [
+    (24, 2304, 768, 5.0, 3.0), (64, 768, 768, 6.6, 3.4), (64, 3072, 768, 7.4, 5.4), (48, 6144, 1024, 9.8, 8.4), (24, 8192, 4096, 17.6, 15.4),
+    (64, 2304, 4096, 15.8, 10.9), (12, 16000, 768, 9.6, 8.6), (16, 1600, 8192, 10.3, 10.1), (24, 8192, 6400, 23.7, 22.9),
+    (32, 8192, 1024, 9.0, 9.7), (64, 4096, 2048, 10.1, 13.2), (64, 8192, 2048, 15.0, 24.4), (24, 12288, 1024, 10.6, 12.3),
+    (64, 12288, 4096, 28.6, 41.5), (32, 16000, 768, 9.8, 14.9), (24, 1600, 6400, 9.2, 10.7), (24, 1600, 11008, 12.2, 16.0), (64, 50257, 768, 21.4, 58.9)])
+def test_products_of_few_tokens_take_the_faster_tiles(narrow_plan, m, n, k, swapped, narrow):
+    assert (narrow_plan(m, n, k, SMS) != 0) == (narrow < swapped)

@@ -350,6 +350,19 @@ def test_narrow_products(m, n, k, epilogue):
     assert int(status) == 0
 
 
+# both sides of the line between narrow and swapped tiles: blocks that fit the SMs at once, a second round of them, a long K that blocks share or not
+@pytest.mark.parametrize("m, n, k", [(17, 9472, 64), (17, 9480, 64), (33, 7104, 72), (64, 4096, 2048), (64, 7120, 64), (24, 1600, 6400), (24, 4096, 6400), (16, 16376, 64)])
+def test_products_at_the_edge_of_the_narrow_tiles(m, n, k):
+    from mini_llm_b200.kernels import ops
+    rng = np.random.default_rng(m + n + k)
+    a, w = dev(rng.normal(size=(m, k)), torch.bfloat16), dev(rng.normal(size=(n, k)) / math.sqrt(k), torch.bfloat16)
+    status, out = torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((m + 1, n), 0.5, device="cuda")
+    ops.gemm_bf16(out[:m], a, w, None, "add", status)
+    # (as above: 6,400 terms whose sizes add up to 80)
+    np.testing.assert_allclose(f64(out)[:m], 0.5 + f64(a) @ f64(w).T, rtol=0, atol=1e-4)
+    assert bool((out[m] == 0.5).all()) and int(status) == 0
+
+
 # widths: a ring that holds all of K, rows whose end is no block of 32 of K, K shared by two and by four warps; tokens: of which nearly
 # every expert has one and hardly any, tiles of 8, 16 and 32 pairs, more than fit shared memory beside the weights
 @pytest.mark.parametrize("tokens, experts, top, inner, width", [(1, 24, 1, 40, 768), (2, 8, 2, 136, 776), (16, 3, 2, 264, 1000), (31, 2, 2, 72, 1032),
