@@ -2422,8 +2422,9 @@ __device__ __forceinline__ int pairs_of_expert(const int* choice, int n_pairs, i
 }
 
 // Whether the weights of all experts are asked for ahead of the wait, before their tokens are known: where the tokens choose half as many
-// experts as there are or more.  (What is read in vain costs less than the wait for what is not: the router's kernel runs meanwhile.  One
-// token of 8 experts, two and a shared one: 15.4 us behind the wait, 16.7 ahead; two: 18.4 and 17.7.)
+// experts as there are or more, a token's last pair not counted (where there is a shared expert it is that one's; where there is none, two tokens of 8
+// experts, two each, are the faster behind the wait, too: 15.5 us ahead and 14.3).  What is read in vain costs less than the wait for what is
+// not: the router's kernel runs meanwhile.  With a shared expert one token of 8, two each: 15.4 us behind the wait, 16.7 ahead; two: 18.4 and 17.7.
 __device__ __forceinline__ bool experts_ahead(int n_tokens, int pairs, int n_experts) {
     return n_tokens * (pairs > 1 ? pairs - 1 : 1) * 2 >= n_experts;
 }
@@ -2527,14 +2528,18 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
         ask(0, 0);
         ask(1, half);
     };
-    // the other kernel's weights come into L2 meanwhile, an expert's piece of a row at a time
+    // the other kernel's weights come into L2 meanwhile, an expert's piece of a row at a time (the launcher sees to width <= walkers; with a
+    // division to find each piece's expert, those without a token cost as much as those with one: one token of 60 experts 21.4 us, 18.5 so)
     auto down_ahead = [&](auto has) {
-        for (int i = walker; i < n_tables * width; i += walkers) {
-            const int e = i / width;
-            if (!has(e)) continue;
-            const char* row = reinterpret_cast<const char*>(down_here[e]) + (long)(i - e * width) * ld_down * 2;
-            const int bytes = inner_here[e] * 2;
-            for (int at = lane * 128; at < bytes; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + at));
+        int at_row = walker;
+        for (int e = 0; e < n_tables; e++) {
+            if (at_row < width && has(e)) {
+                const char* row = reinterpret_cast<const char*>(down_here[e]) + (long)at_row * ld_down * 2;
+                const int bytes = inner_here[e] * 2;
+                for (int at = lane * 128; at < bytes; at += 32 * 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + at));
+            }
+            at_row -= width;
+            if (at_row < 0) at_row += walkers;
         }
     };
     int part = walker, e = 0, f0 = 0;
@@ -2727,6 +2732,8 @@ expert_down_tiles_kernel(float* hidden, long ld_hidden, const bf16* act, long ld
         }
         copies_end();
     };
+    // (all experts may be more units than there is room for where the chosen ones are not: planning again for those behind the wait was slower, 24 experts
+    // of 768, 16 and 31 tokens 31.5 and 35.8 us so, 33.7 and 37.1 then)
     const bool early = experts_ahead(n_tokens, pairs, n_experts);
     if (early) {
         plan([](int) { return true; });

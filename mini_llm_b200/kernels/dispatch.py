@@ -184,17 +184,29 @@ class Kernels:
     def experts(self, hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
                 ld_down=None, assign=False, identity_weight=None, eights=False, features=0, **form):
         """``eights``: every expert's inner size is a multiple of 8; ``features``: inner features of all experts of a token.
-        Pair by pair a block has 32 features of a pair, and an expert's weights are read once a pair: as fast as the tiles, which
-        find every expert's pairs first, or faster, while those blocks fit the GPU at once (592, four an SM).  Only one or two
-        tokens, whose blocks are few, go through the tiles all the same.  A layer of 8 experts of 768, two and a shared one of
-        1,536 a token, at 1, 4, 7, 16 tokens: tiles 14.7, 18.3, 18.7, 20.8 us, pairs 20.5, 21.6, 25.9, 37.8; 16 experts of 512, two and a shared one of
-        512, at 3, 8, 13, 31: tiles 16.6, 20.6, 21.8, 27.0, pairs 16.9, 18.1, 24.7, 37.5."""
+        Pair by pair a block has 32 features of a pair, and an expert's weights are read once a pair; the tiles find every expert's pairs
+        first and read its weights once.  The line lies where the pairs' blocks no longer fit the GPU at once (592, four an SM), and one or
+        two tokens, whose blocks are few, take the tiles all the same.  Back to back, tiles and pairs: 16 experts of 512, two and a shared
+        one of 512 a token, 1, 2, 4, 8, 12, 13, 31 tokens 13.4 and 14.1 us, 14.2 and 15.4, 18.4 and 16.9, 19.8 and 18.5, 21.8 and 18.5, 20.8 and 25.0, 25.4
+        and 38.5; 8 of 2,048, two a token, 1, 4, 5, 16 tokens 17.1 and 24.3, 31.7 and 27.6, 33.6 and 36.7, 37.4 and 59.6.  (Where a shared expert has
+        half of a token's features the tiles are ahead on the pairs' side too: 8 of 768, two and a shared one of 1,536, 3 and 6 tokens 17.2 and
+        21.1, 17.9 and 20.8.)  Of many experts few tokens share none, and the tables cost the tiles time: 48 of 512, two a token, 1, 2, 24 tokens
+        15.4 and 9.1, 16.6 and 9.5, 43.4 and 32.1; 60 of 256, four a token, 1, 2, 20, 24 tokens 18.5 and 10.9, 20.0 and 12.5, 42.4 and 34.5, 43.3
+        and 37.8; 24 of 768, two a token, 1, 16, 31 tokens 13.6 and 9.6, 31.5 and 30.0, 35.8 and 40.4: more than 20 go pair by pair until there are
+        half as many pairs again as experts."""
         self.launches += 2
         tiles = (eights and not self.plain_only and ld_down is not None and ops.expert_tiles_take(x, act, inner_of.shape[0], ld_down)
-                 and (x.shape[0] <= 2 or x.shape[0] * features > 592 * 32))
+                 and self.experts_in_tiles(x.shape[0], inner_of.shape[0], pairs, features))
         self.chose("experts", "expert_tiles" if tiles else "expert_pairs", x.shape[0], max_inner, x.shape[1])
         return ops.experts(hidden, act, x, choice, in_weight, out_weight, gate_of, up_of, down_of, inner_of, max_inner, pairs,
                            ld_down, assign, identity_weight, tiles=tiles, **form)
+
+    @staticmethod
+    def experts_in_tiles(n_tokens, n_tables, pairs, features) -> bool:
+        """The line that ``experts`` gives the reasons for."""
+        if n_tables > 20 and 2 * n_tokens * pairs < 3 * n_tables:
+            return False
+        return n_tokens <= 2 or n_tokens * features > 592 * 32
 
     EXPERTS_AT_ONCE_TOKENS = 32    # from here on a step's tokens go through all experts as two products
 

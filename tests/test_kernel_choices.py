@@ -20,3 +20,13 @@ def narrow_plan():
     (64, 12288, 4096, 28.6, 41.5), (32, 16000, 768, 9.8, 14.9), (24, 1600, 6400, 9.2, 10.7), (24, 1600, 11008, 12.2, 16.0), (64, 50257, 768, 21.4, 58.9)])
 def test_products_of_few_tokens_take_the_faster_tiles(narrow_plan, m, n, k, swapped, narrow):
     assert (narrow_plan(m, n, k, SMS) != 0) == (narrow < swapped)
+
+
+# measured (us, in tiles and pair by pair): tokens, tables, pairs a token, features a token
+@pytest.mark.parametrize("tokens, tables, pairs, features, tiles, by_pairs", [
+    (1, 17, 3, 1536, 13.4, 14.1), (2, 17, 3, 1536, 14.2, 15.4), (8, 17, 3, 1536, 19.8, 18.5), (13, 17, 3, 1536, 20.8, 25.0), (1, 9, 3, 3072, 14.4, 20.9),
+    (16, 9, 3, 3072, 19.8, 38.5), (4, 8, 2, 4096, 31.7, 27.6), (5, 8, 2, 4096, 33.6, 36.7), (1, 24, 2, 1536, 13.6, 9.6), (31, 24, 2, 1536, 35.8, 40.4),
+    (1, 48, 2, 1024, 15.4, 9.1), (2, 48, 2, 1024, 16.6, 9.5), (24, 48, 2, 1024, 43.4, 32.1), (1, 60, 4, 1024, 18.5, 10.9), (20, 60, 4, 1024, 42.4, 34.5)])
+def test_experts_take_the_faster_kernels(tokens, tables, pairs, features, tiles, by_pairs):
+    from mini_llm_b200.kernels.dispatch import Kernels
+    assert Kernels.experts_in_tiles(tokens, tables, pairs, features) == (tiles < by_pairs)

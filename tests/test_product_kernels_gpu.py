@@ -400,6 +400,12 @@ def test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, ga
     assert np.abs(f64(hidden) - expected).max() <= 0.03
 
 
+# more units of all experts than there is room for, chosen by few tokens and by many; tables of nearly 64 experts, whose rows are all warps' or nearly so
+@pytest.mark.parametrize("tokens, experts, top, inner, width", [(13, 24, 2, 768, 768), (31, 24, 2, 768, 768), (2, 60, 4, 256, 1024), (20, 64, 4, 264, 1184)])
+def test_experts_of_more_units_than_there_is_room_for(tokens, experts, top, inner, width):
+    test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, True)
+
+
 @pytest.mark.parametrize("ints", [4, 1020, 4096, 4100, 70000])       # a piece, a thread's, a block's and all blocks' edges
 def test_control_block_from_the_ring(ints):
     from mini_llm_b200.kernels import ops
