@@ -175,7 +175,7 @@ class Kernels:
         self.launches += 1
         return ops.linear_recurrence(out, q, k, v, gate_a, gate_b, log_rate, step_bias, state, ctx.item_slot, ctx.item_offset,
                                      ctx.item_count, heads, qk_heads, dim, vdim, delta, unit_norm, q_scale, skip, writes,
-                                     channel_decay, ctx.steps_apart)
+                                     channel_decay, ctx.steps_apart and writes)      # (as in memory_scan)
 
     def route(self, x, router, shared_gate, top, choice, in_weight, out_weight, **how):
         self.launches += 1
@@ -318,7 +318,10 @@ class Kernels:
     def memory_scan(self, ctx, out, q, k, v, state, heads, dim, vdim, writes=True, **how):
         self.launches += 1
         # prompt portions go through the kernel that takes 32 tokens at a time; a step of single
-        # tokens walks each token's one update (the state is read and written once either way)
+        # tokens walks each token's one update (the state is read and written once either way), and asks for its states ahead of the
+        # wait (4 heads of 96 x 192, gated, between two products: 13.1 -> 11.9 us).  Long portions of key sizes that the chunks do not
+        # take walk behind the wait: launched early, a walk's blocks crowd on the SMs that have room (two of 1,000 tokens 1,411 us, 2,972
+        # early).  A state that this entry does not write is another one's, whose kernel may run still.
         chunked = not ctx.decode_only and ops.memory_chunk_takes(dim)
         passes = None
         if chunked and q.shape[0] >= self.MEMORY_PASSES_TOKENS:
@@ -332,7 +335,8 @@ class Kernels:
         self.chose("memory_scan", "memory_passes" if passes else ("memory_chunk" if chunked else "memory_scan"),
                    q.shape[0], heads, dim, vdim)
         return ops.memory_scan(out, q, k, v, state, ctx.item_slot, ctx.item_offset, ctx.item_count, heads, dim, vdim,
-                               writes=writes, chunked=chunked, passes=passes, state_ahead=ctx.steps_apart, **how)
+                               writes=writes, chunked=chunked, passes=passes,
+                               state_ahead=ctx.steps_apart and ctx.decode_only and writes, **how)
 
     MEMORY_PASSES_TOKENS = 128     # from here on a step's chunks are worth four launches
 

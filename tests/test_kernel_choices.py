@@ -1,7 +1,9 @@
 """Which kernel a launcher takes, where the launcher decides by sizes alone (host code of the kernel libraries, no device)."""
 import ctypes
+from types import SimpleNamespace
 
 import pytest
+import torch
 
 SMS = 148
 
@@ -30,3 +32,21 @@ def test_products_of_few_tokens_take_the_faster_tiles(narrow_plan, m, n, k, swap
 def test_experts_take_the_faster_kernels(tokens, tables, pairs, features, tiles, by_pairs):
     from mini_llm_b200.kernels.dispatch import Kernels
     assert Kernels.experts_in_tiles(tokens, tables, pairs, features) == (tiles < by_pairs)
+
+
+@pytest.mark.parametrize("steps_apart, decode_only, writes, ahead", [(True, True, True, True), (True, False, True, False), (True, True, False, False),
+                                                                     (False, True, True, False)])
+def test_states_are_read_ahead_of_the_wait_by_single_tokens_of_their_writer(monkeypatch, steps_apart, decode_only, writes, ahead):
+    """512 is a key size that the kernels for chunks do not take: portions walk token by token, as single tokens do."""
+    from mini_llm_b200.kernels import dispatch
+    from mini_llm_b200.kernels.dispatch import Kernels
+    seen = {}
+    monkeypatch.setattr(dispatch.ops, "memory_scan", lambda *a, state_ahead=None, **k: seen.update(memory=state_ahead, chunked=k["chunked"]))
+    monkeypatch.setattr(dispatch.ops, "linear_recurrence", lambda *a: seen.update(recurrence=a[-1]))
+    rows, ints = torch.zeros(3, 512), torch.zeros(3, dtype=torch.int32)
+    ctx = SimpleNamespace(steps_apart=steps_apart, decode_only=decode_only, n_items=3, item_slot=ints, item_offset=ints, item_count=ints, device=rows.device)
+    kernels = Kernels(torch.float32)
+    kernels.memory_scan(ctx, rows, rows, rows, rows, rows, 1, 512, 512, writes=writes, decay=rows[0, :1])
+    kernels.linear_recurrence(ctx, rows, rows, rows, rows, rows, rows, rows, rows, rows, 1, 1, 512, 512, True, True, 1.0, None, writes, False)
+    assert bool(seen["memory"]) == ahead and not seen["chunked"]
+    assert bool(seen["recurrence"]) == (steps_apart and writes)       # (only its kernel for few tokens an entry reads ahead)
