@@ -920,6 +920,7 @@ struct LatentTiledParams {
     const float* gate;             // [T, >= heads] (rows ld_gate apart) or null: head h's result times sigmoid(gate[t, h])
     long ld_gate;
     int rows_ahead;                // single tokens: of the cached rows only the tokens' own are written by kernels that may still run
+    int most_blocks;               // single tokens: blocks of a cluster (0: 16, or 8 where those are refused)
 };
 
 template <typename T> struct Chunk4;
@@ -1479,9 +1480,9 @@ latent_step_kernel(LatentTiledParams p) {
         ask(key_begin + KEYS, 1, position);
     }
     {
-        // the token's own row, if it lies in the first two tiles
+        // the token's own row, if it lies in the first two tiles (a block without keys begins behind it)
         const int j = position - key_begin;
-        if (position < key_end && j < 2 * KEYS && warp == 0) {
+        if (position < key_end && j >= 0 && j < 2 * KEYS && warp == 0) {
             const bf16* from = reinterpret_cast<const bf16*>(behind_the_wait(p.pages)) +
                                ((long)bt[position / p.page_size] * p.page_size + position % p.page_size) * row_width;
             for (int c = lane; c < pieces; c += 32) copy_16(tiles + j * ld + c * 8, from + c * 8, true);
@@ -1628,16 +1629,21 @@ static int latent_step_parts(int n_tokens) { return n_tokens <= 18 ? 16 : n_toke
 template <int RANK>
 static int launch_latent_step(const LatentTiledParams& p, int n_tokens, cudaStream_t s) {
     const size_t shared = LatentStep<RANK>::bytes(p.rank + p.rot);
-    // (at every launch, as the limits are a device's own)
-    if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess ||
-        cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-        return fail("latent_attention: the steps' shared memory or clusters were refused");
-    const int parts = latent_step_parts(n_tokens);
-    if (launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p) != cudaSuccess) {
+    // (at every launch, as the limit is a device's own)
+    if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared) != cudaSuccess)
+        return fail("latent_attention: the steps' shared memory was refused");
+    int parts = latent_step_parts(n_tokens);
+    if (p.most_blocks > 0 && parts > p.most_blocks) parts = p.most_blocks;
+    // every device takes clusters of up to 8 blocks; 16 need as many SMs side by side, of which a part of a device may not have enough
+    if (parts > 8) {
+        if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p) == cudaSuccess)
+            return check_launch("latent_step_kernel");
         cudaGetLastError();
-        return fail("latent_attention: the clusters of a step were refused");
+        parts = 8;
     }
-    return check_launch("latent_step_kernel");
+    return launched(launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p),
+                    "latent_step_kernel");
 }
 
 // The parts of a (token, head) into one result, in the order of the parts.
@@ -1712,6 +1718,8 @@ extern "C" int mllm_sequence_latent_attention_tiled(const LatentTiledParams* par
     const int rows = p.HB * p.TQ;
     if (p.HB <= 0 || p.TQ <= 0 || (rows != 32 && rows != 16) || 128 % p.TQ != 0) return fail("latent_attention_tiled: a block takes 32 or 16 rows");
     if (p.tiles == nullptr && p.TQ != 1) return fail("latent_attention_tiled: single tokens come one per block");
+    if (p.most_blocks != 0 && p.most_blocks != 1 && p.most_blocks != 2 && p.most_blocks != 4 && p.most_blocks != 8 && p.most_blocks != 16)
+        return fail("latent_attention_tiled: clusters are of 1, 2, 4, 8 or 16 blocks");
     if (p.parts < 1 || p.parts > 32 || (p.parts > 1 && (p.tiles != nullptr || p.part_out == nullptr || p.part_ml == nullptr)))
         return fail("latent_attention_tiled: parts are for single tokens and need scratch");
     if (latent_mma_takes(p, dtype))

@@ -1084,7 +1084,7 @@ class _LatentTiledParams(ctypes.Structure):
                 ("positions", P), ("token_item", P), ("tiles", P), ("max_blocks", I), ("page_size", I), ("n_tokens", I),
                 ("heads", I), ("rank", I), ("rot", I), ("TQ", I), ("HB", I), ("parts", I),
                 ("scale", F), ("out_bf16", I), ("key_buffers", I), ("window", I), ("gate", P), ("ld_gate", L),
-                ("rows_ahead", I)]
+                ("rows_ahead", I), ("most_blocks", I)]
 
 
 _latent_attention_tiled = Function("sequence", "mllm_sequence_latent_attention_tiled",
@@ -1109,14 +1109,15 @@ def latent_heads_per_block(heads: int) -> int:
 
 
 def latent_attention_tiled(out, q_eff, pages, block_table, positions, token_item, heads, rank, rot, page_size, scale,
-                           tiles=None, n_tiles=0, parts=1, scratch=None, window=0, gate=None, rows_ahead=False):
+                           tiles=None, n_tiles=0, parts=1, scratch=None, window=0, gate=None, rows_ahead=False, most_blocks=0):
     """``latent_attention_plain`` in tiles of 32 query rows that share their keys.  With ``tiles``
     (the step's work list, device int32 records of 8, ``n_tiles`` of them) for prompt portions;
     without, for single tokens, the keys of each in ``parts`` runs (the token's context length over
     ``parts``, in whole blocks of 32) whose results are merged (``scratch``: fp32 (T * heads * parts * rank, T * heads * parts * 2)).
     ``out`` may be bfloat16: the sums are 32-bit either way, the result is rounded once.  ``gate`` as in the plain form.
     Single tokens of up to 16 heads over bfloat16 rows with a latent of 128 or 256 go to a kernel that merges the parts itself (their
-    number is its own); ``rows_ahead``: kernels that may still run write no cached row but the tokens' own."""
+    number is its own); ``rows_ahead``: kernels that may still run write no cached row but the tokens' own; ``most_blocks``: of a token at
+    most so many blocks share the rows (0: as many as are worth it and the device takes)."""
     _check(out, "latent_attention.out", None, 2)
     if out.dtype not in (torch.float32, torch.bfloat16):
         raise KernelError("latent_attention_tiled: out must be float32 or bfloat16")
@@ -1138,7 +1139,7 @@ def latent_attention_tiled(out, q_eff, pages, block_table, positions, token_item
     params.window = int(window or 0)           # (> 0: a query sees the last ``window`` positions only)
     _check_gate(gate, n, heads, "latent_attention")
     params.gate, params.ld_gate = _ptr(gate), gate.stride(0) if gate is not None else 0
-    params.rows_ahead = int(bool(rows_ahead))
+    params.rows_ahead, params.most_blocks = int(bool(rows_ahead)), int(most_blocks)
     if tiles is not None:
         _check(tiles, "latent_attention.tiles", torch.int32)
         if tiles.numel() < ATTENTION_TILE_RECORD * n_tiles or parts != 1:

@@ -445,7 +445,7 @@ def test_an_emptied_slot_and_draws_on_the_host():
 @pytest.mark.parametrize("tokens, heads, rank, rot, window", [(1, 12, 256, 32, 0), (3, 16, 256, 64, 70), (5, 3, 128, 0, 0), (19, 5, 128, 48, 0), (40, 12, 256, 32, 33), (90, 2, 128, 16, 0),
                                                               (150, 1, 128, 32, 200)])
 @pytest.mark.parametrize("ahead", [True, False])
-def test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, ahead):
+def test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, ahead, most_blocks=0):
     from mini_llm_b200.kernels import ops
     rng = np.random.default_rng(tokens + rank)
     page, row = 16, rank + rot
@@ -462,7 +462,7 @@ def test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, ahe
     common = (q, pages, dev(table, torch.int32), dev(np.array(lengths) - 1, torch.int32), dev(np.arange(tokens), torch.int32), heads, rank, rot, page, 0.1)
     got = torch.full((tokens, heads * rank), math.nan, device="cuda")
     scratch = (torch.empty(tokens * heads * 2 * rank, device="cuda"), torch.empty(tokens * heads * 4, device="cuda"))
-    ops.latent_attention_tiled(got, *common, parts=2, scratch=scratch, window=window, gate=gate, rows_ahead=ahead)
+    ops.latent_attention_tiled(got, *common, parts=2, scratch=scratch, window=window, gate=gate, rows_ahead=ahead, most_blocks=most_blocks)
     for i, n in enumerate(lengths):
         rows = f64(pages[table[i, :blocks[i]]]).reshape(-1, row)[max(0, n - window) if window else 0:n]
         s = f64(q)[i].reshape(heads, row) @ rows.T * 0.1
@@ -470,3 +470,11 @@ def test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, ahe
         want = w / w.sum(axis=1, keepdims=True) @ rows[:, :rank] / (1.0 + np.exp(-f64(gate)[i]))[:, None]
         # queries and weights keep all 24 bits and sums are 32-bit: scores of up to 8 off by some 2^-21, weights by as much
         np.testing.assert_allclose(f64(got)[i].reshape(heads, rank), want, rtol=2e-5, atol=1e-5)
+
+
+# clusters smaller than the launcher would take (on a part of a device that refuses 16 blocks they are of 8); rows of more than 320 entries, of which one
+# block fits an SM, and the widest ones
+@pytest.mark.parametrize("tokens, heads, rank, rot, window, most_blocks", [(3, 12, 256, 32, 0, 8), (5, 7, 128, 16, 40, 4), (2, 16, 256, 32, 0, 2), (2, 3, 128, 0, 0, 1),
+                                                                           (3, 12, 256, 80, 0, 0), (2, 16, 128, 384, 0, 0), (20, 16, 256, 256, 90, 0), (80, 4, 256, 112, 0, 0)])
+def test_latent_attention_of_single_tokens_in_other_clusters(tokens, heads, rank, rot, window, most_blocks):
+    test_latent_attention_of_single_tokens(tokens, heads, rank, rot, window, True, most_blocks)
