@@ -1616,10 +1616,10 @@ latent_step_kernel(LatentTiledParams p) {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-static bool latent_step_takes(const LatentTiledParams& p, int dtype) {
-    const int row_width = p.rank + p.rot;
-    return dtype == DT_BF16 && p.tiles == nullptr && p.heads <= 16 && (p.rank == 128 || p.rank == 256) && row_width % 16 == 0 && row_width <= 512 &&
-           (reinterpret_cast<uintptr_t>(p.pages) & 15) == 0 && (reinterpret_cast<uintptr_t>(p.q_eff) & 15) == 0;
+extern "C" int mllm_sequence_latent_step_takes(int dtype, int heads, int rank, int rot, const void* pages, const float* q_eff) {
+    const int row_width = rank + rot;
+    return dtype == DT_BF16 && heads <= 16 && (rank == 128 || rank == 256) && row_width % 16 == 0 && row_width <= 512 &&
+           (reinterpret_cast<uintptr_t>(pages) & 15) == 0 && (reinterpret_cast<uintptr_t>(q_eff) & 15) == 0;
 }
 
 // Blocks that share a token's rows: 16 while no more than two come to an SM (17 tokens of up to 981 rows, heads of 128: 14.6 us with 8,
@@ -1724,7 +1724,7 @@ extern "C" int mllm_sequence_latent_attention_tiled(const LatentTiledParams* par
         return fail("latent_attention_tiled: parts are for single tokens and need scratch");
     if (latent_mma_takes(p, dtype))
         return p.rank == 128 ? launch_latent_mma<128>(p, n_units, (cudaStream_t)stream) : launch_latent_mma<256>(p, n_units, (cudaStream_t)stream);
-    if (latent_step_takes(p, dtype))
+    if (p.tiles == nullptr && mllm_sequence_latent_step_takes(dtype, p.heads, p.rank, p.rot, p.pages, p.q_eff))
         return p.rank == 128 ? launch_latent_step<128>(p, n_units, (cudaStream_t)stream) : launch_latent_step<256>(p, n_units, (cudaStream_t)stream);
     const int element_bytes = dtype == DT_F32 ? 4 : 2;
     // prompt portions take 64 keys a block where two such blocks, or one, fit beside the queries

@@ -298,6 +298,9 @@ class Kernels:
                 # prompt portions: 32 rows (tokens x heads) a block share every cached row they read
                 self.chose("latent_attention", "latent_attention_tiled", n, heads, rank + rot)
                 return ops.latent_attention_tiled(*common, tiles=ctx.att_tiles, n_tiles=ctx.n_att_tiles, window=window, gate=gate)
+            if ctx.decode_only and ops.latent_step_takes(q_eff, cache.k_pages, heads, rank, rot):
+                self.chose("latent_attention", "latent_step", n, heads, rank + rot)
+                return ops.latent_attention_tiled(*common, window=window, gate=gate, rows_ahead=ctx.steps_apart)
             if ctx.decode_only:
                 # single tokens: all heads of a token share the cached rows; while the (token, head
                 # block) pairs are fewer than twice the SMs, each token's keys come in parts
@@ -306,7 +309,7 @@ class Kernels:
                 scratch = self._latent_scratch(ctx.device, n * heads * parts * rank, n * heads * parts * 2) if parts > 1 else None
                 self.launches += 1 if parts > 1 else 0
                 self.chose("latent_attention", "latent_attention_tiled_parts", n, heads, rank + rot)
-                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate, rows_ahead=ctx.steps_apart)
+                return ops.latent_attention_tiled(*common, parts=parts, scratch=scratch, window=window, gate=gate)
         self.chose("latent_attention", "latent_attention_plain", n, heads, rank + rot)
         plain_out = out if out.dtype == torch.float32 else ctx.buffer("latent_mixed_32", out.shape, torch.float32)
         ops.latent_attention_plain(plain_out, q_eff, cache.k_pages, cache.block_table, ctx.positions, ctx.token_item,

@@ -78,6 +78,12 @@ class Function:
         self._err = getattr(lib, f"mllm_{self.library}_last_error")
         self._fn = fn
 
+    def value(self, *args) -> int:
+        """What the function returns, for one that answers a question instead of launching."""
+        if self._fn is None:
+            self._resolve()
+        return self._fn(*args)
+
     def __call__(self, *args):
         if self._fn is None:
             self._resolve()

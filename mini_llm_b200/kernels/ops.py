@@ -1100,6 +1100,15 @@ def latent_attention_tiled_takes(pages, rank, rot) -> bool:
     return row % 4 == 0 and rank % 8 == 0 and rank <= 1024 and shared <= 220 * 1024
 
 
+_latent_step_takes = Function("sequence", "mllm_sequence_latent_step_takes", [I, I, I, I, P, P])
+
+
+def latent_step_takes(q_eff, pages, heads, rank, rot) -> bool:
+    """Whether ``latent_attention_tiled`` takes single tokens of these sizes with the kernel that merges a token's parts itself (the
+    launcher's own question); it wants no scratch and is one launch."""
+    return bool(_latent_step_takes.value(dtype_code(pages.dtype), heads, rank, rot, pages.data_ptr(), q_eff.data_ptr()))
+
+
 def latent_heads_per_block(heads: int) -> int:
     """Heads of one block of 32 rows in prompt portions: the power of two (32 at most) that leaves
     the fewest rows for heads that do not exist, the larger one on a tie; the block then takes

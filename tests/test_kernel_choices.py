@@ -50,3 +50,20 @@ def test_states_are_read_ahead_of_the_wait_by_single_tokens_of_their_writer(monk
     kernels.linear_recurrence(ctx, rows, rows, rows, rows, rows, rows, rows, rows, rows, 1, 1, 512, 512, True, True, 1.0, None, writes, False)
     assert bool(seen["memory"]) == ahead and not seen["chunked"]
     assert bool(seen["recurrence"]) == (steps_apart and writes)       # (only its kernel for few tokens an entry reads ahead)
+
+
+@pytest.mark.parametrize("heads, rank, dtype, step", [(12, 256, torch.bfloat16, True), (16, 128, torch.bfloat16, True), (17, 256, torch.bfloat16, False),
+                                                      (4, 64, torch.bfloat16, False), (4, 128, torch.float32, False)])
+def test_single_tokens_over_a_latent_are_one_launch_where_the_kernel_merges_itself(monkeypatch, heads, rank, dtype, step):
+    from mini_llm_b200.kernels import dispatch
+    from mini_llm_b200.kernels.dispatch import Kernels
+    seen, rot, ints = {}, 32, torch.zeros(2, dtype=torch.int32)
+    monkeypatch.setattr(dispatch.ops, "latent_attention_tiled", lambda *a, **k: seen.update(k))
+    pages, q = torch.zeros(4, 16, 1, rank + rot, dtype=dtype), torch.zeros(2, heads * (rank + rot))
+    ctx = SimpleNamespace(steps_apart=True, decode_only=True, att_tiles=None, positions=ints, token_item=ints, device=q.device)
+    cache = SimpleNamespace(k_pages=pages, block_table=ints.view(1, 2), page_size=16)
+    kernels = Kernels(torch.bfloat16)
+    kernels.latent_attention(ctx, torch.zeros(2, heads * rank), q, cache, heads, rank, rot, 0.1)
+    assert kernels.launches == (1 if step else 2) and kernels.scratch_generation == (0 if step else 1)
+    assert ("scratch" in seen) != step and seen.get("rows_ahead", False) == step
+    assert {kernel for kernel in kernels.choices.values()} == {"latent_step" if step else "latent_attention_tiled_parts"}
