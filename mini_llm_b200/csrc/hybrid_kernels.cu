@@ -2464,17 +2464,16 @@ __device__ __forceinline__ int expert_of_part(const int* first_part, int n_table
 
 // A warp: eight inner features of an expert with a gate (16 without): its tile's 16 rows are the gates and the ups of the same features,
 // so that a lane holds both of a result; the tile's columns are pairs, eight at a time.  The weights lie in a ring of the lane's own
-// in shared memory (`depth` blocks of 32 of K: all of them at a width of 768), the tokens beside them where they fit.
+// in shared memory (`depth` blocks of 32 of K: all of them at a width of 768), the tokens beside them.
 constexpr int EXPERT_UP_WARPS = 8, EXPERT_UP_SHARED = 224 * 1024, EXPERT_UP_BLOCK = EXPERT_UP_WARPS * 2 * 32 * 16;     // (bytes of a block of 32 of K)
 constexpr int EXPERT_UP_STATIC = (EXPERT_UP_WARPS * 32 + EXPERT_TABLES + 1) * 4 + EXPERT_TABLES * 28 + 64;
 
-template <int FORM, bool HELD>         // HELD: the tokens are copied into shared memory
+template <int FORM>
 __global__ void __launch_bounds__(EXPERT_UP_WARPS * 32, 1)
 expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long ld_x, const int* choice, const float* in_weight,
                        const long long* __restrict__ gate_of, const long long* __restrict__ up_of, const long long* __restrict__ down_of,
                        const int* __restrict__ inner_of, int n_tables, long ld_down, int width, int pairs, int n_tokens, float limit,
                        float shared_limit, float alpha, int n_experts, int depth) {
-    const int held_tokens = HELD ? n_tokens : 0;
     constexpr bool GATED = FORM != EXPERT_RELU_SQUARED;
     constexpr int FEATURES = GATED ? 8 : 16, THREADS = EXPERT_UP_WARPS * 32;
     __shared__ int lists[EXPERT_UP_WARPS][32], first_part[EXPERT_TABLES + 1], inner_here[EXPERT_TABLES];
@@ -2484,7 +2483,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
     const int n_pairs = n_tokens * pairs, pieces = width / 8, all = (width + 31) / 32;
     const int ld_held = width * 2 + (width % 64 == 0 ? 64 : 16);              // bytes: neighbouring rows in other banks
     unsigned char* held = up_shared + (size_t)depth * EXPERT_UP_BLOCK;
-    int* chosen = reinterpret_cast<int*>(held + (size_t)held_tokens * ld_held);
+    int* chosen = reinterpret_cast<int*>(held + (size_t)n_tokens * ld_held);
     float* scales = reinterpret_cast<float*>(chosen + n_pairs);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int half = depth / 2;
@@ -2551,7 +2550,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
     choice = behind_the_wait(choice);
     x = behind_the_wait(x);
     in_weight = behind_the_wait(in_weight);
-    for (int t = warp; t < held_tokens; t += EXPERT_UP_WARPS)
+    for (int t = warp; t < n_tokens; t += EXPERT_UP_WARPS)
         for (int c = lane; c < pieces; c += 32) copy_16(held + (size_t)t * ld_held + c * 16, x + (long)t * ld_x + c * 8, true);
     copies_end();
     for (int i = threadIdx.x; i < n_pairs; i += THREADS) {
@@ -2584,7 +2583,7 @@ expert_up_tiles_kernel(bf16* __restrict__ act, long ld_act, const bf16* x, long 
         for (int t = 0; t < TILES; t++) {
             // (a column without a pair repeats the first one's and is not stored)
             const int pair = list[t * 8 + g < here ? t * 8 + g : 0], token = pair / pairs;
-            row[t] = HELD ? held + (size_t)token * ld_held : reinterpret_cast<const unsigned char*>(x + (long)token * ld_x);
+            row[t] = held + (size_t)token * ld_held;
             scale[t] = scales[pair];
             scaled |= scale[t] != 1.0f;
         }
@@ -3237,7 +3236,11 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
         if (n_pairs > 16384) return fail("experts: too many pairs for the tiles");
         const bf16* xb = (const bf16*)x;
         bf16* ab = (bf16*)act;
-        if ((width + 7) / 8 > sm_count()) {
+        // the first kernel's shared memory: the tokens, the pairs' choices and weights, and as much again or more for the ring of weights
+        const size_t room = EXPERT_UP_SHARED - EXPERT_UP_STATIC;
+        const size_t beside = n_pairs * 8 + (size_t)n_tokens * (width * 2 + (width % 64 == 0 ? 64 : 16));
+        // (widths of two rounds of the second kernel's blocks, and tokens of more than some 150 pairs)
+        if ((width + 7) / 8 > sm_count() || beside > room / 2) {
             const dim3 tiles((max_inner + 15) / 16, n_tables);
 #define UP_BLOCKS(FORM)                                                                                                          \
     launch_kernel(g_dependent_launch != 0, expert_up_blocks_kernel<FORM>, tiles, dim3(256), 0, s, ab, ld_act, xb, ld_x, choice, in_weight, \
@@ -3254,35 +3257,24 @@ extern "C" int mllm_hybrid_experts(float* hidden, long ld_hidden, void* act, lon
                           out_weight, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, assign, xb, ld_x, identity_weight);
             return check_launch("expert blocks");
         }
-        // the first kernel's shared memory: the pairs' choices and weights, then the tokens if they leave half of it, then the ring of weights
-        const size_t room = EXPERT_UP_SHARED - EXPERT_UP_STATIC, chosen_bytes = n_pairs * 8;
-        const size_t token_bytes = (size_t)n_tokens * (width * 2 + (width % 64 == 0 ? 64 : 16));
-        const int held_tokens = chosen_bytes + token_bytes <= room / 2 ? n_tokens : 0;
-        const size_t beside = chosen_bytes + (held_tokens > 0 ? token_bytes : 0);
         int depth = (int)((room - beside) / EXPERT_UP_BLOCK) / 2 * 2;
         const int blocks_of_k = (width + 31) / 32;
         if (depth > (blocks_of_k + 1) / 2 * 2) depth = (blocks_of_k + 1) / 2 * 2;
         const size_t up_bytes = (size_t)depth * EXPERT_UP_BLOCK + beside;
         const dim3 walkers(sm_count());
         // (the limits at every launch, as they are a device's own)
-#define UP_TILES_AS(FORM, HELD)                                                                                                  \
+#define UP_TILES(FORM)                                                                                                           \
     do {                                                                                                                         \
-        if (cudaFuncSetAttribute(expert_up_tiles_kernel<FORM, HELD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess) \
+        if (cudaFuncSetAttribute(expert_up_tiles_kernel<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room) != cudaSuccess) \
             return fail("experts: cannot raise the shared memory limit");                                                        \
-        launch_kernel(g_dependent_launch != 0, expert_up_tiles_kernel<FORM, HELD>, walkers, dim3(EXPERT_UP_WARPS * 32), up_bytes, s, ab, ld_act, xb, ld_x, \
+        launch_kernel(g_dependent_launch != 0, expert_up_tiles_kernel<FORM>, walkers, dim3(EXPERT_UP_WARPS * 32), up_bytes, s, ab, ld_act, xb, ld_x, \
                       choice, in_weight, gate_of, up_of, down_of, inner_of, n_tables, ld_down, width, pairs, n_tokens, limit, shared_limit, alpha, \
-                      n_experts, depth);                                                                                       \
-    } while (0)
-#define UP_TILES(FORM)                                  \
-    do {                                                \
-        if (held_tokens > 0) UP_TILES_AS(FORM, true);   \
-        else UP_TILES_AS(FORM, false);                  \
+                      n_experts, depth);                                                                                         \
     } while (0)
         if (form == EXPERT_GATED_SILU) UP_TILES(EXPERT_GATED_SILU);
         else if (form == EXPERT_RELU_SQUARED) UP_TILES(EXPERT_RELU_SQUARED);
         else UP_TILES(EXPERT_CLAMPED_GLU);
 #undef UP_TILES
-#undef UP_TILES_AS
         if (cudaFuncSetAttribute(expert_down_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)EXPERT_DOWN_SHARED) != cudaSuccess)
             return fail("experts: cannot raise the shared memory limit");
         // the second kernel's: the sums, the pairs' places, and as far as they fit the weights that are asked for ahead and the pairs' choices

@@ -363,8 +363,8 @@ def test_products_at_the_edge_of_the_narrow_tiles(m, n, k):
     assert bool((out[m] == 0.5).all()) and int(status) == 0
 
 
-# widths: a ring that holds all of K, rows whose end is no block of 32 of K, K shared by two and by four warps; tokens: of which nearly
-# every expert has one and hardly any, tiles of 8, 16 and 32 pairs, more than fit shared memory beside the weights
+# widths: a ring that holds all of K, rows whose end is no block of 32 of K, rows of two rounds of the second kernel's blocks, which other kernels
+# take; tokens: of which nearly every expert has one and hardly any, tiles of 8, 16 and 32 pairs
 @pytest.mark.parametrize("tokens, experts, top, inner, width", [(1, 24, 1, 40, 768), (2, 8, 2, 136, 776), (16, 3, 2, 264, 1000), (31, 2, 2, 72, 1032),
                                                                 (9, 4, 2, 80, 2056), (31, 5, 1, 48, 4096), (3, 40, 2, 64, 2048)])
 @pytest.mark.parametrize("gated", [True, False])
@@ -404,6 +404,28 @@ def test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, ga
 @pytest.mark.parametrize("tokens, experts, top, inner, width", [(13, 24, 2, 768, 768), (31, 24, 2, 768, 768), (2, 60, 4, 256, 1024), (20, 64, 4, 264, 1184)])
 def test_experts_of_more_units_than_there_is_room_for(tokens, experts, top, inner, width):
     test_experts_in_tiles_of_other_widths(tokens, experts, top, inner, width, True)
+
+
+# tokens that name their experts again and again, on both sides of what shared memory holds beside the weights
+@pytest.mark.parametrize("top, width", [(150, 1184), (160, 1184)])
+def test_experts_named_by_a_token_many_times(top, width):
+    from mini_llm_b200.kernels import ops
+    tokens, experts, inner = 31, 40, 16
+    rng = np.random.default_rng(top)
+    ups, downs = (dev(rng.normal(size=shape) / math.sqrt(shape[1]), torch.bfloat16) for shape in ((experts * inner, width), (width, experts * inner)))
+    x = dev(rng.normal(size=(tokens, width)), torch.bfloat16)
+    chosen = rng.integers(0, experts, size=(tokens, top)).astype(np.int32)
+    weights = rng.uniform(0.5, 1.5, size=(tokens, top)).astype(np.float32)
+    table = lambda matrix, step: torch.tensor([matrix.data_ptr() + 2 * e * step for e in range(experts)], dtype=torch.int64, device="cuda")
+    act, hidden = torch.full((tokens * top, inner), math.nan, dtype=torch.bfloat16, device="cuda"), dev(rng.normal(size=(tokens, width)), torch.float32)
+    rows = f64(dev(np.maximum(f64(x) @ f64(ups).T, 0.0) ** 2, torch.bfloat16))
+    of_pairs = np.zeros((tokens, experts))
+    np.add.at(of_pairs, (np.arange(tokens)[:, None], chosen), weights)
+    expected = f64(hidden) + (rows * np.repeat(of_pairs, inner, axis=1)) @ f64(downs).T
+    ops.experts(hidden, act, x, dev(chosen.reshape(-1)), dev(np.ones(tokens * top), torch.float32), dev(weights.reshape(-1), torch.float32), None,
+                table(ups, inner * width), table(downs, inner), dev(np.full(experts, inner, np.int32)), inner, top, ld_down=experts * inner, tiles=True, n_experts=experts)
+    # (as above: activations rounded to 8 bits, some the other way)
+    assert np.linalg.norm(f64(hidden) - expected) <= 1e-3 * np.linalg.norm(expected)
 
 
 @pytest.mark.parametrize("ints", [4, 1020, 4096, 4100, 70000])       # a piece, a thread's, a block's and all blocks' edges
