@@ -126,11 +126,23 @@ __device__ __forceinline__ void mma_bf16_16816(float& c0, float& c1, float& c2, 
 // on the stream still runs: its CTAs take the SMs that the earlier kernel's CTAs leave, set up
 // what needs no memory of the step (barriers, tensor memory, index arithmetic) and then wait
 // in wait_for_earlier_kernels(), which returns when every earlier kernel has completed and its
-// writes are visible.  No thread reads or writes global memory that another kernel of the
-// stream touches before it has passed that wait.  A kernel says with dependents_may_start(),
-// at its start, that the next one may be scheduled as soon as all of its own CTAs run.  Both
-// calls do nothing in a kernel that was launched the ordinary way, and stream capture keeps the
-// dependency as an edge of the graph.
+// writes are visible.  A kernel says with dependents_may_start(), at its start, that the next one
+// may be scheduled as soon as all of its own CTAs run.  Both calls do nothing in a kernel that was
+// launched the ordinary way, and stream capture keeps the dependency as an edge of the graph.
+//
+// Before it has passed that wait no thread writes global memory, and none reads what another
+// kernel of the same step writes.  What it may read there:
+//   - weights and what lies beside them, which no kernel writes;
+//   - the step's arrays (positions, block tables, entries, work lists), which a step's first kernel
+//     brings, but for the token ids, which resolve_tokens may write;
+//   - where its caller says so (first_new, rows_ahead, state_ahead): cached rows of positions before an
+//     entry's first new one, and the state that this kernel alone writes.  (A state that another kernel
+//     of the step writes is not read ahead, whatever its caller knows about the steps.)
+// The last two hold because steps are apart: control_kernel, which brings the arrays, waits for all
+// kernels ahead and lets no dependents start, and the kernel behind it (resolve_tokens or an embedding)
+// is launched AFTER_THE_KERNELS_AHEAD, so that everything behind that one runs when the arrays are there
+// and every earlier step has ended.  An embedding whose first kernel is launched as a dependent must
+// not say `begins_apart` (parts/base.py): the engine then puts resolve_tokens before it.
 __device__ __forceinline__ void dependents_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_earlier_kernels() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -147,8 +159,8 @@ template <typename T> __device__ __forceinline__ T* behind_the_wait(T* p) {
 // A kernel of few long blocks is launched the second way: as a dependent its blocks go to whatever SMs have room while other
 // kernels' waiting blocks hold the rest, several to an SM, and stay there (per launch within a replayed step, early against
 // not: a gated delta rule over two prompts of 1,000 tokens 680 against 513 us, latent attention of one token in 32 parts 23.5 against
-// 12.4, a 32-bit product of 240 x 768 x 768 73 against 41).  A step's first kernels are, too: those behind them may read the step's
-// arrays, which the very first one brings, ahead of their waits.
+// 12.4, a 32-bit product of 240 x 768 x 768 73 against 41).  So is the kernel behind the one that brings a step's
+// arrays (see above).
 constexpr bool AFTER_THE_KERNELS_AHEAD = false;
 
 // (cluster: the CTAs of a thread block cluster, or x = 0 for a launch without clusters)

@@ -260,6 +260,8 @@ class StepContext:
         self.next_norm = None         # the norm that reads the stream first in the next run entry, where it is known
         self.normed_ahead = None      # (that norm, its rows) once a pass over the stream has applied it
         self.streams_pending = None   # a layer's last write onto the streams, waiting to go with the next read-out
+        self.in_ring = False          # the step's arrays come from the ring of control blocks, by the step's first kernel
+        self.turn = None              # device int32 [1]: the step's number modulo two, where its draws go on the host
         self.steps_apart = False      # no kernel of an earlier step still runs when this step's kernels start, but for its first one: what
                                       # earlier steps left (cached rows, states) may be read ahead of the wait for the kernels ahead
         self.decode_only = False      # every entry brings exactly one token

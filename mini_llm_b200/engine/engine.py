@@ -101,8 +101,7 @@ class Engine:
         self.workspace = Workspace(self.device, min_rows=min(self.max_tokens_per_step, 256))
         self.control = ControlBlock(self.device, self.cache.groups)
         self.ctx = StepContext(self.kernels, self.workspace, self.dtype, self.device)
-        # (a step's first kernel is launched behind the step before, and the second one behind the first)
-        self.ctx.steps_apart = True
+        self.ctx.steps_apart = True           # (see ``_forward_on_stream``)
         self.steps = 0
         self._sampled = None
         self.kept_tokens = torch.zeros(self.max_requests, dtype=torch.int32, device=self.device)
@@ -465,9 +464,11 @@ class Engine:
             return self._forward_on_stream(ctx, sample_views)
 
     def _forward_on_stream(self, ctx, sample_views):
+        # ``take`` waits for the step before and lets nothing start early; behind it comes a kernel that starts when it has ended
+        # (and that leaves ids as they are where there is none to resolve): what follows finds every earlier step ended.
         if ctx.in_ring:
             self.control.take()
-        if ctx.any_previous:
+        if ctx.any_previous or not self.model.begins_apart:
             self.kernels.resolve_tokens(ctx.token_ids, self.kept_tokens)
         logits = self.model.forward(ctx, self.storage.views)
         self._sampled = None

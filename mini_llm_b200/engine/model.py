@@ -37,6 +37,8 @@ class Model:
         # A step may be captured into a CUDA graph only if every part launches nothing but
         # kernels whose arguments stay valid from step to step; parts say so themselves.
         self.graph_safe = all(getattr(part, "graph_safe", False) for part in self.parts())
+        # (an embedding that is no ``Embedding`` says nothing)
+        self.begins_apart = getattr(type(self.embedding), "forward_begins_apart", lambda: False)()
         # The step makes a work list of attention tiles only if some part says it reads one.
         self.wants_attention_tiles = any(getattr(part, "wants_attention_tiles", False) for part in self.parts())
         # A step of long portions may bring its work list as units of 256 tokens instead, if

@@ -104,6 +104,16 @@ class PositionEncoding(Part):
 
 
 class Embedding(Part):
+    # Whether the first kernel that ``forward`` launches starts only when every kernel ahead of it has ended (is not launched as
+    # a dependent).  Kernels behind it read the step's arrays and what earlier steps left early, so an engine puts
+    # such a kernel before an embedding that does not say so.  Said by the class that defines ``forward``, for its own one.
+    begins_apart = False
+
+    @classmethod
+    def forward_begins_apart(cls) -> bool:
+        owner = next(c for c in cls.__mro__ if "forward" in vars(c))
+        return bool(vars(owner).get("begins_apart", False))
+
     def cache_need(self):
         return NoCache()
 

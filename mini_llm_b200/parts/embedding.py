@@ -19,6 +19,8 @@ from .spec import FixedState, WeightSpec
 
 class TokenEmbedding(Embedding):
     graph_safe = True
+    begins_apart = True
+
     def __init__(self, prefix, vocab_size: int, width: int, name: str = "wte.weight", scale: float = 1.0):
         super().__init__(prefix)
         self.vocab_size, self.width, self.name, self.scale = int(vocab_size), int(width), name, float(scale)
@@ -39,6 +41,8 @@ class PairedTokenEmbedding(TokenEmbedding):
     """The token's row plus a row for the pair of it and the token before it: row
     ``(previous * mul_prev + token * mul_cur) mod buckets`` of a table of ``buckets + 1`` rows, the last of which is for a
     sequence's first token.  A request's last token is its state."""
+
+    begins_apart = True
 
     def __init__(self, prefix, vocab_size: int, width: int, buckets: int, mul_prev: int, mul_cur: int, name: str = "wte.weight",
                  pair_name: str = "bigram", scale: float = 1.0):

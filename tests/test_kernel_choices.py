@@ -67,3 +67,18 @@ def test_single_tokens_over_a_latent_are_one_launch_where_the_kernel_merges_itse
     assert kernels.launches == (1 if step else 2) and kernels.scratch_generation == (0 if step else 1)
     assert ("scratch" in seen) != step and seen.get("rows_ahead", False) == step
     assert {kernel for kernel in kernels.choices.values()} == {"latent_step" if step else "latent_attention_tiled_parts"}
+
+
+def test_an_embedding_with_a_forward_of_its_own_says_itself_how_it_begins():
+    from mini_llm_b200.parts.base import Embedding
+    from mini_llm_b200.parts.embedding import PairedTokenEmbedding, TokenEmbedding
+
+    class Other(TokenEmbedding):
+        def forward(self, ctx, position=None, cache=None):
+            raise NotImplementedError
+
+    class Same(TokenEmbedding):
+        pass
+
+    assert TokenEmbedding.forward_begins_apart() and PairedTokenEmbedding.forward_begins_apart() and Same.forward_begins_apart()
+    assert not Other.forward_begins_apart() and not Embedding.forward_begins_apart()
