@@ -2397,8 +2397,8 @@ expert_down_kernel(float* __restrict__ hidden, long ld_hidden, const T* __restri
 // cores', every product added by a rounded addition.  What bounds the two kernels are the weights' way from HBM (35 MB at 8 experts of 768 and a shared one of
 // 1,536 with a width of 768: 5.4 us) and the chain of choice, lists, operands and sums behind the router.  So all of a block's
 // weights are asked for at once, ahead of the wait for the kernels ahead where the tokens choose half as many experts as there are, and the
-// first kernel's idle lanes bring the second one's into L2.  Both kernels, 1, 2, 7, 16, 31 tokens of such experts, replayed back to back:
-// 14.7, 17.7, 18.8, 20.8, 26.5 us (16.0, 21.2, 24.8, 26.9, 34.2 by the kernels for wide rows below); in a decode step of 16 requests 17.8 us a
+// first kernel's idle lanes bring the second one's into L2.  Both kernels, 1, 2, 8, 16, 31 tokens of such experts, replayed back to back:
+// 14.2, 17.0, 18.0, 19.8, 24.5 us (16.1, 21.4, 24.3, 26.1, 32.3 by the kernels for wide rows below); in a decode step of 16 requests 17.8 us a
 // layer where it was 25.4.
 constexpr int EXPERT_TILE_TOKENS = 31, EXPERT_TABLES = 64, EXPERT_UNITS = 64, EXPERT_UNIT_K = 256;
 
