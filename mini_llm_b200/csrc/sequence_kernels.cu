@@ -1635,12 +1635,20 @@ static int launch_latent_step(const LatentTiledParams& p, int n_tokens, cudaStre
     int parts = latent_step_parts(n_tokens);
     if (p.most_blocks > 0 && parts > p.most_blocks) parts = p.most_blocks;
     // every device takes clusters of up to 8 blocks; 16 need as many SMs side by side, of which a part of a device may not have enough
+    // (asked for rather than tried: a launch that fails may end a capture)
     if (parts > 8) {
-        if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-            launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p) == cudaSuccess)
-            return check_launch("latent_step_kernel");
-        cudaGetLastError();
-        parts = 8;
+        cudaLaunchAttribute size = {};
+        size.id = cudaLaunchAttributeClusterDimension;
+        size.val.clusterDim.x = size.val.clusterDim.y = 1, size.val.clusterDim.z = parts;
+        cudaLaunchConfig_t config = {};
+        config.gridDim = dim3(n_tokens, 1, parts), config.blockDim = dim3(256), config.dynamicSmemBytes = shared, config.stream = s;
+        config.attrs = &size, config.numAttrs = 1;
+        int at_once = 0;
+        if (cudaFuncSetAttribute(latent_step_kernel<RANK>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&at_once, latent_step_kernel<RANK>, &config) != cudaSuccess || at_once < 1) {
+            cudaGetLastError();
+            parts = 8;
+        }
     }
     return launched(launch_kernel_in_clusters(g_dependent_launch != 0, dim3(1, 1, parts), latent_step_kernel<RANK>, dim3(n_tokens, 1, parts), dim3(256), shared, s, p),
                     "latent_step_kernel");
